@@ -183,7 +183,7 @@ int pg_lora_delta(const void* x, long long ldx, const void* A, const void* B, co
 
 // ---- Gated DeltaNet (gdn.cu) ------------------------------------------------------
 int pg_gdn_conv1d(const void* x, long long ldx, const void* w, void* state, void* out, long long ldo, const void* q_indptr, const void* slots,
-                  int num_seqs, int channels, int K, long long state_slot_stride, cudaStream_t stream);
+                  int num_seqs, int channels, int K, long long state_slot_stride, int max_q_len, cudaStream_t stream);
 int pg_gdn_gates(const void* a, long long lda, const void* b, long long ldb, const void* a_log, const void* dt_bias, void* g, void* beta,
                  int tokens, int hv, cudaStream_t stream);
 int pg_gdn_recurrent(const void* q, const void* k, long long ld_qk, const void* v, long long ld_v, const void* g, const void* beta, void* state,

@@ -790,7 +790,7 @@ def gdn_conv1d(x, conv_w, conv_state, meta: AttnMeta):
     c = ctx(x.device)
     k = conv_w.shape[1]
     rc = lib().pg_gdn_conv1d(_ptr(x), _ll(x.stride(0)), _ptr(conv_w), _ptr(conv_state), _ptr(out), _ll(out.stride(0)), _ptr(meta.q_indptr), _ptr(meta.state_slots),
-                             _ci(meta.num_seqs), _ci(ch), _ci(k), _ll(conv_state.stride(0)), _stream())
+                             _ci(meta.num_seqs), _ci(ch), _ci(k), _ll(conv_state.stride(0)), _ci(max(int(meta.max_q_len), 1)), _stream())
     _check(rc, c)
     return out
 
