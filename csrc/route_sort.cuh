@@ -1,11 +1,13 @@
 // Stable counting sort of expert routes inside one CTA (shared by the local MoE path and
 // the expert-parallel receive path).
 //
-// Routes arrive as a flat list of local expert ids (anything outside [0, e_local) means
-// "not for this rank").  The list is staged through shared memory in chunks; every warp
-// owns a subset of the experts and walks a chunk 32 entries at a time, ranking matches with
-// a ballot, so the order inside an expert is the route order (stable: the f32 summation
-// order downstream never depends on scheduling) while the scan is 32-wide.
+// Routes arrive as a flat list of local expert ids (anything outside [0, e_local) means "not for this rank").  Every warp
+// owns one contiguous slice of the list and walks it 32 entries at a time: lanes with the same expert find each other by a
+// ballot per bit of the id (a warp match takes several times as long), the first of them moves the warp's counter of it.  A first walk counts, a scan over (expert, warp)
+// turns the counts into cursors, a second walk hands out positions, so the order inside an expert is the route order
+// (stable: the f32 summation order downstream never depends on scheduling).  Bound by the latency of the walks,
+// n / 512 steps each; with every warp scanning the whole list for its own experts instead, 10266 routes to 64 experts took
+// 140 us and 1024 routes 14 us; 20 us and 4.6 us now.
 //
 // Takes the place of the reference's per-layer host-side routing bookkeeping and of the
 // align step of its Marlin MoE path (pegainfer-kernels/csrc/kimi_k2/kimi_marlin_wna16.cu
@@ -13,13 +15,13 @@
 #pragma once
 #include "common.cuh"
 
-constexpr int ROUTE_SORT_CHUNK = 8192;
 constexpr int ROUTE_SORT_THREADS = 512;
+constexpr int ROUTE_SORT_WARPS = ROUTE_SORT_THREADS / 32;
+constexpr int ROUTE_SORT_EXPERTS = 512;
 
 struct RouteSortSmem {
-  int ids[ROUTE_SORT_CHUNK];
-  int cnt[512];
-  int start[513];
+  int cursor[ROUTE_SORT_WARPS][ROUTE_SORT_EXPERTS];
+  int warp_total[ROUTE_SORT_WARPS];
 };
 
 // `load(i)` returns the local expert id of flat entry i (0 <= i < n); `emit(i, pos)` is called
@@ -27,53 +29,69 @@ struct RouteSortSmem {
 // for a local expert.  Writes offsets[0..e_local].  All ROUTE_SORT_THREADS threads call this.
 template <typename Load, typename Emit>
 __device__ __forceinline__ void route_sort(RouteSortSmem& sm, int n, int e_local, int* __restrict__ offsets, Load load, Emit emit) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = ROUTE_SORT_THREADS / 32;
-  for (int e = threadIdx.x; e < 512; e += ROUTE_SORT_THREADS) sm.cnt[e] = 0;
-  __syncthreads();
-  // pass 1: counts
-  for (int base = 0; base < n; base += ROUTE_SORT_CHUNK) {
-    const int m = min(ROUTE_SORT_CHUNK, n - base);
-    for (int i = threadIdx.x; i < m; i += ROUTE_SORT_THREADS) sm.ids[i] = load(base + i);
-    __syncthreads();
-    for (int e = warp; e < e_local; e += nwarps) {
-      int c = 0;
-      for (int i = lane; i < m; i += 32) c += (sm.ids[i] == e);
-      c = (int)warp_sum((float)c);  // exact: counts stay far below 2^24
-      if (lane == 0) sm.cnt[e] += c;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int i = 0; i < e_local; ++i) {
-      sm.start[i] = acc;
-      acc += sm.cnt[i];
-    }
-    sm.start[e_local] = acc;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i <= e_local; i += ROUTE_SORT_THREADS) offsets[i] = sm.start[i];
-  // pass 2: positions (sm.start[e] becomes the running cursor of expert e)
-  for (int base = 0; base < n; base += ROUTE_SORT_CHUNK) {
-    const int m = min(ROUTE_SORT_CHUNK, n - base);
-    __syncthreads();
-    for (int i = threadIdx.x; i < m; i += ROUTE_SORT_THREADS) {
-      const int id = load(base + i);
-      sm.ids[i] = id;
-      if (id < 0 || id >= e_local) emit(base + i, -1);
-    }
-    __syncthreads();
-    for (int e = warp; e < e_local; e += nwarps) {
-      int running = sm.start[e];
-      for (int i0 = 0; i0 < m; i0 += 32) {
-        const int i = i0 + lane;
-        const bool hit = i < m && sm.ids[i] == e;
-        const uint32_t mask = __ballot_sync(0xffffffffu, hit);
-        if (hit) emit(base + i, running + __popc(mask & ((1u << lane) - 1u)));
-        running += __popc(mask);
+  static_assert(ROUTE_SORT_THREADS == ROUTE_SORT_EXPERTS, "the scan gives every expert a thread");
+  constexpr int AHEAD = 4;  // groups of 32 entries whose ids are loaded together
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int slice = ((n + ROUTE_SORT_WARPS - 1) / ROUTE_SORT_WARPS + 31) & ~31;
+  const int i_begin = min(n, warp * slice), i_end = min(n, i_begin + slice);
+  int* cursor = sm.cursor[warp];
+  const int bits = 32 - __clz(e_local - 1);  // of a local expert id (none for a single expert)
+  // `place`: the second walk
+  auto walk = [&](bool place) {
+    for (int base = i_begin; base < i_end; base += 32 * AHEAD) {
+      int id[AHEAD];
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a) {
+        const int i = base + 32 * a + lane;
+        id[a] = i < i_end ? load(i) : -1;
       }
-      __syncwarp();
-      if (lane == 0) sm.start[e] = running;
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a) {
+        const int i = base + 32 * a + lane;
+        const bool mine = id[a] >= 0 && id[a] < e_local;
+        uint32_t peers = __ballot_sync(0xffffffffu, mine);  // for a lane with a local expert: the lanes that have the same one
+#pragma unroll 1
+        for (int bit = 0; bit < bits; ++bit) {
+          const bool one = id[a] >> bit & 1;
+          const uint32_t ones = __ballot_sync(0xffffffffu, one);
+          peers &= one ? ones : ~ones;
+        }
+        const int before = mine ? cursor[id[a]] : 0;
+        __syncwarp();
+        if (mine && lane == __ffs(peers) - 1) cursor[id[a]] = before + __popc(peers);
+        __syncwarp();
+        if (place && i < i_end) emit(i, mine ? before + __popc(peers & ((1u << lane) - 1u)) : -1);
+      }
     }
+  };
+#pragma unroll
+  for (int w = 0; w < ROUTE_SORT_WARPS; ++w) sm.cursor[w][tid] = 0;
+  __syncthreads();
+  walk(false);
+  __syncthreads();
+  int total = 0;  // of expert `tid`
+#pragma unroll
+  for (int w = 0; w < ROUTE_SORT_WARPS; ++w) total += sm.cursor[w][tid];
+  int upto = total;  // inclusive scan over the experts
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += x;
   }
+  if (lane == 31) sm.warp_total[warp] = upto;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < ROUTE_SORT_WARPS; ++w)
+    if (w < warp) upto += sm.warp_total[w];
+  int at = upto - total;
+  if (tid < e_local) offsets[tid] = at;
+  if (tid == e_local - 1) offsets[e_local] = upto;
+#pragma unroll
+  for (int w = 0; w < ROUTE_SORT_WARPS; ++w) {
+    const int c = sm.cursor[w][tid];
+    sm.cursor[w][tid] = at;
+    at += c;
+  }
+  __syncthreads();
+  walk(true);
 }

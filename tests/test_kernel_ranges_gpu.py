@@ -22,3 +22,20 @@ def test_gdn_conv1d_segments(channels, taps):
     # the sum is rounded to bf16 once; its order may move it by one step, and SiLU's slope is at most 1.1: two steps of bf16
     assert ((y1.float() - y2.float()).abs() <= 2 ** -7 * y2.float().abs() + 2 ** -9).all()
     assert torch.equal(st1, st2)
+
+
+@pytest.mark.parametrize("routes,e0,e_local,total", [(1, 0, 1, 1), (31, 0, 3, 5), (512, 8, 64, 96), (513, 0, 384, 384), (8193, 16, 48, 384), (40007, 0, 512, 512)])
+def test_route_sort_is_stable(routes, e0, e_local, total):
+    g = torch.Generator().manual_seed(routes)
+    ids = torch.randint(0, total, (routes, 1), generator=g, dtype=torch.int32)
+    if routes > 600:
+        ids[100:400] = e0 + e_local - 1  # a run of one expert
+    offsets, src, pos = cu().moe_route_plan(ids.to(DEV), e0, e_local)
+    local = ids.flatten().long() - e0
+    local[(local < 0) | (local >= e_local)] = e_local
+    order = torch.argsort(local, stable=True)
+    n = int((local < e_local).sum())
+    want = torch.full((routes,), -1)
+    want[order[:n]] = torch.arange(n)
+    assert torch.equal(offsets.cpu().long(), torch.searchsorted(local[order], torch.arange(e_local + 1)))
+    assert torch.equal(pos.cpu().long()[:routes], want) and torch.equal(src.cpu().long()[:n], order[:n])
