@@ -39,3 +39,34 @@ def test_route_sort_is_stable(routes, e0, e_local, total):
     want[order[:n]] = torch.arange(n)
     assert torch.equal(offsets.cpu().long(), torch.searchsorted(local[order], torch.arange(e_local + 1)))
     assert torch.equal(pos.cpu().long()[:routes], want) and torch.equal(src.cpu().long()[:n], order[:n])
+
+
+@pytest.mark.parametrize("dv", [64, 128])
+def test_kda_blocks_of_four_tokens(dv):
+    torch.manual_seed(dv)
+    heads, dk, q_lens, slots = 3, 128, [5, 1, 16, 17, 4, 33, 130, 9], [3, 1, 4, 2, 8, 5, 7, -1]  # around blocks of 4 and stages of 16
+    meta, t = _state_meta(q_lens, slots), sum(q_lens)
+    qkv = torch.randn(t, heads * (2 * dk + dv) + 8, device=DEV).bfloat16()
+    q, k = (qkv[:, j * heads * dk : (j + 1) * heads * dk].view(t, heads, dk) for j in range(2))
+    v = qkv[:, 2 * heads * dk : 2 * heads * dk + heads * dv].view(t, heads, dv)
+    f, b = torch.randn(t, heads * dk, device=DEV).bfloat16(), torch.randn(t, heads + 5, device=DEV).bfloat16()[:, :heads]
+    a_log, dt = torch.randn(heads, device=DEV) * 0.5, torch.randn(heads * dk, device=DEV) - 2
+    st1 = torch.randn(9, heads, dk, dv, device=DEV)
+    st2 = st1.double()
+    o1 = cu().kda_recurrent(q, k, v, f, b, a_log, dt, -5.0, st1, meta)
+    # the rule in 64 bits: the kernel works in f32 (2^-23 a step, fewer than 2^6 steps that matter) and rounds its output to bf16
+    unit = lambda x: x * torch.rsqrt(x.pow(2).sum(-1, keepdim=True) + 1e-6)  # noqa: E731
+    qd, kd = unit(q.double()) * dk ** -0.5, unit(k.double())
+    dec = torch.exp(-5.0 * torch.sigmoid(a_log.double().exp().view(heads, 1) * (f.double() + dt.double()).view(t, heads, dk)))
+    beta, at = torch.sigmoid(b.double()), 0
+    for n, slot in zip(q_lens, slots):
+        for i in range(at, at + n):
+            if slot < 0:
+                continue
+            S = st2[slot] * dec[i].unsqueeze(-1)
+            d = (v[i].double() - torch.einsum("hkv,hk->hv", S, kd[i])) * beta[i].unsqueeze(-1)
+            st2[slot] = S + kd[i].unsqueeze(-1) * d.unsqueeze(1)
+            want = torch.einsum("hkv,hk->hv", st2[slot], qd[i])
+            assert (o1[i].double() - want).abs().max() <= 2 ** -8 * want.abs().max() + 1e-5
+        at += n
+    assert (st1.double() - st2).abs().max() < 2 ** -17 * st2.abs().max()
