@@ -281,52 +281,97 @@ __global__ void __launch_bounds__(ST) sample_kernel(const T* __restrict__ logits
 }
 
 // ---------------------------------------------------------------------------------
-// Cluster sampler: one thread-block cluster per row.  Each CTA of the cluster reads its slice
-// of the row ONCE into shared memory (as tempered f32 logits) and every later pass -- the
-// normaliser, the four radix levels of the threshold search, the inverse-CDF walk -- runs out
-// of shared memory, with the per-CTA partial results combined across the cluster through
-// distributed shared memory.  Probability mass is carried as 2^-40 fixed point in 64-bit
-// integers, so every sum is exact and independent of the order in which threads add to it:
-// the same (logits, controls, uniform) always pick the same token, and the CDF target
+// Cluster sampler: one thread-block cluster per row.  Each CTA of the cluster reads its slice of the row ONCE into shared
+// memory and every later pass runs there, with the per-CTA partial results combined across the cluster through distributed
+// shared memory.  A token is represented by e = exp(s - max) in [0, 1], whose bit pattern orders the tokens as their logits
+// do.  Probability mass is carried as 2^-40 fixed point in 64-bit integers, so every sum is exact and independent of the
+// order in which threads add to it: the same (logits, controls, uniform) always pick the same token, and the CDF target
 // floor(u * total) is always strictly inside the kept mass (no rounding fallback).
+//
+// The threshold of the keep-set is found in two steps.  A histogram of counts over 32 bins per factor of two (tokens below
+// 2^-40 have no mass and are left out) brackets it: a bin's count times its edges bounds its mass from both sides, and the
+// walk from the top with the lower (upper) bounds ends at or below (above) the bin that the exact walk ends in.  Then the
+// mass above the bracket is summed exactly and only the tokens inside it, some hundred as a rule, go through a radix
+// descent with counts and masses.  Bound by the latency of the passes and of the eight cluster barriers between them, with
+// every row of a batch of 64 resident at once (clusters of four).  64 x 151936 bf16, top-k 50, top-p 0.9: 200 us with all tokens
+// taking part in each of four radix levels, one warp match per 32 tokens; 61 us now (1 row: 36 us).
 // ---------------------------------------------------------------------------------
 constexpr int SC_THREADS = 512;
+constexpr int SC_WARPS = SC_THREADS / 32;
 constexpr int SC_MAX_CLUSTER = 8;
-constexpr float SC_FX = 1099511627776.f;  // 2^40
+constexpr uint32_t SC_ONE = 0x3f800000u;  // key of e = 1, the largest
+constexpr uint32_t SC_LOW = (127u - 40u) << 23;  // key of 2^-40: tokens below have no mass
+constexpr int SC_BIN_SHIFT = 18;          // 32 coarse bins per factor of two
+constexpr int SC_BINS = (int)((SC_ONE - SC_LOW) >> SC_BIN_SHIFT) + 1;  // 1281
+constexpr int SC_BINS_PER_THREAD = (SC_BINS + SC_THREADS - 1) / SC_THREADS;
+constexpr int SC_LIST = 1024;             // bracketed tokens kept in a list; more of them are found by walking the slice
 
+// (no memory clobber: several of these are in flight together; the cluster barriers around them have one)
 __device__ __forceinline__ unsigned long long ld_dsmem_u64(uint32_t cluster_addr) {
   unsigned long long v;
-  asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(cluster_addr) : "memory");
+  asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(cluster_addr));
   return v;
 }
 __device__ __forceinline__ uint32_t ld_dsmem_u32(uint32_t cluster_addr) {
   uint32_t v;
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr));
   return v;
 }
 
+struct ScLevel {
+  unsigned long long mass[256];
+  uint32_t cnt[256];
+};
 struct ScShared {
-  unsigned long long h_mass[2][256];  // per-CTA histogram of the level being searched (double buffered)
-  uint32_t h_cnt[2][256];
-  unsigned long long m_mass[256];     // histogram merged over the cluster (every CTA computes the same)
-  uint32_t m_cnt[256];
-  unsigned long long x_u64;           // this CTA's contribution to a cluster-wide sum
-  float x_f32;                        // this CTA's contribution to a cluster-wide max
-  uint32_t prefix, cnt_above;
+  // a level's histogram is read by the peers until the next level's barrier, so two take turns; the coarse counts are
+  // read for the last time in front of the first level's barrier
+  ScLevel even;
+  union {
+    ScLevel odd;
+    uint32_t coarse[SC_BINS_PER_THREAD * SC_THREADS];
+  };
+  ScLevel merged;  // the cluster's sum (every CTA forms the same)
+  uint32_t list[SC_LIST];
+  unsigned long long x_u64[4];  // this CTA's contributions to cluster-wide sums: normaliser, mass and count above the bracket, kept mass
+  float x_f32;                  // and to the cluster-wide maximum
+  uint32_t list_n, prefix, cnt_above;
+  int bin_lo, bin_hi;
   unsigned long long mass_above;
-  unsigned long long warp_tot[SC_THREADS / 32];
-  int owner;
+  unsigned long long warp_tot[SC_WARPS], warp_ub[SC_WARPS];
+  uint32_t warp_cnt[SC_WARPS];
 };
 
+// floor(e * 2^40) of a token by its bits (2^-40 <= e < 2^24), in integer instructions: a conversion to 64 bits takes several
+// times as long as the rest of a token's work
+__device__ __forceinline__ unsigned long long sc_fx(uint32_t key) {
+  const unsigned long long mant = (key & 0x7fffffu) | 0x800000u;
+  const int shift = (int)(key >> 23) - (127 - 40 + 23);
+  return shift >= 0 ? mant << shift : mant >> -shift;
+}
+
+// Totals of the lanes above this one, of three quantities.
+__device__ __forceinline__ void sc_suffix(uint32_t& c, unsigned long long& m, unsigned long long& n, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t cu = __shfl_down_sync(0xffffffffu, c, o);
+    const unsigned long long mu = __shfl_down_sync(0xffffffffu, m, o), nu = __shfl_down_sync(0xffffffffu, n, o);
+    if (lane + o < 32) {
+      c += cu;
+      m += mu;
+      n += nu;
+    }
+  }
+}
+
 template <typename T>
-__global__ void __launch_bounds__(SC_THREADS) sample_cluster_kernel(const T* __restrict__ logits, long long ld, int vocab, int slice,
+__global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* __restrict__ logits, long long ld, int vocab, int slice,
                                                                     const float* __restrict__ temperature, const int* __restrict__ top_k,
                                                                     const float* __restrict__ top_p, const float* __restrict__ min_p,
                                                                     const float* __restrict__ uniform, int* __restrict__ out, int csize) {
   PG_PDL_ENTRY();
   extern __shared__ __align__(16) uint8_t sc_raw[];
   ScShared& sh = *reinterpret_cast<ScShared*>(sc_raw);
-  float* vals = reinterpret_cast<float*>(sc_raw + ((sizeof(ScShared) + 15) & ~size_t(15)));
+  T* vals = reinterpret_cast<T*>(sc_raw + ((sizeof(ScShared) + 15) & ~size_t(15)));
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t cr = csize > 1 ? cluster_ctarank() : 0u;
   const int row = blockIdx.x / csize;
@@ -334,220 +379,337 @@ __global__ void __launch_bounds__(SC_THREADS) sample_cluster_kernel(const T* __r
   const float inv_t = 1.f / fmaxf(temperature[row], 1e-6f);
   const int i0 = min(vocab, (int)cr * slice), i1 = min(vocab, i0 + slice);
   const int n = i1 - i0;
-  const int n_pad = (n + SC_THREADS - 1) / SC_THREADS * SC_THREADS;
   __shared__ float red[32];
+  auto cluster_barrier = [&]() {
+    if (csize > 1) cluster_sync_all(); else __syncthreads();
+  };
+  // sums over the cluster's CTAs (a lone CTA is a cluster of its own)
+  auto sum_u64 = [&](const unsigned long long* at) {
+    unsigned long long x[SC_MAX_CLUSTER], t = 0ull;
+#pragma unroll
+    for (int q = 0; q < SC_MAX_CLUSTER; ++q) x[q] = q < csize ? ld_dsmem_u64(dsmem_addr(smem_u32(at), (uint32_t)q)) : 0ull;
+#pragma unroll
+    for (int q = 0; q < SC_MAX_CLUSTER; ++q) t += x[q];
+    return t;
+  };
+  auto sum_u32 = [&](const uint32_t* at) {
+    uint32_t x[SC_MAX_CLUSTER], t = 0u;
+#pragma unroll
+    for (int q = 0; q < SC_MAX_CLUSTER; ++q) x[q] = q < csize ? ld_dsmem_u32(dsmem_addr(smem_u32(at), (uint32_t)q)) : 0u;
+#pragma unroll
+    for (int q = 0; q < SC_MAX_CLUSTER; ++q) t += x[q];
+    return t;
+  };
 
-  // the slice, tempered, into shared memory; local max
+  // the slice into shared memory (slices start at multiples of eight tokens); local max
   float m = -FLT_MAX;
-  for (int i = tid; i < n; i += SC_THREADS) {
-    const float s = ldf(r, (long long)i0 + i) * inv_t;
-    vals[i] = s;
-    m = fmaxf(m, s);
+  constexpr int VEC = 16 / sizeof(T);
+  int done = 0;
+  if (((reinterpret_cast<uintptr_t>(r) | (uintptr_t)(i0 * sizeof(T))) & 15) == 0) {
+    done = n / VEC * VEC;
+    for (int i = tid; i < n / VEC; i += SC_THREADS) {
+      const uint4 x = reinterpret_cast<const uint4*>(r + i0)[i];
+      reinterpret_cast<uint4*>(vals)[i] = x;
+      const T* e = reinterpret_cast<const T*>(&x);
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) m = fmaxf(m, ldf(e, j) * inv_t);
+    }
+  }
+  for (int i = done + tid; i < n; i += SC_THREADS) {
+    const T x = r[i0 + i];
+    vals[i] = x;
+    m = fmaxf(m, ldf(&x, 0) * inv_t);
   }
   m = block_max_f(m, red);
   if (tid == 0) {
     sh.x_f32 = m;
-    sh.prefix = 0u;
-    sh.cnt_above = 0u;
-    sh.mass_above = 0ull;
+    sh.list_n = 0u;
+    sh.bin_lo = SC_BINS;
+    sh.bin_hi = SC_BINS;
   }
-  for (int b = tid; b < 256; b += SC_THREADS) {
-    sh.h_cnt[0][b] = 0u;
-    sh.h_mass[0][b] = 0ull;
-  }
-  if (csize > 1) cluster_sync_all(); else __syncthreads();
+#pragma unroll
+  for (int j = 0; j < SC_BINS_PER_THREAD; ++j) sh.coarse[tid + j * SC_THREADS] = 0u;
+  cluster_barrier();
   if (csize > 1) {
     float mm = -FLT_MAX;
     for (int q = 0; q < csize; ++q) mm = fmaxf(mm, ld_dsmem_f32(dsmem_addr(smem_u32(&sh.x_f32), (uint32_t)q)));
     m = mm;
   }
+  // bits of a token's e; the maximum (infinite ones too) has e = 1, a NaN has none
+  auto key_of = [&](float logit) -> uint32_t {
+    const float s = logit * inv_t;
+    const float e = s >= m ? 1.f : __expf(s - m);
+    return e > 0.f ? min(__float_as_uint(e), SC_ONE) : 0u;
+  };
+  // f(key) for the slice's tokens `from` + VEC * first .. `to`, 16 bytes of them at a time, every `step` pieces
+  auto walk = [&](int from, int to, int first, int step, auto&& f) {
+    for (int i = from + first * VEC; i < to; i += step * VEC) {
+      const uint4 x = *reinterpret_cast<const uint4*>(vals + i);
+      uint32_t key[VEC];
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) key[j] = i + j < to ? key_of(ldf(reinterpret_cast<const T*>(&x), j)) : 0u;
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) f(key[j]);
+    }
+  };
 
-  const int kk = top_k[row] > 0 ? min(top_k[row], vocab) : vocab;
+  const uint32_t kk = top_k[row] > 0 ? (uint32_t)min(top_k[row], vocab) : (uint32_t)vocab;
   const float tp = top_p[row];
   const float mp = min_p[row];
-
-  // From here on a token is represented by e = exp(s - max) in (0, 1]: the exponential is taken
-  // once, when the first radix level walks the slice, and stored over the tempered logit.  e
-  // orders the tokens exactly as s does, so the threshold search runs on the bits of e; the
-  // first level's histogram masses also add up to the normaliser.
-  unsigned long long p_lim = ~0ull;
-  for (int level = 0; level < 4; ++level) {
-    const int shift = 24 - 8 * level;
-    const uint32_t hi_mask = level == 0 ? 0u : (0xffffffffu << (shift + 8));
-    const int hb = level & 1;
-    const uint32_t prefix = sh.prefix;
-    for (int i = tid; i < n_pad; i += SC_THREADS) {
-      uint32_t bin = 256u;
-      unsigned long long fx = 0ull;
-      if (i < n) {
-        float e = vals[i];
-        if (level == 0) {
-          e = __expf(e - m);
-          vals[i] = e;
-        }
-        const uint32_t key = __float_as_uint(e);  // e >= 0: the bit pattern is already order preserving
-        if ((key & hi_mask) == prefix) {
-          bin = (key >> shift) & 255u;
-          fx = (unsigned long long)(e * SC_FX);
-        }
+  uint32_t thr_key = 0u;
+  if (kk < (uint32_t)vocab || tp < 1.f) {  // the same for the whole cluster: every CTA reads the row's controls
+    // ---- coarse counts and the normaliser ----
+    unsigned long long z = 0ull;
+    walk(0, n, tid, SC_THREADS, [&](uint32_t key) {
+      if (key >= SC_LOW) {
+        z += sc_fx(key);
+        atomicAdd(&sh.coarse[(key - SC_LOW) >> SC_BIN_SHIFT], 1u);
       }
-      if (!__any_sync(0xffffffffu, bin < 256u)) continue;  // below the first level most warps have no candidate left
-      // one shared-memory atomic per distinct bin of the warp
-      const uint32_t peers = __match_any_sync(0xffffffffu, bin);
-      if (bin < 256u) {
-        const uint32_t lo = __reduce_add_sync(peers, (uint32_t)(fx & 0xFFFFFull));
-        const uint32_t hi = __reduce_add_sync(peers, (uint32_t)(fx >> 20));
-        if (lane == __ffs(peers) - 1) {
-          atomicAdd(&sh.h_cnt[hb][bin], (uint32_t)__popc(peers));
-          atomicAdd(&sh.h_mass[hb][bin], ((unsigned long long)hi << 20) + (unsigned long long)lo);
-        }
-      }
+    });
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+    if (lane == 0) sh.warp_tot[warp] = z;
+    __syncthreads();
+    if (tid == 0) {
+      unsigned long long t = 0ull;
+      for (int w = 0; w < SC_WARPS; ++w) t += sh.warp_tot[w];
+      sh.x_u64[0] = t;
     }
-    if (csize > 1) cluster_sync_all(); else __syncthreads();
-    for (int b = tid; b < 256; b += SC_THREADS) {
-      // The other buffer is free now: peers read it (the previous level's merge) before they arrived
-      // at the barrier above.  The next level adds into it after the __syncthreads below.
-      sh.h_cnt[hb ^ 1][b] = 0u;
-      sh.h_mass[hb ^ 1][b] = 0ull;
-      uint32_t c = 0u;
-      unsigned long long ms = 0ull;
-      if (csize > 1) {
-        for (int q = 0; q < csize; ++q) {
-          c += ld_dsmem_u32(dsmem_addr(smem_u32(&sh.h_cnt[hb][b]), (uint32_t)q));
-          ms += ld_dsmem_u64(dsmem_addr(smem_u32(&sh.h_mass[hb][b]), (uint32_t)q));
-        }
-      } else {
-        c = sh.h_cnt[hb][b];
-        ms = sh.h_mass[hb][b];
-      }
-      sh.m_cnt[b] = c;
-      sh.m_mass[b] = ms;
+    cluster_barrier();
+    z = sum_u64(&sh.x_u64[0]);
+    const unsigned long long lim = tp >= 1.f ? ~0ull : (unsigned long long)((double)tp * (double)z);
+    // thread t owns bins SC_BINS_PER_THREAD * t ..; walking the bins from the top, a bin is kept while (count above < k) and
+    // (mass above < top-p limit); both grow as the bin index falls, so the last one kept is the LOWEST non-empty bin that
+    // satisfies them
+    uint32_t c[SC_BINS_PER_THREAD], csum = 0u;
+    unsigned long long lb[SC_BINS_PER_THREAD], ub[SC_BINS_PER_THREAD], lsum = 0ull, usum = 0ull;
+#pragma unroll
+    for (int j = 0; j < SC_BINS_PER_THREAD; ++j) {
+      const int bin = tid * SC_BINS_PER_THREAD + j;
+      c[j] = sum_u32(&sh.coarse[bin]);  // (zero behind the last bin)
+      lb[j] = c[j] ? c[j] * sc_fx(SC_LOW + ((uint32_t)bin << SC_BIN_SHIFT)) : 0ull;
+      ub[j] = c[j] ? c[j] * sc_fx(SC_LOW + ((uint32_t)(bin + 1) << SC_BIN_SHIFT)) : 0ull;
+      csum += c[j];
+      lsum += lb[j];
+      usum += ub[j];
+    }
+    uint32_t c_hi = csum;
+    unsigned long long l_hi = lsum, u_hi = usum;
+    sc_suffix(c_hi, l_hi, u_hi, lane);
+    __syncthreads();  // warp_tot is read above
+    if (lane == 0) {
+      sh.warp_cnt[warp] = c_hi;
+      sh.warp_tot[warp] = l_hi;
+      sh.warp_ub[warp] = u_hi;
     }
     __syncthreads();
-    if (warp == 0) {
-      // Warp-parallel threshold step.  Lane l owns bins 8l .. 8l+7.  Walking the bins from the top, a
-      // bin is kept while (count above < k) and (mass above < top-p limit); both grow as the bin index
-      // falls, so the chosen bin is the LOWEST non-empty bin that still satisfies them.
-      uint32_t c8[8];
-      unsigned long long m8[8];
-      uint32_t csum = 0u;
-      unsigned long long msum = 0ull;
+    c_hi -= csum;
+    l_hi -= lsum;
+    u_hi -= usum;
+    for (int w = warp + 1; w < SC_WARPS; ++w) {
+      c_hi += sh.warp_cnt[w];
+      l_hi += sh.warp_tot[w];
+      u_hi += sh.warp_ub[w];
+    }
+    int lo = SC_BINS, hi = SC_BINS;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        c8[j] = sh.m_cnt[lane * 8 + j];
-        m8[j] = sh.m_mass[lane * 8 + j];
-        csum += c8[j];
-        msum += m8[j];
-      }
-      // totals of the lanes above this one (exclusive suffix sum)
-      uint32_t c_hi = csum;
-      unsigned long long m_hi = msum;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t cu = __shfl_down_sync(0xffffffffu, c_hi, o);
-        const unsigned long long mu = __shfl_down_sync(0xffffffffu, m_hi, o);
-        if (lane + o < 32) {
-          c_hi += cu;
-          m_hi += mu;
-        }
-      }
-      if (level == 0) {
-        const unsigned long long z = __shfl_sync(0xffffffffu, m_hi, 0);  // exact, whatever order the threads added in
-        if (lane == 0) sh.x_u64 = tp >= 1.f ? ~0ull : (unsigned long long)((double)tp * (double)z);
-        __syncwarp();
-      }
-      const unsigned long long lim = sh.x_u64;
-      uint32_t cnt = sh.cnt_above + (c_hi - csum);
-      unsigned long long mass = sh.mass_above + (m_hi - msum);
-      int chosen = 256;
-      uint32_t c_cnt = 0u;
-      unsigned long long c_mass = 0ull;
-#pragma unroll
-      for (int j = 7; j >= 0; --j) {
-        if (c8[j] != 0u && cnt < (uint32_t)kk && mass < lim) {
-          chosen = lane * 8 + j;
-          c_cnt = cnt;
-          c_mass = mass;
-        }
-        cnt += c8[j];
-        mass += m8[j];
-      }
-      int best = chosen;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-      __syncwarp();
-      if (best == 256) {  // cannot happen (the top element is always kept); keep the top bin
-        if (lane == 31) {
-          sh.prefix = prefix | (255u << shift);
-        }
-      } else if (chosen == best) {  // exactly one lane owns the chosen bin
-        sh.prefix = prefix | ((uint32_t)best << shift);
-        sh.cnt_above = c_cnt;
-        sh.mass_above = c_mass;
-      }
+    for (int j = SC_BINS_PER_THREAD - 1; j >= 0; --j) {
+      const int bin = tid * SC_BINS_PER_THREAD + j;
+      if (c[j] != 0u && c_hi < kk && l_hi < lim) lo = bin;
+      if (c[j] != 0u && c_hi < kk && u_hi < lim) hi = bin;
+      c_hi += c[j];
+      l_hi += lb[j];
+      u_hi += ub[j];
+    }
+    // (a limit of zero mass keeps no bin by these rules: the top element is always kept)
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_min_sync(0xffffffffu, hi);
+    if (lane == 0) {
+      atomicMin(&sh.bin_lo, lo);
+      atomicMin(&sh.bin_hi, hi);
     }
     __syncthreads();
+    lo = sh.bin_lo;
+    hi = min(sh.bin_hi, SC_BINS - 1);
+    if (lo == SC_BINS) {
+      thr_key = SC_ONE;
+    } else {
+      // ---- exact mass above the bracket lo .. hi, and the tokens inside it ----
+      const uint32_t k_lo = SC_LOW + ((uint32_t)lo << SC_BIN_SHIFT), k_hi = SC_LOW + ((uint32_t)(hi + 1) << SC_BIN_SHIFT);  // [k_lo, k_hi)
+      unsigned long long above = 0ull;
+      uint32_t n_above = 0u;
+      walk(0, n, tid, SC_THREADS, [&](uint32_t key) {
+        if (key >= k_hi) {
+          above += sc_fx(key);
+          ++n_above;
+        } else if (key >= k_lo) {
+          const uint32_t at = atomicAdd(&sh.list_n, 1u);
+          if (at < SC_LIST) sh.list[at] = key;
+        }
+      });
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        above += __shfl_xor_sync(0xffffffffu, above, o);
+        n_above += __shfl_xor_sync(0xffffffffu, n_above, o);
+      }
+      if (lane == 0) {
+        sh.warp_ub[warp] = above;
+        sh.warp_cnt[warp] = n_above;
+      }
+      if (tid < 256) {
+        sh.even.cnt[tid] = 0u;
+        sh.even.mass[tid] = 0ull;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        unsigned long long t = 0ull, k = 0ull;
+        for (int w = 0; w < SC_WARPS; ++w) {
+          t += sh.warp_ub[w];
+          k += sh.warp_cnt[w];
+        }
+        sh.x_u64[1] = t;
+        sh.x_u64[2] = k;
+      }
+      // ---- radix descent over key - k_lo ----
+      const int bits = 32 - __clz((int)(k_hi - k_lo - 1u));
+      const int levels = (bits + 7) / 8, step = (bits + levels - 1) / levels;
+      const uint32_t listed = sh.list_n;
+      uint32_t prefix = 0u;  // of key - k_lo
+      for (int level = 0; level < levels; ++level) {
+        const int shift = max(0, bits - step * (level + 1)), above_shift = bits - step * level;
+        ScLevel& h = level & 1 ? sh.odd : sh.even;
+        ScLevel& next = level & 1 ? sh.even : sh.odd;
+        auto add = [&](uint32_t key) {
+          const uint32_t d = key - k_lo;
+          if (level > 0 && (d >> above_shift) != (prefix >> above_shift)) return;
+          const uint32_t bin = (d >> shift) & ((1u << (above_shift - shift)) - 1u);
+          atomicAdd(&h.cnt[bin], 1u);
+          atomicAdd(&h.mass[bin], sc_fx(key));
+        };
+        if (listed <= SC_LIST) {
+          for (int i = tid; i < (int)listed; i += SC_THREADS) add(sh.list[i]);
+        } else {
+          walk(0, n, tid, SC_THREADS, [&](uint32_t key) {
+            if (key >= k_lo && key < k_hi) add(key);
+          });
+        }
+        cluster_barrier();
+        if (tid < 256) {  // a thread merges one bin
+          sh.merged.cnt[tid] = sum_u32(&h.cnt[tid]);
+          sh.merged.mass[tid] = sum_u64(&h.mass[tid]);
+          if (level == 0 && tid == 0) {
+            sh.mass_above = sum_u64(&sh.x_u64[1]);
+            sh.cnt_above = (uint32_t)sum_u64(&sh.x_u64[2]);
+          }
+        } else {
+          // the other histogram is free: peers read it (the previous level, or the coarse counts) before they arrived
+          next.cnt[tid - 256] = 0u;
+          next.mass[tid - 256] = 0ull;
+        }
+        __syncthreads();
+        if (warp == 0) {
+          // Lane l owns bins 8l .. 8l + 7; the same walk as over the coarse bins, with exact masses
+          uint32_t c8[8], cs = 0u;
+          unsigned long long m8[8], ms = 0ull, none = 0ull;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            c8[j] = sh.merged.cnt[lane * 8 + j];
+            m8[j] = sh.merged.mass[lane * 8 + j];
+            cs += c8[j];
+            ms += m8[j];
+          }
+          const uint32_t cnt0 = sh.cnt_above;
+          const unsigned long long mass0 = sh.mass_above;
+          __syncwarp();
+          uint32_t ch = cs;
+          unsigned long long mh = ms;
+          sc_suffix(ch, mh, none, lane);
+          uint32_t cnt = cnt0 + (ch - cs);
+          unsigned long long mass = mass0 + (mh - ms);
+          int chosen = 256;
+          uint32_t c_cnt = 0u;
+          unsigned long long c_mass = 0ull;
+#pragma unroll
+          for (int j = 7; j >= 0; --j) {
+            if (c8[j] != 0u && cnt < kk && mass < lim) {
+              chosen = lane * 8 + j;
+              c_cnt = cnt;
+              c_mass = mass;
+            }
+            cnt += c8[j];
+            mass += m8[j];
+          }
+          const int best = __reduce_min_sync(0xffffffffu, chosen);
+          if (chosen == best && best < 256) {  // exactly one lane owns the chosen bin
+            sh.prefix = prefix | ((uint32_t)best << shift);
+            sh.cnt_above = c_cnt;
+            sh.mass_above = c_mass;
+          } else if (best == 256 && lane == 0) {  // cannot happen: the bracket holds the last kept bin
+            sh.prefix = prefix;
+          }
+        }
+        __syncthreads();
+        prefix = sh.prefix;
+      }
+      thr_key = k_lo + prefix;
+    }
   }
-  (void)p_lim;
   // min-p: e >= min_p (e is relative to the row maximum, whose e is 1)
-  const uint32_t thr_key = max(sh.prefix, mp > 0.f ? __float_as_uint(fminf(mp, 1.f)) : 0u);
-  __syncthreads();  // every thread has read the threshold before x_u64 is reused below
+  if (mp > 0.f) thr_key = max(thr_key, __float_as_uint(fminf(mp, 1.f)));
+  thr_key = max(thr_key, SC_LOW);  // tokens below have no mass
 
-  // inverse CDF in vocabulary order over the kept set: a contiguous chunk per thread
-  const int chunk = (n + SC_THREADS - 1) / SC_THREADS;
-  const int c0 = min(n, tid * chunk), c1 = min(n, c0 + chunk);
+  // inverse CDF in vocabulary order over the kept set: a contiguous run of tokens per warp
+  const int run = ((n + SC_WARPS - 1) / SC_WARPS + 31) & ~31;  // (a multiple of a 16-byte piece)
+  const int c0 = min(n, warp * run), c1 = min(n, c0 + run);
   unsigned long long local = 0ull;
-  for (int i = c0; i < c1; ++i) {
-    const float e = vals[i];
-    if (__float_as_uint(e) >= thr_key) local += (unsigned long long)(e * SC_FX);
-  }
-  unsigned long long incl = local;
+  walk(c0, c1, lane, 32, [&](uint32_t key) {
+    if (key >= thr_key) local += sc_fx(key);
+  });
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += up;
-  }
-  if (lane == 31) sh.warp_tot[warp] = incl;
+  for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
+  __syncthreads();  // warp_tot is read above
+  if (lane == 0) sh.warp_tot[warp] = local;
   __syncthreads();
-  unsigned long long warp_before = 0ull, cta_total = 0ull;
-  for (int w = 0; w < SC_THREADS / 32; ++w) {
+  unsigned long long before = 0ull, cta_total = 0ull;
+  for (int w = 0; w < SC_WARPS; ++w) {
     const unsigned long long t = sh.warp_tot[w];
-    if (w < warp) warp_before += t;
+    if (w < warp) before += t;
     cta_total += t;
   }
-  const unsigned long long before = warp_before + incl - local;
-  if (tid == 0) {
-    sh.x_u64 = cta_total;
-    sh.owner = -1;
-  }
-  // x_u64 held the top-p limit, which only this CTA's thread 0 read (every CTA computes its own copy)
-  if (csize > 1) cluster_sync_all(); else __syncthreads();
+  if (tid == 0) sh.x_u64[3] = cta_total;
+  cluster_barrier();
   unsigned long long total = 0ull, cta_before = 0ull;
-  for (int q = 0; q < csize; ++q) {
-    const unsigned long long t = csize > 1 ? ld_dsmem_u64(dsmem_addr(smem_u32(&sh.x_u64), (uint32_t)q)) : sh.x_u64;
+#pragma unroll
+  for (int q = 0; q < SC_MAX_CLUSTER; ++q) {
+    const unsigned long long t = q < csize ? ld_dsmem_u64(dsmem_addr(smem_u32(&sh.x_u64[3]), (uint32_t)q)) : 0ull;
     if (q < (int)cr) cta_before += t;
     total += t;
   }
   // u < 1, so the target lies strictly inside [0, total)
   const float u = fminf(fmaxf(uniform[row], 0.f), 0.99999994f);
   unsigned long long target = (unsigned long long)((double)u * (double)total);
-  if (target >= total) target = total - 1ull;
-  const bool mine = total > 0ull && target >= cta_before && target < cta_before + cta_total;
-  if (mine) {
-    const unsigned long long tl = target - cta_before;
-    if (local > 0ull && before <= tl && tl < before + local) {
-      unsigned long long acc = before;
-      int pick = -1;
-      for (int i = c0; i < c1; ++i) {
-        const float e = vals[i];
-        if (__float_as_uint(e) >= thr_key) {
-          acc += (unsigned long long)(e * SC_FX);
-          pick = i;
-          if (acc > tl) break;
-        }
+  if (target >= total && total > 0ull) target = total - 1ull;
+  before += cta_before;
+  if (local > 0ull && before <= target && target < before + local) {
+    for (int b = c0; b < c1; b += 32) {
+      const int i = b + lane;
+      const uint32_t key = i < c1 ? key_of(ldf(vals, i)) : 0u;
+      unsigned long long incl = i < c1 && key >= thr_key ? sc_fx(key) : 0ull;
+      if (!__any_sync(0xffffffffu, incl > 0ull)) continue;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
       }
-      out[row] = i0 + pick;
+      const uint32_t past = __ballot_sync(0xffffffffu, before + incl > target);
+      if (past) {
+        if (lane == 0) out[row] = i0 + b + __ffs(past) - 1;
+        break;
+      }
+      before += __shfl_sync(0xffffffffu, incl, 31);
     }
+  } else if (total == 0ull && cr == 0u && tid == 0) {
+    out[row] = 0;  // no token has mass: nothing but NaN and minus infinity
   }
   // a CTA must not exit while a peer may still read its shared memory
   if (csize > 1) cluster_sync_all();
@@ -636,23 +798,30 @@ static int g_force_cluster = 0;
 // Test hook: pin the cluster size of the cluster sampler (1, 2, 4 or 8; 0 = chosen from the vocabulary).
 extern "C" void pg_sample_force_cluster(int c) { g_force_cluster = c; }
 
-// Cluster size and slice length of the cluster sampler for a vocabulary, or 0 when the row does
-// not fit the shared memory of eight CTAs (the one-CTA kernel serves those).
-static int sampler_cluster_plan(int vocab, int max_smem, int* slice_out) {
-  const int room = (max_smem - 2048 - (int)sizeof(ScShared) - 64) / 4;  // floats per CTA (2 KB left for static shared memory)
-  int c = 1;
-  while (c < SC_MAX_CLUSTER && (ceil_div(vocab, c) > 24 * 1024 || ceil_div(vocab, c) > room)) c *= 2;
-  if (g_force_cluster > 0) c = g_force_cluster;
-  const int slice = (ceil_div(vocab, c) + 3) & ~3;
-  if (slice > room) return 0;
-  *slice_out = slice;
-  return c;
+// Cluster size and slice length of the cluster sampler for a vocabulary, or 0 when the row does not fit the shared memory of
+// eight CTAs (the one-CTA kernel serves those).  A wave holds so many clusters of 1, 2, 4, 8 CTAs at one or two CTAs an SM
+// (74 / 33 / 15 clusters of 2 / 4 / 8 fit the GPCs); a row's time is about that of 40 K tokens more than its slice has.
+// 64 x 151936, top-k 50: 102 us with clusters of 8 (three waves of 30), 62 us with 4 (one wave of 66), 83 us with 2; 8 rows:
+// 42 us with 8, 51 us with 4.
+static int sampler_cluster_plan(int rows, int vocab, int elem, int max_smem, int* slice_out) {
+  const int room = (max_smem - 2048 - (int)sizeof(ScShared) - 64) / elem;  // tokens per CTA (2 KB left for static shared memory)
+  static const int per_wave[4] = {148, 74, 33, 15};
+  int best = 0;
+  double least = 0;
+  for (int l = 0; l < 4; ++l) {
+    const int c = 1 << l, slice = (ceil_div(vocab, c) + 7) & ~7;
+    if (slice > room || (g_force_cluster > 0 && c != g_force_cluster)) continue;
+    const int wave = per_wave[l] * (2 * (slice * elem + (int)sizeof(ScShared) + 2048) <= max_smem ? 2 : 1);
+    const double cost = (double)ceil_div(rows, wave) * (slice + 40.0 * 1024);
+    if (best == 0 || cost < least) best = c, least = cost, *slice_out = slice;
+  }
+  return best;
 }
 
 template <typename T>
 static int launch_sample_cluster(const T* logits, long long ld, int rows, int vocab, int c, int slice, const float* temperature, const int* top_k,
                                  const float* top_p, const float* min_p, const float* uniform, int* out, cudaStream_t stream) {
-  const size_t smem = ((sizeof(ScShared) + 15) & ~size_t(15)) + (size_t)slice * 4;
+  const size_t smem = ((sizeof(ScShared) + 15) & ~size_t(15)) + (size_t)slice * sizeof(T);
   static bool attr_done[2] = {false, false};
   const int which = sizeof(T) == 4 ? 1 : 0;
   if (!attr_done[which]) {
@@ -701,7 +870,7 @@ extern "C" int pg_sample(const void* logits, int is_f32, int rows, int vocab, lo
     use_cluster = (e && e[0] == '0') ? 0 : 1;
   }
   int slice = 0;
-  const int c = use_cluster ? sampler_cluster_plan(vocab, max_smem, &slice) : 0;
+  const int c = use_cluster ? sampler_cluster_plan(rows, vocab, is_f32 ? 4 : 2, max_smem, &slice) : 0;
   if (c > 0) {
     if (is_f32)
       return launch_sample_cluster<float>((const float*)logits, ld, rows, vocab, c, slice, (const float*)temperature, (const int*)top_k, (const float*)top_p,

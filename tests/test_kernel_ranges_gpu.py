@@ -70,3 +70,46 @@ def test_kda_blocks_of_four_tokens(dv):
             assert (o1[i].double() - want).abs().max() <= 2 ** -8 * want.abs().max() + 1e-5
         at += n
     assert (st1.double() - st2).abs().max() < 2 ** -17 * st2.abs().max()
+
+
+@pytest.mark.parametrize("vocab,dtype", [(9, torch.bfloat16), (1023, torch.float32), (24577, torch.bfloat16), (49160, torch.float32), (151936, torch.bfloat16), (163841, torch.bfloat16)])
+def test_sampler_brackets(vocab, dtype):
+    """Thresholds where the coarse bracket is hard: every token alike, tokens spread over few bins (more of them than the
+    list holds), a limit of no mass, masked tokens, infinities; odd vocabularies (rows that are not 16-byte aligned)."""
+    g = torch.Generator(device=DEV).manual_seed(vocab)
+    lg = torch.randn(12, vocab, device=DEV, generator=g)
+    lg[1] = 1.25
+    lg[2] *= 0.002
+    lg[3] = lg[3] * 2.5
+    lg[4, vocab // 2 :] = float("-inf")
+    lg[5] = float("-inf")
+    lg[5, vocab - 1] = 0.0
+    lg[6, 3] = float("inf")
+    lg[7, 0] = float("nan")
+    lg[8] *= 30
+    lg = lg.to(dtype)
+    one = torch.ones(12, device=DEV)
+    for k, p, m in ((0, 0.95, 0.0), (0, 0.5, 0.0), (40, 1.0, 0.0), (3, 0.9, 0.0), (1, 1.0, 0.0), (0, 0.0, 0.0), (0, 1.0, 0.05), (0, 1.0, 0.0), (vocab - 1, 0.999, 0.001)):
+        u = torch.rand(12, device=DEV, generator=g)
+        got = cu().sample(lg, one, torch.full((12,), k, dtype=torch.int32, device=DEV), one * p, one * m, u).long()
+        assert ((got >= 0) & (got < vocab)).all()
+        assert got[5] == vocab - 1 and got[6] == 3 and (got[7] != 0 or p == 0.0)
+        rows = [0, 1, 2, 3, 4, 8]  # finite maxima: the kernel's e = exp(s - max) is within 2^-20 of this one
+        s = lg[rows].double()
+        e = torch.exp(s - s.amax(-1, keepdim=True))
+        srt = e.sort(-1, descending=True).values
+        before = srt.cumsum(-1) - srt
+        keep = (torch.arange(vocab, device=DEV) < (k if 0 < k < vocab else vocab)).expand(len(rows), -1)
+        if p < 1:
+            keep = keep & (before < p * e.sum(-1, keepdim=True) * (1 + 1e-5))  # a hair wide: the tokens at the crossing
+        keep = keep | (torch.arange(vocab, device=DEV) == 0)
+        thr = torch.where(keep, srt, torch.full_like(srt, 2.0)).amin(-1, keepdim=True)
+        pick = e.gather(-1, got[rows, None])
+        assert (pick >= thr * (1 - 1e-5)).all() and (pick >= m * (1 - 1e-5)).all()
+        if p == 1.0:  # the keep-set is known: the draw is the one that the cumulative mass in vocabulary order names
+            mass = torch.where((e >= thr * (1 - 1e-9)) & (e >= m), e, torch.zeros_like(e))
+            cdf = mass.cumsum(-1)
+            target = u[rows, None].double() * cdf[:, -1:]
+            slack = cdf[:, -1:] * 2e-5
+            at = cdf.gather(-1, got[rows, None])
+            assert (at >= target - slack).all() and (at - mass.gather(-1, got[rows, None]) <= target + slack).all()
