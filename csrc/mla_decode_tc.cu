@@ -1,0 +1,403 @@
+// Absorbed latent attention of single query rows on tcgen05 (latents of 512 columns with 64 rotated ones or none).
+//
+// All heads of a row read the same keys, so the heads are the narrow side of both products and everything is transposed:
+// with a tile of 64 keys in shared memory, S^T [64 keys, heads] = K Q^T and O^T [512, heads] += V^T P^T, four accumulators of
+// 128 value columns x heads in tensor memory.  K is the tile read K-major, V^T the same bytes read MN-major, Q stays in
+// shared memory, P^T is written back MN-major (a key's row of heads).  A tile is made of eight boxes of eight keys, each one
+// copy of [block of 64 columns][8 keys][128 bytes] (a 16-token page is two of them; boxes of one block and a page's keys are
+// 36 copies of 2 KB a tile, which took 1.25 us to issue), and the operand descriptors step from box to box.  Two tiles of
+// 72 KB, Q (72 KB at 64 heads) and P fill the shared memory, so a CTA owns an SM; a split of a row's keys over CTAs is merged
+// by a second kernel.
+//
+// A product of 64 rows leaves them in the lower half of each warp's tensor-memory lanes: a warp has 16 keys, and a thread
+// reads two of them for a quarter of the heads.  Rows are reduced across threads only when it matters: exponentials refer to
+// a reference value per head that moves only if some score exceeds it by more than 2^8 (the tile's maxima are formed then, and
+// O and the sums rescaled), and each thread sums its own keys' weights, added up once at the end.
+//
+// Against the mma.sync kernel, in which a CTA of 16 heads exchanges partial scores through shared memory for every 32 keys
+// (128 rows x 64 heads x 1150 keys): 284 us before, 90 us now.  What
+// bounds it: the chain copy, scores, softmax, output product of a tile, 2.3 us with two tiles in flight; the keys' bytes take 26 us.
+#include "api.h"
+#include "attention_tc.cuh"
+#include "mla_decode_tc.h"
+
+namespace {
+
+constexpr int DT_KEYS = 64;
+constexpr int DT_P = DT_KEYS * 128;      // weights: 64 keys x 64 heads
+constexpr int DT_THREADS = 192;          // producer, MMA, four softmax / epilogue warps
+constexpr float DT_NONE = -1e30f;        // reference of a head that has seen no key; also "no keys" among the partial results
+
+template <int HN>
+struct DtSync {
+  uint64_t full[2], empty[2], cleared, s_full[2], p_ready, o_full;
+  uint32_t tmem_slot;
+  int abort_flag;
+  alignas(16) int grew[2][4];          // by tile parity and warp: some score exceeds its reference by too much
+  float ref[HN], fac[HN];  // log2 units; factor on what was summed so far, at the end on the output
+  float part[4][HN];       // per warp: maxima of a tile, at the end sums of weights
+};
+
+__device__ __forceinline__ void dt_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
+// 16 lanes x HN columns of tensor memory as mma fragments: r[4 i + e] = lane (lane / 4, + 8 for e >= 2), column 8 i + 2 (lane % 4) + (e & 1).
+template <int HN>
+__device__ __forceinline__ void dt_ld_frag(uint32_t taddr, uint32_t* r) {
+#pragma unroll
+  for (int c = 0; c < HN / 16; ++c)
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[8 * c]), "=r"(r[8 * c + 1]), "=r"(r[8 * c + 2]), "=r"(r[8 * c + 3]), "=r"(r[8 * c + 4]), "=r"(r[8 * c + 5]), "=r"(r[8 * c + 6]), "=r"(r[8 * c + 7])
+                 : "r"(taddr + 16 * c)
+                 : "memory");
+}
+// K-major operand whose groups of eight rows are `sbo` bytes apart
+__device__ __forceinline__ uint64_t dt_desc_k(uint32_t smem_addr, uint32_t sbo) {
+  return (umma_desc_k_sw128(smem_addr) & ~((uint64_t)0x3FFF << 32)) | (uint64_t)(sbo >> 4) << 32;
+}
+
+// CTA = (token row, group of HN heads, split).  QKB: 64-column blocks of a key.
+template <int HN, int QKB>
+__global__ void __launch_bounds__(DT_THREADS, 1) mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tm, const MlaDecodeTc p) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = smem_u32(smem_raw);
+  uint8_t* tiles = smem_raw + (((base + 1023u) & ~1023u) - base);
+  constexpr int BOX = QKB * 1024, STAGE = DT_KEYS / 8 * BOX, QBLK = HN * 128;
+  uint8_t* q_sm = tiles + 2 * STAGE;
+  uint8_t* p_sm = q_sm + QKB * QBLK;
+  DtSync<HN>* sh = reinterpret_cast<DtSync<HN>*>(p_sm + DT_P);
+  constexpr uint32_t TMEM_COLS = HN == 64 ? 512 : HN == 32 ? 256 : 128;  // S twice, O four times
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int groups = (p.heads + HN - 1) / HN;
+  const int split = blockIdx.x % p.splits;
+  const int h0 = blockIdx.x / p.splits % groups * HN;
+  const int t = blockIdx.x / (p.splits * groups);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&sh->full[s], 1);
+      mbar_init(&sh->empty[s], 1);
+      mbar_init(&sh->s_full[s], 1);
+    }
+    mbar_init(&sh->cleared, 4);
+    mbar_init(&sh->p_ready, 4);
+    mbar_init(&sh->o_full, 1);
+    sh->abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tm);
+  }
+  if (warp == 1) {
+    tmem_alloc(&sh->tmem_slot, TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sh->tmem_slot;
+  volatile int* abort_flag = &sh->abort_flag;
+  PG_PDL_ENTRY();
+
+  const int b = p.unit_seq[p.first_row + t];
+  const int q0 = p.q_indptr[b], q1 = p.q_indptr[b + 1];
+  const int kv_len = p.kv_lens[b];
+  const int pos = kv_len - (q1 - q0) + (p.first_row + t - q0);  // of this query token
+  const int kv_end = kv_len == 0 ? 0 : pos + 1;
+  const int kv_begin = p.window > 0 ? max(0, kv_end - p.window) : 0;
+  const int tile0 = kv_begin / DT_KEYS, all_tiles = (kv_end + DT_KEYS - 1) / DT_KEYS;
+  const int per_split = (all_tiles - tile0 + p.splits - 1) / p.splits;
+  const int first = tile0 + split * per_split, n_tiles = max(0, min(all_tiles, first + per_split) - first);
+
+  const int ragged = kv_end % DT_KEYS ? all_tiles - 1 - first : -1;  // tile whose last rows are no keys (of another split if it is not below n_tiles)
+
+  if (warp == 0) {
+    const uint64_t pol = l2_policy_evict_first();
+    const int* table = p.table + (long long)b * p.table_stride;
+    bool ok = true;
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      const int st = j & 1, key = (first + j) * DT_KEYS + lane * 8;  // of this lane's box
+      const int boxes = min(DT_KEYS / 8, (kv_end - (first + j) * DT_KEYS + 7) / 8);
+      const int page = lane < boxes ? table[min(key / p.page_size, p.table_stride - 1)] : 0;
+      if (j >= 2) ok = mbar_wait(&sh->empty[st], (uint32_t)(((j >> 1) - 1) & 1), abort_flag);
+      ok = __all_sync(0xFFFFFFFFu, ok);
+      if (!ok) break;
+      if (lane == 0) mbar_expect_tx(&sh->full[st], (uint32_t)(boxes * BOX));
+      __syncwarp();
+      if (lane < boxes) tma_load_3d(tiles + st * STAGE + lane * BOX, &tm, &sh->full[st], 0, page * p.page_size + key % p.page_size, 0, pol);
+    }
+  } else {
+    // queries into shared memory while the first tiles are on their way: [block][head][128 B], 128-byte swizzle
+    for (int i = threadIdx.x - 32; i < HN * QKB * 8; i += DT_THREADS - 32) {
+      const int h = i / (QKB * 8), ch = i % (QKB * 8), head = min(h0 + h, p.heads - 1);  // heads past the last: any row, not stored
+      uint4* dst = reinterpret_cast<uint4*>(q_sm + (ch >> 3) * QBLK + h * 128 + (((ch & 7) ^ (h & 7)) << 4));
+      const bf16* src = ch < 64 ? p.q_abs + t * p.q_tok + head * p.q_head + ch * 8 : p.q_pe + t * p.pe_tok + head * p.pe_head + (ch - 64) * 8;
+      if (ch < 64 || p.cos == nullptr) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+      } else {
+        uint4 v = *reinterpret_cast<const uint4*>(src);
+        const long long at = (long long)min(max(pos, 0), p.max_pos - 1) * 32 + (ch - 64) * 4;
+        uint32_t* w = &v.x;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = __bfloat1622float2(*reinterpret_cast<const bf162*>(&w[j]));
+          const float cs = p.cos[at + j], sn = p.sin[at + j];
+          const bf162 r = __floats2bfloat162_rn(f.x * cs - f.y * sn, f.y * cs + f.x * sn);
+          w[j] = *reinterpret_cast<const uint32_t*>(&r);
+        }
+        *dst = v;
+      }
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    fence_proxy_async_smem();
+    asm volatile("bar.sync 2, 160;" ::: "memory");
+  }
+  if (warp == 1) {
+    if (lane == 0 && n_tiles > 0) {
+      constexpr uint32_t idesc_s = idesc_bf16(DT_KEYS, HN, 0);
+      constexpr uint32_t idesc_o = idesc_bf16(128, HN, 1) | (1u << 15);  // both operands MN-major
+      const uint32_t qa = smem_u32(q_sm), pa = smem_u32(p_sm);
+      // Whatever is ready goes first: the product with V as soon as P is there (it frees the tile's memory), the scores of the
+      // next tile as soon as it has landed.  (Scores always first left a finished P waiting for a tile that could only be
+      // fetched after that product: 3.9 us a tile.)
+      int s_next = 0, o_next = 0;
+      uint32_t spins = 0;
+      uint64_t since = globaltimer_ns();
+      while (o_next < n_tiles) {
+        const int ss = s_next & 1, os = o_next & 1;
+        if (s_next > o_next && mbar_try_wait(&sh->p_ready, (uint32_t)(o_next & 1))) {
+          tc_fence_after();
+          const uint32_t va = smem_u32(tiles + os * STAGE);
+#pragma unroll
+          for (int mb = 0; mb < 4; ++mb)
+#pragma unroll
+            for (int ks = 0; ks < DT_KEYS / 16; ++ks)
+              umma_bf16_ss(tmem + (uint32_t)((2 + mb) * HN), umma_desc_mn_sw128(va + mb * 2048 + ks * 2 * BOX, 1024u, BOX), umma_desc_mn_sw128(pa + ks * 2048, DT_P, 1024u), idesc_o,
+                           (o_next | ks) ? 1u : 0u);
+          umma_commit(&sh->o_full);
+          umma_commit(&sh->empty[os]);
+          ++o_next;
+        } else if (s_next < n_tiles && s_next <= o_next + 1 && mbar_try_wait(&sh->full[ss], (uint32_t)((s_next >> 1) & 1)) && (s_next != ragged || mbar_try_wait(&sh->cleared, 0))) {
+          tc_fence_after();
+          const uint32_t ka = smem_u32(tiles + ss * STAGE);
+#pragma unroll
+          for (int cb = 0; cb < QKB; ++cb)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              umma_bf16_ss(tmem + (uint32_t)(ss * HN), dt_desc_k(ka + cb * 1024 + k * 32, BOX), umma_desc_k_sw128(qa + cb * QBLK + k * 32), idesc_s, (cb | k) ? 1u : 0u);
+          umma_commit(&sh->s_full[ss]);
+          ++s_next;
+        } else {
+          if ((++spins & 63u) == 0u && (*abort_flag || globaltimer_ns() - since > PG_WAIT_LIMIT_NS)) {
+            *abort_flag = 1;
+            break;
+          }
+          continue;
+        }
+        since = globaltimer_ns();
+      }
+    }
+  } else if (warp >= 2) {
+    const int wq = warp & 3, tid = wq * 32 + lane;  // tensor-memory lanes of this warp: 32 wq ..
+    const uint32_t row = tmem + ((uint32_t)(wq * 32) << 16);
+    const int key_a = wq * 16 + (lane >> 2), col = 2 * (lane & 3);  // keys key_a and key_a + 8, heads 8 i + col and the next one
+    constexpr int HB = HN / 8;
+    float l[HB][2], ref[HB][2];
+#pragma unroll
+    for (int i = 0; i < HB; ++i) l[i][0] = l[i][1] = 0.f, ref[i][0] = ref[i][1] = DT_NONE;
+    if (tid < HN) sh->ref[tid] = DT_NONE;
+    bool ok = true;  // after a wait that ran out the warps go on through the barriers, without work
+    for (int j = 0; j < n_tiles; ++j) {
+      const int st = j & 1, key0 = (first + j) * DT_KEYS;
+      if (j == ragged) {
+        // rows behind the last key may hold anything, and zero weights do not silence a NaN: clear their values
+        ok = ok && mbar_wait(&sh->full[st], (uint32_t)((j >> 1) & 1), abort_flag);
+        const int live = kv_end - key0;
+        if (ok)
+          for (int i = tid; i < (DT_KEYS - live) * 64; i += 128) {
+            const int r = live + (i >> 6);
+            *reinterpret_cast<uint4*>(tiles + st * STAGE + (r >> 3) * BOX + (i & 7) * 1024 + (r & 7) * 128 + ((i >> 3) & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+          }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->cleared);
+      }
+      float v[HB][4];  // columns col, col + 1 of key_a, then of key_a + 8
+      bool grew = false;
+      ok = ok && mbar_wait(&sh->s_full[st], (uint32_t)((j >> 1) & 1), abort_flag);
+      ok = __all_sync(0xFFFFFFFFu, ok);
+      if (ok) {
+        tc_fence_after();
+        dt_ld_frag<HN>(row + (uint32_t)(st * HN), reinterpret_cast<uint32_t*>(&v[0][0]));
+        tmem_ld_wait();
+        const int ka = key0 + key_a, kb = ka + 8;
+        const bool live_a = ka < kv_end && ka >= kv_begin, live_b = kb < kv_end && kb >= kv_begin;
+        float over = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < HB; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            v[i][e] = (e < 2 ? live_a : live_b) ? v[i][e] * p.scale_log2 : -INFINITY;
+            over = fmaxf(over, v[i][e] - ref[i][e & 1]);
+          }
+        grew = __any_sync(0xFFFFFFFFu, over > RESCALE_LOG2);
+      }
+      if (lane == 0) sh->grew[st][wq] = grew;
+      dt_barrier();
+      // the previous product is complete: O may be rescaled, P written again
+      if (j > 0) {
+        ok = ok && mbar_wait(&sh->o_full, (uint32_t)((j - 1) & 1), abort_flag);
+        ok = __all_sync(0xFFFFFFFFu, ok);
+        tc_fence_after();
+      }
+      const int4 any = *reinterpret_cast<const int4*>(sh->grew[st]);
+      if (any.x | any.y | any.z | any.w) {
+#pragma unroll
+        for (int i = 0; i < HB; ++i)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float mx = ok ? fmaxf(v[i][e], v[i][e + 2]) : -INFINITY;
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+            if (lane < 4) sh->part[wq][8 * i + col + e] = mx;
+          }
+        dt_barrier();
+        if (tid < HN) {
+          const float old = sh->ref[tid], mx = fmaxf(fmaxf(sh->part[0][tid], sh->part[1][tid]), fmaxf(sh->part[2][tid], sh->part[3][tid]));
+          const bool move = mx > old + RESCALE_LOG2;
+          sh->fac[tid] = move ? exp2f(old - mx) : 1.f;  // 0 for the first keys
+          if (move) sh->ref[tid] = mx;
+        }
+        dt_barrier();
+#pragma unroll
+        for (int i = 0; i < HB; ++i)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            l[i][e] *= sh->fac[8 * i + col + e];
+            ref[i][e] = sh->ref[8 * i + col + e];
+          }
+        if (j > 0 && ok) {
+#pragma unroll 1
+          for (int mb = 0; mb < 4; ++mb)
+#pragma unroll 1
+            for (int c = 0; c < HN; c += 16) {
+              uint32_t w[16];
+              tmem_ld16(row + (uint32_t)((2 + mb) * HN + c), w);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(__uint_as_float(w[i]) * sh->fac[c + i]);
+              tmem_st16(row + (uint32_t)((2 + mb) * HN + c), w);
+            }
+          tmem_st_wait();
+        }
+      }
+      if (ok) {
+#pragma unroll
+        for (int i = 0; i < HB; ++i) {
+          const float a0 = ex2_approx(v[i][0] - ref[i][0]), a1 = ex2_approx(v[i][1] - ref[i][1]), b0 = ex2_approx(v[i][2] - ref[i][0]), b1 = ex2_approx(v[i][3] - ref[i][1]);
+          l[i][0] += a0 + b0;
+          l[i][1] += a1 + b1;
+          uint8_t* at = p_sm + key_a * 128 + ((i ^ (key_a & 7)) << 4) + col * 2;  // (key_a + 8 has the same swizzle)
+          *reinterpret_cast<bf162*>(at) = __floats2bfloat162_rn(a0, a1);
+          *reinterpret_cast<bf162*>(at + 8 * 128) = __floats2bfloat162_rn(b0, b1);
+        }
+      }
+      fence_proxy_async_smem();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh->p_ready);
+    }
+#pragma unroll
+    for (int i = 0; i < HB; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float x = l[i][e];
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) x += __shfl_xor_sync(0xFFFFFFFFu, x, o);
+        if (lane < 4) sh->part[wq][8 * i + col + e] = x;
+      }
+    if (n_tiles > 0) {
+      ok = ok && mbar_wait(&sh->o_full, (uint32_t)((n_tiles - 1) & 1), abort_flag);
+      ok = __all_sync(0xFFFFFFFFu, ok);
+      tc_fence_after();
+    }
+    dt_barrier();
+    if (tid < HN && h0 + tid < p.heads) {
+      const int head = h0 + tid;
+      const float m = sh->ref[tid];
+      float sum = (sh->part[0][tid] + sh->part[1][tid]) + (sh->part[2][tid] + sh->part[3][tid]), f = 0.f;
+      if (p.splits > 1) p.part_lse[((long long)t * p.heads + head) * p.splits + split] = sum > 0.f ? m + log2f(sum) : DT_NONE;
+      if (sum > 0.f) {
+        if (p.splits == 1 && p.sink) sum += exp2f(p.sink[head] * 1.4426950408889634f - m);
+        f = 1.f / sum;
+        if (p.splits == 1 && p.gate) f /= 1.f + __expf(-__bfloat162float(p.gate[t * p.ld_gate + head]));
+      }
+      sh->fac[tid] = f;
+    }
+    dt_barrier();
+    if (ok) {
+#pragma unroll 1
+      for (int mb = 0; mb < 4; ++mb)
+#pragma unroll 1
+        for (int c = 0; c < HN; c += 16) {
+          uint32_t w[16];
+          if (n_tiles > 0) {
+            tmem_ld16(row + (uint32_t)((2 + mb) * HN + c), w);
+            tmem_ld_wait();
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int head = h0 + c + i, d = mb * 128 + tid;
+            if (head >= p.heads) break;
+            const float x = n_tiles > 0 ? __uint_as_float(w[i]) * sh->fac[c + i] : 0.f;
+            if (p.splits == 1)
+              p.out[t * p.o_tok + head * p.o_head + d] = __float2bfloat16(x);
+            else if (n_tiles > 0)
+              p.part_o[(((long long)t * p.heads + head) * p.splits + split) * 512 + d] = x;
+          }
+        }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem, TMEM_COLS);
+  }
+  if (threadIdx.x == 0 && sh->abort_flag) atomicCAS(p.status, PG_ST_OK, PG_ST_TIMEOUT | (58u << 8));
+}
+
+template <int HN, int QKB>
+int launch(const CUtensorMap& tm, const MlaDecodeTc& p, cudaStream_t stream) {
+  constexpr size_t smem = (size_t)2 * QKB * DT_KEYS * 128 + QKB * HN * 128 + DT_P + sizeof(DtSync<HN>) + 1024;
+  static bool set = false;
+  if (!set) {
+    PG_CUDA(cudaFuncSetAttribute(mla_decode_tc_kernel<HN, QKB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    set = true;
+  }
+  const unsigned grid = (unsigned)(p.tokens * ((p.heads + HN - 1) / HN) * p.splits);
+  PG_CUDA(launch_pdl(mla_decode_tc_kernel<HN, QKB>, dim3(grid), dim3(DT_THREADS), smem, stream, tm, p));
+  PG_LAUNCH_CHECK();
+  return PG_OK;
+}
+
+}  // namespace
+
+int mla_decode_tc(const MlaDecodeTc& p, int r, long long pages, cudaStream_t stream) {
+  CUtensorMap tm;
+  // eight keys of all blocks of 64 columns per copy
+  const cuuint64_t dims[3] = {64u, (cuuint64_t)(pages * p.page_size), (cuuint64_t)((512 + r) / 64)}, strides[2] = {(cuuint64_t)(512 + r) * 2, 128u};
+  const cuuint32_t box[3] = {64u, 8u, (cuuint32_t)((512 + r) / 64)};
+  if (int rc = make_tmap_bf16(&tm, p.latent, 3, dims, strides, box)) return rc;
+  // A block of 64 heads reads a key once for all of them; steps that leave SMs idle get blocks of fewer heads, whose start, first
+  // tile and output take less (one row of 64 heads, 100 keys: 45 us for the whole operation with blocks of 64, 37 us with 16).
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? n : 148;
+  }();
+  int hn = 64;
+  while (hn > 16 && (p.heads <= hn / 2 || p.tokens * p.splits * ((p.heads + hn / 2 - 1) / (hn / 2)) <= sms)) hn /= 2;
+  switch (hn) {
+    case 16: return r ? launch<16, 9>(tm, p, stream) : launch<16, 8>(tm, p, stream);
+    case 32: return r ? launch<32, 9>(tm, p, stream) : launch<32, 8>(tm, p, stream);
+    default: return r ? launch<64, 9>(tm, p, stream) : launch<64, 8>(tm, p, stream);
+  }
+}

@@ -1544,6 +1544,13 @@ def _head_offsets(heads: int, tokens: int, device):
     return o
 
 
+def _latent_splits(rows: int, heads: int, lat: int, rot: int, longest: int, sms: int) -> int:
+    """Blocks that share one row's keys in the absorbed kernels."""
+    if lat == 512 and rot in (0, 64):  # csrc/mla_decode_tc.cu: a block owns an SM and serves up to 64 heads, so as many as there are SMs, of 256 keys or more
+        return max(1, min(16, sms // (rows * ((heads + 63) // 64)), (longest + 255) // 256))
+    return max(1, min(16, (4 * sms) // (rows * ((heads + 15) // 16)), (min(longest, 4096) + 127) // 128))
+
+
 def _mla_expanded_seqs(q: "_MlaQ", w_uk, w_uv, meta: AttnMeta, kv_lora) -> int:
     """How many leading sequences of the step take the expanded-form tcgen05 prefill: the prefill chunks (at least
     two rows each) in front of the step's single-row decodes, when they have the 128 + 64 / 128 head shape and are
@@ -1659,11 +1666,7 @@ def mla_attention(q: "_MlaQ", w_uk, w_uv, latent_layer, meta: AttnMeta, scale, k
         for b in range(meta.num_seqs):
             seq_of.extend([b] * (qi[b + 1] - qi[b]))
         unit_seq = torch.tensor(seq_of, dtype=torch.int32, device=dev)
-    groups = h // 16
-    if meta.decode_only:
-        splits = max(1, min(16, (4 * c.sms) // max(1, t * groups), (min(meta.max_kv_len, 4096) + 127) // 128))
-    else:
-        splits = 1
+    splits = _latent_splits(t, h, kv_lora, rope, meta.max_kv_len, c.sms) if meta.decode_only else 1
     need = t * h * splits * (kv_lora + 1) * 4
     if need > c.attn_part.numel():
         splits = 1
@@ -1672,7 +1675,7 @@ def mla_attention(q: "_MlaQ", w_uk, w_uv, latent_layer, meta: AttnMeta, scale, k
     lat_out = torch.empty((h * t, kv_lora), dtype=torch.bfloat16, device=dev)
     rc = lib().pg_mla_attention(_ptr(q_abs), _ptr(q.pe), _ptr(latent_layer), _ptr(lat_out), _ptr(meta.q_indptr), _ptr(meta.kv_lens), _ptr(meta.block_table),
                                 _ci(meta.block_table.stride(0)), _ptr(unit_seq), _ci(meta.num_seqs), _ci(t), _ci(h), _ci(kv_lora), _ci(rope), _ci(page_size), _cf(scale),
-                                _ci(splits), _ptr(part_o), _ptr(part_lse), _ptr(c.status), _stream())
+                                _ci(splits), _ptr(part_o), _ptr(part_lse), _ll(latent_layer.shape[0]), _ptr(c.status), _stream())
     _check(rc, c, 2 if splits > 1 else 1)
     v_hm = grouped_gemm(lat_out, offs, w_uv, None, bn)  # [H*T, v]
     vdim = w_uv.shape[1]
@@ -1790,11 +1793,10 @@ def latent_attention(q, uk_t, uv, ukv, cache, meta: AttnMeta, rot: int, scale: f
     where = (_ptr(cache), _ptr(o), *strides, _ptr(meta.q_indptr), _ptr(meta.kv_lens), _ptr(table), _ci(table.stride(0)), _ptr(_unit_seq(meta, dev)))
     if aligned and lat <= 512 and rot <= 64:
         longest = max(meta.max_kv_len, 1)
-        longest = min(longest, window + 31) if window else min(longest, 4096)
-        splits = max(1, min(16, (4 * c.sms) // (n * ((heads + 15) // 16)), (longest + 127) // 128))
+        splits = _latent_splits(n, heads, lat, rot, min(longest, window + 31) if window else longest, c.sms)
         splits = max(1, min(splits, c.attn_part.numel() // (n * heads * (lat + 1) * 4)))
         rc = lib().pg_latent_attention(_ptr(q_abs), *strides, *pe, *where, _ci(row0), _ci(meta.num_seqs), _ci(n), _ci(heads), _ci(lat), _ci(rot), _ci(ps), _cf(scale), _ci(window), *extra, _ci(splits),
-                                       _ptr(c.attn_part), _ptr(c.attn_part[n * heads * splits * lat * 4 :]), _stream())
+                                       _ptr(c.attn_part), _ptr(c.attn_part[n * heads * splits * lat * 4 :]), _ll(cache.shape[0]), _ptr(c.status), _stream())
         _check(rc, c, 2 if splits > 1 else 1)
     else:
         assert row0 == 0

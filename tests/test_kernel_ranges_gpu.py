@@ -113,3 +113,35 @@ def test_sampler_brackets(vocab, dtype):
             slack = cdf[:, -1:] * 2e-5
             at = cdf.gather(-1, got[rows, None])
             assert (at >= target - slack).all() and (at - mass.gather(-1, got[rows, None]) <= target + slack).all()
+
+
+@pytest.mark.parametrize("heads,page,splits", [(16, 16, 1), (16, 64, 5), (32, 32, 2), (64, 16, 1), (64, 16, 3), (96, 16, 2)])
+def test_latent_decode_tiles(heads, page, splits, monkeypatch):
+    """Absorbed attention around tiles of 64 keys, padding rows, splits without keys, and rows behind a sequence's end that
+    hold NaN."""
+    torch.manual_seed(heads + page)
+    kv_lens = [1, 63, 64, 65, 0, 129, 200, 511, 1000, 77]
+    n = len(kv_lens)
+    per = [(x + page - 1) // page for x in kv_lens]
+    table, at = torch.zeros(n, max(per), dtype=torch.int32), 1
+    for i, m in enumerate(per):
+        table[i, :m] = torch.arange(at, at + m)
+        at += m
+    cache = torch.randn(at, page, 576, device=DEV).bfloat16()
+    for i, (x, m) in enumerate(zip(kv_lens, per)):
+        if m and x % page:
+            cache[table[i, m - 1].item(), x % page :] = float("nan")
+    pos = torch.tensor([max(x - 1, 0) for x in kv_lens], dtype=torch.int32, device=DEV)
+    meta = R.AttnMeta(torch.arange(n + 1, dtype=torch.int32, device=DEV), torch.tensor(kv_lens, dtype=torch.int32, device=DEV), table.to(DEV), pos, pos, page, n, n, 1, max(kv_lens), True,
+                      list(range(n + 1)), kv_lens)
+    q = torch.randn(n, heads, 192, device=DEV).bfloat16()
+    uk, uv = (torch.randn(heads, 128, 512, device=DEV) * 0.05).bfloat16(), (torch.randn(heads, 128, 512, device=DEV) * 0.05).bfloat16()
+    q[2] *= 8  # scores that pass the reference value by far in a later tile
+    cos, sin = R.rope_tables(2048, 64, 1e4, torch.bfloat16, DEV)
+    monkeypatch.setattr(cu(), "_latent_splits", lambda *a: splits)
+    got = cu().mla_attention(cu().mla_rope_q(q, cos, sin, meta, 128), uk, uv, cache, meta, 0.07, 512)
+    want = R.mla_attention(R.mla_rope_q(q, cos, sin, meta, 128), uk, uv, cache, meta, 0.07, 512)
+    assert not got[4].any() and torch.isfinite(got.float()).all()
+    # weights and outputs of both are rounded to bf16 (2^-8 each), the sums are of some hundred terms: 2^-6 of the largest
+    assert (got.float() - want.float()).abs().max() <= 2 ** -6 * want.float().abs().max()
+    assert cu().read_status(DEV) == 0
