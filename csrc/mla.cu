@@ -124,6 +124,39 @@ __global__ void __launch_bounds__(128) mla_q_prep_kernel(const bf16* __restrict_
   }
 }
 
+// The same for heads of 128 + 64 columns in groups of four, in 16-byte pieces: a warp's 32 lanes are the rotary parts of four
+// heads, and twice two heads' unrotated parts.  Bound by the rows (2999 x 16 heads: 17 us with a warp per head and two-byte
+// accesses to the rotary part, 5.9 us now).
+__global__ void __launch_bounds__(128) mla_q_prep_x4_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cos, const bf16* __restrict__ sin, const int* __restrict__ positions,
+                                                            bf16* __restrict__ q_nope_hm, bf16* __restrict__ q_pe, int tokens, int heads, int max_pos) {
+  const unsigned unit = blockIdx.x * 4u + (threadIdx.x >> 5), quads = heads / 4;
+  const int lane = threadIdx.x & 31;
+  if (unit >= (unsigned)tokens * quads) return;
+  const int t = (int)(unit / quads), h0 = (int)(unit % quads) * 4;
+  const bf16* src = q + ((long long)t * heads + h0) * 192;
+  uint4 a[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) a[i] = reinterpret_cast<const uint4*>(src + (2 * i + (lane >> 4)) * 192)[lane & 15];
+  const int h = lane >> 3, c = lane & 7;  // pairs 4 c .. 4 c + 3 of head h's rotary part
+  float x[8], cs[4], sn[4], lo[4], hi[4];
+  unpack8(*reinterpret_cast<const bf16x8*>(src + h * 192 + 128 + c * 8), x);
+  const int pos = min(max(positions[t], 0), max_pos - 1);
+  const uint2 cr = *reinterpret_cast<const uint2*>(cos + (long long)pos * 32 + c * 4), sr = *reinterpret_cast<const uint2*>(sin + (long long)pos * 32 + c * 4);
+  const bf16 *cp = reinterpret_cast<const bf16*>(&cr), *sp = reinterpret_cast<const bf16*>(&sr);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    cs[i] = __bfloat162float(cp[i]);
+    sn[i] = __bfloat162float(sp[i]);
+    lo[i] = x[2 * i] * cs[i] - x[2 * i + 1] * sn[i];
+    hi[i] = x[2 * i + 1] * cs[i] + x[2 * i] * sn[i];
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) reinterpret_cast<uint4*>(q_nope_hm + ((long long)(h0 + 2 * i + (lane >> 4)) * tokens + t) * 128)[lane & 15] = a[i];
+  bf16* dp = q_pe + ((long long)t * heads + h0 + h) * 64 + c * 4;
+  *reinterpret_cast<uint2*>(dp) = make_uint2(pack_bf16(lo[0], lo[1]), pack_bf16(lo[2], lo[3]));
+  *reinterpret_cast<uint2*>(dp + 32) = make_uint2(pack_bf16(hi[0], hi[1]), pack_bf16(hi[2], hi[3]));
+}
+
 __global__ void permute_021_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, int A, int B, int D) {
   const long long row = blockIdx.x;  // output row index b * A + a
   const int b = (int)(row / A), a = (int)(row % A);
@@ -616,6 +649,11 @@ extern "C" int pg_mla_q_prep(const void* q, const void* cos, const void* sin, co
   PG_REQUIRE(nope % 8 == 0 && rope % 2 == 0, "mla_q_prep: nope %d / rope %d not supported", nope, rope);
   if (tokens == 0) return PG_OK;
   const long long units = (long long)tokens * heads;
+  if (nope == 128 && rope == 64 && heads % 4 == 0 && units < (1ll << 31) && (((uintptr_t)q | (uintptr_t)q_nope_hm | (uintptr_t)q_pe) & 15) == 0 && (((uintptr_t)cos | (uintptr_t)sin) & 7) == 0) {
+    mla_q_prep_x4_kernel<<<(unsigned)((units / 4 + 3) / 4), 128, 0, stream>>>((const bf16*)q, (const bf16*)cos, (const bf16*)sin, (const int*)positions, (bf16*)q_nope_hm, (bf16*)q_pe, tokens, heads, max_pos);
+    PG_LAUNCH_CHECK();
+    return PG_OK;
+  }
   mla_q_prep_kernel<<<(unsigned)((units + 3) / 4), 128, 0, stream>>>((const bf16*)q, (const bf16*)cos, (const bf16*)sin, (const int*)positions,
                                                                     (bf16*)q_nope_hm, (bf16*)q_pe, tokens, heads, nope, rope, max_pos);
   PG_LAUNCH_CHECK();
