@@ -78,7 +78,7 @@ int pg_rms_norm(const void* x, void* residual, const void* w, void* y, int rows,
                 long long ldx, long long ldr, long long ldy, cudaStream_t stream);
 int pg_gated_rms_norm(const void* x, const void* gate, const void* w_f32, void* y, long long rows, int dim, float eps, cudaStream_t stream);
 // act 0: SiLU gate (as above); 1: bf16(norm * w) * bf16(sigmoid(gate))
-int pg_gated_rms_norm_act(const void* x, const void* gate, const void* w_f32, void* y, long long rows, int dim, float eps, int act, cudaStream_t stream);
+int pg_gated_rms_norm_act(const void* x, const void* gate, long long ld_gate, const void* w_f32, void* y, long long rows, int heads, int dim, float eps, int act, cudaStream_t stream);
 int pg_swiglu(const void* gate_up, void* out, int rows, int inter, long long ldin, long long ldout, int interleaved, cudaStream_t stream);
 int pg_sigmoid_gate_mul(void* x, const void* gate, long long n, cudaStream_t stream);
 int pg_qk_norm_rope_append(const void* qkv, long long ld, const void* q_w, const void* k_w, const void* cos, const void* sin,

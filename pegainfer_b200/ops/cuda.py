@@ -194,12 +194,16 @@ def gated_rms_norm(x, gate, w, eps, act: str = "silu"):
     """Per-head ``rms_norm(x) * w * silu(gate)``; ``act="sigmoid"``: ``bf16(rms_norm(x) * w) * bf16(sigmoid(gate))``."""
     _bf16(x)
     x = x.contiguous()
-    gate = gate.contiguous()
     w = w.float().contiguous()
+    dim, heads = x.shape[-1], x.shape[-2] if x.dim() == 3 else 1
+    if x.dim() == 3 and gate.dim() == 3 and gate.stride(2) == 1 and gate.stride(1) == dim:
+        ld = gate.stride(0)  # a column slice of a fused projection
+    else:
+        gate, ld = gate.contiguous(), heads * dim
     y = torch.empty_like(x)
-    rows = x.numel() // x.shape[-1]
+    rows = x.numel() // dim
     c = ctx(x.device)
-    _check(lib().pg_gated_rms_norm_act(_ptr(x), _ptr(gate), _ptr(w), _ptr(y), _ll(rows), _ci(x.shape[-1]), _cf(eps), _ci({"silu": 0, "sigmoid": 1}[act]), _stream()), c)
+    _check(lib().pg_gated_rms_norm_act(_ptr(x), _ptr(gate), _ll(ld), _ptr(w), _ptr(y), _ll(rows), _ci(heads), _ci(dim), _cf(eps), _ci({"silu": 0, "sigmoid": 1}[act]), _stream()), c)
     return y
 
 

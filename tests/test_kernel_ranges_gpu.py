@@ -145,3 +145,16 @@ def test_latent_decode_tiles(heads, page, splits, monkeypatch):
     # weights and outputs of both are rounded to bf16 (2^-8 each), the sums are of some hundred terms: 2^-6 of the largest
     assert (got.float() - want.float()).abs().max() <= 2 ** -6 * want.float().abs().max()
     assert cu().read_status(DEV) == 0
+
+
+@pytest.mark.parametrize("dim,heads,act", [(128, 6, "silu"), (128, 5, "sigmoid"), (256, 3, "silu"), (64, 7, "silu"), (96, 3, "sigmoid")])
+def test_gated_norm_reads_the_gate_in_place(dim, heads, act):
+    torch.manual_seed(dim)
+    t = 37  # rows that do not fill the last block
+    x = torch.randn(t, heads, dim, device=DEV).bfloat16()
+    fused = torch.randn(t, heads * dim + 24, device=DEV).bfloat16()
+    w = torch.rand(dim, device=DEV) + 0.5
+    for gate in (fused[:, 8 : 8 + heads * dim].reshape(t, heads, dim), fused[:, 1 : 1 + heads * dim].reshape(t, heads, dim)):  # 16-byte pieces; not even aligned
+        got, want = cu().gated_rms_norm(x, gate, w, 1e-6, act), R.gated_rms_norm(x, gate, w, 1e-6, act)
+        # f32 sums in another order: one step of bf16, two where two rounded factors meet
+        assert ((got.float() - want.float()).abs() <= 2 ** -7 * want.float().abs() + 1e-6).all()
