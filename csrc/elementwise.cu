@@ -184,12 +184,14 @@ __global__ void __launch_bounds__(128) gated_rms_norm_kernel(const bf16* __restr
 // `interleaved` = 0: a row is [gate_0 .. gate_{I-1}, up_0 .. up_{I-1}]; 1: (gate_0, up_0, gate_1, up_1, ...).
 // `flags`: bit 0 = gate / up columns interleaved, bit 1 = tanh GELU instead of SiLU on the gate (GeGLU), bit 2 = the
 // saturating form 4 tanh(g / 4) sigmoid(g) * 25 tanh(u / 25), rounded once (pegainfer-k3/kernels/tilelang_defs.py:244-262)
+// I: index type, 32-bit where the output has fewer than 2^31 pieces (a 64-bit division per piece is half of the kernel's work)
+template <typename I>
 __global__ void swiglu_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, int rows, int inter, long long ldin, long long ldout, int flags) {
   PG_PDL_ENTRY();
   const int interleaved = flags & 1, gelu = flags & 2, situ = flags & 4;
   const int nvec = inter / 8;
-  const long long total = (long long)rows * nvec;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
+  const I total = (I)rows * nvec;
+  for (I idx = (I)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (I)gridDim.x * blockDim.x) {
     const int row = (int)(idx / nvec), i = (int)(idx % nvec);
     float gf[8], uf[8], o[8];
     if (interleaved) {
@@ -229,8 +231,18 @@ __global__ void softcap_kernel(const bf16* __restrict__ x, bf16* __restrict__ y,
     y[i] = __float2bfloat16(tanhf(__bfloat162float(x[i]) * inv) * cap);
 }
 
-__global__ void sigmoid_gate_mul_kernel(bf16* __restrict__ x, const bf16* __restrict__ gate, long long n) {
+__global__ void sigmoid_gate_mul_kernel(bf16* __restrict__ x, const bf16* __restrict__ gate, long long n, long long vecs) {
   PG_PDL_ENTRY();
+  // `vecs` 16-byte pieces, then the rest
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += (long long)gridDim.x * blockDim.x) {
+    float xf[8], gf[8];
+    unpack8(reinterpret_cast<const bf16x8*>(x)[i], xf);
+    unpack8(reinterpret_cast<const bf16x8*>(gate)[i], gf);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) xf[j] = xf[j] / (1.f + __expf(-gf[j]));
+    reinterpret_cast<bf16x8*>(x)[i] = pack8(xf);
+  }
+  x += vecs * 8, gate += vecs * 8, n -= vecs * 8;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     float g = __bfloat162float(gate[i]);
     x[i] = __float2bfloat16(__bfloat162float(x[i]) / (1.f + __expf(-g)));
@@ -515,7 +527,8 @@ extern "C" int pg_swiglu(const void* gate_up, void* out, int rows, int inter, lo
   long long total = (long long)rows * (inter / 8);
   int blocks = (int)((total + 255) / 256);
   if (blocks > 148 * 16) blocks = 148 * 16;
-  PG_CUDA(launch_pdl(swiglu_kernel, dim3(blocks), dim3(256), (size_t)(0), stream, (const bf16*)gate_up, (bf16*)out, rows, inter, ldin, ldout, interleaved));
+  auto kernel = total < (1ll << 31) ? swiglu_kernel<unsigned> : swiglu_kernel<long long>;
+  PG_CUDA(launch_pdl(kernel, dim3(blocks), dim3(256), (size_t)(0), stream, (const bf16*)gate_up, (bf16*)out, rows, inter, ldin, ldout, interleaved));
   PG_LAUNCH_CHECK();
   return PG_OK;
 }
@@ -532,9 +545,10 @@ extern "C" int pg_softcap(const void* x, void* y, long long n, float cap, cudaSt
 
 extern "C" int pg_sigmoid_gate_mul(void* x, const void* gate, long long n, cudaStream_t stream) {
   if (n == 0) return PG_OK;
-  long long blocks = (n + 255) / 256;
+  const long long vecs = (((uintptr_t)x | (uintptr_t)gate) & 15) == 0 ? n / 8 : 0;
+  long long blocks = ((vecs ? vecs : n) + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  PG_CUDA(launch_pdl(sigmoid_gate_mul_kernel, dim3((int)blocks), dim3(256), (size_t)(0), stream, (bf16*)x, (const bf16*)gate, n));
+  PG_CUDA(launch_pdl(sigmoid_gate_mul_kernel, dim3((int)blocks), dim3(256), (size_t)(0), stream, (bf16*)x, (const bf16*)gate, n, vecs));
   PG_LAUNCH_CHECK();
   return PG_OK;
 }
