@@ -123,6 +123,12 @@ class Qwen35Model:
         self.wp = wp
         source = source or RandomSource(qwen35_shapes(cfg, wp), seed=seed, dtype=dtype, kind=_kind)
         self._load(source)
+        # On one GPU the rows of every gate_up weight alternate (gate_i, up_i), so that SwiGLU runs in the GEMM's epilogue
+        self.gate_up_interleaved = w == 1 and self.device.type == "cuda" and dtype == torch.bfloat16
+        if self.gate_up_interleaved:
+            for L in self.layers:
+                i = L.gate_up.shape[0] // 2
+                L.gate_up = torch.stack((L.gate_up[:i], L.gate_up[i:]), 1).reshape(L.gate_up.shape).contiguous()
         self.cos, self.sin = rope_tables(min(cfg.max_position, 65536), cfg.rotary_dim, cfg.rope_theta, dtype, self.device)
         self.rec: Optional[RecurrentState] = None
 
@@ -230,7 +236,10 @@ class Qwen35Model:
             else:
                 a = self.linear_attention(L.linear, x, meta)
                 x = tp.row_linear_add_norm(a, L.linear.out, residual, L.post_norm, eps, offset=True)
-            act = ops.swiglu(tp.col_linear(x, L.gate_up))
+            if self.gate_up_interleaved and ops.get_mode() == "sm100":
+                act = ops.dense_glu(x, L.gate_up, True)
+            else:
+                act = ops.swiglu(tp.col_linear(x, L.gate_up), self.gate_up_interleaved)
             nxt = self.layers[i + 1].input_norm if i + 1 < n else self.final_norm
             x = tp.row_linear_add_norm(act, L.down, residual, nxt, eps, offset=True)
         tp.sync()
