@@ -39,6 +39,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "decode_rows.h"
 
 namespace {
 
@@ -993,6 +994,34 @@ static int decode_chain_impl(const PgChainPhase* phases, int nphase, int T, void
                  "decode chain: residual, output and norm weight must be 8-byte aligned");
     }
     // a k-range never spans more than two tiles: per_cta <= kblocks because rem_tiles < G
+  }
+  if (tp == nullptr && T <= DR_MAX_ROWS) {
+    // Few rows: streams of weight rows instead of tiles (decode_rows.cu); the phases' results are the same.
+    DecodeRows r;
+    memset(&r, 0, sizeof(r));
+    r.nphase = nphase;
+    r.residual = p.residual, r.ld_res = ld_res;
+    r.scratch = p.ws;
+    r.counters = p.counters, r.status = p.status;
+    r.barriers = nphase > 1 || phases[0].epi == CH_QKV_ROPE || phases[0].epi == CH_RESID_NORM;
+    bool room = true;
+    for (int i = 0; i < nphase; ++i) {
+      const PgChainPhase& s = phases[i];
+      const Phase& P = p.ph[i];
+      DecodeRowsPhase& d = r.ph[i];
+      d.M = s.M, d.K = s.K, d.epi = s.epi;
+      d.x = (const bf16*)s.x, d.ldx = s.ldx, d.w = (const bf16*)s.w, d.ldw = s.ldw, d.out = (bf16*)s.out, d.ld_out = s.ld_out;
+      d.norm_w = (const bf16*)s.norm_w, d.norm_offset = s.norm_offset;
+      d.in_ssp = (const float*)s.in_ssp, d.in_parts = s.in_parts, d.in_ld = s.in_ld, d.in_width = s.in_width, d.in_eps = s.in_eps;
+      d.out_ssp = (float*)s.out_ssp, d.out_ld = s.out_ld;
+      d.q_w = P.q_w, d.k_w = P.k_w, d.cos = P.cos, d.sin = P.sin, d.positions = P.positions, d.slots = P.slots, d.kv = P.kv;
+      d.hq = P.hq, d.hkv = P.hkv, d.rot = P.rot, d.page_size = P.page_size, d.max_pos = P.max_pos, d.num_slots = P.num_slots, d.qk_eps = P.qk_eps;
+      room = room && (s.epi != CH_QKV_ROPE || (i == nphase - 1 && ws_bytes >= (long long)T * s.M * 4));
+    }
+    if (room && decode_rows_plan(r, T)) return decode_rows_run(r, T, stream);
+  }
+  for (int i = 0; i < nphase; ++i) {
+    const PgChainPhase& s = phases[i];
     int rc = pg_make_tmap_bf16_2d(&tm.w[i], s.w, s.M, s.K, s.ldw, BM, BK);
     if (rc) return rc;
     rc = pg_make_tmap_bf16_2d(&tm.x[i], s.x, T, s.K, s.ldx, BN, BK);

@@ -27,6 +27,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "decode_rows.h"
 
 namespace {
 
@@ -1262,12 +1263,36 @@ static int g_tp_last_site = 0;
 // Profiling hook: device buffer of 8 x uint64 per site (nullptr switches it off).
 extern "C" void pg_tp_set_timing(void* buf) { g_tp_timing = (unsigned long long*)buf; }
 
+// One to four token rows: a stream of weight rows (decode_rows.cu) where sizes and alignment allow it; false: not launched.
+// One row, us on the tile kernel -> here: 4096 x 4096 12.2 -> 8.2, 151936 x 4096 201 -> 186, 1024 x 3072 6.9 -> 3.6; four rows:
+// 12.2 -> 10.1, 201 -> 188, 6.9 -> 4.5.  The tile kernel keeps several rows of long k, which every block reads before its first
+// product (four rows of 4096 x 12288: 22.3, here 25.1), and two rows of the largest matrices (151936 x 4096: 201, here 225).
+static bool try_decode_rows(const void* x, const void* w, void* y, int y_is_f32, int T, int M, int K, long long ldx, long long ldw, long long ldy, int epi, const void* in_ssp, int in_parts, int in_ld,
+                            int in_width, float in_eps, void* status, cudaStream_t stream, int* rc) {
+  if (T < 1 || T > DR_MAX_ROWS || x == nullptr || w == nullptr || y == nullptr || status == nullptr) return false;
+  if ((T > 1 && K > 8192) || (T == 2 && (long long)M * K > 100'000'000)) return false;
+  DecodeRows r;
+  memset(&r, 0, sizeof(r));
+  r.nphase = 1;
+  r.status = (uint32_t*)status;
+  DecodeRowsPhase& d = r.ph[0];
+  d.M = M, d.K = K, d.epi = epi;
+  d.x = (const bf16*)x, d.ldx = ldx, d.w = (const bf16*)w, d.ldw = ldw, d.out = (bf16*)y, d.out_f32 = y_is_f32, d.ld_out = ldy;
+  d.in_ssp = (const float*)in_ssp, d.in_parts = in_parts, d.in_ld = in_ld, d.in_width = in_width, d.in_eps = in_eps;
+  if (!decode_rows_plan(r, T)) return false;
+  pg_gemm_prefetch_next(nullptr, 0);  // the hint was for this GEMM
+  *rc = decode_rows_run(r, T, stream);
+  return true;
+}
+
 extern "C" int pg_gemm_bf16_tn(const void* x, const void* w, void* y, int y_is_f32, int T, int M, int K, long long ldx, long long ldw,
                                long long ldy, void* ws, long long ws_bytes, void* counters, long long counter_bytes, void* status,
                                int force_splits, cudaStream_t stream) {
   // tensor-bound problems go to the two-SM kernel; a pinned split count (batch-invariant
   // serving) keeps every problem size on this one kernel
   if (!y_is_f32 && force_splits <= 0 && pg_gemm2sm_eligible(T, M, K)) return pg_gemm2sm_bf16_tn(x, w, y, T, M, K, ldx, ldw, ldy, status, stream);
+  int rc = PG_OK;
+  if (force_splits <= 0 && try_decode_rows(x, w, y, y_is_f32, T, M, K, ldx, ldw, ldy, DR_PLAIN, nullptr, 0, 0, 0, 0.f, status, stream, &rc)) return rc;
   return gemm_impl(x, w, y, y_is_f32, T, M, K, ldx, ldw, ldy, ws, ws_bytes, counters, counter_bytes, status, force_splits, nullptr, nullptr, stream);
 }
 
@@ -1358,6 +1383,8 @@ extern "C" int pg_gemm_bf16_tn_fused(const void* x, const void* w, void* y, int 
     PG_REQUIRE(residual && norm_w && out_ssp && ld_res % 4 == 0 && ldy % 4 == 0 && ((uintptr_t)residual & 7) == 0 && ((uintptr_t)norm_w & 7) == 0 && ((uintptr_t)y & 7) == 0,
                "gemm fused: residual, norm weight and output must be given and 8-byte aligned");
   }
+  int rc = PG_OK;
+  if (!gelu && epi != EPI_RESID_NORMW && try_decode_rows(x, w, y, 0, T, M, K, ldx, ldw, ldy, epi == EPI_SWIGLU ? DR_SWIGLU : DR_PLAIN, in_ssp, in_parts, in_ld, in_width, in_eps, status, stream, &rc)) return rc;
   FuseSpec f;
   memset(&f, 0, sizeof(f));
   f.epi = epi;

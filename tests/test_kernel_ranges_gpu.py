@@ -158,3 +158,57 @@ def test_gated_norm_reads_the_gate_in_place(dim, heads, act):
         got, want = cu().gated_rms_norm(x, gate, w, 1e-6, act), R.gated_rms_norm(x, gate, w, 1e-6, act)
         # f32 sums in another order: one step of bf16, two where two rounded factors meet
         assert ((got.float() - want.float()).abs() <= 2 ** -7 * want.float().abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("t", [1, 2, 3, 4])
+@pytest.mark.parametrize("h,hq,hkv,inter", [(1024, 16, 8, 3072), (2560, 32, 8, 9728), (256, 2, 1, 512), (4096, 32, 8, 12288)])
+def test_chain_of_few_rows(t, h, hq, hkv, inter):
+    """One to four rows through the streamed form of the decode chain, phase by phase against f64 of the same bf16 inputs."""
+    K = cu()
+    torch.manual_seed(t + h)
+    page, eps, d = 16, 1e-6, 128
+    mat = lambda m, k: (torch.randn(m, k, device=DEV) * 0.03).bfloat16()  # noqa: E731
+    o, gu, down, qkv = mat(h, hq * d), mat(2 * inter, h), mat(h, inter), mat((hq + 2 * hkv) * d, h)
+    n1, n2, qn, kn = ((torch.rand(s, device=DEV) + 0.5).bfloat16() for s in (h, h, d, d))
+    a, res = torch.randn(t, hq * d, device=DEV).bfloat16(), torch.randn(t, h, device=DEV).bfloat16()
+    cos, sin = R.rope_tables(512, d, 1e4, torch.bfloat16, DEV)
+    kv = torch.zeros(8, 2, page, hkv, d, device=DEV).bfloat16()
+    pos = torch.tensor([3, 77, 5, 400][:t], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([18, 35, 100, 127][:t], dtype=torch.int32, device=DEV)
+    meta = R.AttnMeta(torch.arange(t + 1, dtype=torch.int32, device=DEV), pos + 1, torch.zeros(t, 8, dtype=torch.int32, device=DEV), slots, pos, page, t, t, 1, 512, True)
+    spec = dict(q_norm=qn, k_norm=kn, cos=cos, sin=sin, meta=meta, kv_layer=kv, hq=hq, hkv=hkv, eps=eps)
+    r1 = res.clone()
+    outs = K.decode_chain(a, [(o, K.CH_RESID_NORM, n1, False), (gu, K.CH_SWIGLU, None, False), (down, K.CH_RESID_NORM, n2, True), (qkv, K.CH_QKV_ROPE, spec, False)], residual=r1, eps=eps)
+
+    def near(got, want, roundings):  # every rounding to bf16 on the way is at most 2^-9 of a value; products add up as their squares
+        err = (got.double() - want.double()).norm() / want.double().norm()
+        assert err < roundings * 2 ** -9, float(err)
+
+    h1 = res.double() + a.double() @ o.double().t()
+    near(outs[0].xw, h1 * n1.double(), 2)
+    inv = lambda x: torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps)  # noqa: E731
+    x1 = outs[0].xw.double() * torch.rsqrt(outs[0].ssp[:, : outs[0].parts].double().sum(-1, keepdim=True) / h + eps)
+    near(x1, h1 * inv(h1) * n1.double(), 2)
+    y = x1 @ gu.double().t()
+    near(outs[1], torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2], 3)
+    h2 = h1 + outs[1].double() @ down.double().t()
+    near(r1, h2, 2)
+    near(outs[2].xw, h2 * (n2.double() + 1), 3)
+    x2 = outs[2].xw.double() * torch.rsqrt(outs[2].ssp[:, : outs[2].parts].double().sum(-1, keepdim=True) / h + eps)
+    z = (x2 @ qkv.double().t()).bfloat16()
+    kv2 = torch.zeros_like(kv)
+    q = R.qk_norm_rope_append(z, qn, kn, cos, sin, meta, kv2, hq, hkv, d, eps)
+    near(outs[3], q, 4)
+    near(kv, kv2, 4)
+    assert not K.ctx(DEV).chain_counters.any() and K.read_status(DEV) == 0
+
+
+@pytest.mark.parametrize("t,m,k", [(1, 2, 256), (2, 130, 512), (3, 4098, 768), (4, 1000, 12288), (1, 40000, 256), (4, 64, 5120)])
+def test_linear_of_few_rows(t, m, k):
+    torch.manual_seed(m)
+    x, w = torch.randn(t, k + 8, device=DEV).bfloat16()[:, :k], torch.randn(m, k, device=DEV).bfloat16()
+    want = x.double() @ w.double().t()
+    lim = k * 2 ** -24 * (x.double().abs() @ w.double().abs().t())  # f32 sums of k products
+    for dtype in (torch.bfloat16, torch.float32):
+        got = cu().linear(x, w, dtype).double()
+        assert ((got - want).abs() <= lim + (2 ** -8 * want.abs() if dtype == torch.bfloat16 else 0)).all()
