@@ -62,12 +62,13 @@ int pg_ipc_import(const void* handle64, void** out);
 int pg_ipc_close(void* p);
 // Two-SM (cta_group::2) bf16 GEMM for tensor-bound problems (gemm2sm_sm100.cu); pg_gemm_bf16_tn
 // routes eligible problems to it (PEGAINFER_GEMM_2SM=0 turns that off).
+int pg_gemm2sm_takes(int T, int M, int K);
 int pg_gemm2sm_eligible(int T, int M, int K);
-int pg_gemm2sm_bf16_tn(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, void* status,
+int pg_gemm2sm_bf16_tn(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, void* ws, long long ws_bytes, void* counters, long long counter_bytes, void* status,
                        cudaStream_t stream);
-int pg_gemm2sm_bf16_tn_swiglu(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, int gelu, void* status,
+int pg_gemm2sm_bf16_tn_swiglu(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, int gelu, void* ws, long long ws_bytes, void* counters, long long counter_bytes, void* status,
                        cudaStream_t stream);
-int pg_gemm2sm_bf16_tn_xielu(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, const void* act, void* status,
+int pg_gemm2sm_bf16_tn_xielu(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, const void* act, void* ws, long long ws_bytes, void* counters, long long counter_bytes, void* status,
                              cudaStream_t stream);
 int pg_make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, long long rows, long long cols, long long ld, int box_rows, int box_cols);
 

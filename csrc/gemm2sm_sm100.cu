@@ -13,12 +13,12 @@
 //   CTA rank 0 (leader)                          CTA rank 1
 //   warp 0  TMA producer (own halves)            warp 0  TMA producer (own halves)
 //   warp 1  TMEM alloc, issues every MMA          warp 1  TMEM alloc / dealloc only
-//   warps 2..5 epilogue of rows 0..127            warps 2..5 epilogue of rows 128..255
+//   warps 2..9 epilogue of rows 0..127            warps 2..9 epilogue of rows 128..255
 //
 // Barriers: `full[s]` lives in the leader and counts the bytes of BOTH CTAs' loads (each
 // CTA's TMA names the leader's barrier); `empty[s]` and `tfull[a]` exist in both CTAs and
 // are signalled by tcgen05.commit with a two-CTA multicast mask; `tempty[a]` lives in the
-// leader and counts the eight epilogue warps of the pair.  Every wait is bounded.
+// leader and counts the epilogue warps of the pair.  Every wait is bounded.
 //
 // Takes the place of the reference's cuBLAS/cuBLASLt layer for prefill-sized problems
 // (pegainfer-kernels/csrc/shared/linear.cu:294-596).
@@ -36,7 +36,9 @@ constexpr int BM = 128;  // weight rows per CTA (256 per pair)
 constexpr int BK = 64;
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int MAX_STAGES = 12;
-constexpr int NUM_THREADS = 192;
+constexpr int MAX_SPLITS = 4;
+constexpr int EPI_WARPS = 8;
+constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;
 constexpr int RASTER_GROUP = 8;  // weight-row pairs per raster group
 
 struct Gemm2Params {
@@ -50,7 +52,29 @@ struct Gemm2Params {
   uint32_t* status;
   int epi;  // 0: y = x W^T; 1: the weight rows alternate (gate_i, up_i) and y [T, M / 2] = bf16(silu(gate)) * up
   const float* xielu;  // epi 0: the two constants of xIELU on every output (nullptr = none)
+  int whole;           // tiles that one pair computes over all of K; the `rem` tiles behind them are cut in `splits` ranges of k (1: none are)
+  int rem, splits;
+  float4* part;        // partial sums [rem][splits][CTA of the pair][bn / 4][128 rows][4]
+  uint32_t* counters;  // [rem][CTA of the pair][epilogue warp], zero between launches
 };
+
+struct Work {
+  int tile, part, kb0, kb1;  // part < 0: a whole tile
+};
+// The i-th piece of work of a pair: whole tiles in rounds, then at most one range of a cut tile.  Neighbouring pairs take
+// neighbouring tiles at the same range of k, so that they share operands through L2.
+__device__ __forceinline__ bool work_at(const Gemm2Params& p, int pair, int pairs, int i, Work& w) {
+  const int item = pair + i * pairs;
+  if (item < p.whole) {
+    w = {item, -1, 0, p.kblocks};
+    return true;
+  }
+  const int q = item - p.whole;
+  if (q >= p.rem * p.splits) return false;
+  const int part = q / p.rem;
+  w = {p.whole + q % p.rem, part, part * p.kblocks / p.splits, (part + 1) * p.kblocks / p.splits};
+  return true;
+}
 
 // Work item -> (weight-row pair, token tile).  Items walk RASTER_GROUP weight-row pairs across
 // all token tiles before moving on, so the CTA pairs that run at the same time cover a
@@ -127,7 +151,7 @@ gemm2sm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 8);
+      mbar_init(&tempty[a], 2 * EPI_WARPS);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -146,8 +170,6 @@ gemm2sm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
   if (threadIdx.x == 0) pdl_launch_dependents();
   pdl_wait();
 
-  const int total = p.m_pairs * p.n_tiles;
-
   if (warp == 0) {
     if (lane == 0) {
       // both operands are re-read (weights by every token tile, tokens by every weight-row pair)
@@ -163,12 +185,13 @@ gemm2sm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
         last_phase[s] = 0;
       }
       bool ok = true;
-      for (int item = pair; item < total && ok; item += pairs) {
+      Work wk;
+      for (int i = 0; ok && work_at(p, pair, pairs, i, wk); ++i) {
         int m_pair, n_tile;
-        tile_of(p, item, m_pair, n_tile);
+        tile_of(p, wk.tile, m_pair, n_tile);
         const int w_row = m_pair * (2 * BM) + (int)rank * BM;
         const int x_row = n_tile * p.bn + (int)rank * bnh;
-        for (int kb = 0; kb < p.kblocks; ++kb) {
+        for (int kb = wk.kb0; kb < wk.kb1; ++kb) {
           if (!mbar_wait_cluster(&empty[stage], phase ^ 1u, abort_flag)) {
             ok = false;
             break;
@@ -204,11 +227,12 @@ gemm2sm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int item = pair; item < total && ok; item += pairs) {
+      Work wk;
+      for (int i = 0; ok && work_at(p, pair, pairs, i, wk); ++i) {
         if (!mbar_wait_cluster(&tempty[acc], acc_phase ^ 1u, abort_flag)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * p.bn);
-        for (int kb = 0; kb < p.kblocks; ++kb) {
+        for (int kb = wk.kb0; kb < wk.kb1; ++kb) {
           if (!mbar_wait_cluster(&full[stage], phase, abort_flag)) {
             ok = false;
             break;
@@ -218,7 +242,7 @@ gemm2sm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
           const uint32_t b_addr = a_addr + A_BYTES;
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
-            umma_bf16_ss_pair(d_tmem, umma_desc_k_sw128(a_addr + k * 32), umma_desc_k_sw128(b_addr + k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_bf16_ss_pair(d_tmem, umma_desc_k_sw128(a_addr + k * 32), umma_desc_k_sw128(b_addr + k * 32), idesc, (kb > wk.kb0 || k > 0) ? 1u : 0u);
           }
           umma_commit_pair(&empty[stage], (uint16_t)3);
           if (++stage == p.stages) {
@@ -233,25 +257,84 @@ gemm2sm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
       }
     }
   } else {
-    // epilogue: warp w may touch TMEM lanes 32*(w%4) .. 32*(w%4)+31 of its own CTA
-    const int wq = warp & 3;
+    // epilogue: warp w may touch TMEM lanes 32*(w%4) .. 32*(w%4)+31 of its own CTA; two warps share the lanes, alternating in
+    // steps of 32 columns
+    const int wq = warp & 3, c0 = ((warp - 2) >> 2) * 32;
     const int r = wq * 32 + lane;
     int acc = 0;
     uint32_t acc_phase = 0;
-    for (int item = pair; item < total; item += pairs) {
+    Work wk;
+    for (int i = 0; work_at(p, pair, pairs, i, wk); ++i) {
       int m_pair, n_tile;
-      tile_of(p, item, m_pair, n_tile);
+      tile_of(p, wk.tile, m_pair, n_tile);
       if (!mbar_wait_cluster(&tfull[acc], acc_phase, abort_flag)) break;
       tc_fence_after();
       const int m = m_pair * (2 * BM) + (int)rank * BM + r;
       const int n0 = n_tile * p.bn;
       const uint32_t t_row = tmem_base + ((uint32_t)(wq * 32) << 16) + (uint32_t)(acc * p.bn);
       bf16* yc = p.y + m;
-      for (int c = 0; c < p.bn; c += 32) {
+      // A cut tile: every range leaves its sums in scratch, and for each 32 rows the last one to arrive adds them up, in the
+      // order of the ranges whoever is last, and stores the output.  Nobody waits.
+      const long long part_stride = 2ll * (p.bn / 4) * BM;
+      float4* parts = nullptr;
+      bool last = true;
+      if (wk.part >= 0) {
+        const int cut = wk.tile - p.whole;
+        parts = p.part + ((long long)cut * p.splits * 2 + rank) * (p.bn / 4) * BM + r;
+        float4* mine = parts + wk.part * part_stride;
+        for (int c = c0; c < p.bn; c += 64) {
+          uint32_t v[2][16];
+          tmem_ld16(t_row + c, v[0]);
+          tmem_ld16(t_row + c + 16, v[1]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint32_t* u = v[q / 4] + q % 4 * 4;
+            __stcg(mine + (c / 4 + q) * BM, make_float4(__uint_as_float(u[0]), __uint_as_float(u[1]), __uint_as_float(u[2]), __uint_as_float(u[3])));
+          }
+        }
+        __threadfence();
+        __syncwarp();
+        uint32_t* counter = p.counters + (cut * 2 + (int)rank) * EPI_WARPS + warp - 2;
+        uint32_t before = 0;
+        if (lane == 0) before = atomicAdd(counter, 1u);
+        last = __shfl_sync(0xFFFFFFFFu, before, 0) == (uint32_t)(p.splits - 1);
+        if (last) {
+          __threadfence();
+          if (lane == 0) *counter = 0u;
+        }
+      }
+      for (int c = c0; last && c < p.bn; c += 64) {
         uint32_t v[2][16];
+        float4 o[MAX_SPLITS - 1][8];  // the other ranges
+        if (wk.part >= 0) {
+#pragma unroll
+          for (int j = 0; j < MAX_SPLITS - 1; ++j)
+            if (j < p.splits - 1) {
+#pragma unroll
+              for (int q = 0; q < 8; ++q) o[j][q] = __ldcg(parts + (j < wk.part ? j : j + 1) * part_stride + (c / 4 + q) * BM);
+            }
+        }
         tmem_ld16(t_row + c, v[0]);
         tmem_ld16(t_row + c + 16, v[1]);
         tmem_ld_wait();
+        if (wk.part >= 0) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const float4 own = make_float4(__uint_as_float(v[q / 4][q % 4 * 4]), __uint_as_float(v[q / 4][q % 4 * 4 + 1]), __uint_as_float(v[q / 4][q % 4 * 4 + 2]), __uint_as_float(v[q / 4][q % 4 * 4 + 3]));
+            float4 sum = wk.part == 0 ? own : o[0][q];
+#pragma unroll
+            for (int s = 1; s < MAX_SPLITS; ++s)
+              if (s < p.splits) {
+                const float4 x = s == wk.part ? own : s < wk.part ? o[min(s, MAX_SPLITS - 2)][q] : o[s - 1][q];
+                sum = make_float4(sum.x + x.x, sum.y + x.y, sum.z + x.z, sum.w + x.w);
+              }
+            v[q / 4][q % 4 * 4] = __float_as_uint(sum.x);
+            v[q / 4][q % 4 * 4 + 1] = __float_as_uint(sum.y);
+            v[q / 4][q % 4 * 4 + 2] = __float_as_uint(sum.z);
+            v[q / 4][q % 4 * 4 + 3] = __float_as_uint(sum.w);
+          }
+        }
         if (p.epi != 0) {
           // SwiGLU (1) or its form with tanh-GELU (3): lanes 2 i and 2 i + 1 hold gate and up of output column m / 2 (both rounded to bf16 first, as the
           // separate kernel sees them); the shuffles run on all lanes, the even ones store
@@ -319,48 +402,57 @@ int g_enabled = -1;
 
 }  // namespace
 
-// 1 if the two-SM kernel would take this problem on the current device.
-extern "C" int pg_gemm2sm_eligible(int T, int M, int K) {
+static bool gemm2sm_enabled() {
   if (g_enabled < 0) {
     const char* e = getenv("PEGAINFER_GEMM_2SM");
     g_enabled = (e && e[0] == '0') ? 0 : 1;
   }
-  if (!g_enabled) return 0;
-  // Tensor-bound problems with at least about one full round of CTA pairs: below that the
-  // one-CTA kernel's narrower token tiles and k-splits fill the machine better.  Very deep
-  // problems (K > 8192) stay on the one-CTA kernel as well: there the operand slabs that the
-  // concurrently running 256 x 256 tiles share (17 slabs of 256 x K) approach the L2 capacity
-  // and this kernel measured slower (493 vs 372 us at T = M = 4096, K = 12288).
-  static int max_k = 0;
-  if (max_k == 0) {
-    const char* e = getenv("PEGAINFER_GEMM_2SM_MAXK");
-    max_k = e ? atoi(e) : 8192;
-    if (max_k <= 0) max_k = 8192;
-  }
-  if (T < 256 || M < 1024 || K < 256 || K > max_k || K % 8 != 0) return 0;
+  return g_enabled == 1;
+}
+
+// 1 if the two-SM kernel takes this problem in a GEMM with bf16 results: above the 64 rows of the decode plans it measured faster
+// than the one-CTA kernel at every size.  Us there -> here: T = 65, M x K = 1024 x 1024 20 -> 11, 4096 x 12288 58 -> 34; T = 256,
+// 64 x 512 20 -> 9, 5120 x 17408 109 -> 57; T = 1100, 4096 x 12288 144 -> 101; T = 4096, 4096 x 12288 377 -> 280.  At 64 rows and
+// below the one-CTA kernel's narrow tiles win (4096 x 4096: 14, here 19).
+extern "C" int pg_gemm2sm_takes(int T, int M, int K) { return gemm2sm_enabled() && T > 64 && M >= 64 && K >= 256 && K % 8 == 0 ? 1 : 0; }
+
+// 1 for the problems whose f32 results callers leave to a bf16 GEMM on this kernel (at least about a round of CTA pairs, k up to
+// 8192): a narrower set than pg_gemm2sm_takes, so that no other results lose their 32 bits.
+extern "C" int pg_gemm2sm_eligible(int T, int M, int K) {
+  if (!gemm2sm_enabled() || T < 256 || M < 1024 || K < 256 || K > 8192 || K % 8 != 0) return 0;
   return (long long)ceil_div(M, 2 * BM) * ceil_div(T, 256) >= 64 ? 1 : 0;
 }
 
-static int gemm2sm_impl(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, void* status, int epi, cudaStream_t stream, const void* xielu = nullptr);
+struct Scratch2 {
+  void* ws;
+  long long ws_bytes;
+  void* counters;
+  long long counter_bytes;
+};
+static int gemm2sm_impl(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, const Scratch2& sc, void* status, int epi, cudaStream_t stream,
+                        const void* xielu = nullptr);
 
-extern "C" int pg_gemm2sm_bf16_tn(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, void* status,
-                                  cudaStream_t stream) {
-  return gemm2sm_impl(x, w, y, T, M, K, ldx, ldw, ldy, status, 0, stream);
+// ws, counters: scratch as for pg_gemm_bf16_tn (null: no tile is cut)
+extern "C" int pg_gemm2sm_bf16_tn(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, void* ws, long long ws_bytes, void* counters,
+                                  long long counter_bytes, void* status, cudaStream_t stream) {
+  return gemm2sm_impl(x, w, y, T, M, K, ldx, ldw, ldy, {ws, ws_bytes, counters, counter_bytes}, status, 0, stream);
 }
 
 // The same product with SwiGLU (gelu: tanh-GELU on the gate) in the epilogue: w [M, K] with rows alternating (gate_i, up_i), y [T, M / 2].
-extern "C" int pg_gemm2sm_bf16_tn_swiglu(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, int gelu, void* status,
-                                         cudaStream_t stream) {
+extern "C" int pg_gemm2sm_bf16_tn_swiglu(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, int gelu, void* ws, long long ws_bytes, void* counters,
+                                         long long counter_bytes, void* status, cudaStream_t stream) {
   PG_REQUIRE(M % 2 == 0, "gemm2sm swiglu: M %d must be even (interleaved gate / up rows)", M);
-  return gemm2sm_impl(x, w, y, T, M, K, ldx, ldw, ldy, status, gelu ? 3 : 1, stream);
+  return gemm2sm_impl(x, w, y, T, M, K, ldx, ldw, ldy, {ws, ws_bytes, counters, counter_bytes}, status, gelu ? 3 : 1, stream);
 }
 
 // The same product with xIELU in the epilogue; act: f32 softplus(p), 1/2 + softplus(q).
-extern "C" int pg_gemm2sm_bf16_tn_xielu(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, const void* act, void* status, cudaStream_t stream) {
-  return gemm2sm_impl(x, w, y, T, M, K, ldx, ldw, ldy, status, 0, stream, act);
+extern "C" int pg_gemm2sm_bf16_tn_xielu(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, const void* act, void* ws, long long ws_bytes,
+                                        void* counters, long long counter_bytes, void* status, cudaStream_t stream) {
+  return gemm2sm_impl(x, w, y, T, M, K, ldx, ldw, ldy, {ws, ws_bytes, counters, counter_bytes}, status, 0, stream, act);
 }
 
-static int gemm2sm_impl(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, void* status, int epi, cudaStream_t stream, const void* xielu) {
+static int gemm2sm_impl(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, const Scratch2& sc, void* status, int epi, cudaStream_t stream,
+                        const void* xielu) {
   PG_REQUIRE(T > 0 && M > 0 && K > 0 && K % 8 == 0, "gemm2sm: bad problem %dx%dx%d", T, M, K);
   PG_REQUIRE(status != nullptr, "gemm2sm: a device status word is required");
   int dev = 0;
@@ -401,22 +493,35 @@ static int gemm2sm_impl(const void* x, const void* w, void* y, int T, int M, int
   p.T = T;
   p.K = K;
   p.m_pairs = ceil_div(M, 2 * BM);
-  // token-tile width: fewest rounds of CTA pairs; a round costs about (width + 256): the MMA
-  // time follows the width, the 128 weight rows per CTA and the per-k-block hand-offs do not
+  p.kblocks = ceil_div(K, BK);
+  // Token-tile width, and ranges of k for the tiles of the last round where it leaves most pairs idle: least time on the busiest
+  // pair.  A k-block costs about (width + 256): the MMA time follows the width, the 128 weight rows per CTA and the hand-offs do
+  // not.  Cutting tiles costs as much as CUT_KBLOCKS k-blocks (10 us: partial sums out and in again).
   {
+    constexpr int CUT_KBLOCKS = 25;
     long long best_cost = -1;
     for (int bn = 256; bn >= 128; bn -= 32) {
-      const long long tiles = (long long)p.m_pairs * ceil_div(T, bn);
-      const long long rounds = (tiles + di.max_pairs - 1) / di.max_pairs;
-      const long long cost = rounds * (bn + 256);
-      if (best_cost < 0 || cost < best_cost) {
-        best_cost = cost;
-        p.bn = bn;
+      const long long tiles = (long long)p.m_pairs * ceil_div(T, bn), rounds = tiles / di.max_pairs, rem = tiles % di.max_pairs;
+      for (int s = 1; s <= MAX_SPLITS; ++s) {
+        if (s > 1) {
+          if (rem == 0 || rem * s > di.max_pairs || p.kblocks < 8 * s) break;
+          if (sc.ws == nullptr || sc.counters == nullptr || (((uintptr_t)sc.ws) & 15) != 0 || rem * s * 2 * bn * BM * 4 > sc.ws_bytes || rem * 2 * EPI_WARPS * 4 > sc.counter_bytes) break;
+        }
+        const long long cost = (rounds * p.kblocks + (rem == 0 ? 0 : s == 1 ? p.kblocks : (p.kblocks + s - 1) / s + CUT_KBLOCKS)) * (bn + 256);
+        if (best_cost < 0 || cost < best_cost) {
+          best_cost = cost;
+          p.bn = bn;
+          p.splits = s;
+        }
       }
     }
   }
   p.n_tiles = ceil_div(T, p.bn);
-  p.kblocks = ceil_div(K, BK);
+  const int total = p.m_pairs * p.n_tiles;
+  p.rem = p.splits > 1 ? total % di.max_pairs : 0;
+  p.whole = total - p.rem;
+  p.part = (float4*)sc.ws;
+  p.counters = (uint32_t*)sc.counters;
   const int stage_bytes = A_BYTES + (p.bn / 2) * 128;
   p.stages = (di.max_smem - 1024 - tail) / stage_bytes;
   if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
@@ -431,8 +536,8 @@ static int gemm2sm_impl(const void* x, const void* w, void* y, int T, int M, int
   if (rc) return rc;
   rc = pg_make_tmap_bf16_2d(&tm_x, x, T, K, ldx, p.bn / 2, BK);
   if (rc) return rc;
-  const int total = p.m_pairs * p.n_tiles;
-  const int npairs = total < di.max_pairs ? total : di.max_pairs;
+  const int items = p.whole + p.rem * p.splits;
+  const int npairs = items < di.max_pairs ? items : di.max_pairs;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)(2 * npairs));

@@ -1290,7 +1290,7 @@ extern "C" int pg_gemm_bf16_tn(const void* x, const void* w, void* y, int y_is_f
                                int force_splits, cudaStream_t stream) {
   // tensor-bound problems go to the two-SM kernel; a pinned split count (batch-invariant
   // serving) keeps every problem size on this one kernel
-  if (!y_is_f32 && force_splits <= 0 && pg_gemm2sm_eligible(T, M, K)) return pg_gemm2sm_bf16_tn(x, w, y, T, M, K, ldx, ldw, ldy, status, stream);
+  if (!y_is_f32 && force_splits <= 0 && pg_gemm2sm_takes(T, M, K)) return pg_gemm2sm_bf16_tn(x, w, y, T, M, K, ldx, ldw, ldy, ws, ws_bytes, counters, counter_bytes, status, stream);
   int rc = PG_OK;
   if (force_splits <= 0 && try_decode_rows(x, w, y, y_is_f32, T, M, K, ldx, ldw, ldy, DR_PLAIN, nullptr, 0, 0, 0, 0.f, status, stream, &rc)) return rc;
   return gemm_impl(x, w, y, y_is_f32, T, M, K, ldx, ldw, ldy, ws, ws_bytes, counters, counter_bytes, status, force_splits, nullptr, nullptr, stream);
@@ -1300,7 +1300,7 @@ extern "C" int pg_gemm_bf16_tn(const void* x, const void* w, void* y, int y_is_f
 extern "C" int pg_gemm_bf16_tn_xielu(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, const void* act, void* ws, long long ws_bytes, void* counters,
                                      long long counter_bytes, void* status, int force_splits, cudaStream_t stream) {
   PG_REQUIRE(act != nullptr, "gemm xielu: the activation's constants are required");
-  if (force_splits <= 0 && pg_gemm2sm_eligible(T, M, K)) return pg_gemm2sm_bf16_tn_xielu(x, w, y, T, M, K, ldx, ldw, ldy, act, status, stream);
+  if (force_splits <= 0 && pg_gemm2sm_takes(T, M, K)) return pg_gemm2sm_bf16_tn_xielu(x, w, y, T, M, K, ldx, ldw, ldy, act, ws, ws_bytes, counters, counter_bytes, status, stream);
   FuseSpec f;
   memset(&f, 0, sizeof(f));
   f.epi = EPI_PLAIN;

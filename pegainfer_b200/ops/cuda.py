@@ -432,7 +432,8 @@ def linear_2sm(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     m = w.shape[0]
     out = torch.empty((t, m), dtype=torch.bfloat16, device=x.device)
     c = ctx(x.device)
-    rc = lib().pg_gemm2sm_bf16_tn(_ptr(x2), _ptr(w), _ptr(out), _ci(t), _ci(m), _ci(k), _ll(x2.stride(0)), _ll(w.stride(0)), _ll(out.stride(0)), _ptr(c.status), _stream())
+    rc = lib().pg_gemm2sm_bf16_tn(_ptr(x2), _ptr(w), _ptr(out), _ci(t), _ci(m), _ci(k), _ll(x2.stride(0)), _ll(w.stride(0)), _ll(out.stride(0)),
+                                  _ptr(c.gemm_ws), _ll(c.gemm_ws.numel()), _ptr(c.gemm_counters), _ll(c.gemm_counters.numel() * 4), _ptr(c.status), _stream())
     _check(rc, c)
     return out.view(*x.shape[:-1], m)
 
@@ -444,11 +445,12 @@ def linear_swiglu_2sm(x: torch.Tensor, w: torch.Tensor, gelu: bool = False) -> O
     x2 = _rows2d(x)
     t, k = x2.shape
     m = w.shape[0]
-    if not lib().pg_gemm2sm_eligible(_ci(t), _ci(m), _ci(k)) or _BATCH_INVARIANT or w.stride(-1) != 1:
+    if not lib().pg_gemm2sm_takes(_ci(t), _ci(m), _ci(k)) or _BATCH_INVARIANT or w.stride(-1) != 1:
         return None
     out = torch.empty((t, m // 2), dtype=torch.bfloat16, device=x.device)
     c = ctx(x.device)
-    rc = lib().pg_gemm2sm_bf16_tn_swiglu(_ptr(x2), _ptr(w), _ptr(out), _ci(t), _ci(m), _ci(k), _ll(x2.stride(0)), _ll(w.stride(0)), _ll(out.stride(0)), _ci(int(gelu)), _ptr(c.status), _stream())
+    rc = lib().pg_gemm2sm_bf16_tn_swiglu(_ptr(x2), _ptr(w), _ptr(out), _ci(t), _ci(m), _ci(k), _ll(x2.stride(0)), _ll(w.stride(0)), _ll(out.stride(0)), _ci(int(gelu)),
+                                         _ptr(c.gemm_ws), _ll(c.gemm_ws.numel()), _ptr(c.gemm_counters), _ll(c.gemm_counters.numel() * 4), _ptr(c.status), _stream())
     _check(rc, c)
     return out.view(*x.shape[:-1], m // 2)
 

@@ -212,3 +212,18 @@ def test_linear_of_few_rows(t, m, k):
     for dtype in (torch.bfloat16, torch.float32):
         got = cu().linear(x, w, dtype).double()
         assert ((got - want).abs() <= lim + (2 ** -8 * want.abs() if dtype == torch.bfloat16 else 0)).all()
+
+
+@pytest.mark.parametrize("t,m,k", [(257, 1024, 2048), (1337, 4096, 1024), (700, 5008, 1096), (4100, 4112, 512), (300, 1280, 8704), (1200, 1504, 776)])
+def test_two_sm_gemm_cuts_the_last_round(t, m, k):
+    """Tiles of the last round cut in ranges of k: a few tiles only, tiles behind whole rounds, ragged edges, uneven ranges."""
+    K = cu()
+    torch.manual_seed(m)
+    x, w = torch.randn(t, k + 8, device=DEV).bfloat16()[:, :k], torch.randn(m, k, device=DEV).bfloat16()
+    want = x.double() @ w.double().t()
+    lim = 2 ** -8 * want.abs() + k * 2 ** -24 * (x.double().abs() @ w.double().abs().t())  # f32 sums of k products, rounded to bf16
+    y = K.linear_2sm(x, w)
+    assert ((y.double() - want).abs() <= lim).all()
+    assert torch.equal(y, K.linear_2sm(x, w)) and not K.ctx(DEV).gemm_counters.any() and K.read_status(DEV) == 0
+    glu = K.linear_swiglu_2sm(x, w)
+    assert glu is None or torch.equal(glu, K.swiglu(y, True))
