@@ -455,6 +455,7 @@ static int gemm2sm_impl(const void* x, const void* w, void* y, int T, int M, int
                         const void* xielu) {
   PG_REQUIRE(T > 0 && M > 0 && K > 0 && K % 8 == 0, "gemm2sm: bad problem %dx%dx%d", T, M, K);
   PG_REQUIRE(status != nullptr, "gemm2sm: a device status word is required");
+  pg_gemm_prefetch_next(nullptr, 0);  // a hint was for this GEMM, which has no use for it: it must not outlive the weights it names
   int dev = 0;
   PG_CUDA(cudaGetDevice(&dev));
   Dev2& di = g_dev2[dev & 63];
