@@ -227,9 +227,10 @@ int pg_token_mix(const void* h, long long ldh, const void* mu, void* carried, vo
 int pg_attnres_mix(const void* cur, long long ld_cur, const void* snaps, long long ld_tok, const void* score_w, void* out, long long ld_out,
                    int tokens, int nb, int hidden, float eps, cudaStream_t stream);
 // Chunk-wise (64-token) tensor-core form of the same rule for sequences of >= min_len tokens (gdn_chunk.cu).
+long long pg_gdn_chunk_bytes(int hv, int dv);
 int pg_gdn_chunked(const void* q, const void* k, long long ld_qk, const void* v, long long ld_v, const void* g, const void* beta, void* state,
                    void* out, const void* q_indptr, const void* slots, int num_seqs, int hk, int hv, int dk, int dv, int min_len,
-                   cudaStream_t stream);
+                   int chunks, int long_seqs, int longest, void* ws, long long ws_bytes, cudaStream_t stream);
 
 // ---- attention (attention.cu) ------------------------------------------------------
 int pg_decode_splits(int num_seqs, int hkv, int max_kv_len, int sms);

@@ -813,6 +813,7 @@ def gdn_gates(a, b, a_log, dt_bias):
 
 
 _GDN_CHUNKED = os.environ.get("PEGAINFER_GDN_CHUNKED", "1") != "0"
+_GDN_WS_BYTES = 256 << 20  # scratch of a step's chunks at most; longer steps go through it in segments
 _GDN_CHUNK_MIN = 32  # sequences of at least this many tokens in a step take the chunk-wise kernel
 
 
@@ -828,13 +829,21 @@ def gdn_recurrent(q, k, v, g, beta, state, meta: AttnMeta, chunked: Optional[boo
     chunked = (_GDN_CHUNKED if chunked is None else chunked) and int(meta.max_q_len) >= _GDN_CHUNK_MIN and dk == 128 and dv % 64 == 0 and q.stride(0) % 8 == 0 and v.stride(0) % 8 == 0
     args = (_ptr(q), _ptr(k), _ll(q.stride(0)), _ptr(v), _ll(v.stride(0)), _ptr(g), _ptr(beta), _ptr(state), _ptr(out),
             _ptr(meta.q_indptr), _ptr(meta.state_slots), _ci(meta.num_seqs), _ci(hk), _ci(hv), _ci(dk), _ci(dv))
-    if chunked:
-        rc = lib().pg_gdn_chunked(*args, _ci(_GDN_CHUNK_MIN), _stream())
-        _check(rc, c)
     short_rows = True  # is there a sequence below the chunk threshold (decode rows in a unified step)?
-    if chunked and meta.h_q_indptr is not None:
-        qi = meta.h_q_indptr
-        short_rows = any(qi[i + 1] - qi[i] < _GDN_CHUNK_MIN for i in range(meta.num_seqs))
+    if chunked:
+        # chunks of 64 tokens, sequences that have some and the longest of them: counted where the lengths are known here, else bounded
+        if meta.h_q_indptr is not None:
+            lens = [meta.h_q_indptr[i + 1] - meta.h_q_indptr[i] for i in range(meta.num_seqs)]
+            short_rows = any(n < _GDN_CHUNK_MIN for n in lens)
+            counts = [-(-n // 64) for n in lens if n >= _GDN_CHUNK_MIN]
+            chunks, rows, longest = sum(counts), len(counts), max(counts, default=0)
+        else:
+            rows = min(meta.num_seqs, t // _GDN_CHUNK_MIN)
+            chunks, longest = t // 64 + rows, -(-t // 64)
+        one = int(lib().pg_gdn_chunk_bytes(_ci(hv), _ci(dv)))
+        ws = torch.empty(one * max(1, min(chunks, _GDN_WS_BYTES // one)) if longest > 2 else 0, dtype=torch.uint8, device=q.device)
+        rc = lib().pg_gdn_chunked(*args, _ci(_GDN_CHUNK_MIN), _ci(chunks), _ci(rows), _ci(longest), _ptr(ws), _ll(ws.numel()), _stream())
+        _check(rc, c, 2)
     if not chunked or short_rows:
         rc = lib().pg_gdn_recurrent(*args, _ci(int(meta.max_q_len)), _ci(_GDN_CHUNK_MIN if chunked else 0), _stream())
         _check(rc, c)

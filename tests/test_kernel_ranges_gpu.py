@@ -214,6 +214,41 @@ def test_linear_of_few_rows(t, m, k):
         assert ((got - want).abs() <= lim + (2 ** -8 * want.abs() if dtype == torch.bfloat16 else 0)).all()
 
 
+@pytest.mark.parametrize("dv", [64, 128])
+@pytest.mark.parametrize("lens,room", [([32, 63, 64, 65, 1, 129, 0, 31], None), ([700, 33, 450], 7), ([140] * 9 + [3] + [200] * 4, 5), ([260], 1)])
+def test_gated_delta_chunks_in_segments(lens, room, dv, monkeypatch):
+    """All chunks at once, segments of the sequences, groups of sequences, and (short ones) one kernel give the same bytes, and the
+    token-by-token rule's values."""
+    torch.manual_seed(sum(lens) + dv)
+    hk, hv, dk = 2, 4, 128
+    meta = _state_meta(lens, list(range(1, len(lens) + 1)))
+    t = meta.num_tokens
+    x = torch.randn(t, 2 * hk * dk + hv * dv, device=DEV).bfloat16()
+    q, k, v = (y.view(t, -1, d) for y, d in zip(x.split([hk * dk, hk * dk, hv * dv], 1), (dk, dk, dv)))
+    g, beta = -torch.rand(t, hv, device=DEV), torch.rand(t, hv, device=DEV)
+    s0 = torch.randn(len(lens) + 2, hv, dk, dv, device=DEV) * 0.1
+    want_s, runs = s0.clone(), []
+    want = R.gdn_recurrent(q, k, v, g, beta, want_s, meta)
+    for limit, known in ((256 << 20, True), (256 << 20, False)) + (((room * hv * (16384 * 3 + 8192 * 2 + 256 + 128 * dv), True),) if room else ()):
+        monkeypatch.setattr(cu(), "_GDN_WS_BYTES", limit)
+        meta.h_q_indptr = meta.q_indptr.tolist() if known else None
+        s = s0.clone()
+        runs.append((cu().gdn_recurrent(q, k, v, g, beta, s, meta, chunked=True), s))
+    for o, s in runs[1:]:
+        assert torch.equal(o, runs[0][0]) and torch.equal(s, runs[0][1])
+    short = _state_meta([128], [1])  # the first 128 tokens of the first sequence, in one kernel and beside a longer sequence
+    if lens[0] > 128:
+        both = _state_meta([128, lens[0]], [1, 2])
+        sa, sb = s0.clone(), s0.clone()
+        cat = lambda y: torch.cat((y[:128], y[: lens[0]]))  # noqa: E731
+        a = cu().gdn_recurrent(q[:128], k[:128], v[:128], g[:128], beta[:128], sa, short, chunked=True)
+        b = cu().gdn_recurrent(cat(q), cat(k), cat(v), cat(g), cat(beta), sb, both, chunked=True)
+        assert torch.equal(a, b[:128]) and torch.equal(sa[1], sb[1])
+    # operands of the products are bf16 (2^-9 each), sums f32: the limits of the chunk scan against the f32 rule
+    assert (runs[0][0].float() - want.float()).abs().max() < 0.03 * want.float().abs().max() + 2e-3
+    assert (runs[0][1] - want_s).abs().max() < 0.03 * want_s.abs().max()
+
+
 @pytest.mark.parametrize("t,m,k", [(257, 1024, 2048), (1337, 4096, 1024), (700, 5008, 1096), (4100, 4112, 512), (300, 1280, 8704), (1200, 1504, 776)])
 def test_two_sm_gemm_cuts_the_last_round(t, m, k):
     """Tiles of the last round cut in ranges of k: a few tiles only, tiles behind whole rounds, ragged edges, uneven ranges."""
