@@ -80,10 +80,10 @@ BUILDERS = {"nonetar": _nonetar, "zeripel": _zeripel, "vekalorn": _vekalorn, "ne
 
 # Translation units (csrc/<name>.cu) that a family's kernels come from, for programs that build only what one model needs
 KERNEL_UNITS = {
-    "nemipel": ("runtime", "gemm_sm100", "gemm2sm_sm100", "elementwise", "stream32", "attention", "attention_tc", "attention_general", "kda", "lightning", "sampling"),
-    "vekalorn": ("runtime", "gemm_sm100", "gemm2sm_sm100", "elementwise", "stream32", "mla", "mla_prefill", "moe_route", "moe_gemm", "sampling"),
-    "zeripel": ("runtime", "gemm_sm100", "gemm2sm_sm100", "elementwise", "stream32", "attention", "attention_tc", "attention_general", "kda", "wkv", "mla", "mla_prefill", "moe_route", "moe_gemm", "sampling"),
-    "nonetar": ("runtime", "gemm_sm100", "gemm2sm_sm100", "elementwise", "stream32", "streams", "attention", "attention_tc", "attention_general", "kda", "lightning", "lru", "moe_gemm", "sampling"),
+    "nemipel": ("runtime", "gemm_sm100", "gemm2sm_sm100", "decode_rows", "elementwise", "stream32", "attention", "attention_tc", "attention_general", "kda", "lightning", "sampling"),
+    "vekalorn": ("runtime", "gemm_sm100", "gemm2sm_sm100", "decode_rows", "elementwise", "stream32", "mla", "mla_decode_tc", "mla_prefill", "moe_route", "moe_gemm", "sampling"),
+    "zeripel": ("runtime", "gemm_sm100", "gemm2sm_sm100", "decode_rows", "elementwise", "stream32", "attention", "attention_tc", "attention_general", "kda", "wkv", "mla", "mla_decode_tc", "mla_prefill", "moe_route", "moe_gemm", "sampling"),
+    "nonetar": ("runtime", "gemm_sm100", "gemm2sm_sm100", "decode_rows", "elementwise", "stream32", "streams", "attention", "attention_tc", "attention_general", "kda", "lightning", "lru", "moe_gemm", "sampling"),
 }
 
 
