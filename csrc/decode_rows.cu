@@ -379,7 +379,10 @@ bool decode_rows_plan(DecodeRows& p, int T) {
     const int pieces = P.K / DR_PIECE;
     if (P.K % DR_PIECE != 0 || pieces == 0 || P.ldw % 8 != 0 || P.ldx % 8 != 0 || (((uintptr_t)P.w | (uintptr_t)P.x) & 15) != 0 || P.M < 2 || P.M % 2 != 0) return false;
     if (P.epi == DR_RESID_NORM && P.M % 128 != 0) return false;
-    if (i > 0 && P.in_ssp != nullptr && (p.ph[i - 1].epi != DR_RESID_NORM || p.ph[i - 1].M != P.K || P.in_width != P.K || p.ld_res % 8 != 0 || ((uintptr_t)p.residual & 15) != 0)) return false;
+    // a phase behind RESID_NORM forms the sums of squares of the residual rows that phase left: it must not write them itself (the
+    // tile kernel takes such chains), and sums that it takes in must be those
+    if (i > 0 && P.epi == DR_RESID_NORM && p.ph[i - 1].epi == DR_RESID_NORM) return false;
+    if (i > 0 && P.in_ssp != nullptr && (p.ph[i - 1].epi != DR_RESID_NORM || P.in_ssp != p.ph[i - 1].out_ssp || p.ph[i - 1].M != P.K || P.in_width != P.K || p.ld_res % 8 != 0 || ((uintptr_t)p.residual & 15) != 0)) return false;
     const int unit = P.M >= d.sms * 2 * DR_QUAD ? DR_QUAD : 2;
     P.rows = ceil_div(ceil_div(P.M, d.sms), unit) * unit;
     // warps split k only as far as that evens out the rows: the least work on the busiest warp, where the sums over the lanes that

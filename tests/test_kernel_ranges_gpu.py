@@ -262,3 +262,28 @@ def test_two_sm_gemm_cuts_the_last_round(t, m, k):
     assert torch.equal(y, K.linear_2sm(x, w)) and not K.ctx(DEV).gemm_counters.any() and K.read_status(DEV) == 0
     glu = K.linear_swiglu_2sm(x, w)
     assert glu is None or torch.equal(glu, K.swiglu(y, True))
+
+
+@pytest.mark.parametrize("t", [1, 3, 4, 64])
+def test_chain_of_two_residual_phases(t):
+    """Two residual + norm phases in a row update the same residual rows: the second may not do so before the sums of squares of
+    the first are formed."""
+    K = cu()
+    torch.manual_seed(t)
+    h, eps = 1024, 1e-6
+    w1, w2 = ((torch.randn(h, h, device=DEV) * 0.03).bfloat16() for _ in range(2))
+    n1, n2 = ((torch.rand(h, device=DEV) + 0.5).bfloat16() for _ in range(2))
+    a, res = torch.randn(t, h, device=DEV).bfloat16(), torch.randn(t, h, device=DEV).bfloat16()
+    inv = lambda x: torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps)  # noqa: E731
+    for _ in range(5):
+        r = res.clone()
+        o1, o2 = K.decode_chain(a, [(w1, K.CH_RESID_NORM, n1, False), (w2, K.CH_RESID_NORM, n2, False)], residual=r, eps=eps)
+        h1 = res.double() + a.double() @ w1.double().t()
+        s1 = o1.ssp[:, : o1.parts].double().sum(-1)
+        # the residual is rounded to bf16 (2^-9 a value) before it is squared: the sum of 1024 squares is within 2^-8 of the exact one
+        assert ((s1 - h1.pow(2).sum(-1)).abs() <= 2 ** -8 * s1).all()
+        h2 = h1 + (h1 * inv(h1) * n1.double()) @ w2.double().t()
+        err = (r.double() - h2).norm() / h2.norm()
+        assert err < 3 * 2 ** -9  # three roundings to bf16: the residual twice, the rows between
+        assert ((o2.ssp[:, : o2.parts].double().sum(-1) - r.double().pow(2).sum(-1)).abs() <= 2 ** -16 * r.double().pow(2).sum(-1)).all()
+    assert not K.ctx(DEV).chain_counters.any() and K.read_status(DEV) == 0
