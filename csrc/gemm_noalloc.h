@@ -22,7 +22,7 @@
 //  * The first call on a device looks up the scratch address (cudaGetSymbolAddress, with
 //    that device current).  Make that first call outside any stream capture.
 //  * All calls on a device share the one array, and it keeps whatever the previous call
-//    left there.  Each call clears the counters it needs on `stream` before launching.
+//    left there.  Each call clears the counters on `stream` before launching.
 //    Two calls that overlap on the GPU (different streams, or graphs replayed
 //    concurrently) race on it: serialise them.
 //  * Nothing here calls cudaMalloc, cudaFree or any allocating library routine.

@@ -1481,8 +1481,8 @@ extern "C" int pg_gemm_bf16_tn_noalloc(const void* x, const void* w, void* y, in
              "gemm_noalloc: %lld output tiles (M=%d, T=%d) exceed the built-in scratch limit of %d tiles; use pg_gemm_bf16_tn with caller scratch",
              tiles, M, T, (int)PG_NOALLOC_MAX_TILES);
   unsigned char* base = static_cast<unsigned char*>(scratch);
-  // the counters must start at zero; the partial sums are fully written before they are read
-  PG_CUDA(cudaMemsetAsync(base, 0, (size_t)tiles * 4, stream));
+  // the counters must start at zero, whichever kernel takes the problem (their layouts differ); the partial sums are fully written before they are read
+  PG_CUDA(cudaMemsetAsync(base, 0, PG_NOALLOC_COUNTER_BYTES, stream));
   return pg_gemm_bf16_tn(x, w, y, 0, T, M, K, ldx, ldw, ldy, base + PG_NOALLOC_COUNTER_BYTES,
                          (long long)PG_NOALLOC_SCRATCH_BYTES - PG_NOALLOC_COUNTER_BYTES, base, PG_NOALLOC_COUNTER_BYTES, status, 0, stream);
 }
