@@ -331,6 +331,7 @@ __device__ __forceinline__ void decode_rows(const DecodeRows& p) {
       *reinterpret_cast<uint2*>(dst + lane * 4) = pk;
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");  // a block that gave up has pieces of the next phase in flight
   // the last block out leaves the counters at zero for the next launch
   if (p.barriers && tid == 0 && atomicAdd(p.counters + DR_MAX_PHASES, 1u) == gridDim.x - 1) {
     for (int i = 0; i <= DR_MAX_PHASES; ++i) p.counters[i] = 0u;

@@ -287,3 +287,26 @@ def test_chain_of_two_residual_phases(t):
         assert err < 3 * 2 ** -9  # three roundings to bf16: the residual twice, the rows between
         assert ((o2.ssp[:, : o2.parts].double().sum(-1) - r.double().pow(2).sum(-1)).abs() <= 2 ** -16 * r.double().pow(2).sum(-1)).all()
     assert not K.ctx(DEV).chain_counters.any() and K.read_status(DEV) == 0
+
+
+@pytest.mark.parametrize("t", [1, 4])
+def test_chain_that_gives_up_leaves_nothing_behind(t):
+    """A chain whose status word is set gives up at a barrier that it has to wait at: counters back at zero, the next launch right."""
+    K = cu()
+    torch.manual_seed(t)
+    w = [(torch.randn(m, k, device=DEV) * 0.03).bfloat16() for m, k in ((1024, 2048), (6144, 1024), (1024, 3072))]
+    n1, n2 = ((torch.rand(1024, device=DEV) + 0.5).bfloat16() for _ in range(2))
+    a, res = torch.randn(t, 2048, device=DEV).bfloat16(), torch.randn(t, 1024, device=DEV).bfloat16()
+
+    def chain():
+        r = res.clone()
+        K.decode_chain(a, [(w[0], K.CH_RESID_NORM, n1, False), (w[1], K.CH_SWIGLU, None, False), (w[2], K.CH_RESID_NORM, n2, False)], residual=r, eps=1e-6)
+        return r
+
+    want = chain()
+    for _ in range(20):
+        K.ctx(DEV).status[0] = 2
+        chain()
+        assert not K.ctx(DEV).chain_counters.any()
+        K.clear_status(DEV)
+        assert torch.equal(chain(), want) and K.read_status(DEV) == 0
