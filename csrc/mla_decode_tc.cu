@@ -106,7 +106,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1) mla_decode_tc_kernel(const __gr
   const int per_split = (all_tiles - tile0 + p.splits - 1) / p.splits;
   const int first = tile0 + split * per_split, n_tiles = max(0, min(all_tiles, first + per_split) - first);
 
-  const int ragged = kv_end % DT_KEYS ? all_tiles - 1 - first : -1;  // tile whose last rows are no keys (of another split if it is not below n_tiles)
+  // tiles whose last rows, and whose first rows (in front of a window), are no keys; one of another split is not in 0 .. n_tiles - 1
+  const int ragged = kv_end % DT_KEYS ? all_tiles - 1 - first : -1, head = kv_begin % DT_KEYS ? tile0 - first : -1;
 
   if (warp == 0) {
     const uint64_t pol = l2_policy_evict_first();
@@ -174,7 +175,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1) mla_decode_tc_kernel(const __gr
           umma_commit(&sh->o_full);
           umma_commit(&sh->empty[os]);
           ++o_next;
-        } else if (s_next < n_tiles && s_next <= o_next + 1 && mbar_try_wait(&sh->full[ss], (uint32_t)((s_next >> 1) & 1)) && (s_next != ragged || mbar_try_wait(&sh->cleared, 0))) {
+        } else if (s_next < n_tiles && s_next <= o_next + 1 && mbar_try_wait(&sh->full[ss], (uint32_t)((s_next >> 1) & 1)) &&
+                   ((s_next != ragged && s_next != head) || mbar_try_wait(&sh->cleared, s_next != head && head >= 0 ? 1u : 0u))) {
           tc_fence_after();
           const uint32_t ka = smem_u32(tiles + ss * STAGE);
 #pragma unroll
@@ -206,13 +208,13 @@ __global__ void __launch_bounds__(DT_THREADS, 1) mla_decode_tc_kernel(const __gr
     bool ok = true;  // after a wait that ran out the warps go on through the barriers, without work
     for (int j = 0; j < n_tiles; ++j) {
       const int st = j & 1, key0 = (first + j) * DT_KEYS;
-      if (j == ragged) {
-        // rows behind the last key may hold anything, and zero weights do not silence a NaN: clear their values
+      if (j == ragged || j == head) {
+        // rows behind the last key or in front of the window may hold anything, and zero weights do not silence a NaN: clear their values
         ok = ok && mbar_wait(&sh->full[st], (uint32_t)((j >> 1) & 1), abort_flag);
-        const int live = kv_end - key0;
+        const int lo = max(0, kv_begin - key0), hi = min(DT_KEYS, kv_end - key0);
         if (ok)
-          for (int i = tid; i < (DT_KEYS - live) * 64; i += 128) {
-            const int r = live + (i >> 6);
+          for (int i = tid; i < (lo + DT_KEYS - hi) * 64; i += 128) {
+            const int r = (i >> 6) < lo ? i >> 6 : hi + (i >> 6) - lo;
             *reinterpret_cast<uint4*>(tiles + st * STAGE + (r >> 3) * BOX + (i & 7) * 1024 + (r & 7) * 128 + ((i >> 3) & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
           }
         fence_proxy_async_smem();

@@ -310,3 +310,39 @@ def test_chain_that_gives_up_leaves_nothing_behind(t):
         assert not K.ctx(DEV).chain_counters.any()
         K.clear_status(DEV)
         assert torch.equal(chain(), want) and K.read_status(DEV) == 0
+
+
+@pytest.mark.parametrize("extras", [False, True])
+@pytest.mark.parametrize("heads,rot,window,splits", [(16, 64, 70, 1), (64, 64, 70, 3), (5, 0, 33, 1), (40, 64, 200, 2), (64, 0, 64, 16), (16, 64, 0, 16)])
+def test_latent_window_and_empty_splits(heads, rot, window, splits, extras, monkeypatch):
+    """Rows in front of a window and behind the last key hold NaN (pages that others have written since); splits without keys,
+    also with a sink and a gate per head, which belong to the merged row."""
+    torch.manual_seed(heads + window)
+    kv_lens, page, lat, dim, vdim = [1, 63, 64, 65, 0, 129, 200, 511, 1000, 77, 96, 270], 16, 512, 128, 128
+    n = len(kv_lens)
+    per = [(x + page - 1) // page for x in kv_lens]
+    table, at = torch.zeros(n, max(per), dtype=torch.int32), 1
+    for i, m in enumerate(per):
+        table[i, :m] = torch.arange(at, at + m)
+        at += m
+    cache = torch.randn(at * page, lat + rot, device=DEV).bfloat16()
+    for i, (x, m) in enumerate(zip(kv_lens, per)):
+        rows = (table[i, :m].long()[:, None] * page + torch.arange(page)).flatten().to(DEV)
+        cache[rows[x:]] = float("nan")
+        if window:
+            cache[rows[: max(0, x - window)]] = float("nan")
+    pos = torch.tensor([max(x - 1, 0) for x in kv_lens], dtype=torch.int32, device=DEV)
+    meta = R.AttnMeta(torch.arange(n + 1, dtype=torch.int32, device=DEV), torch.tensor(kv_lens, dtype=torch.int32, device=DEV), table.to(DEV), pos, pos, page, n, n, 1, max(kv_lens), True,
+                      list(range(n + 1)), kv_lens)
+    q = torch.randn(n, heads * (dim + rot), device=DEV).bfloat16()
+    uk_t, uv = (torch.randn(heads, 512, 128, device=DEV) * 0.05).bfloat16(), (torch.randn(heads, vdim, lat, device=DEV) * 0.05).bfloat16()
+    a = torch.randn(2048, max(rot // 2, 1), device=DEV)
+    more = dict(head_gate=torch.randn(n, heads, device=DEV).bfloat16(), sink=torch.randn(heads, device=DEV)) if extras else {}
+    monkeypatch.setattr(cu(), "_latent_splits", lambda *a: splits)
+    args = (uk_t, uv, None)
+    got = cu().latent_attention(q, *args, cache.view(at, -1), meta, rot, 0.07, window, a.cos(), a.sin(), **more)
+    want = R.latent_attention(q, *args, torch.nan_to_num(cache).view(at, -1), meta, rot, 0.07, window, a.cos(), a.sin(), **more)
+    assert not got[4].any() and torch.isfinite(got.float()).all()
+    # weights and outputs of both are rounded to bf16 (2^-8 each), the sums are of some hundred terms: 2^-6 of the largest
+    assert (got.float() - want.float()).abs().max() <= 2 ** -6 * want.float().abs().max()
+    assert cu().read_status(DEV) == 0
