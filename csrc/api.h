@@ -230,7 +230,7 @@ int pg_attnres_mix(const void* cur, long long ld_cur, const void* snaps, long lo
 long long pg_gdn_chunk_bytes(int hv, int dv);
 int pg_gdn_chunked(const void* q, const void* k, long long ld_qk, const void* v, long long ld_v, const void* g, const void* beta, void* state,
                    void* out, const void* q_indptr, const void* slots, int num_seqs, int hk, int hv, int dk, int dv, int min_len,
-                   int chunks, int long_seqs, int longest, void* ws, long long ws_bytes, cudaStream_t stream);
+                   int short_seqs, int chunks, int long_seqs, int longest, void* ws, long long ws_bytes, cudaStream_t stream);
 
 // ---- attention (attention.cu) ------------------------------------------------------
 int pg_decode_splits(int num_seqs, int hkv, int max_kv_len, int sms);

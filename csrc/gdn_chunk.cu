@@ -19,14 +19,17 @@
 // order with what is left: four products and three barriers a chunk, its operands copied ahead by cp.async (block = (sequence,
 // value head, 64 of the Dv columns)).  The operands pass through scratch (88 KB a chunk and head).  48 value heads, us with
 // everything in the walk (10 us a chunk, both halves of Dv forming the same T, W and P) -> in two kernels: 842 + 1935 tokens
-// 414 -> 247, 4096 tokens 589 -> 402, 8 x 300 291 -> 229, 300 tokens 49 -> 40.  Sequences of up to SHORT_CHUNKS chunks stay on the one
-// kernel, whose operands never leave the SM (64 tokens 13, in two kernels 20; 40 x 100 557, in two 616).  The results are the same
+// 414 -> 247, 4096 tokens 589 -> 405, 8 x 300 290 -> 225, 300 tokens 49 -> 39.  Sequences of up to SHORT_CHUNKS chunks stay on the one
+// kernel, whose operands never leave the SM (64 tokens 13, in two kernels 20; 40 x 100 557, in two 616), also beside longer ones, and
+// the two kernels are launched for the longer ones alone: a block of the walk owns an SM, and one for every sequence of the step made 200 tokens beside 255
+// decode rows 1496 us instead of 539 (585 on the one kernel), 500 beside 100 x 64 2457 instead of 870 (881).  The results are the same
 // bytes: every operation and its order are those of the one kernel.
 //
 // Takes the place of the reference's chunk-wise Triton pipeline (pegainfer-kernels/tools/triton/
 // gated_delta_rule_chunkwise_kernels.py:28-708, chunk 64); the oracle is the token-by-token
 // recurrence of gdn.cu.
 #include <algorithm>
+#include <climits>
 #include <cuda_fp16.h>
 
 #include "api.h"
@@ -66,14 +69,14 @@ struct ChunkSmem {
 __global__ void __launch_bounds__(256, 1)
 gdn_chunk_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long long ld_qk, const bf16* __restrict__ v, long long ld_v,
                  const float* __restrict__ g, const float* __restrict__ beta, float* __restrict__ state, bf16* __restrict__ out,
-                 const int* __restrict__ q_indptr, const int* __restrict__ slots, int hk, int hv, int dv, int min_len) {
+                 const int* __restrict__ q_indptr, const int* __restrict__ slots, int hk, int hv, int dv, int min_len, int max_len) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   ChunkSmem& sm = *reinterpret_cast<ChunkSmem*>(smem_raw);
   const int splits = dv / DVC;
   const int h = blockIdx.x / splits, dv0 = (blockIdx.x % splits) * DVC, b = blockIdx.y;
   const int slot = slots[b];
   const int q0 = q_indptr[b], q1 = q_indptr[b + 1];
-  if (q1 - q0 < min_len || q1 == q0 || slot < 0) return;
+  if (q1 - q0 < min_len || q1 - q0 > max_len || q1 == q0 || slot < 0) return;
   const int kh = h / (hv / hk);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int gq = lane >> 2, t4 = lane & 3;
@@ -438,23 +441,50 @@ struct ChunkArgs {
   __device__ ChunkWs& chunk(int i, int h) const { return *reinterpret_cast<ChunkWs*>(ws + ((size_t)i * hv + h) * chunk_bytes(dv)); }
 };
 
+// Chunks of sequence b in this launch (b may lie behind the last: none)
 __device__ __forceinline__ int chunks_here(const ChunkArgs& p, int b) {
-  const int n = p.q_indptr[b + 1] - p.q_indptr[b];
-  if (n < p.min_len || n == 0 || p.slots[b] < 0) return 0;
-  return max(0, min(p.seg, (n + C - 1) / C - p.seg0));
+  const int i = min(b, p.num_seqs - 1), n = p.q_indptr[i + 1] - p.q_indptr[i];
+  const bool live = b < p.num_seqs && n >= p.min_len && n > 0 && p.slots[i] >= 0;
+  return live ? max(0, min(p.seg, (n + C - 1) / C - p.seg0)) : 0;
+}
+
+// The sequence that chunk `key` of the launch belongs to (BY_CHUNK), or the key-th one that has chunks; its first chunk in the
+// scratch, and its chunks (none: there is no such sequence).  All lanes of a warp call it; 32 sequences a step.
+struct Located {
+  int b, first, chunks;
+};
+template <bool BY_CHUNK>
+__device__ __forceinline__ Located locate(const ChunkArgs& p, int key) {
+  const int lane = threadIdx.x & 31;
+  int chunks = 0, keys = 0;
+  for (int base = 0; base < p.num_seqs; base += 32) {
+    const int n = chunks_here(p, base + lane);
+    int upto = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += x;
+    }
+    const uint32_t some = __ballot_sync(0xffffffffu, n > 0);
+    const int behind = BY_CHUNK ? chunks + upto : keys + __popc(some & (0xffffffffu >> (31 - lane)));  // keys up to and with this sequence
+    const uint32_t hit = __ballot_sync(0xffffffffu, n > 0 && behind > key);
+    if (hit) {
+      const int l = __ffs(hit) - 1;
+      return {base + l, chunks + __shfl_sync(0xffffffffu, upto - n, l), __shfl_sync(0xffffffffu, n, l)};
+    }
+    chunks += __shfl_sync(0xffffffffu, upto, 31);
+    keys += __popc(some);
+  }
+  return {0, 0, 0};
 }
 
 __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const ChunkArgs p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(smem_raw);
   const int h = blockIdx.x;
-  int b = 0, c = blockIdx.y;
-  for (; b < p.num_seqs; ++b) {
-    const int n = chunks_here(p, b);
-    if (c < n) break;
-    c -= n;
-  }
-  if (b == p.num_seqs) return;
+  const Located at = locate<true>(p, blockIdx.y);
+  if (at.chunks == 0) return;
+  const int b = at.b, c = blockIdx.y - at.first;
   const int t0 = p.q_indptr[b] + (p.seg0 + c) * C, nt = min(C, p.q_indptr[b + 1] - t0);
   ChunkWs& ws = p.chunk(blockIdx.y, h);
   bf16* vb = reinterpret_cast<bf16*>(&ws + 1);
@@ -676,25 +706,42 @@ __global__ void __launch_bounds__(256, 3 - STAGES) gdn_walk_kernel(const ChunkAr
   WalkSmem<STAGES>& sm = *reinterpret_cast<WalkSmem<STAGES>*>(smem_raw);
   const int splits = p.dv / DVC;
   const int h = blockIdx.x / splits, part = blockIdx.x % splits, dv0 = part * DVC;
-  // long sequences first: their walks bound the launch (the lengths are ranked in the state's place)
-  __shared__ int s_b;
-  int b = blockIdx.y;
-  if (p.num_seqs > 1 && p.num_seqs <= 256) {
-    int* len = reinterpret_cast<int*>(sm.s);
-    const int own = threadIdx.x < p.num_seqs ? chunks_here(p, threadIdx.x) : 0;
-    len[threadIdx.x] = own;
+  // Block row y walks the y-th longest sequence, since the long ones bound the launch (with more sequences than threads: the y-th).
+  // The sequences that have chunks are listed in the state's place, in their order, then ranked.
+  Located at;
+  if (p.num_seqs <= 256) {
+    __shared__ int s_count[8];
+    __shared__ Located s_at;
+    int2* list = reinterpret_cast<int2*>(sm.s);
+    const int own = chunks_here(p, threadIdx.x), w = threadIdx.x >> 5;
+    const uint32_t some = __ballot_sync(0xffffffffu, own > 0);
+    if ((threadIdx.x & 31) == 0) s_count[w] = __popc(some);
     __syncthreads();
-    if (threadIdx.x < p.num_seqs) {
-      int rank = 0;
-      for (int i = 0; i < p.num_seqs; ++i) rank += len[i] > own || (len[i] == own && i < threadIdx.x);
-      if (rank == b) s_b = threadIdx.x;
+    int place = __popc(some & ((1u << (threadIdx.x & 31)) - 1u)), total = 0;
+    for (int i = 0; i < 8; ++i) {
+      if (i < w) place += s_count[i];
+      total += s_count[i];
+    }
+    if ((int)blockIdx.y >= total) return;
+    if (own > 0) list[place] = make_int2(own, threadIdx.x);
+    __syncthreads();
+    if ((int)threadIdx.x < total) {
+      const int2 mine = list[threadIdx.x];
+      int rank = 0, first = 0;
+#pragma unroll 4
+      for (int i = 0; i < total; ++i) {
+        const int n = list[i].x;
+        rank += n > mine.x || (n == mine.x && i < (int)threadIdx.x);
+        first += i < (int)threadIdx.x ? n : 0;
+      }
+      if (rank == (int)blockIdx.y) s_at = {mine.y, first, mine.x};
     }
     __syncthreads();
-    b = s_b;
+    at = s_at;
+  } else {
+    at = locate<false>(p, blockIdx.y);
   }
-  int c0 = 0;  // this sequence's first chunk in the scratch
-  for (int i = 0; i < b; ++i) c0 += chunks_here(p, i);
-  const int n_chunks = min(chunks_here(p, b), p.cap - c0);
+  const int b = at.b, c0 = at.first, n_chunks = min(at.chunks, p.cap - c0);
   if (n_chunks <= 0) return;
   const int slot = p.slots[b], q1 = p.q_indptr[b + 1], dv = p.dv;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -853,17 +900,18 @@ __global__ void __launch_bounds__(256, 3 - STAGES) gdn_walk_kernel(const ChunkAr
 extern "C" long long pg_gdn_chunk_bytes(int hv, int dv) { return (long long)chunk_bytes(dv) * hv; }
 
 // Chunk-wise gated delta rule for every sequence of at least `min_len` tokens (shorter ones,
-// decode rows in particular, are left to pg_gdn_recurrent).  dk must be 128, dv a multiple of 64.  There are at most `long_seqs` such
-// sequences, of `chunks` chunks in all and `longest` each; what exceeds the scratch is done in segments of the sequences (their
-// states carry over), and groups of sequences where not even one chunk of each fits.
+// decode rows in particular, are left to pg_gdn_recurrent).  dk must be 128, dv a multiple of 64.  Sequences of up to
+// SHORT_CHUNKS chunks (is there one: `short_seqs`) run on the one kernel.  There are at most `long_seqs` longer ones, of `chunks` chunks in
+// all and `longest` each; what exceeds the scratch, which has room for one chunk of each, is done in segments of the sequences
+// (their states carry over).
 extern "C" int pg_gdn_chunked(const void* q, const void* k, long long ld_qk, const void* v, long long ld_v, const void* g, const void* beta,
                               void* state, void* out, const void* q_indptr, const void* slots, int num_seqs, int hk, int hv, int dk, int dv,
-                              int min_len, int chunks, int long_seqs, int longest, void* ws, long long ws_bytes, cudaStream_t stream) {
+                              int min_len, int short_seqs, int chunks, int long_seqs, int longest, void* ws, long long ws_bytes, cudaStream_t stream) {
   PG_REQUIRE(dk == DK && dv % DVC == 0 && hv % hk == 0, "gdn_chunked: dk=%d must be 128, dv=%d a multiple of 64", dk, dv);
   PG_REQUIRE(ld_qk % 8 == 0 && ld_v % 8 == 0, "gdn_chunked: row strides must be multiples of 8 elements");
   PG_REQUIRE((((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)ws) & 15) == 0 && (((uintptr_t)state | (uintptr_t)out) & 7) == 0,
              "gdn_chunked: q, k, v and the scratch must be 16-byte aligned, state and out 8-byte aligned");
-  if (num_seqs == 0 || chunks == 0) return PG_OK;
+  if (num_seqs == 0) return PG_OK;
   static bool set = false;
   if (!set) {
     PG_CUDA(cudaFuncSetAttribute(gdn_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChunkSmem)));
@@ -872,30 +920,27 @@ extern "C" int pg_gdn_chunked(const void* q, const void* k, long long ld_qk, con
     PG_CUDA(cudaFuncSetAttribute(gdn_walk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkSmem<2>)));
     set = true;
   }
-  if (longest <= SHORT_CHUNKS) {
+  if (short_seqs) {
+    const int max_len = long_seqs > 0 ? SHORT_CHUNKS * C : INT_MAX;
     gdn_chunk_kernel<<<dim3(hv * (dv / DVC), num_seqs), 256, sizeof(ChunkSmem), stream>>>((const bf16*)q, (const bf16*)k, ld_qk, (const bf16*)v, ld_v, (const float*)g, (const float*)beta, (float*)state, (bf16*)out,
-                                                                                          (const int*)q_indptr, (const int*)slots, hk, hv, dv, min_len);
+                                                                                          (const int*)q_indptr, (const int*)slots, hk, hv, dv, min_len, max_len);
     PG_LAUNCH_CHECK();
-    return PG_OK;
   }
+  if (long_seqs == 0 || chunks == 0) return PG_OK;
+  min_len = std::max(min_len, SHORT_CHUNKS * C + 1);
   const long long room = std::min(ws_bytes / ((long long)chunk_bytes(dv) * hv), 65535ll);
-  PG_REQUIRE(room >= 1, "gdn_chunked: scratch of %lld bytes", ws_bytes);
-  const bool all = chunks <= room;
-  const int group = long_seqs <= room ? std::min(num_seqs, 65535) : (int)room;  // sequences of a launch
-  const int seg = all ? longest : (int)std::max(room / std::min(long_seqs, group), 1ll);
-  for (int b0 = 0; b0 < num_seqs; b0 += group) {
-    const int nb = std::min(group, num_seqs - b0);
-    for (int seg0 = 0; seg0 < longest; seg0 += seg) {
-      const int cap = (int)std::min((long long)chunks, std::min(room, (long long)seg * std::min(long_seqs, nb)));
-      const ChunkArgs p = {(const bf16*)q, (const bf16*)k, (const bf16*)v, ld_qk, ld_v, (const float*)g, (const float*)beta, (float*)state, (bf16*)out,
-                           (const int*)q_indptr + b0, (const int*)slots + b0, nb, hk, hv, dv, min_len, seg0, seg, cap, (uint8_t*)ws};
-      gdn_prep_kernel<<<dim3(hv, cap), 256, sizeof(PrepSmem), stream>>>(p);
-      PG_LAUNCH_CHECK();
-      const dim3 walks(hv * (dv / DVC), nb);
-      if (walks.x * (long long)std::min(nb, long_seqs) > 3 * 148) gdn_walk_kernel<1><<<walks, 256, sizeof(WalkSmem<1>), stream>>>(p);
-      else gdn_walk_kernel<2><<<walks, 256, sizeof(WalkSmem<2>), stream>>>(p);
-      PG_LAUNCH_CHECK();
-    }
+  PG_REQUIRE(room >= std::min(chunks, long_seqs), "gdn_chunked: scratch of %lld bytes for %d sequences", ws_bytes, long_seqs);
+  const int seg = chunks <= room ? longest : (int)(room / long_seqs);
+  const int cap = (int)std::min((long long)chunks, room);
+  for (int seg0 = 0; seg0 < longest; seg0 += seg) {
+    const ChunkArgs p = {(const bf16*)q, (const bf16*)k, (const bf16*)v, ld_qk, ld_v, (const float*)g, (const float*)beta, (float*)state, (bf16*)out,
+                         (const int*)q_indptr, (const int*)slots, num_seqs, hk, hv, dv, min_len, seg0, seg, cap, (uint8_t*)ws};
+    gdn_prep_kernel<<<dim3(hv, cap), 256, sizeof(PrepSmem), stream>>>(p);
+    PG_LAUNCH_CHECK();
+    const dim3 walks(hv * (dv / DVC), long_seqs);
+    if (walks.x * (long long)long_seqs > 3 * 148) gdn_walk_kernel<1><<<walks, 256, sizeof(WalkSmem<1>), stream>>>(p);
+    else gdn_walk_kernel<2><<<walks, 256, sizeof(WalkSmem<2>), stream>>>(p);
+    PG_LAUNCH_CHECK();
   }
   return PG_OK;
 }

@@ -831,19 +831,27 @@ def gdn_recurrent(q, k, v, g, beta, state, meta: AttnMeta, chunked: Optional[boo
             _ptr(meta.q_indptr), _ptr(meta.state_slots), _ci(meta.num_seqs), _ci(hk), _ci(hv), _ci(dk), _ci(dv))
     short_rows = True  # is there a sequence below the chunk threshold (decode rows in a unified step)?
     if chunked:
-        # chunks of 64 tokens, sequences that have some and the longest of them: counted where the lengths are known here, else bounded
+        # sequences of one or two chunks of 64 tokens run on one kernel, longer ones on two with scratch: which there are, and how many
+        # chunks of the longer ones, counted where the lengths are known here, else bounded
         if meta.h_q_indptr is not None:
             lens = [meta.h_q_indptr[i + 1] - meta.h_q_indptr[i] for i in range(meta.num_seqs)]
             short_rows = any(n < _GDN_CHUNK_MIN for n in lens)
-            counts = [-(-n // 64) for n in lens if n >= _GDN_CHUNK_MIN]
+            short_seqs = any(_GDN_CHUNK_MIN <= n <= 128 for n in lens)
+            counts = [-(-n // 64) for n in lens if n > 128]
             chunks, rows, longest = sum(counts), len(counts), max(counts, default=0)
         else:
-            rows = min(meta.num_seqs, t // _GDN_CHUNK_MIN)
+            short_seqs, rows = True, min(meta.num_seqs, t // 129) if int(meta.max_q_len) > 128 else 0
             chunks, longest = t // 64 + rows, -(-t // 64)
         one = int(lib().pg_gdn_chunk_bytes(_ci(hv), _ci(dv)))
-        ws = torch.empty(one * max(1, min(chunks, _GDN_WS_BYTES // one)) if longest > 2 else 0, dtype=torch.uint8, device=q.device)
-        rc = lib().pg_gdn_chunked(*args, _ci(_GDN_CHUNK_MIN), _ci(chunks), _ci(rows), _ci(longest), _ptr(ws), _ll(ws.numel()), _stream())
-        _check(rc, c, 2)
+        room = max(1, _GDN_WS_BYTES // one)
+        if (longest == 3 and rows * hv * (dv // 64) <= c.sms < chunks * hv) or (chunks > room and room < 2 * rows):
+            # the one kernel takes all: three chunks that it walks in one wave of blocks, where the first of the two kernels would need more
+            # than one (8 x 130 tokens, 8 heads: 30 us, in two kernels 33); scratch for less than two chunks of each sequence, whose states
+            # would be read and written for every chunk (40 x 400 tokens, 48 heads: 1735 us, in segments of one chunk 1888)
+            short_seqs, rows = True, 0
+        ws = torch.empty(one * min(chunks, room) if rows else 0, dtype=torch.uint8, device=q.device)
+        rc = lib().pg_gdn_chunked(*args, _ci(_GDN_CHUNK_MIN), _ci(int(short_seqs)), _ci(chunks), _ci(rows), _ci(longest), _ptr(ws), _ll(ws.numel()), _stream())
+        _check(rc, c, int(short_seqs) + (2 if rows else 0))
     if not chunked or short_rows:
         rc = lib().pg_gdn_recurrent(*args, _ci(int(meta.max_q_len)), _ci(_GDN_CHUNK_MIN if chunked else 0), _stream())
         _check(rc, c)

@@ -217,8 +217,8 @@ def test_linear_of_few_rows(t, m, k):
 @pytest.mark.parametrize("dv", [64, 128])
 @pytest.mark.parametrize("lens,room", [([32, 63, 64, 65, 1, 129, 0, 31], None), ([700, 33, 450], 7), ([140] * 9 + [3] + [200] * 4, 5), ([260], 1)])
 def test_gated_delta_chunks_in_segments(lens, room, dv, monkeypatch):
-    """All chunks at once, segments of the sequences, groups of sequences, and (short ones) one kernel give the same bytes, and the
-    token-by-token rule's values."""
+    """All chunks at once, segments of the sequences, and one kernel (short sequences; scratch for less than two chunks of each) give
+    the same bytes, and the token-by-token rule's values."""
     torch.manual_seed(sum(lens) + dv)
     hk, hv, dk = 2, 4, 128
     meta = _state_meta(lens, list(range(1, len(lens) + 1)))
@@ -346,3 +346,35 @@ def test_latent_window_and_empty_splits(heads, rot, window, splits, extras, monk
     # weights and outputs of both are rounded to bf16 (2^-8 each), the sums are of some hundred terms: 2^-6 of the largest
     assert (got.float() - want.float()).abs().max() <= 2 ** -6 * want.float().abs().max()
     assert cu().read_status(DEV) == 0
+
+
+@pytest.mark.parametrize("known", [True, False])
+@pytest.mark.parametrize("rows", [3, 70, 290])  # decode rows beside the prompts: up to and above the 256 sequences that are ranked by length
+def test_gated_delta_prompts_beside_decode_rows(rows, known):
+    """Prompts of one to six chunks among decode rows, empty sequences and one without a state: every sequence's bytes are those of a
+    step of its own, whichever kernel takes it."""
+    torch.manual_seed(rows)
+    lens = [200, 64, 0, 129, 128, 330, 32, 129] + [1] * rows + [260, 31, 100]
+    slots = list(range(1, len(lens) + 1))
+    slots[3] = -1
+    meta = _state_meta(lens, slots)
+    hk, hv, dk, dv, t = 2, 4, 128, 128, sum(lens)
+    x = torch.randn(t, 2 * hk * dk + hv * dv, device=DEV).bfloat16()
+    q, k, v = (y.view(t, -1, d) for y, d in zip(x.split([hk * dk, hk * dk, hv * dv], 1), (dk, dk, dv)))
+    g, beta = -torch.rand(t, hv, device=DEV), torch.rand(t, hv, device=DEV)
+    s0 = torch.randn(len(lens) + 2, hv, dk, dv, device=DEV) * 0.1
+    s = s0.clone()
+    meta.h_q_indptr = meta.q_indptr.tolist() if known else None
+    out, at = cu().gdn_recurrent(q, k, v, g, beta, s, meta, chunked=True), 0
+    for i, n in enumerate(lens):
+        sl = slice(at, at + n)
+        at += n
+        if n < 32 and i != 8 or slots[i] < 0:
+            continue
+        alone, one = s0.clone(), _state_meta([n], [slots[i]])
+        y = cu().gdn_recurrent(q[sl], k[sl], v[sl], g[sl], beta[sl], alone, one, chunked=n >= 32)
+        if n >= 32:
+            assert torch.equal(out[sl], y) and torch.equal(s[slots[i]], alone[slots[i]]), i
+        else:  # (a decode row among prompts may sum in another order: the limits of one f32 step, rounded to bf16)
+            assert (out[sl].float() - y.float()).abs().max() <= 2 ** -7 * y.float().abs().max()
+    assert torch.equal(s[0], s0[0]) and torch.equal(s[4], s0[4]) and torch.equal(s[3], s0[3])  # no one's, the stateless one's, the empty one's
