@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(128) kda_recurrent_kernel(const T* __restrict_
   const int slot = slots[seq];
   const int q0 = q_indptr[seq], q1 = q_indptr[seq + 1];
   if (q1 == q0 || slot < 0) return;
-  if (RULE != RULE_BOUNDED && skip_len > 0 && q1 - q0 >= skip_len) return;
+  if (skip_len > 0 && q1 - q0 >= skip_len) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qtr = XW ? warp : (tid & 3), lc = XW ? lane : (tid >> 2), col = cg * KDA_COLS + lc;
   const bool owner = col < dv;
@@ -290,7 +290,8 @@ int run_rule(int rule, RecArgs<T> p, int num_seqs, int max_q_len, cudaStream_t s
 // A lane holds 16 rows x 4 columns of the state as row pairs for the packed f32x2 instructions; the 8 lanes of a column
 // group read 128 contiguous bytes of a vector at a time, which is what the walk, with 32 elements of one column per thread,
 // was short of: shared-memory reads (three vectors per 32 elements and token there, 13 per 64 elements and 4 tokens here).
-// 3001 tokens in two prompts, 96 heads: 2550 us before, 1145 us now.  What bounds it: FMA issue and shared-memory reads
+// 3001 tokens in two prompts, 96 heads: 2550 us before, 1145 us now; 16 heads, one prompt of 3000: 1644 and 1099.  Decode rows
+// beside a prompt stay on the walk (64 rows and 300 tokens, 96 heads: 398 us with every row in a block of four, 333 now).  What bounds it: FMA issue and shared-memory reads
 // (both near half of their rate) by warps that wait for their own sums, few of them where a step has few sequences.
 constexpr int KB_T = 4;        // tokens per block
 constexpr int KB_BLOCKS = 4;   // blocks per stage: one per warp to prepare
@@ -303,13 +304,14 @@ struct KdaBlock {
   float ab[16];  // A_ts at t (t - 1) / 2 + s, B_ts at 6 + t (t + 1) / 2 + s
   float beta[KB_T];
 };
-struct KdaBlockSmem {
+struct KdaBlockSmem {  // 47 KB: no attribute needed
   KdaBlock blk[KB_BLOCKS];
   bf16 raw[KB_BLOCKS][3][KB_T][KB_DK];  // q, k, f rows of the stage after this one
   bf16 raw_v[KB_BLOCKS][KB_T][KB_COLS];
   float u[4][KB_T][16], o[4][KB_T][16];  // per warp: kd . S0, then d; qd . S0
 };
 
+static_assert(sizeof(KdaBlockSmem) <= 48 * 1024, "more needs the kernel's attribute, on every device");
 __device__ __forceinline__ unsigned long long kb_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
   unsigned long long d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
@@ -348,14 +350,14 @@ __device__ __forceinline__ void kb_reduce_scatter(float* v, int lane, int top) {
 __global__ void __launch_bounds__(128, 3)
 kda_block_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v, long long ld, const bf16* __restrict__ f, long long ldf, const bf16* __restrict__ b, long long ldb,
                  const float* __restrict__ a_log, const float* __restrict__ dt_bias, float lower, float* __restrict__ state, bf16* __restrict__ out, const int* __restrict__ q_indptr,
-                 const int* __restrict__ slots, int heads, int dv) {
+                 const int* __restrict__ slots, int heads, int dv, int min_len) {
   extern __shared__ __align__(16) uint8_t kb_raw[];
   KdaBlockSmem& sm = *reinterpret_cast<KdaBlockSmem*>(kb_raw);
   const int groups = dv / KB_COLS;
   const int h = blockIdx.x / groups, c0 = blockIdx.x % groups * KB_COLS, seq = blockIdx.y;
   const int slot = slots[seq];
   const int q0 = q_indptr[seq], q1 = q_indptr[seq + 1];
-  if (q1 == q0 || slot < 0) return;
+  if (q1 - q0 < min_len || slot < 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rg = lane & 7, cg = lane >> 3;
   const int col = c0 + warp * 16 + cg * 4;  // the lane's first state column
@@ -629,26 +631,28 @@ __global__ void __launch_bounds__(256) attnres_mix_kernel(const bf16* __restrict
 
 }  // namespace
 
+// Sequences of min_len tokens and more go four tokens at a time where rows and state are runs of 16-byte pieces, shorter ones (of
+// up to `short_len` tokens; 0: there are none) token by token in a launch of their own, so that a decode row beside a prompt is
+// what it is in a step of decode rows.
 extern "C" int pg_kda_recurrent(const void* q, const void* k, const void* v, long long ld, const void* f, long long ldf, const void* b, long long ldb,
                                 const void* a_log, const void* dt_bias, float lower, void* state, void* out, const void* q_indptr, const void* slots,
-                                int num_seqs, int heads, int dk, int dv, int max_q_len, cudaStream_t stream) {
+                                int num_seqs, int heads, int dk, int dv, int max_q_len, int min_len, int short_len, cudaStream_t stream) {
   PG_REQUIRE(dv <= 128 && lower < 0.f, "kda_recurrent: dv=%d must be <= 128 and the decay lower bound %f negative", dv, (double)lower);
+  PG_REQUIRE(min_len >= 1, "kda_recurrent: blocks for sequences of %d tokens", min_len);
   if (num_seqs == 0) return PG_OK;
   RecArgs<bf16> p = {(const bf16*)q, (const bf16*)k, (const bf16*)v, ld, f, ldf, (const bf16*)b, ldb, (const float*)a_log, (const float*)dt_bias, nullptr, lower,
                      (float*)state, (bf16*)out, (const int*)q_indptr, (const int*)slots, heads, heads, dk, dv, (dv + KDA_COLS - 1) / KDA_COLS, 0};
-  const dim3 grid(heads * p.col_groups, num_seqs);
-  const bool few = max_q_len <= 4;
-  // prompts: four tokens at a time where rows and state are runs of 16-byte pieces
-  const bool blocks = !few && dk == KB_DK && dv % KB_COLS == 0 && ld % 8 == 0 && ldf % 8 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)f | (uintptr_t)dt_bias | (uintptr_t)state) & 15) == 0;
+  const bool blocks = max_q_len >= min_len && dk == KB_DK && dv % KB_COLS == 0 && ld % 8 == 0 && ldf % 8 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)f | (uintptr_t)dt_bias | (uintptr_t)state) & 15) == 0;
   if (blocks) {
-    static bool set = false;
-    if (!set) {
-      PG_CUDA(cudaFuncSetAttribute(kda_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KdaBlockSmem)));
-      set = true;
-    }
     kda_block_kernel<<<dim3(heads * (dv / KB_COLS), num_seqs), 128, sizeof(KdaBlockSmem), stream>>>(p.q, p.k, p.v, ld, (const bf16*)f, ldf, p.b, ldb, p.a_log, p.dt_bias, lower, p.state, p.out, p.q_indptr, p.slots,
-                                                                                                     heads, dv);
-  } else if (dk == 128)
+                                                                                                     heads, dv, min_len);
+    PG_LAUNCH_CHECK();
+    if (short_len <= 0) return PG_OK;
+    p.skip_len = min_len;
+  }
+  const dim3 grid(heads * p.col_groups, num_seqs);
+  const bool few = (blocks ? short_len : max_q_len) <= 4;
+  if (dk == 128)
     PG_CUDA((launch_rule<bf16, 128, RULE_BOUNDED, false>(p, grid, few, stream)));
   else if (dk == 64)
     PG_CUDA((launch_rule<bf16, 64, RULE_BOUNDED, false>(p, grid, few, stream)));

@@ -378,3 +378,38 @@ def test_gated_delta_prompts_beside_decode_rows(rows, known):
         else:  # (a decode row among prompts may sum in another order: the limits of one f32 step, rounded to bf16)
             assert (out[sl].float() - y.float()).abs().max() <= 2 ** -7 * y.float().abs().max()
     assert torch.equal(s[0], s0[0]) and torch.equal(s[4], s0[4]) and torch.equal(s[3], s0[3])  # no one's, the stateless one's, the empty one's
+
+
+@pytest.mark.parametrize("known", [True, False])
+@pytest.mark.parametrize("lens", [[1] * 5 + [200], [16, 1, 8, 9, 3, 13, 1, 0, 40], [4, 1, 5]])
+def test_kda_rows_beside_prompts(lens, known):
+    """Sequences below the blocks' shortest go token by token, whatever shares their step: decode rows beside prompts have the bytes of a
+    step of decode rows, prompts those of a step of their own."""
+    K = cu()
+    torch.manual_seed(sum(lens))
+    heads, dk, dv, t, slots = 3, 128, 128, sum(lens), list(range(1, len(lens) + 1))
+    qkv = torch.randn(t, 3 * heads * dk, device=DEV).bfloat16()
+    q, k, v = (qkv[:, j * heads * dk : (j + 1) * heads * dk].view(t, heads, dk) for j in range(3))
+    f, b = torch.randn(t, heads * dk, device=DEV).bfloat16(), torch.randn(t, heads, device=DEV).bfloat16()
+    a_log, dt = torch.randn(heads, device=DEV) * 0.5, torch.randn(heads * dk, device=DEV) - 2
+    s0 = torch.randn(len(lens) + 1, heads, dk, dv, device=DEV)
+
+    def run(rows, lens, slots, known):
+        meta, s = _state_meta(lens, slots), s0.clone()
+        meta.h_q_indptr = meta.q_indptr.tolist() if known else None
+        return K.kda_recurrent(q[rows], k[rows], v[rows], f[rows], b[rows], a_log, dt, -5.0, s, meta), s
+
+    out, s = run(slice(0, t), lens, slots, known)
+    short, at = max((n for n in lens if n < K._KDA_BLOCK_MIN), default=0), 0
+    for n, slot in zip(lens, slots):
+        rows = slice(at, at + n)
+        at += n
+        if n == 0:
+            assert torch.equal(s[slot], s0[slot])
+            continue
+        y, alone = run(rows, [n], [slot], True)
+        if n >= K._KDA_BLOCK_MIN or (known and (short <= 4) == (n <= 4)):
+            assert torch.equal(out[rows], y) and torch.equal(s[slot], alone[slot])
+        else:  # beside rows of five tokens and more the sums of a column are formed in another order: f32, then one rounding to bf16
+            assert (out[rows].float() - y.float()).abs().max() <= 2 ** -8 * y.float().abs().max() + 1e-5
+            assert (s[slot] - alone[slot]).abs().max() <= 2 ** -17 * alone[slot].abs().max()
