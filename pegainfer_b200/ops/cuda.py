@@ -1587,9 +1587,44 @@ def _head_offsets(heads: int, tokens: int, device):
     return o
 
 
-def _latent_splits(rows: int, heads: int, lat: int, rot: int, longest: int, sms: int) -> int:
+def _latent_keys(meta: AttnMeta, row0: int = 0, window: int = 0) -> int:
+    """Keys of a typical row of a step from row ``row0`` on, for the choice of a kernel: the rows' mean where the lengths are known here, but at
+    least half of the longest, which one block walks."""
+    longest = min(meta.max_kv_len, window) if window else meta.max_kv_len
+    qi, kvl = meta.h_q_indptr, meta.h_kv_lens
+    if qi is None or kvl is None:
+        return longest
+    rows = keys = 0
+    for b in range(meta.num_seqs):
+        n = qi[b + 1] - max(qi[b], row0)
+        if n > 0:
+            rows += n
+            keys += n * (min(kvl[b] - (n - 1) // 2, window) if window else kvl[b] - (n - 1) // 2)
+    return max(keys // max(rows, 1), longest // 2)
+
+
+def _latent_tc(rows: int, heads: int, lat: int, rot: int, keys: int, decode: bool, sms: int) -> bool:
+    """Does the absorbed form of rows of about ``keys`` keys run on tcgen05 (csrc/mla_decode_tc.cu)?  A block there owns an SM, serves up
+    to 64 heads and works in tiles of 64 keys, whole ones; the mma.sync kernel has four blocks of 16 heads an SM and tiles of 32.
+    Measured with 16, 32, 64 and 128 heads (tcgen05 / mma.sync): within one wave of blocks 1.01 - 1.11 up to 32 keys, 0.90 - 1.02 at 40, 1.02 -
+    1.04 at 65 and 80 with few blocks (prompts of 80 tokens 1.01 - 1.05, of 100 0.94 - 0.97); above, where blocks of 16 heads leave three quarters of their tiles empty, 16 heads
+    1.03 - 1.26 at 128 keys and two waves, 1.03 - 1.08 at 200 and more waves (0.91 - 0.97 at 300), 32 heads 1.0 - 1.06 at 80 (0.90 - 0.98 at
+    100), 64 heads 0.88 - 1.0 at 40, but 1.02 at 80 with a second wave that is nearly empty (150 rows).
+    A captured graph goes by its bound on the keys: 20 keys in a graph for 2048 take 1.02 - 1.10 of the time (8 rows of 128 heads 1.13),
+    500 keys 0.5 - 0.8."""
+    if lat != 512 or rot not in (0, 64):
+        return False
+    blocks = rows * ((heads + 63) // 64)
+    if blocks <= sms:
+        return keys > (32 if decode else 44) and not (64 < keys <= 88 and blocks < 32)
+    if heads <= 16:
+        return keys > (128 if blocks <= 2 * sms else 256)
+    return keys > (96 if heads <= 32 or 3 * blocks < 4 * sms else 32)
+
+
+def _latent_splits(rows: int, heads: int, longest: int, tc: bool, sms: int) -> int:
     """Blocks that share one row's keys in the absorbed kernels."""
-    if lat == 512 and rot in (0, 64):  # csrc/mla_decode_tc.cu: a block owns an SM and serves up to 64 heads, so as many as there are SMs, of 256 keys or more
+    if tc:  # csrc/mla_decode_tc.cu: a block owns an SM and serves up to 64 heads, so as many as there are SMs, of 256 keys or more
         return max(1, min(16, sms // (rows * ((heads + 63) // 64)), (longest + 255) // 256))
     return max(1, min(16, (4 * sms) // (rows * ((heads + 15) // 16)), (min(longest, 4096) + 127) // 128))
 
@@ -1709,7 +1744,8 @@ def mla_attention(q: "_MlaQ", w_uk, w_uv, latent_layer, meta: AttnMeta, scale, k
         for b in range(meta.num_seqs):
             seq_of.extend([b] * (qi[b + 1] - qi[b]))
         unit_seq = torch.tensor(seq_of, dtype=torch.int32, device=dev)
-    splits = _latent_splits(t, h, kv_lora, rope, meta.max_kv_len, c.sms) if meta.decode_only else 1
+    tc = _latent_tc(t, h, kv_lora, rope, _latent_keys(meta), meta.decode_only, c.sms)
+    splits = _latent_splits(t, h, meta.max_kv_len, tc, c.sms) if meta.decode_only else 1
     need = t * h * splits * (kv_lora + 1) * 4
     if need > c.attn_part.numel():
         splits = 1
@@ -1718,7 +1754,7 @@ def mla_attention(q: "_MlaQ", w_uk, w_uv, latent_layer, meta: AttnMeta, scale, k
     lat_out = torch.empty((h * t, kv_lora), dtype=torch.bfloat16, device=dev)
     rc = lib().pg_mla_attention(_ptr(q_abs), _ptr(q.pe), _ptr(latent_layer), _ptr(lat_out), _ptr(meta.q_indptr), _ptr(meta.kv_lens), _ptr(meta.block_table),
                                 _ci(meta.block_table.stride(0)), _ptr(unit_seq), _ci(meta.num_seqs), _ci(t), _ci(h), _ci(kv_lora), _ci(rope), _ci(page_size), _cf(scale),
-                                _ci(splits), _ptr(part_o), _ptr(part_lse), _ll(latent_layer.shape[0]), _ptr(c.status), _stream())
+                                _ci(splits), _ci(int(tc)), _ptr(part_o), _ptr(part_lse), _ll(latent_layer.shape[0]), _ptr(c.status), _stream())
     _check(rc, c, 2 if splits > 1 else 1)
     v_hm = grouped_gemm(lat_out, offs, w_uv, None, bn)  # [H*T, v]
     vdim = w_uv.shape[1]
@@ -1836,10 +1872,12 @@ def latent_attention(q, uk_t, uv, ukv, cache, meta: AttnMeta, rot: int, scale: f
     where = (_ptr(cache), _ptr(o), *strides, _ptr(meta.q_indptr), _ptr(meta.kv_lens), _ptr(table), _ci(table.stride(0)), _ptr(_unit_seq(meta, dev)))
     if aligned and lat <= 512 and rot <= 64:
         longest = max(meta.max_kv_len, 1)
-        splits = _latent_splits(n, heads, lat, rot, min(longest, window + 31) if window else longest, c.sms)
+        longest = min(longest, window + 31) if window else longest
+        tc = _latent_tc(n, heads, lat, rot, _latent_keys(meta, row0, window), meta.decode_only, c.sms)
+        splits = _latent_splits(n, heads, longest, tc, c.sms)
         splits = max(1, min(splits, c.attn_part.numel() // (n * heads * (lat + 1) * 4)))
         rc = lib().pg_latent_attention(_ptr(q_abs), *strides, *pe, *where, _ci(row0), _ci(meta.num_seqs), _ci(n), _ci(heads), _ci(lat), _ci(rot), _ci(ps), _cf(scale), _ci(window), *extra, _ci(splits),
-                                       _ptr(c.attn_part), _ptr(c.attn_part[n * heads * splits * lat * 4 :]), _ll(cache.shape[0]), _ptr(c.status), _stream())
+                                       _ci(int(tc)), _ptr(c.attn_part), _ptr(c.attn_part[n * heads * splits * lat * 4 :]), _ll(cache.shape[0]), _ptr(c.status), _stream())
         _check(rc, c, 2 if splits > 1 else 1)
     else:
         assert row0 == 0

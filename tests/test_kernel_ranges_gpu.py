@@ -313,12 +313,18 @@ def test_chain_that_gives_up_leaves_nothing_behind(t):
 
 
 @pytest.mark.parametrize("extras", [False, True])
-@pytest.mark.parametrize("heads,rot,window,splits", [(16, 64, 70, 1), (64, 64, 70, 3), (5, 0, 33, 1), (40, 64, 200, 2), (64, 0, 64, 16), (16, 64, 0, 16)])
-def test_latent_window_and_empty_splits(heads, rot, window, splits, extras, monkeypatch):
+@pytest.mark.parametrize(
+    "heads,rot,window,splits,reps,tc",
+    # blocks of 16 heads; of 32 (60 rows of 64 heads) and 64 (120 rows), with one and three splits, and a second group of 32 heads
+    [(16, 64, 70, 1, 1, True), (64, 64, 70, 3, 1, True), (5, 0, 33, 1, 1, True), (40, 64, 200, 2, 1, True), (64, 0, 64, 16, 1, True), (16, 64, 0, 16, 1, True),
+     (64, 64, 70, 1, 5, True), (64, 64, 0, 1, 10, True), (64, 64, 70, 3, 10, True), (96, 64, 130, 2, 10, True), (33, 0, 33, 1, 15, True),
+     (16, 64, 70, 1, 1, False), (5, 0, 64, 3, 1, False), (64, 64, 0, 16, 1, False)],
+)
+def test_latent_window_and_empty_splits(heads, rot, window, splits, reps, tc, extras, monkeypatch):
     """Rows in front of a window and behind the last key hold NaN (pages that others have written since); splits without keys,
-    also with a sink and a gate per head, which belong to the merged row."""
+    also with a sink and a gate per head, which belong to the merged row; on both kernels."""
     torch.manual_seed(heads + window)
-    kv_lens, page, lat, dim, vdim = [1, 63, 64, 65, 0, 129, 200, 511, 1000, 77, 96, 270], 16, 512, 128, 128
+    kv_lens, page, lat, dim, vdim = [1, 63, 64, 65, 0, 129, 200, 511, 1000, 77, 96, 270] * reps, 16, 512, 128, 128
     n = len(kv_lens)
     per = [(x + page - 1) // page for x in kv_lens]
     table, at = torch.zeros(n, max(per), dtype=torch.int32), 1
@@ -329,22 +335,49 @@ def test_latent_window_and_empty_splits(heads, rot, window, splits, extras, monk
     for i, (x, m) in enumerate(zip(kv_lens, per)):
         rows = (table[i, :m].long()[:, None] * page + torch.arange(page)).flatten().to(DEV)
         cache[rows[x:]] = float("nan")
-        if window:
-            cache[rows[: max(0, x - window)]] = float("nan")
+        if window:  # (the mma.sync kernel reads the tile of 32 keys that a window begins in)
+            first = max(0, x - window)
+            cache[rows[: first if tc else first // 32 * 32]] = float("nan")
     pos = torch.tensor([max(x - 1, 0) for x in kv_lens], dtype=torch.int32, device=DEV)
     meta = R.AttnMeta(torch.arange(n + 1, dtype=torch.int32, device=DEV), torch.tensor(kv_lens, dtype=torch.int32, device=DEV), table.to(DEV), pos, pos, page, n, n, 1, max(kv_lens), True,
                       list(range(n + 1)), kv_lens)
     q = torch.randn(n, heads * (dim + rot), device=DEV).bfloat16()
     uk_t, uv = (torch.randn(heads, 512, 128, device=DEV) * 0.05).bfloat16(), (torch.randn(heads, vdim, lat, device=DEV) * 0.05).bfloat16()
+    q[2] *= 8  # scores that pass the reference value by far in a later tile
     a = torch.randn(2048, max(rot // 2, 1), device=DEV)
     more = dict(head_gate=torch.randn(n, heads, device=DEV).bfloat16(), sink=torch.randn(heads, device=DEV)) if extras else {}
     monkeypatch.setattr(cu(), "_latent_splits", lambda *a: splits)
+    monkeypatch.setattr(cu(), "_latent_tc", lambda *a: tc)
     args = (uk_t, uv, None)
     got = cu().latent_attention(q, *args, cache.view(at, -1), meta, rot, 0.07, window, a.cos(), a.sin(), **more)
     want = R.latent_attention(q, *args, torch.nan_to_num(cache).view(at, -1), meta, rot, 0.07, window, a.cos(), a.sin(), **more)
     assert not got[4].any() and torch.isfinite(got.float()).all()
     # weights and outputs of both are rounded to bf16 (2^-8 each), the sums are of some hundred terms: 2^-6 of the largest
     assert (got.float() - want.float()).abs().max() <= 2 ** -6 * want.float().abs().max()
+    assert cu().read_status(DEV) == 0
+
+
+@pytest.mark.parametrize("lens,past,heads,tc", [([1] * 8, 31, 16, False), ([1] * 8, 32, 16, True), ([1] * 150, 100, 16, False), ([1] * 150, 130, 16, True), ([1] * 150, 95, 64, False), ([1] * 150, 96, 64, True),
+                                                 ([80], 0, 16, False), ([90], 0, 16, True), ([1] * 60 + [1], 7, 16, False), ([300] * 3, 0, 32, True)])
+def test_latent_kernels_where_the_rule_changes(lens, past, heads, tc, monkeypatch):
+    """The rows on either side of each line of the rule, on the kernel that it names, against the restatement."""
+    torch.manual_seed(past + heads)
+    monkeypatch.setattr(cu(), "_PREFILL_TC", False)
+    n, page, kv_lens = len(lens), 16, [x + past for x in lens]
+    qi = torch.tensor([0] + lens).cumsum(0)
+    per = max((x + page - 1) // page for x in kv_lens)
+    table = torch.randperm(n * per).view(n, per).to(torch.int32).to(DEV)
+    pos = torch.cat([torch.arange(past, x) for x in kv_lens]).to(torch.int32).to(DEV)
+    t, decode = sum(lens), max(lens) == 1
+    meta = R.AttnMeta(qi.to(torch.int32).to(DEV), torch.tensor(kv_lens, dtype=torch.int32, device=DEV), table, pos, pos, page, n, t, max(lens), max(kv_lens), decode, qi.tolist(), kv_lens)
+    assert cu()._latent_tc(t, heads, 512, 64, cu()._latent_keys(meta), decode, 148) == tc
+    cache = torch.randn(n * per, page, 576, device=DEV).bfloat16()
+    q = torch.randn(t, heads, 192, device=DEV).bfloat16()
+    uk, uv = (torch.randn(heads, 128, 512, device=DEV) * 0.05).bfloat16(), (torch.randn(heads, 128, 512, device=DEV) * 0.05).bfloat16()
+    cos, sin = R.rope_tables(2048, 64, 1e4, torch.bfloat16, DEV)
+    got = cu().mla_attention(cu().mla_rope_q(q, cos, sin, meta, 128), uk, uv, cache, meta, 0.07, 512)
+    want = R.mla_attention(R.mla_rope_q(q, cos, sin, meta, 128), uk, uv, cache, meta, 0.07, 512)
+    assert (got.float() - want.float()).abs().max() <= 2 ** -6 * want.float().abs().max()  # as above
     assert cu().read_status(DEV) == 0
 
 
