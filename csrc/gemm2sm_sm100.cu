@@ -503,7 +503,9 @@ static int gemm2sm_impl(const void* x, const void* w, void* y, int T, int M, int
   p.kblocks = ceil_div(K, BK);
   // Token-tile width, and ranges of k for the tiles of the last round where it leaves most pairs idle: least time on the busiest
   // pair.  A k-block costs about (width + 256): the MMA time follows the width, the 128 weight rows per CTA and the hand-offs do
-  // not.  Cutting tiles costs as much as CUT_KBLOCKS k-blocks (10 us: partial sums out and in again).
+  // not.  Cutting tiles costs as much as CUT_KBLOCKS k-blocks (10 us: partial sums out and in again).  A few wide tiles that run alone
+  // behind whole rounds take less than a round (T x M x K = 256 x 19456 x 2560, two of 76 tiles: 38 us whole, 42 cut in four; narrow
+  // ones, 128 x 19456 x 2560: 35 whole, 31 cut; 842 x 5120 x 5120, 20 k-blocks instead of 80: 55 whole and 51 cut).
   {
     constexpr int CUT_KBLOCKS = 25;
     long long best_cost = -1;
@@ -514,7 +516,8 @@ static int gemm2sm_impl(const void* x, const void* w, void* y, int T, int M, int
           if (rem == 0 || rem * s > di.max_pairs || p.kblocks < 8 * s) break;
           if (sc.ws == nullptr || sc.counters == nullptr || (((uintptr_t)sc.ws) & 15) != 0 || rem * s * 2 * bn * BM * 4 > sc.ws_bytes || rem * 2 * EPI_WARPS * 4 > sc.counter_bytes) break;
         }
-        const long long cost = (rounds * p.kblocks + (rem == 0 ? 0 : s == 1 ? p.kblocks : (p.kblocks + s - 1) / s + CUT_KBLOCKS)) * (bn + 256);
+        const long long whole = rounds > 0 && bn > 192 && 4 * rem <= di.max_pairs ? p.kblocks * 4 / 5 : p.kblocks;
+        const long long cost = (rounds * p.kblocks + (rem == 0 ? 0 : s == 1 ? whole : (p.kblocks + s - 1) / s + CUT_KBLOCKS)) * (bn + 256);
         if (best_cost < 0 || cost < best_cost) {
           best_cost = cost;
           p.bn = bn;
