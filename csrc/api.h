@@ -64,6 +64,7 @@ int pg_ipc_close(void* p);
 // routes eligible problems to it (PEGAINFER_GEMM_2SM=0 turns that off).
 int pg_gemm2sm_takes(int T, int M, int K);
 int pg_gemm2sm_eligible(int T, int M, int K);
+int pg_gemm2sm_plan(int T, int M, int K, long long ws_bytes, int* out);
 int pg_gemm2sm_bf16_tn(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, void* ws, long long ws_bytes, void* counters, long long counter_bytes, void* status,
                        cudaStream_t stream);
 int pg_gemm2sm_bf16_tn_swiglu(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, int gelu, void* ws, long long ws_bytes, void* counters, long long counter_bytes, void* status,

@@ -436,7 +436,15 @@ struct Scratch2 {
   long long counter_bytes;
 };
 static int gemm2sm_impl(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, const Scratch2& sc, void* status, int epi, cudaStream_t stream,
-                        const void* xielu = nullptr);
+                        const void* xielu = nullptr, int* plan_out = nullptr);
+
+// How a problem would be launched on the current device with `ws_bytes` of scratch: out = {token-tile width, whole tiles, cut tiles, ranges
+// of k of a cut tile}.
+extern "C" int pg_gemm2sm_plan(int T, int M, int K, long long ws_bytes, int* out) {
+  PG_REQUIRE(out != nullptr, "gemm2sm plan: null output");
+  void* fake = reinterpret_cast<void*>(uintptr_t(256));
+  return gemm2sm_impl(fake, fake, fake, T, M, K, K, K, M, {fake, ws_bytes, fake, 1ll << 40}, fake, 0, nullptr, nullptr, out);
+}
 
 // ws, counters: scratch as for pg_gemm_bf16_tn (null: no tile is cut)
 extern "C" int pg_gemm2sm_bf16_tn(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, void* ws, long long ws_bytes, void* counters,
@@ -458,10 +466,10 @@ extern "C" int pg_gemm2sm_bf16_tn_xielu(const void* x, const void* w, void* y, i
 }
 
 static int gemm2sm_impl(const void* x, const void* w, void* y, int T, int M, int K, long long ldx, long long ldw, long long ldy, const Scratch2& sc, void* status, int epi, cudaStream_t stream,
-                        const void* xielu) {
+                        const void* xielu, int* plan_out) {
   PG_REQUIRE(T > 0 && M > 0 && K > 0 && K % 8 == 0, "gemm2sm: bad problem %dx%dx%d", T, M, K);
   PG_REQUIRE(status != nullptr, "gemm2sm: a device status word is required");
-  pg_gemm_prefetch_next(nullptr, 0);  // a hint was for this GEMM, which has no use for it: it must not outlive the weights it names
+  if (plan_out == nullptr) pg_gemm_prefetch_next(nullptr, 0);  // a hint was for this GEMM, which has no use for it: it must not outlive the weights it names
   int dev = 0;
   PG_CUDA(cudaGetDevice(&dev));
   Dev2& di = g_dev2[dev & 63];
@@ -530,6 +538,10 @@ static int gemm2sm_impl(const void* x, const void* w, void* y, int T, int M, int
   const int total = p.m_pairs * p.n_tiles;
   p.rem = p.splits > 1 ? total % di.max_pairs : 0;
   p.whole = total - p.rem;
+  if (plan_out != nullptr) {
+    plan_out[0] = p.bn, plan_out[1] = p.whole, plan_out[2] = p.rem, plan_out[3] = p.splits;
+    return PG_OK;
+  }
   p.part = (float4*)sc.ws;
   p.counters = (uint32_t*)sc.counters;
   const int stage_bytes = A_BYTES + (p.bn / 2) * 128;

@@ -88,7 +88,7 @@ def trace_calls(module=None):
     trace = CallTrace()
     gpu = module.__name__.endswith(".cuda") and torch.cuda.is_available()
     saved = {}
-    skip = {"ctx", "lib", "launch_count", "read_status", "clear_status", "gemm_plan", "fused_plan_ok", "plan_decode_splits", "set_batch_invariant", "batch_invariant", "prefetch_weights", "quant_code", "paired_int4",
+    skip = {"ctx", "lib", "launch_count", "read_status", "clear_status", "gemm_plan", "gemm2sm_plan", "fused_plan_ok", "plan_decode_splits", "set_batch_invariant", "batch_invariant", "prefetch_weights", "quant_code", "paired_int4",
             "rope_tables"}
     for name, fn in list(vars(module).items()):
         if name.startswith("_") or name in skip or not inspect.isfunction(fn) or fn.__module__ != module.__name__:

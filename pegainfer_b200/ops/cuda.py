@@ -561,6 +561,13 @@ def gemm_plan(t: int, m: int, k: int, force_splits: int = 0) -> dict:
     return dict(zip(("bn", "splits", "cluster", "grid", "stages", "max_clusters"), list(out)))
 
 
+def gemm2sm_plan(t: int, m: int, k: int) -> dict:
+    """Launch plan of the two-SM GEMM for a problem size on the current device."""
+    out = (ctypes.c_int * 4)()
+    _check(lib().pg_gemm2sm_plan(_ci(t), _ci(m), _ci(k), _ll(GEMM_WS_BYTES), out), None)
+    return dict(zip(("bn", "whole", "rem", "splits"), list(out)))
+
+
 def qk_norm_rope_append(qkv, q_norm_w, k_norm_w, cos, sin, meta: AttnMeta, kv_layer, num_q_heads, num_kv_heads, head_dim, eps, offset=False, gated=False, v_norm=False):
     _bf16(qkv)
     t = qkv.shape[0]

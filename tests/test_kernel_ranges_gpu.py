@@ -249,10 +249,18 @@ def test_gated_delta_chunks_in_segments(lens, room, dv, monkeypatch):
     assert (runs[0][1] - want_s).abs().max() < 0.03 * want_s.abs().max()
 
 
-@pytest.mark.parametrize("t,m,k", [(257, 1024, 2048), (1337, 4096, 1024), (700, 5008, 1096), (4100, 4112, 512), (300, 1280, 8704), (1200, 1504, 776)])
-def test_two_sm_gemm_cuts_the_last_round(t, m, k):
+@pytest.mark.parametrize(
+    "t,m,k,splits,rounds",
+    # whole tiles only; cut tiles alone, in two, three and four ranges, some of them uneven, m and t ragged; cut tiles behind a whole round
+    [(257, 1024, 2048, 1, 0), (1337, 4096, 1024, 1, 1), (700, 5008, 1096, 1, 0), (4100, 4112, 512, 1, 3), (1200, 1504, 776, 1, 0), (300, 1280, 8704, 4, 0), (65, 528, 4104, 4, 0), (300, 4096, 4096, 2, 0),
+     (512, 2576, 4104, 3, 0), (1290, 4112, 8200, 2, 1), (1100, 4096, 12288, 3, 1), (842, 5136, 5128, 4, 1)],
+)
+def test_two_sm_gemm_cuts_the_last_round(t, m, k, splits, rounds):
     """Tiles of the last round cut in ranges of k: a few tiles only, tiles behind whole rounds, ragged edges, uneven ranges."""
     K = cu()
+    plan = K.gemm2sm_plan(t, m, k)
+    # with 72 or 74 pairs at once; the rule's lines may move, the ranges that they are to reach may not go untested
+    assert plan["splits"] == splits and (plan["whole"] > 0) == (rounds > 0 or splits == 1), plan
     torch.manual_seed(m)
     x, w = torch.randn(t, k + 8, device=DEV).bfloat16()[:, :k], torch.randn(m, k, device=DEV).bfloat16()
     want = x.double() @ w.double().t()
