@@ -25,6 +25,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <climits>
 #include <mutex>
 
 #include "api.h"
@@ -416,16 +417,25 @@ static bool gemm2sm_enabled() {
   return g_enabled == 1;
 }
 
+// PEGAINFER_GEMM_2SM_MAXK: longest k of the two-SM kernel; `otherwise` where it is not set
+static int gemm2sm_max_k(int otherwise) {
+  static const int limit = [] {
+    const char* e = getenv("PEGAINFER_GEMM_2SM_MAXK");
+    return e ? atoi(e) : 0;
+  }();
+  return limit > 0 ? limit : otherwise;
+}
+
 // 1 if the two-SM kernel takes this problem in a GEMM with bf16 results: above the 64 rows of the decode plans it measured faster
 // than the one-CTA kernel at every size.  Us there -> here: T = 65, M x K = 1024 x 1024 20 -> 11, 4096 x 12288 58 -> 34; T = 256,
 // 64 x 512 20 -> 9, 5120 x 17408 109 -> 57; T = 1100, 4096 x 12288 144 -> 101; T = 4096, 4096 x 12288 377 -> 280.  At 64 rows and
 // below the one-CTA kernel's narrow tiles win (4096 x 4096: 14, here 19).
-extern "C" int pg_gemm2sm_takes(int T, int M, int K) { return gemm2sm_enabled() && T > 64 && M >= 64 && K >= 256 && K % 8 == 0 ? 1 : 0; }
+extern "C" int pg_gemm2sm_takes(int T, int M, int K) { return gemm2sm_enabled() && T > 64 && M >= 64 && K >= 256 && K <= gemm2sm_max_k(INT_MAX) && K % 8 == 0 ? 1 : 0; }
 
 // 1 for the problems whose f32 results callers leave to a bf16 GEMM on this kernel (at least about a round of CTA pairs, k up to
 // 8192): a narrower set than pg_gemm2sm_takes, so that no other results lose their 32 bits.
 extern "C" int pg_gemm2sm_eligible(int T, int M, int K) {
-  if (!gemm2sm_enabled() || T < 256 || M < 1024 || K < 256 || K > 8192 || K % 8 != 0) return 0;
+  if (!gemm2sm_enabled() || T < 256 || M < 1024 || K < 256 || K > gemm2sm_max_k(8192) || K % 8 != 0) return 0;
   return (long long)ceil_div(M, 2 * BM) * ceil_div(T, 256) >= 64 ? 1 : 0;
 }
 

@@ -1,5 +1,9 @@
 """Kernels at the edges of the ranges that their launch rules draw: tile and segment edges, remainders, odd widths, the
 smallest and largest sizes, against the PyTorch restatements."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -454,3 +458,11 @@ def test_kda_rows_beside_prompts(lens, known):
         else:  # beside rows of five tokens and more the sums of a column are formed in another order: f32, then one rounding to bf16
             assert (out[rows].float() - y.float()).abs().max() <= 2 ** -8 * y.float().abs().max() + 1e-5
             assert (s[slot] - alone[slot]).abs().max() <= 2 ** -17 * alone[slot].abs().max()
+
+
+@pytest.mark.parametrize("switch,takes", [({}, "11"), ({"PEGAINFER_GEMM_2SM_MAXK": "8192"}, "10"), ({"PEGAINFER_GEMM_2SM_MAXK": "0"}, "11"), ({"PEGAINFER_GEMM_2SM": "0"}, "00")])
+def test_two_sm_gemm_switches(switch, takes):
+    """The two-SM kernel's switches, read once per process: off, and the longest k that it takes."""
+    code = "from pegainfer_b200 import _native as n; print(n.load().pg_gemm2sm_takes(100, 1024, 8192), n.load().pg_gemm2sm_takes(100, 1024, 8256), sep='')"
+    env = {k: v for k, v in os.environ.items() if not k.startswith("PEGAINFER_GEMM_2SM")}
+    assert subprocess.run([sys.executable, "-c", code], env=env | switch, capture_output=True, text=True, timeout=300).stdout.strip() == takes
