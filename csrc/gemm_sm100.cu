@@ -1266,11 +1266,15 @@ extern "C" void pg_tp_set_timing(void* buf) { g_tp_timing = (unsigned long long*
 // One to four token rows: a stream of weight rows (decode_rows.cu) where sizes and alignment allow it; false: not launched.
 // One row, us on the tile kernel -> here: 4096 x 4096 12.2 -> 8.2, 151936 x 4096 201 -> 186, 1024 x 3072 6.9 -> 3.6; four rows:
 // 12.2 -> 10.1, 201 -> 188, 6.9 -> 4.5.  The tile kernel keeps several rows of long k, which every block reads before its first
-// product (four rows of 4096 x 12288: 22.3, here 25.1), and two rows of the largest matrices (151936 x 4096: 201, here 225).
+// product (four rows of 4096 x 12288: 22.6, here 24.3), and sizes at which the streams of several rows fall behind: two rows of the
+// largest matrices (151936 x 4096: 212, here 232; 151936 x 2560: 127, here 143), three rows of some hundred million weights (24576 x 4096: 39.5, here
+// 41.2; 37984 x 4096: 60.3, here 61.8; 34816 x 5120 and 151936 x 1024: 61.8, 57.5, here 60.2, 51.0), three and four of a thousand million
+// (248320 x 5120: 381, here 450 and 396).
 static bool try_decode_rows(const void* x, const void* w, void* y, int y_is_f32, int T, int M, int K, long long ldx, long long ldw, long long ldy, int epi, const void* in_ssp, int in_parts, int in_ld,
                             int in_width, float in_eps, void* status, cudaStream_t stream, int* rc) {
   if (T < 1 || T > DR_MAX_ROWS || x == nullptr || w == nullptr || y == nullptr || status == nullptr) return false;
-  if ((T > 1 && K > 8192) || (T == 2 && (long long)M * K > 100'000'000)) return false;
+  const long long weights = (long long)M * K;
+  if ((T > 1 && K > 8192) || (T == 2 && weights > 100'000'000) || (T == 3 && K > 1024 && weights > 90'000'000 && weights < 170'000'000) || (T > 2 && weights > 1'000'000'000)) return false;
   DecodeRows r;
   memset(&r, 0, sizeof(r));
   r.nphase = 1;
