@@ -120,64 +120,82 @@ __global__ void __launch_bounds__(256) rms_norm_kernel(const bf16* __restrict__ 
 
 // Per (token, head): y = rms_norm(x, w_f32) * silu(gate); one warp per head row.
 // act 0: rms_norm(x) * w * silu(gate), rounded once; act 1: bf16(rms_norm(x) * w) * bf16(sigmoid(gate))
-// Rows (token, head) of `dim` = 32 VEC elements (VEC = 0: any size), GN_ROWS of them per warp with their loads in flight
-// together.  Gate rows of a token start ld_gate apart, so a column slice of a fused projection is read where it lies.  Bound by
+// Rows (token, head) of `dim` = 32 VEC elements, N of them per warp with their loads in flight together: GN_ROWS where there are
+// many rows, one where there are few, since the chain of a warp's rows is what a short launch waits for (16 x 48 x 128 1.8 us with
+// four, 1.3 with one; 200 x 48 x 128 3.1, 2.8; 400 x 48 x 128 3.5, 5.4; of 256 elements 100 x 16 2.7, 2.4; 300 x 16 3.7, 4.2).  Gate rows of a
+// token start ld_gate apart, so a column slice of a fused projection is read where it lies.  Bound by
 // the rows: 2777 x 48 x 128 took 41 us with a warp per row (39 us with 8-byte accesses: the lives of 133 K warps) and 44 us for
-// a dense copy of the gate in front of it; 30 us now.
+// a dense copy of the gate in front of it; 30 us from a slice, 20 from a dense gate, whose rows need no division.
 constexpr int GN_ROWS = 4;
-template <int VEC>
+template <int VEC, int N>
 __global__ void __launch_bounds__(128) gated_rms_norm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gate, long long ld_gate, const float* __restrict__ w, bf16* __restrict__ y,
                                                              unsigned rows, unsigned heads, int dim, float eps, int act) {
   PG_PDL_ENTRY();
-  constexpr int N = VEC > 0 ? GN_ROWS : 1;
   const unsigned row0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * N;
   if (row0 >= rows) return;
   const int lane = threadIdx.x & 31;
-  auto gate_row = [&](unsigned row) { return gate + (row / heads) * ld_gate + (long long)(row % heads) * dim; };
+  const bool dense = ld_gate == (long long)heads * dim;  // (a division is a good part of a short row's work)
+  auto gate_row = [&](unsigned row) { return dense ? gate + (long long)row * dim : gate + (row / heads) * ld_gate + (long long)(row % heads) * dim; };
   auto finish = [&](float v, float g, float inv, float wi) {
     if (act == 1) return bf16_round(v * inv * wi) * bf16_round(1.f / (1.f + __expf(-g)));
     return v * inv * wi * (g / (1.f + __expf(-g)));
   };
-  if constexpr (VEC > 0) {
-    struct alignas(2 * VEC) Pack {
-      bf16 e[VEC];
-    };
-    Pack xv[N], gv[N];
-    float wv[VEC];
+  struct alignas(2 * VEC) Pack {
+    bf16 e[VEC];
+  };
+  Pack xv[N], gv[N];
+  float wv[VEC];
 #pragma unroll
-    for (int n = 0; n < N; ++n)
-      if (row0 + n < rows) {
-        xv[n] = reinterpret_cast<const Pack*>(x + (long long)(row0 + n) * dim)[lane];
-        gv[n] = reinterpret_cast<const Pack*>(gate_row(row0 + n))[lane];
-      }
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) wv[i] = w[lane * VEC + i];
-#pragma unroll
-    for (int n = 0; n < N; ++n) {
-      if (row0 + n >= rows) break;
-      float v[VEC], ss = 0.f;
-#pragma unroll
-      for (int i = 0; i < VEC; ++i) {
-        v[i] = __bfloat162float(xv[n].e[i]);
-        ss += v[i] * v[i];
-      }
-      ss = warp_sum(ss);
-      const float inv = rsqrtf(ss / (float)dim + eps);
-      Pack o;
-#pragma unroll
-      for (int i = 0; i < VEC; ++i) o.e[i] = __float2bfloat16(finish(v[i], __bfloat162float(gv[n].e[i]), inv, wv[i]));
-      reinterpret_cast<Pack*>(y + (long long)(row0 + n) * dim)[lane] = o;
+  for (int n = 0; n < N; ++n)
+    if (row0 + n < rows) {
+      xv[n] = reinterpret_cast<const Pack*>(x + (long long)(row0 + n) * dim)[lane];
+      gv[n] = reinterpret_cast<const Pack*>(gate_row(row0 + n))[lane];
     }
-  } else {
-    const bf16 *xr = x + (long long)row0 * dim, *gr = gate_row(row0);
-    float ss = 0.f;
-    for (int i = lane; i < dim; i += 32) {
-      const float v = __bfloat162float(xr[i]);
-      ss += v * v;
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) wv[i] = w[lane * VEC + i];
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    if (row0 + n >= rows) break;
+    float v[VEC], ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+      v[i] = __bfloat162float(xv[n].e[i]);
+      ss += v[i] * v[i];
     }
     ss = warp_sum(ss);
     const float inv = rsqrtf(ss / (float)dim + eps);
-    for (int i = lane; i < dim; i += 32) y[(long long)row0 * dim + i] = __float2bfloat16(finish(__bfloat162float(xr[i]), __bfloat162float(gr[i]), inv, w[i]));
+    Pack o;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) o.e[i] = __float2bfloat16(finish(v[i], __bfloat162float(gv[n].e[i]), inv, wv[i]));
+    reinterpret_cast<Pack*>(y + (long long)(row0 + n) * dim)[lane] = o;
+  }
+}
+
+// Rows of any size and alignment, one per warp
+__global__ void gated_rms_norm_any_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gate, long long ld_gate, const float* __restrict__ w, bf16* __restrict__ y, long long rows, unsigned heads, int dim,
+                                          float eps, int act) {
+  PG_PDL_ENTRY();
+  const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int lane = threadIdx.x & 31;
+  const bf16* xr = x + row * dim;
+  const bf16* gr = ld_gate == (long long)heads * dim ? gate + row * dim : gate + (unsigned)row / heads * ld_gate + (long long)((unsigned)row % heads) * dim;
+  float ss = 0.f;
+  for (int i = lane; i < dim; i += 32) {
+    float v = __bfloat162float(xr[i]);
+    ss += v * v;
+  }
+  ss = warp_sum(ss);
+  const float inv = rsqrtf(ss / (float)dim + eps);
+  for (int i = lane; i < dim; i += 32) {
+    float v = __bfloat162float(xr[i]);
+    float g = __bfloat162float(gr[i]);
+    if (act == 1) {
+      y[row * dim + i] = __float2bfloat16(bf16_round(v * inv * w[i]) * bf16_round(1.f / (1.f + __expf(-g))));
+      continue;
+    }
+    float s = g / (1.f + __expf(-g));
+    y[row * dim + i] = __float2bfloat16(v * inv * w[i] * s);
   }
 }
 
@@ -509,8 +527,16 @@ extern "C" int pg_gated_rms_norm_act(const void* x, const void* gate, long long 
   if (rows == 0) return PG_OK;
   const int vec = dim == 128 ? 4 : dim == 256 ? 8 : dim == 64 ? 2 : 0;
   const bool aligned = vec && ld_gate % vec == 0 && (((uintptr_t)x | (uintptr_t)gate | (uintptr_t)y) & (2 * vec - 1)) == 0;
-  auto kernel = !aligned ? gated_rms_norm_kernel<0> : vec == 2 ? gated_rms_norm_kernel<2> : vec == 4 ? gated_rms_norm_kernel<4> : gated_rms_norm_kernel<8>;
-  const int per_block = 4 * (aligned ? GN_ROWS : 1);
+  const bool many = rows >= (vec == 8 ? 2400 : 12000);
+  if (!aligned) {
+    PG_CUDA(launch_pdl(gated_rms_norm_any_kernel, dim3((unsigned)((rows + 3) / 4)), dim3(128), (size_t)(0), stream, (const bf16*)x, (const bf16*)gate, ld_gate, (const float*)w_f32, (bf16*)y, rows, (unsigned)heads, dim, eps,
+                       act));
+    PG_LAUNCH_CHECK();
+    return PG_OK;
+  }
+  auto kernel = many ? (vec == 2 ? gated_rms_norm_kernel<2, GN_ROWS> : vec == 4 ? gated_rms_norm_kernel<4, GN_ROWS> : gated_rms_norm_kernel<8, GN_ROWS>)
+                     : (vec == 2 ? gated_rms_norm_kernel<2, 1> : vec == 4 ? gated_rms_norm_kernel<4, 1> : gated_rms_norm_kernel<8, 1>);
+  const int per_block = 4 * (many ? GN_ROWS : 1);
   PG_CUDA(launch_pdl(kernel, dim3((unsigned)((rows + per_block - 1) / per_block)), dim3(128), (size_t)(0), stream, (const bf16*)x, (const bf16*)gate, ld_gate, (const float*)w_f32, (bf16*)y, (unsigned)rows, (unsigned)heads, dim,
                      eps, act));
   PG_LAUNCH_CHECK();

@@ -152,13 +152,14 @@ def test_latent_decode_tiles(heads, page, splits, monkeypatch):
 
 
 @pytest.mark.parametrize("dim,heads,act", [(128, 6, "silu"), (128, 5, "sigmoid"), (256, 3, "silu"), (64, 7, "silu"), (96, 3, "sigmoid")])
-def test_gated_norm_reads_the_gate_in_place(dim, heads, act):
+@pytest.mark.parametrize("t", [37, 4001])  # one row per warp and several, rows that do not fill the last block
+def test_gated_norm_reads_the_gate_in_place(dim, heads, act, t):
     torch.manual_seed(dim)
-    t = 37  # rows that do not fill the last block
     x = torch.randn(t, heads, dim, device=DEV).bfloat16()
     fused = torch.randn(t, heads * dim + 24, device=DEV).bfloat16()
     w = torch.rand(dim, device=DEV) + 0.5
-    for gate in (fused[:, 8 : 8 + heads * dim].reshape(t, heads, dim), fused[:, 1 : 1 + heads * dim].reshape(t, heads, dim)):  # 16-byte pieces; not even aligned
+    # 16-byte pieces; not even aligned; a dense gate
+    for gate in (fused[:, 8 : 8 + heads * dim].view(t, heads, dim), fused[:, 1 : 1 + heads * dim].view(t, heads, dim), fused[:, 8 : 8 + heads * dim].reshape(t, heads * dim).view(t, heads, dim)):
         got, want = cu().gated_rms_norm(x, gate, w, 1e-6, act), R.gated_rms_norm(x, gate, w, 1e-6, act)
         # f32 sums in another order: one step of bf16, two where two rounded factors meet
         assert ((got.float() - want.float()).abs() <= 2 ** -7 * want.float().abs() + 1e-6).all()
