@@ -249,18 +249,21 @@ __global__ void softcap_kernel(const bf16* __restrict__ x, bf16* __restrict__ y,
     y[i] = __float2bfloat16(tanhf(__bfloat162float(x[i]) * inv) * cap);
 }
 
+// PIECES: `vecs` 16-byte pieces, then the rest
+template <bool PIECES>
 __global__ void sigmoid_gate_mul_kernel(bf16* __restrict__ x, const bf16* __restrict__ gate, long long n, long long vecs) {
   PG_PDL_ENTRY();
-  // `vecs` 16-byte pieces, then the rest
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += (long long)gridDim.x * blockDim.x) {
-    float xf[8], gf[8];
-    unpack8(reinterpret_cast<const bf16x8*>(x)[i], xf);
-    unpack8(reinterpret_cast<const bf16x8*>(gate)[i], gf);
+  if constexpr (PIECES) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += (long long)gridDim.x * blockDim.x) {
+      float xf[8], gf[8];
+      unpack8(reinterpret_cast<const bf16x8*>(x)[i], xf);
+      unpack8(reinterpret_cast<const bf16x8*>(gate)[i], gf);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) xf[j] = xf[j] / (1.f + __expf(-gf[j]));
-    reinterpret_cast<bf16x8*>(x)[i] = pack8(xf);
+      for (int j = 0; j < 8; ++j) xf[j] = xf[j] / (1.f + __expf(-gf[j]));
+      reinterpret_cast<bf16x8*>(x)[i] = pack8(xf);
+    }
+    x += vecs * 8, gate += vecs * 8, n -= vecs * 8;
   }
-  x += vecs * 8, gate += vecs * 8, n -= vecs * 8;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     float g = __bfloat162float(gate[i]);
     x[i] = __float2bfloat16(__bfloat162float(x[i]) / (1.f + __expf(-g)));
@@ -571,10 +574,11 @@ extern "C" int pg_softcap(const void* x, void* y, long long n, float cap, cudaSt
 
 extern "C" int pg_sigmoid_gate_mul(void* x, const void* gate, long long n, cudaStream_t stream) {
   if (n == 0) return PG_OK;
-  const long long vecs = (((uintptr_t)x | (uintptr_t)gate) & 15) == 0 ? n / 8 : 0;
+  // (below some ten thousand elements, one to a thread is as fast: 7 x 6144 1.33 us, in pieces 1.45)
+  const long long vecs = n >= 65536 && (((uintptr_t)x | (uintptr_t)gate) & 15) == 0 ? n / 8 : 0;
   long long blocks = ((vecs ? vecs : n) + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  PG_CUDA(launch_pdl(sigmoid_gate_mul_kernel, dim3((int)blocks), dim3(256), (size_t)(0), stream, (bf16*)x, (const bf16*)gate, n, vecs));
+  PG_CUDA(launch_pdl(vecs ? sigmoid_gate_mul_kernel<true> : sigmoid_gate_mul_kernel<false>, dim3((int)blocks), dim3(256), (size_t)(0), stream, (bf16*)x, (const bf16*)gate, n, vecs));
   PG_LAUNCH_CHECK();
   return PG_OK;
 }
