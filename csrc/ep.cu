@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(128) ep_dispatch_kernel(const bf16* __restrict
 // One CTA: wait for all sources, then the same stable counting sort as moe_align over the
 // live part of the receive table (`live` routes per source; entries beyond that are left
 // over from larger steps and must not be read).  The table is written by peers, so it is
-// read past L1 (ld.cg) while being staged into shared memory.
+// read past L1 (ld.cg).
 __global__ void __launch_bounds__(ROUTE_SORT_THREADS) ep_align_kernel(const int* __restrict__ recv_ids, int world, int cap, int live, int e_local,
                                                                        int* __restrict__ offsets, int* __restrict__ sorted_src,
                                                                        const uint32_t* __restrict__ flags, unsigned long long wait_ns, uint32_t* status) {

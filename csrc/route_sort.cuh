@@ -3,11 +3,12 @@
 //
 // Routes arrive as a flat list of local expert ids (anything outside [0, e_local) means "not for this rank").  Every warp
 // owns one contiguous slice of the list and walks it 32 entries at a time: lanes with the same expert find each other by a
-// ballot per bit of the id (a warp match takes several times as long), the first of them moves the warp's counter of it.  A first walk counts, a scan over (expert, warp)
-// turns the counts into cursors, a second walk hands out positions, so the order inside an expert is the route order
-// (stable: the f32 summation order downstream never depends on scheduling).  Bound by the latency of the walks,
-// n / 512 steps each; with every warp scanning the whole list for its own experts instead, 10266 routes to 64 experts took
-// 140 us and 1024 routes 14 us; 20 us and 4.6 us now.
+// ballot per bit of the id (a warp match takes several times as long), the first of them moves the warp's counter of it.  A
+// first walk counts, a scan over (expert, warp) turns the counts into cursors, a second walk hands out positions, so the order
+// inside an expert is the route order (stable: the f32 summation order downstream never depends on scheduling).  Bound by the
+// latency of the walks, n / 512 steps each; with every warp scanning the whole list for its own experts instead, 10266 routes
+// to 64 experts took 140 us and 1024 routes 14 us; 20 us and 4.6 us now.  Up to 256 routes to at most 16 experts, a warp per
+// expert does scan the list, which it holds in registers (8 experts, 48 routes: 2.0 us, with slices 3.3).
 //
 // Takes the place of the reference's per-layer host-side routing bookkeeping and of the
 // align step of its Marlin MoE path (pegainfer-kernels/csrc/kimi_k2/kimi_marlin_wna16.cu
@@ -24,16 +25,15 @@ struct RouteSortSmem {
   int warp_total[ROUTE_SORT_WARPS];
 };
 
-// `load(i)` returns the local expert id of flat entry i (0 <= i < n); `emit(i, pos)` is called
-// once per entry with its position in the sorted order, or pos = -1 when the entry is not
-// for a local expert.  Writes offsets[0..e_local].  All ROUTE_SORT_THREADS threads call this.
-template <typename Load, typename Emit>
-__device__ __forceinline__ void route_sort(RouteSortSmem& sm, int n, int e_local, int* __restrict__ offsets, Load load, Emit emit) {
+// The sort by slices.  AHEAD: groups of 32 entries whose ids are loaded, and ranked, together; 1 for lists that may leave warps without
+// a slice (up to ROUTE_SORT_THREADS entries).
+template <int AHEAD, typename Load, typename Emit>
+__device__ __forceinline__ void route_sort_sliced(RouteSortSmem& sm, int n, int e_local, int* __restrict__ offsets, Load load, Emit emit) {
   static_assert(ROUTE_SORT_THREADS == ROUTE_SORT_EXPERTS, "the scan gives every expert a thread");
-  constexpr int AHEAD = 4;  // groups of 32 entries whose ids are loaded together
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int slice = ((n + ROUTE_SORT_WARPS - 1) / ROUTE_SORT_WARPS + 31) & ~31;
   const int i_begin = min(n, warp * slice), i_end = min(n, i_begin + slice);
+  const int used = AHEAD == 1 ? (n + 31) / 32 : ROUTE_SORT_WARPS;  // warps that are looked at
   int* cursor = sm.cursor[warp];
   const int bits = 32 - __clz(e_local - 1);  // of a local expert id (none for a single expert)
   // `place`: the second walk
@@ -65,13 +65,15 @@ __device__ __forceinline__ void route_sort(RouteSortSmem& sm, int n, int e_local
     }
   };
 #pragma unroll
-  for (int w = 0; w < ROUTE_SORT_WARPS; ++w) sm.cursor[w][tid] = 0;
+  for (int w = 0; w < ROUTE_SORT_WARPS; ++w)
+    if (w < used) sm.cursor[w][tid] = 0;
   __syncthreads();
   walk(false);
   __syncthreads();
   int total = 0;  // of expert `tid`
 #pragma unroll
-  for (int w = 0; w < ROUTE_SORT_WARPS; ++w) total += sm.cursor[w][tid];
+  for (int w = 0; w < ROUTE_SORT_WARPS; ++w)
+    if (w < used) total += sm.cursor[w][tid];
   int upto = total;  // inclusive scan over the experts
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -87,11 +89,54 @@ __device__ __forceinline__ void route_sort(RouteSortSmem& sm, int n, int e_local
   if (tid < e_local) offsets[tid] = at;
   if (tid == e_local - 1) offsets[e_local] = upto;
 #pragma unroll
-  for (int w = 0; w < ROUTE_SORT_WARPS; ++w) {
-    const int c = sm.cursor[w][tid];
-    sm.cursor[w][tid] = at;
-    at += c;
-  }
+  for (int w = 0; w < ROUTE_SORT_WARPS; ++w)
+    if (w < used) {
+      const int c = sm.cursor[w][tid];
+      sm.cursor[w][tid] = at;
+      at += c;
+    }
   __syncthreads();
   walk(true);
+}
+
+// `load(i)` returns the local expert id of flat entry i (0 <= i < n); `emit(i, pos)` is called
+// once per entry with its position in the sorted order, or pos = -1 when the entry is not
+// for a local expert.  Writes offsets[0..e_local].  All ROUTE_SORT_THREADS threads call this.
+template <typename Load, typename Emit>
+__device__ __forceinline__ void route_sort(RouteSortSmem& sm, int n, int e_local, int* __restrict__ offsets, Load load, Emit emit) {
+  constexpr int FEW = 8;  // groups of 32 entries that a warp holds
+  if (n > ROUTE_SORT_THREADS) {
+    route_sort_sliced<4>(sm, n, e_local, offsets, load, emit);
+    return;
+  }
+  if (e_local > ROUTE_SORT_WARPS || n > 32 * FEW) {
+    route_sort_sliced<1>(sm, n, e_local, offsets, load, emit);
+    return;
+  }
+  // few routes and experts: a warp per expert, which reads the whole list
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int id[FEW], count = 0;
+  uint32_t mine[FEW];
+#pragma unroll
+  for (int a = 0; a < FEW; ++a) id[a] = 32 * a + lane < n ? load(32 * a + lane) : -1;
+#pragma unroll
+  for (int a = 0; a < FEW; ++a) {
+    mine[a] = __ballot_sync(0xffffffffu, warp < e_local && id[a] == warp);
+    count += __popc(mine[a]);
+  }
+  if (lane == 0) sm.warp_total[warp] = count;
+  __syncthreads();
+  int at = 0;
+#pragma unroll
+  for (int w = 0; w < ROUTE_SORT_WARPS; ++w)
+    if (w < warp) at += sm.warp_total[w];
+  if (lane == 0 && warp < e_local) offsets[warp] = at;
+  if (lane == 0 && warp == e_local - 1) offsets[e_local] = at + count;
+#pragma unroll
+  for (int a = 0; a < FEW; ++a) {
+    const int i = 32 * a + lane;
+    if (mine[a] >> lane & 1u) emit(i, at + __popc(mine[a] & ((1u << lane) - 1u)));
+    if (warp == a && i < n && (id[a] < 0 || id[a] >= e_local)) emit(i, -1);
+    at += __popc(mine[a]);
+  }
 }

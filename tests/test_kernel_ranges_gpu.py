@@ -28,7 +28,7 @@ def test_gdn_conv1d_segments(channels, taps):
     assert torch.equal(st1, st2)
 
 
-@pytest.mark.parametrize("routes,e0,e_local,total", [(1, 0, 1, 1), (31, 0, 3, 5), (512, 8, 64, 96), (513, 0, 384, 384), (8193, 16, 48, 384), (40007, 0, 512, 512)])
+@pytest.mark.parametrize("routes,e0,e_local,total", [(1, 0, 1, 1), (31, 0, 3, 5), (256, 3, 16, 40), (255, 0, 16, 16), (257, 3, 16, 40), (200, 5, 17, 30), (100, 0, 1, 4), (512, 8, 64, 96), (513, 0, 384, 384), (8193, 16, 48, 384), (40007, 0, 512, 512)])
 def test_route_sort_is_stable(routes, e0, e_local, total):
     g = torch.Generator().manual_seed(routes)
     ids = torch.randint(0, total, (routes, 1), generator=g, dtype=torch.int32)
