@@ -22,16 +22,19 @@
 
 namespace {
 
-// Bound by the rows it reads and writes.  A thread owns VEC adjacent channels and CONV_SEG tokens of a sequence and reads the
+// Bound by the rows it reads and writes.  A thread owns VEC adjacent channels and `seg` tokens of a sequence and reads the
 // K - 1 rows in front of its segment again, so a prompt spreads over tokens as well as channels (one thread per channel
 // walking all of a prompt's tokens took 968 us for 2777 x 10240; 49 us now, 114 MB read and written;
 // 32 decode rows 6.6 us before, 5.8 now).  The block of a sequence's
 // first segment is the only one that touches the carried inputs: it reads them, and leaves the sequence's last K - 1 inputs.
+// Segments have CONV_SEG tokens; beside many sequences, whose blocks behind their last segment are launched for nothing,
+// twice as many until at most CONV_BLOCKS blocks are.
 constexpr int CONV_SEG = 16;
+constexpr long long CONV_BLOCKS = 16384;
 template <int VEC>
 __global__ void __launch_bounds__(128) gdn_conv1d_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ w, bf16* __restrict__ state,
                                                          bf16* __restrict__ out, long long ldo, const int* __restrict__ q_indptr, const int* __restrict__ slots,
-                                                         int channels, int K, long long state_slot_stride) {
+                                                         int channels, int K, long long state_slot_stride, int seg) {
   constexpr int U = 4;  // rows in flight per thread
   struct alignas(2 * VEC) Vec {
     bf16 e[VEC];
@@ -40,7 +43,7 @@ __global__ void __launch_bounds__(128) gdn_conv1d_kernel(const bf16* __restrict_
   const int c = (blockIdx.x * 128 + threadIdx.x) * VEC;
   if (c >= channels) return;
   const int q0 = q_indptr[b], q1 = q_indptr[b + 1];
-  const int t0 = q0 + blockIdx.y * CONV_SEG, t1 = min(q1, t0 + CONV_SEG);
+  const int t0 = q0 + (int)blockIdx.y * seg, t1 = min(q1, t0 + seg);
   const int slot = slots[b];
   if (t0 >= q1) return;
   if (slot < 0) {
@@ -338,15 +341,18 @@ __global__ void __launch_bounds__(128) gdn_recurrent_kernel(const bf16* __restri
 extern "C" int pg_gdn_conv1d(const void* x, long long ldx, const void* w, void* state, void* out, long long ldo, const void* q_indptr,
                              const void* slots, int num_seqs, int channels, int K, long long state_slot_stride, int max_q_len, cudaStream_t stream) {
   PG_REQUIRE(K >= 2 && K <= 4, "gdn_conv1d: kernel size %d not supported (2..4)", K);
-  PG_REQUIRE(num_seqs <= 65535 && max_q_len <= 65535 * CONV_SEG, "gdn_conv1d: %d sequences of up to %d tokens", num_seqs, max_q_len);
+  PG_REQUIRE(num_seqs <= 65535, "gdn_conv1d: %d sequences", num_seqs);
   if (num_seqs == 0 || max_q_len <= 0) return PG_OK;
   // eight channels per thread where rows, taps and carried inputs are runs of 16-byte pieces, else one
   const bool wide = K == 4 && channels % 8 == 0 && ldx % 8 == 0 && ldo % 8 == 0 && state_slot_stride % 8 == 0 &&
                     (((uintptr_t)x | (uintptr_t)out | (uintptr_t)w | (uintptr_t)state) & 15) == 0;
   const int threads = wide ? channels / 8 : channels;
-  const dim3 grid((threads + 127) / 128, (max_q_len + CONV_SEG - 1) / CONV_SEG, num_seqs);
+  const unsigned pieces = (threads + 127) / 128;
+  long long seg = CONV_SEG;
+  while (seg < max_q_len && pieces * (long long)num_seqs * ((max_q_len + seg - 1) / seg) > CONV_BLOCKS) seg *= 2;
+  const dim3 grid(pieces, (unsigned)((max_q_len + seg - 1) / seg), num_seqs);
   auto kernel = wide ? gdn_conv1d_kernel<8> : gdn_conv1d_kernel<1>;
-  kernel<<<grid, 128, 0, stream>>>((const bf16*)x, ldx, (const bf16*)w, (bf16*)state, (bf16*)out, ldo, (const int*)q_indptr, (const int*)slots, channels, K, state_slot_stride);
+  kernel<<<grid, 128, 0, stream>>>((const bf16*)x, ldx, (const bf16*)w, (bf16*)state, (bf16*)out, ldo, (const int*)q_indptr, (const int*)slots, channels, K, state_slot_stride, (int)seg);
   PG_LAUNCH_CHECK();
   return PG_OK;
 }

@@ -467,3 +467,18 @@ def test_two_sm_gemm_switches(switch, takes):
     code = "from pegainfer_b200 import _native as n; print(n.load().pg_gemm2sm_takes(100, 1024, 8192), n.load().pg_gemm2sm_takes(100, 1024, 8256), sep='')"
     env = {k: v for k, v in os.environ.items() if not k.startswith("PEGAINFER_GEMM_2SM")}
     assert subprocess.run([sys.executable, "-c", code], env=env | switch, capture_output=True, text=True, timeout=300).stdout.strip() == takes
+
+
+def test_gdn_conv1d_beside_many_sequences():
+    """Prompts beside so many decode rows that the segments are longer."""
+    torch.manual_seed(0)
+    q_lens = [70, 1, 33] + [1] * 400 + [64, 65, 2]
+    channels, n = 10240, len(q_lens)
+    meta = _state_meta(q_lens, list(range(1, n + 1)))
+    x = torch.randn(sum(q_lens), channels, device=DEV).bfloat16()
+    w = (torch.randn(channels, 4, device=DEV) * 0.5).bfloat16()
+    st1 = torch.randn(n + 1, channels, 3, device=DEV).bfloat16()
+    st2 = st1.clone()
+    y1, y2 = cu().gdn_conv1d(x, w, st1, meta), R.gdn_conv1d(x, w, st2, meta)
+    assert ((y1.float() - y2.float()).abs() <= 2 ** -7 * y2.float().abs() + 2 ** -9).all()  # as above
+    assert torch.equal(st1, st2)
