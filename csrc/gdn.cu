@@ -343,8 +343,10 @@ extern "C" int pg_gdn_conv1d(const void* x, long long ldx, const void* w, void* 
   PG_REQUIRE(K >= 2 && K <= 4, "gdn_conv1d: kernel size %d not supported (2..4)", K);
   PG_REQUIRE(num_seqs <= 65535, "gdn_conv1d: %d sequences", num_seqs);
   if (num_seqs == 0 || max_q_len <= 0) return PG_OK;
-  // eight channels per thread where rows, taps and carried inputs are runs of 16-byte pieces, else one
-  const bool wide = K == 4 && channels % 8 == 0 && ldx % 8 == 0 && ldo % 8 == 0 && state_slot_stride % 8 == 0 &&
+  // eight channels per thread where rows, taps and carried inputs are runs of 16-byte pieces, else one; also one for decode rows up to
+  // some two million channels in all, which wait for a thread's chain (8 x 2048 3.3 us with eight, 2.4 with one; 200 x 10240 19.3,
+  // 19.4; 512 x 10240 43.5, 46.6)
+  const bool wide = (max_q_len > 4 || channels * (long long)num_seqs > 2000000) && K == 4 && channels % 8 == 0 && ldx % 8 == 0 && ldo % 8 == 0 && state_slot_stride % 8 == 0 &&
                     (((uintptr_t)x | (uintptr_t)out | (uintptr_t)w | (uintptr_t)state) & 15) == 0;
   const int threads = wide ? channels / 8 : channels;
   const unsigned pieces = (threads + 127) / 128;

@@ -482,3 +482,16 @@ def test_gdn_conv1d_beside_many_sequences():
     y1, y2 = cu().gdn_conv1d(x, w, st1, meta), R.gdn_conv1d(x, w, st2, meta)
     assert ((y1.float() - y2.float()).abs() <= 2 ** -7 * y2.float().abs() + 2 ** -9).all()  # as above
     assert torch.equal(st1, st2)
+
+
+@pytest.mark.parametrize("channels,seqs", [(1040, 6), (2048, 976), (2048, 978)])  # one channel per thread; either side of two million channels
+def test_gdn_conv1d_rows(channels, seqs):
+    torch.manual_seed(seqs)
+    q_lens = ([1, 2, 3, 4, 1, 1] * seqs)[:seqs]
+    meta = _state_meta(q_lens, [-1] + list(range(1, seqs)))
+    x, w = torch.randn(sum(q_lens), channels, device=DEV).bfloat16(), (torch.randn(channels, 4, device=DEV) * 0.5).bfloat16()
+    st1 = torch.randn(seqs, channels, 3, device=DEV).bfloat16()
+    st2 = st1.clone()
+    y1, y2 = cu().gdn_conv1d(x, w, st1, meta), R.gdn_conv1d(x, w, st2, meta)
+    assert ((y1.float() - y2.float()).abs() <= 2 ** -7 * y2.float().abs() + 2 ** -9).all()  # as above
+    assert torch.equal(st1, st2)
