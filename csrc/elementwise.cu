@@ -526,8 +526,8 @@ extern "C" int pg_rms_norm(const void* x, void* residual, const void* w, void* y
 // x, y [rows / heads, heads, dim] contiguous; gate rows of a token start ld_gate elements apart
 extern "C" int pg_gated_rms_norm_act(const void* x, const void* gate, long long ld_gate, const void* w_f32, void* y, long long rows, int heads, int dim, float eps, int act, cudaStream_t stream) {
   PG_REQUIRE(act == 0 || act == 1, "gated_rms_norm: gate activation %d (0 = SiLU, 1 = sigmoid)", act);
-  PG_REQUIRE(heads >= 1 && rows < (1ll << 32), "gated_rms_norm: %lld rows of %d heads", rows, heads);
   if (rows == 0) return PG_OK;
+  PG_REQUIRE(heads >= 1 && rows < (1ll << 32), "gated_rms_norm: %lld rows of %d heads", rows, heads);
   const int vec = dim == 128 ? 4 : dim == 256 ? 8 : dim == 64 ? 2 : 0;
   const bool aligned = vec && ld_gate % vec == 0 && (((uintptr_t)x | (uintptr_t)gate | (uintptr_t)y) & (2 * vec - 1)) == 0;
   const bool many = rows >= (vec == 8 ? 2400 : 12000);

@@ -165,6 +165,13 @@ def test_gated_norm_reads_the_gate_in_place(dim, heads, act, t):
         assert ((got.float() - want.float()).abs() <= 2 ** -7 * want.float().abs() + 1e-6).all()
 
 
+def test_gated_norm_of_no_rows():
+    w = torch.ones(128, device=DEV)
+    for shape in ((0, 4, 128), (5, 0, 128), (0, 128)):
+        x = torch.zeros(shape, device=DEV).bfloat16()
+        assert cu().gated_rms_norm(x, x, w, 1e-6).shape == shape
+
+
 @pytest.mark.parametrize("t", [1, 2, 3, 4])
 @pytest.mark.parametrize("h,hq,hkv,inter", [(1024, 16, 8, 3072), (2560, 32, 8, 9728), (256, 2, 1, 512), (4096, 32, 8, 12288)])
 def test_chain_of_few_rows(t, h, hq, hkv, inter):
