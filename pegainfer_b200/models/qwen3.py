@@ -173,7 +173,7 @@ class Qwen3Model:
                 return self._forward_chain(x, residual, meta, kv, aux_layers, K)
         for i, l in enumerate(self.layers):
             ls = meta.lora_slots if self.lora is not None else None
-            decode = ls is None and meta.num_tokens <= 256  # weight-streaming regime: chain L2 prefetches GEMM to GEMM
+            decode = ls is None and meta.num_tokens <= 256  # weight-streaming regime: L2 prefetches from GEMM to GEMM, on the one-CTA kernel (5 to 64 rows, batch-invariant steps); the others drop them
             if decode:
                 ops.prefetch_weights(l.o)
             if fused:
