@@ -835,19 +835,21 @@ extern "C" void pg_sample_force_cluster(int c) { g_force_cluster = c; }
 
 // Cluster size and slice length of the cluster sampler for a vocabulary, or 0 when the row does not fit the shared memory of
 // eight CTAs (the one-CTA kernel serves those).  A wave holds so many clusters of 1, 2, 4, 8 CTAs at one or two CTAs an SM
-// (74 / 33 / 15 clusters of 2 / 4 / 8 fit the GPCs); a row's time is about that of 40 K tokens more than its slice has.
-// 64 x 151936, top-k 50: 102 us with clusters of 8 (three waves of 30), 62 us with 4 (one wave of 66), 83 us with 2; 8 rows:
-// 42 us with 8, 51 us with 4.
+// (74 / 33 / 15 clusters of 2 / 4 / 8 fit the GPCs).  A row takes the time of its slice and of so many thousand tokens more: the
+// barriers of its cluster, and the other clusters of a wave that is full.  Us with clusters of 1 / 2 / 4 / 8, top-k 50: 16 rows of
+// 4096 15 / 16 / 18 / 30, of 32000 41 / 29 / 23 / 32, of 102400 103 / 61 / 41 / 41; 4 rows of 102400 94 / 58 / 38 / 33; 64 rows of
+// 151936 - / 83 / 62 / 102.
 static int sampler_cluster_plan(int rows, int vocab, int elem, int max_smem, int* slice_out) {
   const int room = (max_smem - 2048 - (int)sizeof(ScShared) - 64) / elem;  // tokens per CTA (2 KB left for static shared memory)
   static const int per_wave[4] = {148, 74, 33, 15};
+  static const double alone[4] = {13.2, 15.8, 17.8, 23.3}, crowded[4] = {5.0, 4.4, 6.7, 14.4};
   int best = 0;
   double least = 0;
   for (int l = 0; l < 4; ++l) {
     const int c = 1 << l, slice = (ceil_div(vocab, c) + 7) & ~7;
     if (slice > room || (g_force_cluster > 0 && c != g_force_cluster)) continue;
     const int wave = per_wave[l] * (2 * (slice * elem + (int)sizeof(ScShared) + 2048) <= max_smem ? 2 : 1);
-    const double cost = (double)ceil_div(rows, wave) * (slice + 40.0 * 1024);
+    const double cost = ceil_div(rows, wave) * (slice / 1000.0 + alone[l] + crowded[l] * (rows < wave ? (double)rows / wave : 1.0));
     if (best == 0 || cost < least) best = c, least = cost, *slice_out = slice;
   }
   return best;
