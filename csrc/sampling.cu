@@ -292,7 +292,8 @@ __global__ void __launch_bounds__(ST) sample_kernel(const T* __restrict__ logits
 // 2^-40 have no mass and are left out) brackets it: a bin's count times its edges bounds its mass from both sides, and the
 // walk from the top with the lower (upper) bounds ends at or below (above) the bin that the exact walk ends in.  Then the
 // mass above the bracket is summed exactly and only the tokens inside it, some hundred as a rule, go through a radix
-// descent with counts and masses.  Bound by the latency of the passes and of the eight cluster barriers between them, with
+// descent with counts and masses, which ends after its first level where they are all alike (64 rows of 151936 equal logits: 114 us;
+// 237 with the four radix levels of all tokens).  Bound by the latency of the passes and of the eight cluster barriers between them, with
 // every row of a batch of 64 resident at once (clusters of four).  64 x 151936 bf16, top-k 50, top-p 0.9: 200 us with all tokens
 // taking part in each of four radix levels, one warp match per 32 tokens; 61 us now (1 row: 36 us).
 // ---------------------------------------------------------------------------------
@@ -335,6 +336,7 @@ struct ScShared {
   unsigned long long x_u64[4];  // this CTA's contributions to cluster-wide sums: normaliser, mass and count above the bracket, kept mass
   float x_f32;                  // and to the cluster-wide maximum
   uint32_t list_n, prefix, cnt_above;
+  uint32_t own_min, own_max, key_min, key_max;  // least and largest key in the bracket, of this CTA and of the cluster
   int bin_lo, bin_hi;
   unsigned long long mass_above;
   unsigned long long warp_tot[SC_WARPS], warp_ub[SC_WARPS];
@@ -424,6 +426,8 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
   if (tid == 0) {
     sh.x_f32 = m;
     sh.list_n = 0u;
+    sh.own_min = SC_ONE;
+    sh.own_max = 0u;
     sh.bin_lo = SC_BINS;
     sh.bin_hi = SC_BINS;
   }
@@ -549,17 +553,24 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
       const uint32_t k_lo = SC_LOW + ((uint32_t)lo << SC_BIN_SHIFT), k_hi = SC_LOW + ((uint32_t)(hi + 1) << SC_BIN_SHIFT);  // [k_lo, k_hi)
       unsigned long long above = 0ull;
       uint32_t n_above = 0u;
+      uint32_t least = SC_ONE, most = 0u;
       walk(0, n, tid, SC_THREADS, [&](const uint32_t (&key)[VEC]) {
 #pragma unroll
         for (int j = 0; j < VEC; ++j)
           if (key[j] >= k_hi) {
             above += sc_fx(key[j]);
             ++n_above;
-          } else if (key[j] >= k_lo && *(volatile uint32_t*)&sh.list_n <= SC_LIST) {  // (a list that is too short takes no more)
-            const uint32_t at = atomicAdd(&sh.list_n, 1u);
-            if (at < SC_LIST) sh.list[at] = key[j];
+          } else if (key[j] >= k_lo) {
+            least = min(least, key[j]);
+            most = max(most, key[j]);
+            if (*(volatile uint32_t*)&sh.list_n <= SC_LIST) {  // (a list that is too short takes no more)
+              const uint32_t at = atomicAdd(&sh.list_n, 1u);
+              if (at < SC_LIST) sh.list[at] = key[j];
+            }
           }
       });
+      least = __reduce_min_sync(0xffffffffu, least);
+      most = __reduce_max_sync(0xffffffffu, most);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         above += __shfl_xor_sync(0xffffffffu, above, o);
@@ -568,6 +579,10 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
       if (lane == 0) {
         sh.warp_ub[warp] = above;
         sh.warp_cnt[warp] = n_above;
+        if (most > 0u) {
+          atomicMin(&sh.own_min, least);
+          atomicMax(&sh.own_max, most);
+        }
       }
       if (tid < 256) {
         sh.even.cnt[tid] = 0u;
@@ -634,6 +649,15 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
             sh.mass_above = sum_u64(&sh.x_u64[1]);
             sh.cnt_above = (uint32_t)sum_u64(&sh.x_u64[2]);
           }
+          if (level == 0 && tid == 32) {
+            uint32_t least = SC_ONE, most = 0u;
+            for (int q = 0; q < csize; ++q) {
+              least = min(least, ld_dsmem_u32(dsmem_addr(smem_u32(&sh.own_min), (uint32_t)q)));
+              most = max(most, ld_dsmem_u32(dsmem_addr(smem_u32(&sh.own_max), (uint32_t)q)));
+            }
+            sh.key_min = least;
+            sh.key_max = most;
+          }
         } else {
           // the other histogram is free: peers read it (the previous level, or the coarse counts) before they arrived
           next.cnt[tid - 256] = 0u;
@@ -683,6 +707,10 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
         }
         __syncthreads();
         prefix = sh.prefix;
+        if (sh.key_min == sh.key_max) {  // ties, as many as they are: the bracket has one key
+          prefix = sh.key_min - k_lo;
+          break;
+        }
       }
       thr_key = k_lo + prefix;
     }
