@@ -1612,25 +1612,29 @@ def _latent_keys(meta: AttnMeta, row0: int = 0, window: int = 0) -> int:
     return max(keys // max(rows, 1), longest // 2)
 
 
-def _latent_tc(rows: int, heads: int, lat: int, rot: int, keys: int, sms: int) -> bool:
+def _latent_tc(rows: int, heads: int, lat: int, rot: int, keys: int, max_q_len: int, sms: int) -> bool:
     """Does the absorbed form of rows of about ``keys`` keys run on tcgen05 (csrc/mla_decode_tc.cu)?  A block there owns an SM, serves up
     to 64 heads and works in tiles of 64 keys, whole ones; the mma.sync kernel has four blocks of 16 heads an SM and tiles of 32.
-    Measured with 16, 32, 64 and 128 heads (tcgen05 / mma.sync): within one wave of blocks 1.01 - 1.11 up to 32 keys, 0.90 - 1.02 at 40, 1.02 -
-    1.04 at 65 and 80 with few blocks (prompts of 80 tokens 1.01 - 1.05, of 100 0.94 - 0.97); above, where blocks of 16 heads leave three quarters of their tiles empty, 16 heads
+    Steps of a few rows a sequence do whatever their keys: a captured graph knows no more than a bound on them, and a drafter's tokens are
+    checked in steps of their own, so that a row has to be summed on one kernel in all of them to be the same (tcgen05 / mma.sync: up to 32
+    keys 1.01 - 1.13, 500 keys 0.5 - 0.8).
+    Rows of prompts go by their keys.  Measured with 16, 32, 64 and 128 heads: within one wave of blocks 1.01 - 1.11 up to 32 keys, 1.01 -
+    1.05 at 80 (prompts of 100 tokens 0.94 - 0.97); above, where blocks of 16 heads leave three quarters of their tiles empty, 16 heads
     1.03 - 1.26 at 128 keys and two waves, 1.03 - 1.08 at 200 and more waves (0.91 - 0.97 at 300), 32 heads 1.0 - 1.06 at 80 (0.90 - 0.98 at
-    100), 64 heads 0.88 - 1.0 at 40, but 1.02 at 80 with a second wave that is nearly empty (150 rows).
-    Decode rows gain from 33 keys on, rows of short prompts from 45; one line serves both, so that the rows that check a
-    drafter's tokens are summed as the decode rows are that they stand for.
-    A captured graph goes by its bound on the keys: 20 keys in a graph for 2048 take 1.02 - 1.10 of the time (8 rows of 128 heads 1.13),
-    500 keys 0.5 - 0.8."""
+    100), 64 heads 0.88 - 1.0 at 40, but 1.02 at 80 with a second wave that is nearly empty (150 rows)."""
     if lat != 512 or rot not in (0, 64):
         return False
+    if max_q_len <= _LATENT_FEW:
+        return True
     blocks = rows * ((heads + 63) // 64)
     if blocks <= sms:
         return keys > 44 and not (64 < keys <= 88 and blocks < 32)
     if heads <= 16:
         return keys > (128 if blocks <= 2 * sms else 256)
     return keys > (96 if heads <= 32 or 3 * blocks < 4 * sms else 32)
+
+
+_LATENT_FEW = 16  # rows of a sequence in a decode step or in one that checks drafted tokens
 
 
 def _latent_splits(rows: int, heads: int, longest: int, tc: bool, sms: int) -> int:
@@ -1755,7 +1759,7 @@ def mla_attention(q: "_MlaQ", w_uk, w_uv, latent_layer, meta: AttnMeta, scale, k
         for b in range(meta.num_seqs):
             seq_of.extend([b] * (qi[b + 1] - qi[b]))
         unit_seq = torch.tensor(seq_of, dtype=torch.int32, device=dev)
-    tc = _latent_tc(t, h, kv_lora, rope, _latent_keys(meta), c.sms)
+    tc = _latent_tc(t, h, kv_lora, rope, _latent_keys(meta), meta.max_q_len, c.sms)
     splits = _latent_splits(t, h, meta.max_kv_len, tc, c.sms) if meta.decode_only else 1
     need = t * h * splits * (kv_lora + 1) * 4
     if need > c.attn_part.numel():
@@ -1884,7 +1888,7 @@ def latent_attention(q, uk_t, uv, ukv, cache, meta: AttnMeta, rot: int, scale: f
     if aligned and lat <= 512 and rot <= 64:
         longest = max(meta.max_kv_len, 1)
         longest = min(longest, window + 31) if window else longest
-        tc = _latent_tc(n, heads, lat, rot, _latent_keys(meta, row0, window), c.sms)
+        tc = _latent_tc(n, heads, lat, rot, _latent_keys(meta, row0, window), meta.max_q_len, c.sms)
         splits = _latent_splits(n, heads, longest, tc, c.sms)
         splits = max(1, min(splits, c.attn_part.numel() // (n * heads * (lat + 1) * 4)))
         rc = lib().pg_latent_attention(_ptr(q_abs), *strides, *pe, *where, _ci(row0), _ci(meta.num_seqs), _ci(n), _ci(heads), _ci(lat), _ci(rot), _ci(ps), _cf(scale), _ci(window), *extra, _ci(splits),

@@ -377,8 +377,8 @@ def test_latent_window_and_empty_splits(heads, rot, window, splits, reps, tc, ex
     assert cu().read_status(DEV) == 0
 
 
-@pytest.mark.parametrize("lens,past,heads,tc", [([1] * 8, 43, 16, False), ([1] * 8, 44, 16, True), ([1] * 150, 100, 16, False), ([1] * 150, 130, 16, True), ([1] * 150, 95, 64, False), ([1] * 150, 96, 64, True),
-                                                 ([80], 0, 16, False), ([90], 0, 16, True), ([1] * 60 + [1], 7, 16, False), ([300] * 3, 0, 32, True)])
+@pytest.mark.parametrize("lens,past,heads,tc", [([1] * 8, 7, 16, True), ([1] * 150, 100, 16, True), ([16] * 3, 0, 16, True), ([17] * 3, 0, 16, False), ([80], 0, 16, False), ([90], 0, 16, True),
+                                                 ([20] * 10, 80, 16, False), ([20] * 10, 130, 16, True), ([20] * 10, 15, 64, False), ([20] * 10, 30, 64, True), ([300] * 3, 0, 32, True)])
 def test_latent_kernels_where_the_rule_changes(lens, past, heads, tc, monkeypatch):
     """The rows on either side of each line of the rule, on the kernel that it names, against the restatement."""
     torch.manual_seed(past + heads)
@@ -390,7 +390,7 @@ def test_latent_kernels_where_the_rule_changes(lens, past, heads, tc, monkeypatc
     pos = torch.cat([torch.arange(past, x) for x in kv_lens]).to(torch.int32).to(DEV)
     t, decode = sum(lens), max(lens) == 1
     meta = R.AttnMeta(qi.to(torch.int32).to(DEV), torch.tensor(kv_lens, dtype=torch.int32, device=DEV), table, pos, pos, page, n, t, max(lens), max(kv_lens), decode, qi.tolist(), kv_lens)
-    assert cu()._latent_tc(t, heads, 512, 64, cu()._latent_keys(meta), 148) == tc
+    assert cu()._latent_tc(t, heads, 512, 64, cu()._latent_keys(meta), max(lens), 148) == tc
     cache = torch.randn(n * per, page, 576, device=DEV).bfloat16()
     q = torch.randn(t, heads, 192, device=DEV).bfloat16()
     uk, uv = (torch.randn(heads, 128, 512, device=DEV) * 0.05).bfloat16(), (torch.randn(heads, 128, 512, device=DEV) * 0.05).bfloat16()
