@@ -15,7 +15,7 @@
 // O and the sums rescaled), and each thread sums its own keys' weights, added up once at the end.
 //
 // Rows of a tile that are no keys are cleared in shared memory, adjacent lanes adjacent bytes (lanes a block of columns apart met in the same
-// banks: one row of 8 keys, 16 heads, 25.2 us for the whole operation against 23.4 now; 21.1 on the mma.sync kernel, which short rows go to).
+// banks: one row of 8 keys, 16 heads, 25.2 us for the whole operation against 23.4 now; 21.1 on the mma.sync kernel).
 //
 // Against the mma.sync kernel, in which a CTA of 16 heads exchanges partial scores through shared memory for every 32 keys
 // (128 rows x 64 heads x 1150 keys): 284 us before, 90 us now.  What

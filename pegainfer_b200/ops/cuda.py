@@ -1888,7 +1888,7 @@ def latent_attention(q, uk_t, uv, ukv, cache, meta: AttnMeta, rot: int, scale: f
     if aligned and lat <= 512 and rot <= 64:
         longest = max(meta.max_kv_len, 1)
         longest = min(longest, window + 31) if window else longest
-        tc = _latent_tc(n, heads, lat, rot, _latent_keys(meta, row0, window), meta.max_q_len, c.sms)
+        tc = _latent_tc(n, heads, lat, rot, _latent_keys(meta, row0, window), 1 if row0 else meta.max_q_len, c.sms)  # (behind prompts: decode rows)
         splits = _latent_splits(n, heads, longest, tc, c.sms)
         splits = max(1, min(splits, c.attn_part.numel() // (n * heads * (lat + 1) * 4)))
         rc = lib().pg_latent_attention(_ptr(q_abs), *strides, *pe, *where, _ci(row0), _ci(meta.num_seqs), _ci(n), _ci(heads), _ci(lat), _ci(rot), _ci(ps), _cf(scale), _ci(window), *extra, _ci(splits),
