@@ -20,17 +20,14 @@
 //   bf16   W [E, M, K]: TMA straight into the swizzled A tile.
 //   int4   W packed [E, M, K/8] int32 (offset-binary nibbles, pair-interleaved inside each word:
 //          bits 0-15 hold elements 0,2,4,6 and bits 16-31 elements 1,3,5,7 of the word's eight) with
-//          bf16 scales [E, M, K/32]: TMA brings the packed tile (4 KB per 128x64) into a
-//          raw buffer, the dequantisation warps (four groups of two, each group taking every
-//          fourth k-block) expand it to bf16 ((nibble - 8) * scale,
-//          one rounding) directly into the 128-byte-swizzled A tile and hand it to the MMA
-//          warp through an mbarrier; HBM traffic stays at 4.5 bits per weight.
+//          bf16 scales [E, M, K/32]: a kernel of its own (moe_gemm_int4.cuh); HBM traffic stays
+//          at 4.5 bits per weight.
 //   fp8    W e4m3 [E, M, K] with f32 scale_inv [E, ceil(M/128), ceil(K/128)] (block-scaled
-//          checkpoints): TMA brings the raw 8 KB tile, the same warps convert e4m3 ->
-//          f32 (exact), multiply by the block's scale_inv and round once to bf16 into the
+//          checkpoints): TMA brings the raw 8 KB tile, the dequantisation warps (four groups of two,
+//          each group taking every fourth k-block) convert e4m3 -> f32 (exact), multiply by the block's scale_inv and round once to bf16 into the
 //          swizzled A tile; HBM traffic is one byte per weight.
 //
-// warp 0 TMA producer | warp 1 MMA issuer + TMEM owner | warps 2-5 epilogue | warps 6-13 dequant (int4 / fp8)
+// warp 0 TMA producer | warp 1 MMA issuer + TMEM owner | warps 2-5 epilogue | warps 6-13 dequant (fp8)
 //
 // Takes the place of the reference's Marlin W4A16 MoE kernel
 // (pegainfer-kernels/csrc/kimi_k2/kimi_marlin_wna16.cu:241-340, vllm_marlin/**) and its
@@ -42,13 +39,13 @@
 #include <cuda_fp8.h>
 
 #include "api.h"
+#include "attention_tc.cuh"
 #include "common.cuh"
 
 namespace {
 
 constexpr int BM = 128, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;
-constexpr int RAW_BYTES = BM * BK / 2;  // packed int4 tile
 constexpr int RAW_BYTES_FP8 = BM * BK;  // fp8 tile
 constexpr int MAX_STAGES = 10;
 constexpr int MAX_EXPERTS = 512;
@@ -60,6 +57,7 @@ struct MoeGemmParams {
   int bn, stages, kblocks, m_tiles;
   uint32_t tmem_cols;
   int quant;           // 0 bf16, 1 int4 group-32, 2 fp8 e4m3 with 128x128 block scales
+  int scale_tma;       // int4: a row's scales come in 16-byte pieces by TMA
   const void* scales;  // int4: bf16 [E, M, K/32]; fp8: f32 scale_inv [E, ceil(M/128), ceil(K/128)]
   const int* offsets;  // [E+1]
   uint32_t* status;
@@ -119,6 +117,77 @@ __device__ __forceinline__ bool named_bar_all(int id, int nthreads, bool pred) {
   return r != 0;
 }
 
+// One output tile from tensor memory: the thread's weight row `m`, whose f32 results of the tile's token rows start at `t_row`.
+__device__ __forceinline__ void store_tile(const MoeGemmParams& p, const Item& it, int m, int lane, uint32_t t_row) {
+  for (int c = 0; c < p.bn; c += 16) {
+    if (c >= it.rows) break;  // uniform across the warp
+    uint32_t v[16];
+    tmem_ld16(t_row + c, v);
+    tmem_ld_wait();
+    if (p.act == 2) {  // the shuffles run on all lanes, the even ones store
+      bf16* dst = p.y + (long long)(it.row0 + c) * p.ldy + (m >> 1);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float g = __uint_as_float(v[j]), u = __shfl_xor_sync(0xFFFFFFFFu, g, 1);
+        if (!(lane & 1) && m < p.M && c + j < it.rows) dst[j * p.ldy] = __float2bfloat16(g / (1.f + __expf(-g)) * u);
+      }
+    } else if (m < p.M) {
+      if (p.scatter_src == nullptr) {
+        if (p.act == 1) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float f = fmaxf(__uint_as_float(v[j]), 0.f);
+            v[j] = __float_as_uint(f * f);
+          }
+        }
+        const long long at = (p.head_rows ? it.e * p.y_head : 0ll) + (long long)(it.row0 + c) * p.ldy + m;
+        if (p.y_f32 != nullptr) {
+          float* dst = p.y_f32 + at;
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (c + j < it.rows) dst[(long long)j * p.ldy] = __uint_as_float(v[j]);
+          continue;
+        }
+        bf16* dst = p.y + at;
+        if (p.gate != nullptr) {
+          const bf16* gp = p.gate + it.e * p.g_head + (long long)(it.row0 + c) * p.ldg + m;
+          float gv[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) gv[j] = c + j < it.rows ? __bfloat162float(gp[j * p.ldg]) : 0.f;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) / (1.f + __expf(-gv[j])));
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (c + j < it.rows) dst[j * p.ldy] = __float2bfloat16(__uint_as_float(v[j]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (c + j < it.rows) {
+            const int idx = p.scatter_src[it.row0 + c + j];
+            const int dst_rank = idx / p.cap, slot = idx - dst_rank * p.cap;
+            p.peer_out[dst_rank][(size_t)slot * p.ldy + m] = __float2bfloat16(__uint_as_float(v[j]));
+          }
+        }
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ void raise_returned(const MoeGemmParams& p, uint32_t ep_epoch) {
+  if (p.scatter_src != nullptr && threadIdx.x == 0) {
+    // every output row of this CTA is on its way to its source rank: the last CTA of this
+    // GPU raises the "returned" epoch on all ranks
+    uint32_t* myflags = p.peer_flags[p.rank] + p.site * 32;
+    __threadfence_system();
+    const uint32_t old = atomicAdd(&myflags[17], 1u);
+    if (old == gridDim.x - 1) {
+      myflags[17] = 0u;
+      for (int q = 0; q < p.world; ++q) st_release_sys(p.peer_flags[q] + p.site * 32 + 8 + p.rank, ep_epoch + 1u);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(448, 1)
 moe_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const MoeGemmParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -127,7 +196,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   const uint32_t base = smem_u32(smem_raw);
   uint8_t* tiles = smem_raw + (((base + 1023u) & ~1023u) - base);
   const int b_bytes = p.bn * 128;
-  const int raw_bytes = p.quant == 1 ? RAW_BYTES : p.quant == 2 ? RAW_BYTES_FP8 : 0;
+  const int raw_bytes = p.quant ? RAW_BYTES_FP8 : 0;
   const int stage_bytes = A_BYTES + b_bytes + raw_bytes;
   uint64_t* full = reinterpret_cast<uint64_t*>(tiles + p.stages * stage_bytes);
   uint64_t* empty = full + MAX_STAGES;
@@ -202,7 +271,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
           uint8_t* st = tiles + stage * stage_bytes;
           if (p.quant) {
             mbar_expect_tx(&full[stage], (uint32_t)(raw_bytes + b_bytes));
-            tma_load_3d(st + A_BYTES + b_bytes, &tm_w, &full[stage], p.quant == 1 ? kb * (BK / 8) : kb * BK, it.m_tile * BM, it.e, pol_w);
+            tma_load_3d(st + A_BYTES + b_bytes, &tm_w, &full[stage], kb * BK, it.m_tile * BM, it.e, pol_w);
           } else {
             mbar_expect_tx(&full[stage], (uint32_t)(A_BYTES + b_bytes));
             tma_load_3d(st, &tm_w, &full[stage], kb * BK, it.m_tile * BM, it.e, pol_w);
@@ -276,61 +345,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       ok = named_bar_all(1, 128, ok);
       if (!ok) break;
       tc_fence_after();
-      const int m = it.m_tile * BM + r;
-      const uint32_t t_row = tmem_base + ((uint32_t)(wq * 32) << 16) + (uint32_t)(acc * p.bn);
-      for (int c = 0; c < p.bn; c += 16) {
-        if (c >= it.rows) break;  // uniform across the warp
-        uint32_t v[16];
-        tmem_ld16(t_row + c, v);
-        tmem_ld_wait();
-        if (p.act == 2) {  // the shuffles run on all lanes, the even ones store
-          bf16* dst = p.y + (long long)(it.row0 + c) * p.ldy + (m >> 1);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float g = __uint_as_float(v[j]), u = __shfl_xor_sync(0xFFFFFFFFu, g, 1);
-            if (!(lane & 1) && m < p.M && c + j < it.rows) dst[j * p.ldy] = __float2bfloat16(g / (1.f + __expf(-g)) * u);
-          }
-        } else if (m < p.M) {
-          if (p.scatter_src == nullptr) {
-            if (p.act == 1) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const float f = fmaxf(__uint_as_float(v[j]), 0.f);
-                v[j] = __float_as_uint(f * f);
-              }
-            }
-            const long long at = (p.head_rows ? it.e * p.y_head : 0ll) + (long long)(it.row0 + c) * p.ldy + m;
-            if (p.y_f32 != nullptr) {
-              float* dst = p.y_f32 + at;
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                if (c + j < it.rows) dst[(long long)j * p.ldy] = __uint_as_float(v[j]);
-              continue;
-            }
-            bf16* dst = p.y + at;
-            if (p.gate != nullptr) {
-              const bf16* gp = p.gate + it.e * p.g_head + (long long)(it.row0 + c) * p.ldg + m;
-              float gv[16];
-#pragma unroll
-              for (int j = 0; j < 16; ++j) gv[j] = c + j < it.rows ? __bfloat162float(gp[j * p.ldg]) : 0.f;
-#pragma unroll
-              for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) / (1.f + __expf(-gv[j])));
-            }
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if (c + j < it.rows) dst[j * p.ldy] = __float2bfloat16(__uint_as_float(v[j]));
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              if (c + j < it.rows) {
-                const int idx = p.scatter_src[it.row0 + c + j];
-                const int dst_rank = idx / p.cap, slot = idx - dst_rank * p.cap;
-                p.peer_out[dst_rank][(size_t)slot * p.ldy + m] = __float2bfloat16(__uint_as_float(v[j]));
-              }
-            }
-          }
-        }
-      }
+      store_tile(p, it, it.m_tile * BM + r, lane, tmem_base + ((uint32_t)(wq * 32) << 16) + (uint32_t)(acc * p.bn));
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);
@@ -350,40 +365,15 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     Item it;
     long long kbg0 = 0;  // global index of this item's first k-block
     bool ok = true;
-    const bool int4 = p.quant == 1;
-    const int groups_per_row = p.K / 32;
     const int mb = (p.M + 127) / 128, kbk = (p.K + 127) / 128;
     for (int item = blockIdx.x; item < total && ok; item += gridDim.x, kbg0 += p.kblocks) {
       if (!locate(p, s_tiles, item, cur, it)) break;
       const int first = (int)(((long long)grp - kbg0) & 3);  // first k-block of this item that belongs to the group
-      // scales of the group's next k-block are fetched one turn (four k-blocks) ahead
-      const bf16* srow[2];
-      bool live[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int m = it.m_tile * BM + t + 64 * h;
-        live[h] = m < p.M;
-        srow[h] = reinterpret_cast<const bf16*>(p.scales) + ((size_t)it.e * p.M + (live[h] ? m : 0)) * groups_per_row;
-      }
+      // the scale of the group's next k-block is fetched one turn (four k-blocks) ahead
       const float* frow = reinterpret_cast<const float*>(p.scales) + ((size_t)it.e * mb + it.m_tile) * kbk;
-      const bf16 zero = __float2bfloat16(0.f);
-      bf16 sc[2][2], nx[2][2];
-      float fs = 0.f, fnx = 0.f;
-      auto load_scales = [&](int kb, bf16 (&dst)[2][2], float& fdst) {
-        if (kb >= p.kblocks) return;
-        if (int4) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            dst[h][0] = (live[h] && kb * 2 < groups_per_row) ? srow[h][kb * 2] : zero;
-            dst[h][1] = (live[h] && kb * 2 + 1 < groups_per_row) ? srow[h][kb * 2 + 1] : zero;
-          }
-        } else {
-          fdst = frow[kb >> 1];
-        }
-      };
-      load_scales(first, sc, fs);
+      float fs = first < p.kblocks ? frow[first >> 1] : 0.f;
       for (int kb = first; kb < p.kblocks && ok; kb += 4) {
-        load_scales(kb + 4, nx, fnx);
+        const float fnx = kb + 4 < p.kblocks ? frow[(kb + 4) >> 1] : 0.f;
         const long long kbg = kbg0 + kb;
         const int stage = (int)(kbg % p.stages);
         const uint32_t phase = (uint32_t)((kbg / p.stages) & 1);
@@ -396,61 +386,31 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         for (int h = 0; h < 2; ++h) {
           const int r = t + 64 * h;
           uint8_t* a_row = st + r * 128;
-          if (int4) {
-            const uint4* raw = reinterpret_cast<const uint4*>(st + A_BYTES + b_bytes + r * 32);
-            const bf162 bias = __floats2bfloat162_rn(136.f, 136.f);
+          // fp8 e4m3: exact in half, f32 * scale_inv of the 128x128 block, rounded once to bf16
+          const uint4* raw = reinterpret_cast<const uint4*>(st + A_BYTES + b_bytes + r * 64);
 #pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-              const uint4 rw = raw[hf];
-              const uint32_t words[4] = {rw.x, rw.y, rw.z, rw.w};
-              const bf162 s2 = __halves2bfloat162(sc[h][hf], sc[h][hf]);
+          for (int half = 0; half < 4; ++half) {
+            const uint4 v = raw[half];
+            const uint32_t words[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-              for (int c = 0; c < 4; ++c) {
-                // pair-interleaved nibbles: (w >> 4i) & 0x000F000F | 0x43004300 = bf16 pair (128 + e[2i], 128 + e[2i+1])
-                uint32_t o[4];
+            for (int hh = 0; hh < 2; ++hh) {
+              uint32_t o[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  uint32_t tt = ((words[c] >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
-                  bf162 val = *reinterpret_cast<bf162*>(&tt);
-                  val = __hmul2(__hsub2(val, bias), s2);
-                  o[i] = *reinterpret_cast<uint32_t*>(&val);
-                }
-                const int ch = hf * 4 + c;
-                *reinterpret_cast<uint4*>(a_row + ((ch ^ (r & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+              for (int q = 0; q < 4; ++q) {
+                const uint32_t w = words[hh * 2 + (q >> 1)];
+                const __nv_fp8x2_storage_t pair = (__nv_fp8x2_storage_t)((w >> (16 * (q & 1))) & 0xFFFFu);
+                const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(pair, __NV_E4M3);
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
+                const bf162 b2 = __floats2bfloat162_rn(f.x * fs, f.y * fs);
+                o[q] = *reinterpret_cast<const uint32_t*>(&b2);
               }
-            }
-          } else {
-            // fp8 e4m3: exact in half, f32 * scale_inv of the 128x128 block, rounded once to bf16
-            const uint4* raw = reinterpret_cast<const uint4*>(st + A_BYTES + b_bytes + r * 64);
-#pragma unroll
-            for (int half = 0; half < 4; ++half) {
-              const uint4 v = raw[half];
-              const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-              for (int hh = 0; hh < 2; ++hh) {
-                uint32_t o[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  const uint32_t w = words[hh * 2 + (q >> 1)];
-                  const __nv_fp8x2_storage_t pair = (__nv_fp8x2_storage_t)((w >> (16 * (q & 1))) & 0xFFFFu);
-                  const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(pair, __NV_E4M3);
-                  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
-                  const bf162 b2 = __floats2bfloat162_rn(f.x * fs, f.y * fs);
-                  o[q] = *reinterpret_cast<const uint32_t*>(&b2);
-                }
-                const int ch = half * 2 + hh;
-                *reinterpret_cast<uint4*>(a_row + ((ch ^ (r & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-              }
+              const int ch = half * 2 + hh;
+              *reinterpret_cast<uint4*>(a_row + ((ch ^ (r & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
             }
           }
         }
         fence_proxy_async_smem();
         mbar_arrive(&aready[stage]);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          sc[h][0] = nx[h][0];
-          sc[h][1] = nx[h][1];
-        }
         fs = fnx;
       }
     }
@@ -464,18 +424,10 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     tmem_dealloc(tmem_base, p.tmem_cols);
   }
   if (threadIdx.x == 0 && *abort_flag) atomicCAS(p.status, PG_ST_OK, PG_ST_TIMEOUT | (5u << 8));
-  if (p.scatter_src != nullptr && threadIdx.x == 0) {
-    // every output row of this CTA is on its way to its source rank: the last CTA of this
-    // GPU raises the "returned" epoch on all ranks
-    uint32_t* myflags = p.peer_flags[p.rank] + p.site * 32;
-    __threadfence_system();
-    const uint32_t old = atomicAdd(&myflags[17], 1u);
-    if (old == gridDim.x - 1) {
-      myflags[17] = 0u;
-      for (int q = 0; q < p.world; ++q) st_release_sys(p.peer_flags[q] + p.site * 32 + 8 + p.rank, ep_epoch + 1u);
-    }
-  }
+  raise_returned(p, ep_epoch);
 }
+
+#include "moe_gemm_int4.cuh"
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -494,7 +446,7 @@ EncodeTiledFn moe_get_encode() {
 
 bool g_attr_set[64];
 int g_sms[64], g_max_smem[64];
-int g_static_smem = 0;
+int g_static_smem = 0, g_static_smem_q4 = 0;
 std::mutex g_mu;
 
 }  // namespace
@@ -516,6 +468,7 @@ static int moe_gemm_impl(const void* x, long long ldx, long long x_rows, const v
   PG_REQUIRE(quant == 0 ? K % 8 == 0 : K % 64 == 0, "moe gemm: K=%d must be a multiple of %d", K, quant == 0 ? 8 : 64);
   PG_REQUIRE(bn >= 16 && bn <= 256 && bn % 16 == 0, "moe gemm: token tile %d must be a multiple of 16 in [16, 256]", bn);
   PG_REQUIRE(status != nullptr, "moe gemm: a device status word is required");
+  if (quant == 1 && bn > Q4_MAX_BN) bn = Q4_MAX_BN;  // wider tiles would leave one stage
   if (x_rows == 0 && scatter_src == nullptr) return PG_OK;
   EncodeTiledFn enc = moe_get_encode();
   PG_REQUIRE(enc != nullptr, "cuTensorMapEncodeTiled is not available from this driver");
@@ -530,6 +483,9 @@ static int moe_gemm_impl(const void* x, long long ldx, long long x_rows, const v
       PG_CUDA(cudaFuncGetAttributes(&fa, moe_gemm_kernel));
       g_static_smem = (int)fa.sharedSizeBytes;
       PG_CUDA(cudaFuncSetAttribute(moe_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_max_smem[dev & 63] - g_static_smem));
+      PG_CUDA(cudaFuncGetAttributes(&fa, moe_gemm_int4_kernel));
+      g_static_smem_q4 = (int)fa.sharedSizeBytes;
+      PG_CUDA(cudaFuncSetAttribute(moe_gemm_int4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_max_smem[dev & 63] - g_static_smem_q4));
       g_attr_set[dev & 63] = true;
     }
   }
@@ -569,11 +525,13 @@ static int moe_gemm_impl(const void* x, long long ldx, long long x_rows, const v
     p.world = world;
     p.site = site;
   }
-  const int stage_bytes = A_BYTES + bn * 128 + (quant == 1 ? RAW_BYTES : quant == 2 ? RAW_BYTES_FP8 : 0);
-  const int tail = (3 * MAX_STAGES + 4) * 8 + 64;
-  p.stages = (g_max_smem[dev & 63] - g_static_smem - 1024 - tail) / stage_bytes;
-  if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
-  if (quant) {
+  p.scale_tma = quant == 1 && K % Q4_BK == 0 && ((uintptr_t)scales & 15) == 0;
+  const int stage_bytes = quant == 1 ? Q4_RAW + Q4_SC + 4 * bn * 128 : A_BYTES + bn * 128 + (quant ? RAW_BYTES_FP8 : 0);
+  const int tail = (quant == 1 ? 2 * Q4_STAGES + 2 * Q4_BUFS + 4 : 3 * MAX_STAGES + 4) * 8 + 64;
+  p.stages = (g_max_smem[dev & 63] - (quant == 1 ? g_static_smem_q4 : g_static_smem) - 1024 - tail) / stage_bytes;
+  const int most = quant == 1 ? Q4_STAGES : MAX_STAGES;
+  if (p.stages > most) p.stages = most;
+  if (quant == 2) {
     // The four dequant groups take k-blocks 0,1,2,3 (mod 4).  With a stage count that is a
     // multiple of 4 every stage barrier is only ever waited on by one group, in order; any other
     // count lets a group wait on a barrier that is still two phases behind, and a parity wait
@@ -586,7 +544,7 @@ static int moe_gemm_impl(const void* x, long long ldx, long long x_rows, const v
   while (cols < (uint32_t)(2 * bn)) cols <<= 1;
   p.tmem_cols = cols;
 
-  CUtensorMap tm_w, tm_x;
+  CUtensorMap tm_w, tm_x, tm_s;
   cuuint32_t estr[3] = {1, 1, 1};
   if (quant == 2) {
     cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)M, (cuuint64_t)E};
@@ -598,10 +556,20 @@ static int moe_gemm_impl(const void* x, long long ldx, long long x_rows, const v
   } else if (quant == 1) {
     cuuint64_t dims[3] = {(cuuint64_t)(K / 8), (cuuint64_t)M, (cuuint64_t)E};
     cuuint64_t strides[2] = {(cuuint64_t)(K / 8) * 4, (cuuint64_t)M * (K / 8) * 4};
-    cuuint32_t box[3] = {BK / 8, BM, 1};
+    cuuint32_t box[3] = {Q4_BK / 8, BM, 1};
     CUresult r = enc(&tm_w, CU_TENSOR_MAP_DATA_TYPE_INT32, 3, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     PG_REQUIRE(r == CUDA_SUCCESS, "moe gemm: packed weight tensor map failed (%d)", (int)r);
+    if (p.scale_tma) {
+      cuuint64_t sdims[3] = {(cuuint64_t)(K / 32), (cuuint64_t)M, (cuuint64_t)E};
+      cuuint64_t sstrides[2] = {(cuuint64_t)(K / 32) * 2, (cuuint64_t)M * (K / 32) * 2};
+      cuuint32_t sbox[3] = {Q4_BK / 32, BM, 1};
+      r = enc(&tm_s, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(scales), sdims, sstrides, sbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      PG_REQUIRE(r == CUDA_SUCCESS, "moe gemm: scale tensor map failed (%d)", (int)r);
+    } else {
+      tm_s = tm_w;  // not read
+    }
   } else {
     cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)M, (cuuint64_t)E};
     cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)M * K * 2};
@@ -624,7 +592,10 @@ static int moe_gemm_impl(const void* x, long long ldx, long long x_rows, const v
     if (rc) return rc;
   }
   const size_t smem = 1024 + (size_t)p.stages * stage_bytes + tail;
-  moe_gemm_kernel<<<g_sms[dev & 63], quant ? 448 : 192, smem, stream>>>(tm_w, tm_x, p);
+  if (quant == 1)
+    moe_gemm_int4_kernel<<<g_sms[dev & 63], Q4_THREADS, smem, stream>>>(tm_w, tm_s, tm_x, p);
+  else
+    moe_gemm_kernel<<<g_sms[dev & 63], quant ? 448 : 192, smem, stream>>>(tm_w, tm_x, p);
   PG_LAUNCH_CHECK();
   return PG_OK;
 }

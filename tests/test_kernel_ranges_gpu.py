@@ -502,3 +502,24 @@ def test_gdn_conv1d_rows(channels, seqs):
     y1, y2 = cu().gdn_conv1d(x, w, st1, meta), R.gdn_conv1d(x, w, st2, meta)
     assert ((y1.float() - y2.float()).abs() <= 2 ** -7 * y2.float().abs() + 2 ** -9).all()  # as above
     assert torch.equal(st1, st2)
+
+
+@pytest.mark.parametrize("m,k,bn,aligned", [(128, 64, 16, True), (200, 128, 16, True), (136, 320, 32, True), (256, 256, 48, True), (384, 1024, 128, True), (130, 768, 64, False), (300, 2048, 128, True)])
+def test_int4_experts_of_ragged_rows(m, k, bn, aligned):
+    """Weight rows and k around tiles of 128 and stages of 256, several token tiles and empty experts, scales that TMA can read or not."""
+    torch.manual_seed(m + k)
+    rows = [0, 1, bn, bn + 1, 2 * bn - 1, 0, 3]
+    e, t = len(rows), sum(rows)
+    x = torch.randn(t, k, device=DEV).bfloat16()
+    packed = torch.randint(-(2 ** 31), 2 ** 31 - 1, (e, m, k // 8), dtype=torch.int32, device=DEV)
+    buf = (torch.rand(e * m * k // 32 + 1, device=DEV) * 0.01 + 0.001).bfloat16()
+    scales = (buf[:-1] if aligned else buf[1:]).view(e, m, k // 32)
+    offsets = torch.tensor([0] + rows).cumsum(0).to(torch.int32).to(DEV)
+    got, at = cu().grouped_gemm(x, offsets, packed, scales, bn), 0
+    for i, n in enumerate(rows):
+        a, w = x[at : at + n].double(), R.dequant_int4_g32(packed[i], scales[i]).double()
+        # products of bf16 are exact; f32 sums of k terms, one rounding to bf16
+        bound = 2 ** -8 * (a @ w.T).abs() + k * 2 ** -23 * (a.abs() @ w.abs().T)
+        assert ((got[at : at + n].double() - a @ w.T).abs() <= bound).all()
+        at += n
+    assert cu().read_status(DEV) == 0
