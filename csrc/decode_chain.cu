@@ -471,8 +471,11 @@ __global__ void __launch_bounds__(THREADS, 1) decode_chain_kernel(const __grid_c
     }
   } else if (warp == 2) {
     // ---- MMA issue ----
-    if (lane == 0) {
+    // the whole warp walks the loop and one lane issues: what does not depend on the lane stays in uniform registers
+    {
+      const bool leader = elect_one();
       const uint32_t idesc = umma_idesc_bf16_f32(BM, BN);
+      const uint64_t w_desc0 = umma_desc_k_sw128(smem_u32(wring)), x_desc0 = umma_desc_k_sw128(smem_u32(xring));
       int ws = 0, xs = 0, acc = 0;
       uint32_t wph = 0, xph = 0, acc_phase = 0;
       bool ok = true;
@@ -492,13 +495,13 @@ __global__ void __launch_bounds__(THREADS, 1) decode_chain_kernel(const __grid_c
               break;
             }
             tc_fence_after();
-            const uint32_t a_addr = smem_u32(wring + ws * W_BYTES);
-            const uint32_t b_addr = smem_u32(xring + xs * X_BYTES);
+            if (leader) {
+              const uint64_t a = w_desc0 + (uint32_t)(ws * (W_BYTES >> 4)), b = x_desc0 + (uint32_t)(xs * (X_BYTES >> 4));
 #pragma unroll
-            for (int k = 0; k < BK / 16; ++k)
-              umma_bf16_ss(d_tmem, umma_desc_k_sw128(a_addr + k * 32), umma_desc_k_sw128(b_addr + k * 32), idesc, (kb > it.kb0 || k > 0) ? 1u : 0u);
-            umma_commit(&wempty[ws]);
-            umma_commit(&xempty[xs]);
+              for (int k = 0; k < BK / 16; ++k) umma_bf16_ss(d_tmem, a + (uint32_t)(k * 2), b + (uint32_t)(k * 2), idesc, (kb > it.kb0 || k > 0) ? 1u : 0u);
+              umma_commit(&wempty[ws]);
+              umma_commit(&xempty[xs]);
+            }
             if (++ws == NW) {
               ws = 0;
               wph ^= 1u;
@@ -509,7 +512,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_chain_kernel(const __grid_c
             }
           }
           if (!ok) break;
-          umma_commit(&tfull[acc]);
+          if (leader) umma_commit(&tfull[acc]);
           acc ^= 1;
           if (acc == 0) acc_phase ^= 1u;
         }

@@ -18,8 +18,9 @@
 // banks: one row of 8 keys, 16 heads, 25.2 us for the whole operation against 23.4 now; 21.1 on the mma.sync kernel).
 //
 // Against the mma.sync kernel, in which a CTA of 16 heads exchanges partial scores through shared memory for every 32 keys
-// (128 rows x 64 heads x 1150 keys): 284 us before, 90 us now.  What
-// bounds it: the chain copy, scores, softmax, output product of a tile, 2.3 us with two tiles in flight; the keys' bytes take 26 us.
+// (128 rows x 64 heads x 1150 keys): 284 us before, 75 us now (90 with
+// a lone thread forming the descriptors of the 52 products of a tile).  What bounds it: the longest row, a block's walk; the chain
+// copy, scores, softmax, output product of a tile takes 1.9 us with two tiles in flight; the keys' bytes take 26 us.
 #include "api.h"
 #include "attention_tc.cuh"
 #include "mla_decode_tc.h"
@@ -154,10 +155,14 @@ __global__ void __launch_bounds__(DT_THREADS, 1) mla_decode_tc_kernel(const __gr
     asm volatile("bar.sync 2, 160;" ::: "memory");
   }
   if (warp == 1) {
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0) {
+      // The whole warp walks the loop and one lane issues: descriptors are sums of what does not depend on the lane, so they stay in
+      // uniform registers (formed anew by a lone thread for each product, they took longer than the product).
+      const bool leader = elect_one();
       constexpr uint32_t idesc_s = idesc_bf16(DT_KEYS, HN, 0);
       constexpr uint32_t idesc_o = idesc_bf16(128, HN, 1) | (1u << 15);  // both operands MN-major
-      const uint32_t qa = smem_u32(q_sm), pa = smem_u32(p_sm);
+      const uint32_t t0 = smem_u32(tiles);
+      const uint64_t k_desc = dt_desc_k(t0, BOX), v_desc = umma_desc_mn_sw128(t0, 1024u, BOX), q_desc = umma_desc_k_sw128(smem_u32(q_sm)), p_desc = umma_desc_mn_sw128(smem_u32(p_sm), DT_P, 1024u);
       // Whatever is ready goes first: the product with V as soon as P is there (it frees the tile's memory), the scores of the
       // next tile as soon as it has landed.  (Scores always first left a finished P waiting for a tile that could only be
       // fetched after that product: 3.9 us a tile.)
@@ -166,31 +171,35 @@ __global__ void __launch_bounds__(DT_THREADS, 1) mla_decode_tc_kernel(const __gr
       uint64_t since = globaltimer_ns();
       while (o_next < n_tiles) {
         const int ss = s_next & 1, os = o_next & 1;
-        if (s_next > o_next && mbar_try_wait(&sh->p_ready, (uint32_t)(o_next & 1))) {
+        if (s_next > o_next && __all_sync(0xFFFFFFFFu, mbar_try_wait(&sh->p_ready, (uint32_t)(o_next & 1)))) {
           tc_fence_after();
-          const uint32_t va = smem_u32(tiles + os * STAGE);
+          if (leader) {
+            const uint64_t v = v_desc + (uint32_t)(os * (STAGE >> 4));
 #pragma unroll
-          for (int mb = 0; mb < 4; ++mb)
+            for (int mb = 0; mb < 4; ++mb)
 #pragma unroll
-            for (int ks = 0; ks < DT_KEYS / 16; ++ks)
-              umma_bf16_ss(tmem + (uint32_t)((2 + mb) * HN), umma_desc_mn_sw128(va + mb * 2048 + ks * 2 * BOX, 1024u, BOX), umma_desc_mn_sw128(pa + ks * 2048, DT_P, 1024u), idesc_o,
-                           (o_next | ks) ? 1u : 0u);
-          umma_commit(&sh->o_full);
-          umma_commit(&sh->empty[os]);
+              for (int ks = 0; ks < DT_KEYS / 16; ++ks)
+                umma_bf16_ss(tmem + (uint32_t)((2 + mb) * HN), v + (uint32_t)((mb * 2048 + ks * 2 * BOX) >> 4), p_desc + (uint32_t)(ks * 128), idesc_o, (o_next | ks) ? 1u : 0u);
+            umma_commit(&sh->o_full);
+            umma_commit(&sh->empty[os]);
+          }
           ++o_next;
-        } else if (s_next < n_tiles && s_next <= o_next + 1 && mbar_try_wait(&sh->full[ss], (uint32_t)((s_next >> 1) & 1)) &&
-                   ((s_next != ragged && s_next != head) || mbar_try_wait(&sh->cleared, s_next != head && head >= 0 ? 1u : 0u))) {
+        } else if (s_next < n_tiles && s_next <= o_next + 1 &&
+                   __all_sync(0xFFFFFFFFu, mbar_try_wait(&sh->full[ss], (uint32_t)((s_next >> 1) & 1)) &&
+                                               ((s_next != ragged && s_next != head) || mbar_try_wait(&sh->cleared, s_next != head && head >= 0 ? 1u : 0u)))) {
           tc_fence_after();
-          const uint32_t ka = smem_u32(tiles + ss * STAGE);
+          if (leader) {
+            const uint64_t k = k_desc + (uint32_t)(ss * (STAGE >> 4));
 #pragma unroll
-          for (int cb = 0; cb < QKB; ++cb)
+            for (int cb = 0; cb < QKB; ++cb)
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma_bf16_ss(tmem + (uint32_t)(ss * HN), dt_desc_k(ka + cb * 1024 + k * 32, BOX), umma_desc_k_sw128(qa + cb * QBLK + k * 32), idesc_s, (cb | k) ? 1u : 0u);
-          umma_commit(&sh->s_full[ss]);
+              for (int i = 0; i < 4; ++i)
+                umma_bf16_ss(tmem + (uint32_t)(ss * HN), k + (uint32_t)(cb * 64 + i * 2), q_desc + (uint32_t)(cb * (QBLK >> 4) + i * 2), idesc_s, (cb | i) ? 1u : 0u);
+            umma_commit(&sh->s_full[ss]);
+          }
           ++s_next;
         } else {
-          if ((++spins & 63u) == 0u && (*abort_flag || globaltimer_ns() - since > PG_WAIT_LIMIT_NS)) {
+          if (__any_sync(0xFFFFFFFFu, (++spins & 63u) == 0u && (*abort_flag || globaltimer_ns() - since > PG_WAIT_LIMIT_NS))) {
             *abort_flag = 1;
             break;
           }
