@@ -133,7 +133,6 @@ int pg_mla_append(const void* kv_a, long long ld, const void* norm_w, const void
                   void* latent, int tokens, int c, int rope, int max_pos, long long num_slots, float eps, void* status, cudaStream_t stream);
 int pg_mla_q_prep(const void* q, const void* cos, const void* sin, const void* positions, void* q_nope_hm, void* q_pe, int tokens, int heads,
                   int nope, int rope, int max_pos, cudaStream_t stream);
-int pg_permute_021(const void* in, void* out, int A, int B, int D, cudaStream_t stream);
 int pg_mla_attention(const void* q_abs, const void* q_pe, const void* latent, void* out, const void* q_indptr, const void* kv_lens,
                      const void* table, int table_stride, const void* unit_seq, int num_seqs, int tokens, int heads, int c, int rope,
                      int page_size, float scale, int splits, int tc, void* part_o, void* part_lse, long long num_pages, void* status, cudaStream_t stream);

@@ -22,7 +22,6 @@
 //    rotate_pairs_: the same rotation in place on the query columns, for the expanded prefill form.
 //  * latent_attention_plain: the absorbed form on the CUDA cores for f32 and for sizes the tensor-core
 //    kernel does not address.
-//  * permute_021: [A, B, D] -> [B, A, D] row permutation (head-major <-> token-major).
 //
 // Functional parity with pegainfer-kernels/csrc/kimi_k2/kimi_mla.cu:83-885 (split/norm,
 // rope, paged append, absorbed batch decode), csrc/deepseek_v2_lite/dsv2_lite_attention.cu
@@ -155,14 +154,6 @@ __global__ void __launch_bounds__(128) mla_q_prep_x4_kernel(const bf16* __restri
   bf16* dp = q_pe + ((long long)t * heads + h0 + h) * 64 + c * 4;
   *reinterpret_cast<uint2*>(dp) = make_uint2(pack_bf16(lo[0], lo[1]), pack_bf16(lo[2], lo[3]));
   *reinterpret_cast<uint2*>(dp + 32) = make_uint2(pack_bf16(hi[0], hi[1]), pack_bf16(hi[2], hi[3]));
-}
-
-__global__ void permute_021_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, int A, int B, int D) {
-  const long long row = blockIdx.x;  // output row index b * A + a
-  const int b = (int)(row / A), a = (int)(row % A);
-  const uint4* src = reinterpret_cast<const uint4*>(in + ((long long)a * B + b) * D);
-  uint4* dst = reinterpret_cast<uint4*>(out + row * D);
-  for (int i = threadIdx.x; i < D / 8; i += blockDim.x) dst[i] = src[i];
 }
 
 struct MlaParams {
@@ -660,21 +651,13 @@ extern "C" int pg_mla_q_prep(const void* q, const void* cos, const void* sin, co
   return PG_OK;
 }
 
-extern "C" int pg_permute_021(const void* in, void* out, int A, int B, int D, cudaStream_t stream) {
-  PG_REQUIRE(D % 8 == 0, "permute: inner dim %d must be a multiple of 8", D);
-  if ((long long)A * B == 0) return PG_OK;
-  permute_021_kernel<<<(unsigned)((long long)A * B), 64, 0, stream>>>((const bf16*)in, (bf16*)out, A, B, D);
-  PG_LAUNCH_CHECK();
-  return PG_OK;
-}
-
 extern "C" int pg_mla_attention(const void* q_abs, const void* q_pe, const void* latent, void* out, const void* q_indptr, const void* kv_lens,
                                 const void* table, int table_stride, const void* unit_seq, int num_seqs, int tokens, int heads, int c, int rope,
                                 int page_size, float scale, int splits, int tc, void* part_o, void* part_lse, long long num_pages, void* status, cudaStream_t stream) {
   PG_REQUIRE(c == 512 && rope == 64, "mla_attention: built for kv_lora 512 + rope 64 (got %d + %d)", c, rope);
   PG_REQUIRE(heads % 16 == 0, "mla_attention: heads %d must be a multiple of 16", heads);
-  // head-major absorbed queries and outputs, token-major rotated query parts
-  return pg_latent_attention(q_abs, c, (long long)tokens * c, q_pe, (long long)heads * rope, rope, nullptr, nullptr, 0, latent, out, c, (long long)tokens * c, q_indptr, kv_lens, table, table_stride, unit_seq, 0,
+  // absorbed queries, rotated query parts and outputs [tokens, heads, ..]
+  return pg_latent_attention(q_abs, (long long)heads * c, c, q_pe, (long long)heads * rope, rope, nullptr, nullptr, 0, latent, out, (long long)heads * c, c, q_indptr, kv_lens, table, table_stride, unit_seq, 0,
                              num_seqs, tokens, heads, c, rope, page_size, scale, 0, nullptr, nullptr, 0, splits, tc, part_o, part_lse, num_pages, status, stream);
 }
 

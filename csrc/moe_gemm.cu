@@ -88,6 +88,14 @@ struct ItemCursor {
 };
 
 __device__ __forceinline__ bool locate(const MoeGemmParams& p, const int* s_tiles, int item, ItemCursor& c, Item& out) {
+  if (p.head_rows) {  // all heads alike: no list to walk (64 heads and one item an SM: a microsecond of dependent reads)
+    const int n_tiles = (p.head_rows + p.bn - 1) / p.bn, mt = item / n_tiles;
+    out.e = mt / p.m_tiles;
+    out.m_tile = mt - out.e * p.m_tiles;
+    out.row0 = (item - mt * n_tiles) * p.bn;
+    out.rows = min(p.bn, p.head_rows - out.row0);
+    return true;
+  }
   while (c.e < p.E && item >= c.base + s_tiles[c.e]) {
     c.base += s_tiles[c.e];
     ++c.e;
@@ -98,7 +106,7 @@ __device__ __forceinline__ bool locate(const MoeGemmParams& p, const int* s_tile
   out.e = c.e;
   out.m_tile = local / n_tiles;
   const int n_tile = local - out.m_tile * n_tiles;
-  const int r0 = p.head_rows ? 0 : p.offsets[c.e], r1 = p.head_rows ? p.head_rows : p.offsets[c.e + 1];
+  const int r0 = p.offsets[c.e], r1 = p.offsets[c.e + 1];
   out.row0 = r0 + n_tile * p.bn;
   out.rows = min(p.bn, r1 - out.row0);
   return true;
@@ -115,6 +123,25 @@ __device__ __forceinline__ bool named_bar_all(int id, int nthreads, bool pred) {
       : "r"((uint32_t)pred), "r"(id), "r"(nthreads)
       : "memory");
   return r != 0;
+}
+
+// Per-expert item counts and their sum (every CTA derives the same list from the routing offsets); ends with a barrier over
+// the block, behind which the roles start.
+__device__ __forceinline__ void count_items(const MoeGemmParams& p, int* s_tiles, int* s_total) {
+  for (int e = threadIdx.x; !p.head_rows && e < p.E; e += blockDim.x) {
+    const int n = p.offsets[e + 1] - p.offsets[e];
+    s_tiles[e] = n > 0 ? p.m_tiles * ((n + p.bn - 1) / p.bn) : 0;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (threadIdx.x < 32) {
+    int t = 0;
+    for (int e = threadIdx.x; !p.head_rows && e < p.E; e += 32) t += s_tiles[e];
+    t = __reduce_add_sync(0xffffffffu, t);
+    if (threadIdx.x == 0) *s_total = p.head_rows ? p.E * p.m_tiles * ((p.head_rows + p.bn - 1) / p.bn) : t;
+  }
+  __syncthreads();
 }
 
 // One output tile from tensor memory: the thread's weight row `m`, whose f32 results of the tile's token rows start at `t_row`.
@@ -222,24 +249,13 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     tma_prefetch_desc(&tm_w);
     tma_prefetch_desc(&tm_x);
   }
-  // per-expert item counts (every CTA derives the same list from the routing offsets)
-  for (int e = threadIdx.x; e < p.E; e += blockDim.x) {
-    const int n = p.head_rows ? p.head_rows : p.offsets[e + 1] - p.offsets[e];
-    s_tiles[e] = n > 0 ? p.m_tiles * ((n + p.bn - 1) / p.bn) : 0;
-  }
   if (warp == 1) {
     tmem_alloc(tmem_slot, p.tmem_cols);
     tmem_relinquish();
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int e = 0; e < p.E; ++e) t += s_tiles[e];
-    s_total = t;
-  }
-  __syncthreads();
+  pdl_wait();
+  count_items(p, s_tiles, &s_total);
+  pdl_launch_dependents();  // (behind the allocation above: a dependent that takes tensor memory must not be first)
   const uint32_t tmem_base = *tmem_slot;
   const int total = s_total;
   uint32_t ep_epoch = 0;
@@ -297,8 +313,11 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    // the whole warp walks the loop and one lane issues: what does not depend on the lane stays in uniform registers
+    {
+      const bool leader = elect_one();
       const uint32_t idesc = umma_idesc_bf16_f32(BM, (uint32_t)p.bn);
+      const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(tiles));
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -315,19 +334,19 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             break;
           }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(tiles + stage * stage_bytes);
-          const uint32_t b_addr = a_addr + A_BYTES;
+          if (leader) {
+            const uint64_t a = a_desc0 + (uint32_t)(stage * (stage_bytes >> 4));
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            umma_bf16_ss(d_tmem, umma_desc_k_sw128(a_addr + k * 32), umma_desc_k_sw128(b_addr + k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit(&empty[stage]);
+            for (int k = 0; k < BK / 16; ++k) umma_bf16_ss(d_tmem, a + (uint32_t)(k * 2), a + (uint32_t)((A_BYTES >> 4) + k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_commit(&empty[stage]);
+          }
           if (++stage == p.stages) {
             stage = 0;
             phase ^= 1u;
           }
         }
         if (!ok) break;
-        umma_commit(&tfull[acc]);
+        if (leader) umma_commit(&tfull[acc]);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
       }
@@ -580,7 +599,8 @@ static int moe_gemm_impl(const void* x, long long ldx, long long x_rows, const v
   }
   if (heads) {
     PG_REQUIRE(((uintptr_t)x & 15) == 0 && ldx % 8 == 0 && heads->x_head % 8 == 0, "head gemm: activations must start and step on 16-byte boundaries");
-    PG_REQUIRE(heads->x_head >= K && ldx >= heads->x_head * E, "head gemm: heads lie inside a row (row stride %lld, head stride %lld, %d heads of %d)", ldx, heads->x_head, E, K);
+    PG_REQUIRE((heads->x_head >= K && ldx >= heads->x_head * E) || (ldx >= K && heads->x_head >= ldx * x_rows),
+               "head gemm: heads lie inside a row or rows inside a head (row stride %lld, head stride %lld, %d heads of %d)", ldx, heads->x_head, E, K);
     cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)E, (cuuint64_t)x_rows};
     cuuint64_t strides[2] = {(cuuint64_t)heads->x_head * 2, (cuuint64_t)ldx * 2};
     cuuint32_t box[3] = {BK, 1, (cuuint32_t)bn};
@@ -593,9 +613,9 @@ static int moe_gemm_impl(const void* x, long long ldx, long long x_rows, const v
   }
   const size_t smem = 1024 + (size_t)p.stages * stage_bytes + tail;
   if (quant == 1)
-    moe_gemm_int4_kernel<<<g_sms[dev & 63], Q4_THREADS, smem, stream>>>(tm_w, tm_s, tm_x, p);
+    PG_CUDA(launch_pdl(moe_gemm_int4_kernel, dim3(g_sms[dev & 63]), dim3(Q4_THREADS), smem, stream, tm_w, tm_s, tm_x, p));
   else
-    moe_gemm_kernel<<<g_sms[dev & 63], quant ? 448 : 192, smem, stream>>>(tm_w, tm_x, p);
+    PG_CUDA(launch_pdl(moe_gemm_kernel, dim3(g_sms[dev & 63]), dim3(quant ? 448 : 192), smem, stream, tm_w, tm_x, p));
   PG_LAUNCH_CHECK();
   return PG_OK;
 }

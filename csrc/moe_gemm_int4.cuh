@@ -8,6 +8,10 @@
 // global memory by each thread they were 128 sectors a k-block): 256-deep stages make a row of eight of them the 16 bytes that
 // a TMA row needs.
 //
+// 48 experts of 7168 x 2048, top 8 (routing and both products): 128 tokens 684 us with the A tile in shared memory, 534 now, of
+// which 70 by the issue of products from uniform registers (gemm_sm100.cu).  The weights' bytes take 182 us; a product of 128 rows
+// and few columns occupies the tensor core for 45 cycles whatever its columns, 165 us of this.
+//
 // warp 0 TMA producer | warp 1 MMA issuer + TMEM owner | warps 2-5 epilogue | then Q4_GROUPS groups of four dequant warps.
 // Group g expands the k-blocks g, g + Q4_GROUPS, .. of the four of a stage into one of eight TMEM buffers.
 constexpr int Q4_GROUPS = 2;             // divides 4
@@ -57,23 +61,13 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     tma_prefetch_desc(&tm_x);
     if (p.scale_tma) tma_prefetch_desc(&tm_s);
   }
-  for (int e = threadIdx.x; e < p.E; e += blockDim.x) {
-    const int n = p.offsets[e + 1] - p.offsets[e];
-    s_tiles[e] = n > 0 ? p.m_tiles * ((n + p.bn - 1) / p.bn) : 0;
-  }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int e = 0; e < p.E; ++e) t += s_tiles[e];
-    s_total = t;
-  }
-  __syncthreads();
+  pdl_wait();
+  count_items(p, s_tiles, &s_total);
+  pdl_launch_dependents();  // (behind the allocation above: a dependent that takes tensor memory must not be first)
   const uint32_t tmem_base = *tmem_slot;
   const int total = s_total;
   const int depth = (p.K + Q4_BK - 1) / Q4_BK;  // stages of an item; TMA fills what lies past K with zeros on every operand
@@ -119,8 +113,10 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    const bool leader = elect_one();
+    {
       const uint32_t idesc = umma_idesc_bf16_f32(BM, (uint32_t)p.bn);
+      const uint64_t x_desc0 = umma_desc_k_sw128(smem_u32(tiles) + Q4_RAW + Q4_SC);
       int stage = 0;
       uint32_t phase = 0, turn = 0;
       int acc = 0;
@@ -135,7 +131,8 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             ok = false;
             break;
           }
-          const uint32_t x_addr = smem_u32(tiles + stage * stage_bytes) + Q4_RAW + Q4_SC;
+          const uint64_t x_desc = x_desc0 + (uint32_t)(stage * (stage_bytes >> 4));
+#pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int b = (int)(turn & 1u) * 4 + i;
             if (!mbar_wait(&aready[b], (turn >> 1) & 1u, abort_flag)) {
@@ -143,20 +140,22 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
               break;
             }
             tc_fence_after();
+            if (leader) {
 #pragma unroll
-            for (int k = 0; k < BK / 16; ++k)
-              umma_bf16_ts(d_tmem, tmem_base + 256u + (uint32_t)(b * 32 + k * 8), umma_desc_k_sw128(x_addr + i * x_bytes + k * 32), idesc, (d | i | k) ? 1u : 0u);
-            umma_commit(&afree[b]);
+              for (int k = 0; k < BK / 16; ++k)
+                umma_bf16_ts(d_tmem, tmem_base + 256u + (uint32_t)(b * 32 + k * 8), x_desc + (uint32_t)(i * (x_bytes >> 4) + k * 2), idesc, (d | i | k) ? 1u : 0u);
+              umma_commit(&afree[b]);
+              if (i == 3) umma_commit(&empty[stage]);
+            }
           }
           if (!ok) break;
-          umma_commit(&empty[stage]);
           if (++stage == p.stages) {
             stage = 0;
             phase ^= 1u;
           }
         }
         if (!ok) break;
-        umma_commit(&tfull[acc]);
+        if (leader) umma_commit(&tfull[acc]);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
       }

@@ -45,6 +45,7 @@ __device__ __forceinline__ void warp_argmax(float& v, int& i) {
 }
 
 __global__ void __launch_bounds__(128) router_topk_kernel(const RouterParams p) {
+  PG_PDL_ENTRY();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + warp;
   if (t >= p.tokens) return;
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const RouterParams p) 
 // One CTA: stable counting sort of the routes by local expert (see route_sort.cuh).
 __global__ void __launch_bounds__(ROUTE_SORT_THREADS) moe_align_kernel(const int* __restrict__ ids, int routes, int e0, int e_local, int* __restrict__ offsets,
                                                                         int* __restrict__ sorted_src, int* __restrict__ route_pos) {
+  PG_PDL_ENTRY();
   __shared__ RouteSortSmem sm;
   route_sort(
       sm, routes, e_local, offsets, [&](int i) { return ids[i] - e0; },
@@ -180,6 +182,7 @@ __global__ void __launch_bounds__(ROUTE_SORT_THREADS) moe_align_kernel(const int
 
 __global__ void moe_gather_kernel(const bf16* __restrict__ x, long long ldx, const int* __restrict__ sorted_src, const int* __restrict__ offsets,
                                   int e_local, int k, bf16* __restrict__ out, int width) {
+  PG_PDL_ENTRY();
   const int row = blockIdx.x;
   if (row >= offsets[e_local]) return;
   const int tok = sorted_src[row] / k;
@@ -193,6 +196,7 @@ __global__ void moe_gather_kernel(const bf16* __restrict__ x, long long ldx, con
 // block per token, 7.5 us now).
 __global__ void __launch_bounds__(128) moe_combine_kernel(const bf16* __restrict__ y, long long ldy, const int* __restrict__ route_pos, const float* __restrict__ weights,
                                    int k, float* __restrict__ out, int width, int accumulate) {
+  PG_PDL_ENTRY();
   const int t = blockIdx.x;
   for (int i = blockIdx.y * 128 + threadIdx.x; i < width / 8; i += gridDim.y * 128) {
     float acc[8];
@@ -237,14 +241,14 @@ extern "C" int pg_router_topk(const void* logits, long long ld, const void* bias
   p.group_top = group_top;
   p.norm = norm;
   p.scale = scale;
-  router_topk_kernel<<<(tokens + 3) / 4, 128, 0, stream>>>(p);
+  PG_CUDA(launch_pdl(router_topk_kernel, dim3((tokens + 3) / 4), dim3(128), (size_t)0, stream, p));
   PG_LAUNCH_CHECK();
   return PG_OK;
 }
 
 extern "C" int pg_moe_align(const void* ids, int routes, int e0, int e_local, void* offsets, void* sorted_src, void* route_pos, cudaStream_t stream) {
   PG_REQUIRE(e_local >= 1 && e_local <= 512, "moe_align: %d local experts not supported (<= 512)", e_local);
-  moe_align_kernel<<<1, ROUTE_SORT_THREADS, 0, stream>>>((const int*)ids, routes, e0, e_local, (int*)offsets, (int*)sorted_src, (int*)route_pos);
+  PG_CUDA(launch_pdl(moe_align_kernel, dim3(1), dim3(ROUTE_SORT_THREADS), (size_t)0, stream, (const int*)ids, routes, e0, e_local, (int*)offsets, (int*)sorted_src, (int*)route_pos));
   PG_LAUNCH_CHECK();
   return PG_OK;
 }
@@ -253,7 +257,7 @@ extern "C" int pg_moe_gather(const void* x, long long ldx, const void* sorted_sr
                              int max_rows, cudaStream_t stream) {
   PG_REQUIRE(width % 8 == 0, "moe_gather: width must be a multiple of 8");
   if (max_rows == 0) return PG_OK;
-  moe_gather_kernel<<<max_rows, 128, 0, stream>>>((const bf16*)x, ldx, (const int*)sorted_src, (const int*)offsets, e_local, k, (bf16*)out, width);
+  PG_CUDA(launch_pdl(moe_gather_kernel, dim3(max_rows), dim3(128), (size_t)0, stream, (const bf16*)x, ldx, (const int*)sorted_src, (const int*)offsets, e_local, k, (bf16*)out, width));
   PG_LAUNCH_CHECK();
   return PG_OK;
 }
@@ -264,7 +268,8 @@ extern "C" int pg_moe_combine(const void* y, long long ldy, const void* route_po
   if (tokens == 0) return PG_OK;
   // columns are split only as far as the tokens leave SMs idle: 1711 tokens fill them
   const int pieces = (width / 8 + 127) / 128, parts = tokens >= 1184 ? 1 : (1184 + tokens - 1) / tokens;
-  moe_combine_kernel<<<dim3(tokens, parts < pieces ? parts : pieces), 128, 0, stream>>>((const bf16*)y, ldy, (const int*)route_pos, (const float*)weights, k, (float*)out, width, accumulate);
+  PG_CUDA(launch_pdl(moe_combine_kernel, dim3(tokens, parts < pieces ? parts : pieces), dim3(128), (size_t)0, stream, (const bf16*)y, ldy, (const int*)route_pos, (const float*)weights, k, (float*)out, width,
+                     accumulate));
   PG_LAUNCH_CHECK();
   return PG_OK;
 }

@@ -1583,19 +1583,6 @@ def mla_rope_q(q, cos, sin, meta: AttnMeta, nope):
     return _MlaQ(nope_hm, pe, t, h, nope)
 
 
-_HEAD_OFFSETS: dict = {}
-
-
-def _head_offsets(heads: int, tokens: int, device):
-    key = (heads, tokens, device.index)
-    o = _HEAD_OFFSETS.get(key)
-    if o is None:
-        o = (torch.arange(heads + 1, dtype=torch.int32, device=device) * tokens).contiguous()
-        if len(_HEAD_OFFSETS) < 512:
-            _HEAD_OFFSETS[key] = o
-    return o
-
-
 def _latent_keys(meta: AttnMeta, row0: int = 0, window: int = 0) -> int:
     """Keys of a typical row of a step from row ``row0`` on, for the choice of a kernel: the rows' mean where the lengths are known here, but at
     least half of the longest, which one block walks."""
@@ -1732,6 +1719,7 @@ def mla_attention(q: "_MlaQ", w_uk, w_uv, latent_layer, meta: AttnMeta, scale, k
     """``w_uk`` [H, nope, kv_lora], ``w_uv`` [H, v, kv_lora].  The absorb GEMM wants W_UK as
     an [out = kv_lora, in = nope] weight per head; that transposed copy is made once per
     layer and kept."""
+    assert w_uk.dtype == w_uv.dtype == torch.bfloat16, "mla_attention: bf16 up-projections"
     w_uk_t = getattr(w_uk, "_pg_transposed", None)  # lives and dies with the weight tensor
     if w_uk_t is None:
         w_uk_t = w_uk.transpose(1, 2).contiguous()
@@ -1746,9 +1734,8 @@ def mla_attention(q: "_MlaQ", w_uk, w_uv, latent_layer, meta: AttnMeta, scale, k
         return _mla_prefill_expanded(q, w_uk, w_uv, latent_layer, meta, scale, kv_lora)
     if n_pf > 0:
         return _mla_split_step(q, w_uk, w_uv, latent_layer, meta, scale, kv_lora, n_pf)
-    offs = _head_offsets(h, t, dev)
-    bn = _token_tile(h * t, h)
-    q_abs = grouped_gemm(q.nope_hm.view(h * t, q.nope), offs, w_uk_t, None, bn)  # [H*T, kv_lora]
+    q_abs = torch.empty((t, h, kv_lora), dtype=torch.bfloat16, device=dev)
+    _head_gemm(q.nope_hm, q.nope_hm.stride(1), q.nope_hm.stride(0), w_uk_t, q_abs)
     rope = q.pe.shape[-1]
     page_size = latent_layer.shape[1]
     if meta.decode_only:
@@ -1766,15 +1753,14 @@ def mla_attention(q: "_MlaQ", w_uk, w_uv, latent_layer, meta: AttnMeta, scale, k
         splits = 1
     part_o = c.attn_part
     part_lse = c.attn_part[t * h * splits * kv_lora * 4 :]
-    lat_out = torch.empty((h * t, kv_lora), dtype=torch.bfloat16, device=dev)
+    lat_out = torch.empty((t, h, kv_lora), dtype=torch.bfloat16, device=dev)
     rc = lib().pg_mla_attention(_ptr(q_abs), _ptr(q.pe), _ptr(latent_layer), _ptr(lat_out), _ptr(meta.q_indptr), _ptr(meta.kv_lens), _ptr(meta.block_table),
                                 _ci(meta.block_table.stride(0)), _ptr(unit_seq), _ci(meta.num_seqs), _ci(t), _ci(h), _ci(kv_lora), _ci(rope), _ci(page_size), _cf(scale),
                                 _ci(splits), _ci(int(tc)), _ptr(part_o), _ptr(part_lse), _ll(latent_layer.shape[0]), _ptr(c.status), _stream())
     _check(rc, c, 2 if splits > 1 else 1)
-    v_hm = grouped_gemm(lat_out, offs, w_uv, None, bn)  # [H*T, v]
     vdim = w_uv.shape[1]
     out = torch.empty((t, h * vdim), dtype=torch.bfloat16, device=dev)
-    _check(lib().pg_permute_021(_ptr(v_hm), _ptr(out), _ci(h), _ci(t), _ci(vdim), _stream()), c)
+    _head_gemm(lat_out, h * kv_lora, kv_lora, w_uv, out.view(t, h, vdim))
     return out
 
 
