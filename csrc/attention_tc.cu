@@ -209,10 +209,12 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_attn_tc_kernel(const __gri
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0) {
+      const bool leader = elect_one();  // the warp walks the loop, one lane issues: descriptors in uniform registers (gemm_sm100.cu)
       constexpr uint32_t idesc_s = idesc_bf16(128, 128, 0);
       constexpr uint32_t idesc_o = idesc_bf16(128, 128, 1);
       const uint32_t lbo = p.mn_lbo_first ? (uint32_t)HALF_BYTES : 1024u, sbo = p.mn_lbo_first ? 1024u : (uint32_t)HALF_BYTES;
+      const uint64_t q_desc = umma_desc_k_sw128(smem_u32(q_tile)), k_desc = umma_desc_k_sw128(smem_u32(k_tile)), v_desc = umma_desc_mn_sw128(smem_u32(v_tile), lbo, sbo);
       bool ok = mbar_wait(&sh->q_full, 0, abort_flag);
       int k_seen = -1, v_seen = -1;  // tiles whose K / V arrival this thread has already observed
       // S of group g, tile j.  K_j is released once the last group that needs it has issued its S.  S of tile j
@@ -226,16 +228,17 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_attn_tc_kernel(const __gri
           k_seen = j;
         }
         tc_fence_after();
-        const uint32_t qa = smem_u32(q_tile + g * TILE_BYTES), ka = smem_u32(k_tile + st * TILE_BYTES);
-#pragma unroll
-        for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_bf16_ss(tmem + (uint32_t)(g * 128), umma_desc_k_sw128(qa + kb * HALF_BYTES + k * 32), umma_desc_k_sw128(ka + kb * HALF_BYTES + k * 32), idesc_s,
-                         (kb | k) ? 1u : 0u);
-        umma_commit(&sh->s_full[g]);
         const bool last_user = (g == GROUPS - 1) || j >= n_g[GROUPS - 1];
-        if (last_user) umma_commit(&sh->k_empty[st]);
+        if (leader) {
+          const uint64_t qa = q_desc + (uint32_t)(g * (TILE_BYTES >> 4)), ka = k_desc + (uint32_t)(st * (TILE_BYTES >> 4));
+#pragma unroll
+          for (int kb = 0; kb < 2; ++kb)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              umma_bf16_ss(tmem + (uint32_t)(g * 128), qa + (uint32_t)(kb * (HALF_BYTES >> 4) + k * 2), ka + (uint32_t)(kb * (HALF_BYTES >> 4) + k * 2), idesc_s, (kb | k) ? 1u : 0u);
+          umma_commit(&sh->s_full[g]);
+          if (last_user) umma_commit(&sh->k_empty[st]);
+        }
         return true;
       };
       // O_g (+)= P_g V_j with P_g read from tensor memory.  V_j is released once the last group that needs it has
@@ -249,14 +252,15 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_attn_tc_kernel(const __gri
           v_seen = j;
         }
         tc_fence_after();
-        const uint32_t va = smem_u32(v_tile + st * TILE_BYTES);
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ts(tmem + 256u + (uint32_t)(g * 128), tmem + (uint32_t)(g * 128) + (uint32_t)(ks * 8), umma_desc_mn_sw128(va + ks * 2048, lbo, sbo), idesc_o,
-                       (j | ks) ? 1u : 0u);
-        umma_commit(&sh->o_full[g]);
         const bool last_user = (g == GROUPS - 1) || j >= n_g[GROUPS - 1];
-        if (last_user) umma_commit(&sh->v_empty[st]);
+        if (leader) {
+          const uint64_t va = v_desc + (uint32_t)(st * (TILE_BYTES >> 4));
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks)
+            umma_bf16_ts(tmem + 256u + (uint32_t)(g * 128), tmem + (uint32_t)(g * 128) + (uint32_t)(ks * 8), va + (uint32_t)(ks * 128), idesc_o, (j | ks) ? 1u : 0u);
+          umma_commit(&sh->o_full[g]);
+          if (last_user) umma_commit(&sh->v_empty[st]);
+        }
         return true;
       };
       ok = ok && issue_s(0, 0) && issue_s(1, 0);
@@ -592,10 +596,12 @@ __global__ void __launch_bounds__(THREADS2, 1) prefill_attn_tc256_kernel(const _
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0) {
+      const bool leader = elect_one();  // the warp walks the loop, one lane issues: descriptors in uniform registers (gemm_sm100.cu)
       constexpr uint32_t idesc_s = idesc_bf16(128, BKV2, 0);
       constexpr uint32_t idesc_o = idesc_bf16(128, D2, 1);
       const uint32_t lbo = p.mn_lbo_first ? (uint32_t)KV2_BLOCK : 1024u, sbo = p.mn_lbo_first ? 1024u : (uint32_t)KV2_BLOCK;
+      const uint64_t q_desc = umma_desc_k_sw128(smem_u32(q_tile)), k_desc = umma_desc_k_sw128(smem_u32(k_tile)), v_desc = umma_desc_mn_sw128(smem_u32(v_tile), lbo, sbo);
       bool ok = mbar_wait(&sh->q_full, 0, abort_flag);
       // S of tile j into buffer j & 1.  It overwrites S and P of tile j - 2: the product that read that P was issued
       // before, and the tensor core runs this thread's instructions in order.
@@ -604,15 +610,16 @@ __global__ void __launch_bounds__(THREADS2, 1) prefill_attn_tc256_kernel(const _
         const int st = j & 1;
         if (!mbar_wait(&sh->k_full[st], (uint32_t)((j >> 1) & 1), abort_flag)) return false;
         tc_fence_after();
-        const uint32_t qa = smem_u32(q_tile), ka = smem_u32(k_tile + st * KV2_BYTES);
+        if (leader) {
+          const uint64_t ka = k_desc + (uint32_t)(st * (KV2_BYTES >> 4));
 #pragma unroll
-        for (int cb = 0; cb < 4; ++cb)
+          for (int cb = 0; cb < 4; ++cb)
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_bf16_ss(tmem + 256u + (uint32_t)(st * BKV2), umma_desc_k_sw128(qa + cb * (BQ1 * 128) + k * 32), umma_desc_k_sw128(ka + cb * KV2_BLOCK + k * 32), idesc_s,
-                         (cb | k) ? 1u : 0u);
-        umma_commit(&sh->s_full[st]);
-        umma_commit(&sh->k_empty[st]);
+            for (int k = 0; k < 4; ++k)
+              umma_bf16_ss(tmem + 256u + (uint32_t)(st * BKV2), q_desc + (uint32_t)(cb * (BQ1 * 8) + k * 2), ka + (uint32_t)(cb * (KV2_BLOCK >> 4) + k * 2), idesc_s, (cb | k) ? 1u : 0u);
+          umma_commit(&sh->s_full[st]);
+          umma_commit(&sh->k_empty[st]);
+        }
         return true;
       };
       ok = ok && issue_s(0) && issue_s(1);
@@ -621,12 +628,14 @@ __global__ void __launch_bounds__(THREADS2, 1) prefill_attn_tc256_kernel(const _
         ok = mbar_wait(&sh->p_ready[st], (uint32_t)((j >> 1) & 1), abort_flag) && mbar_wait(&sh->v_full[st], (uint32_t)((j >> 1) & 1), abort_flag);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t va = smem_u32(v_tile + st * KV2_BYTES);
+        if (leader) {
+          const uint64_t va = v_desc + (uint32_t)(st * (KV2_BYTES >> 4));
 #pragma unroll
-        for (int ks = 0; ks < BKV2 / 16; ++ks)
-          umma_bf16_ts(tmem, tmem + 256u + (uint32_t)(st * BKV2) + (uint32_t)(ks * 8), umma_desc_mn_sw128(va + ks * 2048, lbo, sbo), idesc_o, (j | ks) ? 1u : 0u);
-        umma_commit(&sh->o_full);
-        umma_commit(&sh->v_empty[st]);
+          for (int ks = 0; ks < BKV2 / 16; ++ks)
+            umma_bf16_ts(tmem, tmem + 256u + (uint32_t)(st * BKV2) + (uint32_t)(ks * 8), va + (uint32_t)(ks * 128), idesc_o, (j | ks) ? 1u : 0u);
+          umma_commit(&sh->o_full);
+          umma_commit(&sh->v_empty[st]);
+        }
         ok = issue_s(j + 2);
       }
     }

@@ -148,10 +148,12 @@ __global__ void __launch_bounds__(THREADS, 1) mla_prefill_tc_kernel(const __grid
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0) {
+      const bool leader = elect_one();  // the warp walks the loop, one lane issues: descriptors in uniform registers (gemm_sm100.cu)
       constexpr uint32_t idesc_s = idesc_bf16(128, BKV2, 0);
       constexpr uint32_t idesc_o = idesc_bf16(128, 128, 1);
       constexpr uint32_t lbo = 8192u, sbo = 1024u;
+      const uint64_t q_desc = umma_desc_k_sw128(smem_u32(q_tile)), k_desc = umma_desc_k_sw128(smem_u32(k_tile)), v_desc = umma_desc_mn_sw128(smem_u32(v_tile), lbo, sbo);
       bool ok = mbar_wait(&sh->q_full, 0, abort_flag);
       int k_seen = -1, v_seen = -1;
       auto issue_s = [&](int g, int j) {
@@ -162,15 +164,16 @@ __global__ void __launch_bounds__(THREADS, 1) mla_prefill_tc_kernel(const __grid
           k_seen = j;
         }
         tc_fence_after();
-        const uint32_t qa = smem_u32(q_tile + g * MQ_BYTES), ka = smem_u32(k_tile + st * MK_BYTES);
-#pragma unroll
-        for (int cb = 0; cb < QKB; ++cb)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_bf16_ss(tmem + (uint32_t)(g * 128), umma_desc_k_sw128(qa + cb * 16384 + k * 32), umma_desc_k_sw128(ka + cb * 8192 + k * 32), idesc_s, (cb | k) ? 1u : 0u);
-        umma_commit(&sh->s_full[g]);
         const bool last_user = (g == GROUPS - 1) || j >= n_g[GROUPS - 1];
-        if (last_user) umma_commit(&sh->k_empty[st]);
+        if (leader) {
+          const uint64_t qa = q_desc + (uint32_t)(g * (MQ_BYTES >> 4)), ka = k_desc + (uint32_t)(st * (MK_BYTES >> 4));
+#pragma unroll
+          for (int cb = 0; cb < QKB; ++cb)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) umma_bf16_ss(tmem + (uint32_t)(g * 128), qa + (uint32_t)(cb * 1024 + k * 2), ka + (uint32_t)(cb * 512 + k * 2), idesc_s, (cb | k) ? 1u : 0u);
+          umma_commit(&sh->s_full[g]);
+          if (last_user) umma_commit(&sh->k_empty[st]);
+        }
         return true;
       };
       auto issue_pv = [&](int g, int j) {
@@ -182,13 +185,15 @@ __global__ void __launch_bounds__(THREADS, 1) mla_prefill_tc_kernel(const __grid
           v_seen = j;
         }
         tc_fence_after();
-        const uint32_t va = smem_u32(v_tile + st * MV_BYTES);
-#pragma unroll
-        for (int ks = 0; ks < BKV2 / 16; ++ks)
-          umma_bf16_ts(tmem + 256u + (uint32_t)(g * 128), tmem + (uint32_t)(g * 128) + (uint32_t)(ks * 8), umma_desc_mn_sw128(va + ks * 2048, lbo, sbo), idesc_o, (j | ks) ? 1u : 0u);
-        umma_commit(&sh->o_full[g]);
         const bool last_user = (g == GROUPS - 1) || j >= n_g[GROUPS - 1];
-        if (last_user) umma_commit(&sh->v_empty[st]);
+        if (leader) {
+          const uint64_t va = v_desc + (uint32_t)(st * (MV_BYTES >> 4));
+#pragma unroll
+          for (int ks = 0; ks < BKV2 / 16; ++ks)
+            umma_bf16_ts(tmem + 256u + (uint32_t)(g * 128), tmem + (uint32_t)(g * 128) + (uint32_t)(ks * 8), va + (uint32_t)(ks * 128), idesc_o, (j | ks) ? 1u : 0u);
+          umma_commit(&sh->o_full[g]);
+          if (last_user) umma_commit(&sh->v_empty[st]);
+        }
         return true;
       };
       ok = ok && issue_s(0, 0) && issue_s(1, 0);

@@ -160,8 +160,10 @@ __global__ void __launch_bounds__(192) moe_gemm_fp8_kernel(const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();  // the warp walks the loop, one lane issues: descriptors in uniform registers (gemm_sm100.cu)
       constexpr uint32_t idesc = idesc_e4m3(BM, BN);
+      const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(tiles));
       int stage = 0;
       uint32_t phase = 0;
       long long g = 0;  // k groups multiplied so far by this CTA: accumulator g & 1
@@ -178,13 +180,13 @@ __global__ void __launch_bounds__(192) moe_gemm_fp8_kernel(const __grid_constant
             break;
           }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(tiles + stage * stage_bytes);
-          const uint32_t b_addr = a_addr + A_BYTES;
-          const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
+          if (leader) {
+            const uint64_t a = a_desc0 + (uint32_t)(stage * (stage_bytes >> 4));
 #pragma unroll
-          for (int k = 0; k < 4; ++k) umma_f8(d_tmem, umma_desc_k_sw128(a_addr + k * 32), umma_desc_k_sw128(b_addr + k * 32), idesc, k > 0 ? 1u : 0u);
-          umma_commit(&empty[stage]);
-          umma_commit(&tfull[acc]);
+            for (int k = 0; k < 4; ++k) umma_f8(tmem_base + (uint32_t)(acc * BN), a + (uint32_t)(k * 2), a + (uint32_t)((A_BYTES >> 4) + k * 2), idesc, k > 0 ? 1u : 0u);
+            umma_commit(&empty[stage]);
+            umma_commit(&tfull[acc]);
+          }
           if (++stage == p.stages) {
             stage = 0;
             phase ^= 1u;
