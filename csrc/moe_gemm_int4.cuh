@@ -8,13 +8,13 @@
 // global memory by each thread they were 128 sectors a k-block): 256-deep stages make a row of eight of them the 16 bytes that
 // a TMA row needs.
 //
-// 48 experts of 7168 x 2048, top 8 (routing and both products): 128 tokens 684 us with the A tile in shared memory, 534 now, of
+// 48 experts of 7168 x 2048, top 8 (routing and both products): 128 tokens 684 us with the A tile in shared memory, 451 now, of
 // which 70 by the issue of products from uniform registers (gemm_sm100.cu).  The weights' bytes take 182 us; a product of 128 rows
 // and few columns occupies the tensor core for 45 cycles whatever its columns, 165 us of this.
 //
 // warp 0 TMA producer | warp 1 MMA issuer + TMEM owner | warps 2-5 epilogue | then Q4_GROUPS groups of four dequant warps.
 // Group g expands the k-blocks g, g + Q4_GROUPS, .. of the four of a stage into one of eight TMEM buffers.
-constexpr int Q4_GROUPS = 2;             // divides 4
+constexpr int Q4_GROUPS = 4;             // divides 4; two groups: 534 us where four take 474 (128 tokens), 688 and 703 (512)
 constexpr int Q4_BK = 256;               // weights of a row in one stage: 128 bytes
 constexpr int Q4_RAW = BM * Q4_BK / 2;   // packed tile
 constexpr int Q4_SC = BM * (Q4_BK / 32) * 2;
@@ -187,6 +187,8 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     const uint32_t a_row = tmem_base + ((uint32_t)(wq * 32) << 16) + 256u;
     const int groups_per_row = p.K / 32;
     const bf162 bias = __floats2bfloat162_rn(136.f, 136.f);
+    uint32_t mask, magic;  // in registers: as two constants of one operation they make it two (474 us where this takes 451)
+    asm volatile("mov.b32 %0, 0x000F000F;\n\tmov.b32 %1, 0x43004300;" : "=r"(mask), "=r"(magic));
     int stage = 0;
     uint32_t phase = 0, turn = 0;
     ItemCursor cur;
@@ -225,7 +227,8 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
               // pair-interleaved nibbles: (w >> 4j) & 0x000F000F | 0x43004300 = bf16 pair (128 + e[2j], 128 + e[2j+1])
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                uint32_t tt = ((words[h * 4 + c] >> (4 * j)) & 0x000F000Fu) | 0x43004300u;
+                uint32_t tt;
+                asm("lop3.b32 %0, %1, %2, %3, 0xea;" : "=r"(tt) : "r"(words[h * 4 + c] >> (4 * j)), "r"(mask), "r"(magic));  // (a & b) | c
                 bf162 val = *reinterpret_cast<bf162*>(&tt);
                 val = __hmul2(__hsub2(val, bias), s2);
                 o[c * 4 + j] = *reinterpret_cast<uint32_t*>(&val);
