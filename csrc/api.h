@@ -135,14 +135,13 @@ int pg_mla_q_prep(const void* q, const void* cos, const void* sin, const void* p
                   int nope, int rope, int max_pos, cudaStream_t stream);
 int pg_mla_attention(const void* q_abs, const void* q_pe, const void* latent, void* out, const void* q_indptr, const void* kv_lens,
                      const void* table, int table_stride, const void* unit_seq, int num_seqs, int tokens, int heads, int c, int rope,
-                     int page_size, float scale, int splits, int tc, void* part_o, void* part_lse, long long num_pages, void* status, cudaStream_t stream);
+                     int page_size, float scale, int splits, int tc, void* part_o, void* part_lse, long long part_bytes, long long num_pages, void* status, cudaStream_t stream);
 
 // Absorbed latent attention with runtime sizes (latent c, shared rotated key part r, any number of heads), an optional
 // sliding window, and rotation of neighbouring query columns inside the kernel; token / head strides in elements.
 int pg_latent_attention(const void* q_abs, long long q_tok, long long q_head, const void* q_pe, long long pe_tok, long long pe_head, const void* cos, const void* sin, int max_pos, const void* latent,
                         void* out, long long o_tok, long long o_head, const void* q_indptr, const void* kv_lens, const void* table, int table_stride, const void* unit_seq, int first_row, int num_seqs,
-                        int tokens, int heads, int c, int r, int page_size, float scale, int window, const void* sink, const void* head_gate, long long ld_gate, int splits, int tc, void* part_o, void* part_lse,
-                        long long num_pages, void* status, cudaStream_t stream);
+                        int tokens, int heads, int c, int r, int page_size, float scale, int window, const void* sink, const void* head_gate, long long ld_gate, int splits, int tc, void* part_o, void* part_lse, long long part_bytes, long long num_pages, void* status, cudaStream_t stream);
 int pg_latent_attention_plain(const void* q_abs, long long q_tok, long long q_head, const void* q_pe, long long pe_tok, long long pe_head, const void* cos, const void* sin, int max_pos, const void* latent,
                               void* out, long long o_tok, long long o_head, const void* q_indptr, const void* kv_lens, const void* table, int table_stride, const void* unit_seq, int tokens, int heads, int c,
                               int r, int page_size, float scale, int window, const void* sink, const void* head_gate, long long ld_gate, int is_f32, cudaStream_t stream);

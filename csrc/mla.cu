@@ -653,22 +653,23 @@ extern "C" int pg_mla_q_prep(const void* q, const void* cos, const void* sin, co
 
 extern "C" int pg_mla_attention(const void* q_abs, const void* q_pe, const void* latent, void* out, const void* q_indptr, const void* kv_lens,
                                 const void* table, int table_stride, const void* unit_seq, int num_seqs, int tokens, int heads, int c, int rope,
-                                int page_size, float scale, int splits, int tc, void* part_o, void* part_lse, long long num_pages, void* status, cudaStream_t stream) {
+                                int page_size, float scale, int splits, int tc, void* part_o, void* part_lse, long long part_bytes, long long num_pages, void* status, cudaStream_t stream) {
   PG_REQUIRE(c == 512 && rope == 64, "mla_attention: built for kv_lora 512 + rope 64 (got %d + %d)", c, rope);
   PG_REQUIRE(heads % 16 == 0, "mla_attention: heads %d must be a multiple of 16", heads);
   // absorbed queries, rotated query parts and outputs [tokens, heads, ..]
   return pg_latent_attention(q_abs, (long long)heads * c, c, q_pe, (long long)heads * rope, rope, nullptr, nullptr, 0, latent, out, (long long)heads * c, c, q_indptr, kv_lens, table, table_stride, unit_seq, 0,
-                             num_seqs, tokens, heads, c, rope, page_size, scale, 0, nullptr, nullptr, 0, splits, tc, part_o, part_lse, num_pages, status, stream);
+                             num_seqs, tokens, heads, c, rope, page_size, scale, 0, nullptr, nullptr, 0, splits, tc, part_o, part_lse, part_bytes, num_pages, status, stream);
 }
 
 // q_abs, q_pe and out by token / head strides in elements; cos / sin f32 [max_pos, r / 2] turn the q_pe columns (null: they
 // come rotated); window > 0: a row sees its last `window` keys; sink f32 [heads] and head_gate bf16 [tokens, >= heads] as in
 // MlaParams (or null).  Row 0 of this call is row `first_row` of the step that q_indptr and unit_seq describe.
-// tc: the tcgen05 kernel, where sizes and alignment allow it (the caller's rule, and its number of splits).
+// tc: the tcgen05 kernel, where sizes and alignment allow it (the caller's rule); its blocks share the keys by themselves, with part_o
+// as scratch of part_bytes, and `splits` is how many blocks a row may have.
 extern "C" int pg_latent_attention(const void* q_abs, long long q_tok, long long q_head, const void* q_pe, long long pe_tok, long long pe_head, const void* cos, const void* sin, int max_pos,
                                    const void* latent, void* out, long long o_tok, long long o_head, const void* q_indptr, const void* kv_lens, const void* table, int table_stride,
                                    const void* unit_seq, int first_row, int num_seqs, int tokens, int heads, int c, int r, int page_size, float scale, int window, const void* sink, const void* head_gate, long long ld_gate,
-                                   int splits, int tc, void* part_o, void* part_lse, long long num_pages, void* status, cudaStream_t stream) {
+                                   int splits, int tc, void* part_o, void* part_lse, long long part_bytes, long long num_pages, void* status, cudaStream_t stream) {
   PG_REQUIRE(c % 8 == 0 && r % 8 == 0 && c >= 8 && c <= 512 && r >= 0 && r <= 64, "latent_attention: a latent of %d + %d columns is not supported (multiples of 8 up to 512 + 64)", c, r);
   PG_REQUIRE(page_size == 16 || page_size == 32 || page_size == 64, "latent_attention: pages of %d tokens", page_size);
   PG_REQUIRE(q_tok % 2 == 0 && q_head % 2 == 0 && pe_tok % 2 == 0 && pe_head % 2 == 0 && o_tok % 2 == 0 && o_head % 2 == 0, "latent_attention: strides must keep column pairs aligned");
@@ -701,10 +702,8 @@ extern "C" int pg_latent_attention(const void* q_abs, long long q_tok, long long
     const bool pieces = q_tok % 8 == 0 && q_head % 8 == 0 && pe_tok % 8 == 0 && pe_head % 8 == 0 && (((uintptr_t)q_abs | (uintptr_t)q_pe | (uintptr_t)latent) & 15) == 0;
     if (tc && pieces) {  // queries in 16-byte pieces, the cache through a tensor map
       const MlaDecodeTc d = {p.q_abs, p.q_pe, p.latent, p.out, q_tok, q_head, pe_tok, pe_head, o_tok, o_head, p.cos, p.sin, max_pos, window, p.q_indptr, p.kv_lens, p.table, p.unit_seq, table_stride, first_row, tokens,
-                             heads, page_size, p.splits, p.scale_log2, p.part_o, p.part_lse, p.sink, p.gate, ld_gate, (uint32_t*)status};
-      if (int rc = mla_decode_tc(d, r, num_pages, stream)) return rc;
-      if (p.splits > 1) PG_CUDA(launch_pdl(mla_merge_kernel<512>, dim3((unsigned)(((long long)tokens * heads + 3) / 4)), dim3(128), (size_t)0, stream, p));
-      return PG_OK;
+                             heads, page_size, p.splits, 0, p.scale_log2, nullptr, nullptr, nullptr, p.sink, p.gate, ld_gate, (uint32_t*)status};
+      return mla_decode_tc(d, r, num_pages, part_o, part_bytes, stream);
     }
     return r ? launch_mla<512, 64, true>(p, stream) : launch_mla<512, 0, true>(p, stream);
   }

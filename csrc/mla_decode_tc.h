@@ -9,13 +9,17 @@ struct MlaDecodeTc {
   const float *cos, *sin;  // turn the q_pe columns (null: they come rotated)
   int max_pos, window;
   const int *q_indptr, *kv_lens, *table, *unit_seq;
-  int table_stride, first_row, tokens, heads, page_size, splits;
+  int table_stride, first_row, tokens, heads, page_size;
+  int splits;  // blocks that the caller would like to share a row's keys: how small the groups of heads may get
+  int shared;  // the blocks share all rows' keys evenly, rows cut where need be (0: a block walks one row's keys)
   float scale_log2;
-  float *part_o, *part_lse;
+  float *part_o, *part_lse;  // of cut rows: two slots a block, [heads of a group, 512] and [heads of a group]
+  int* cuts;                 // a block's last row, where that ends in other blocks' shares: (unit or -1, pieces)
   const float* sink;
   const bf16* gate;
   long long ld_gate;
   uint32_t* status;
 };
 
-int mla_decode_tc(const MlaDecodeTc& p, int r, long long pages, cudaStream_t stream);
+// part: scratch for cut rows; too little, and no row is cut
+int mla_decode_tc(MlaDecodeTc p, int r, long long pages, void* part, long long part_bytes, cudaStream_t stream);

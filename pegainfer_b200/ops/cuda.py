@@ -1626,7 +1626,7 @@ _LATENT_FEW = 16  # rows of a sequence in a decode step or in one that checks dr
 
 def _latent_splits(rows: int, heads: int, longest: int, tc: bool, sms: int) -> int:
     """Blocks that share one row's keys in the absorbed kernels."""
-    if tc:  # csrc/mla_decode_tc.cu: a block owns an SM and serves up to 64 heads, so as many as there are SMs, of 256 keys or more
+    if tc:  # csrc/mla_decode_tc.cu: a block owns an SM and serves up to 64 heads; blocks share the keys by themselves, this says how few heads one gets
         return max(1, min(16, sms // (rows * ((heads + 63) // 64)), (longest + 255) // 256))
     return max(1, min(16, (4 * sms) // (rows * ((heads + 15) // 16)), (min(longest, 4096) + 127) // 128))
 
@@ -1756,8 +1756,8 @@ def mla_attention(q: "_MlaQ", w_uk, w_uv, latent_layer, meta: AttnMeta, scale, k
     lat_out = torch.empty((t, h, kv_lora), dtype=torch.bfloat16, device=dev)
     rc = lib().pg_mla_attention(_ptr(q_abs), _ptr(q.pe), _ptr(latent_layer), _ptr(lat_out), _ptr(meta.q_indptr), _ptr(meta.kv_lens), _ptr(meta.block_table),
                                 _ci(meta.block_table.stride(0)), _ptr(unit_seq), _ci(meta.num_seqs), _ci(t), _ci(h), _ci(kv_lora), _ci(rope), _ci(page_size), _cf(scale),
-                                _ci(splits), _ci(int(tc)), _ptr(part_o), _ptr(part_lse), _ll(latent_layer.shape[0]), _ptr(c.status), _stream())
-    _check(rc, c, 2 if splits > 1 else 1)
+                                _ci(splits), _ci(int(tc)), _ptr(part_o), _ptr(part_lse), _ll(part_o.numel()), _ll(latent_layer.shape[0]), _ptr(c.status), _stream())
+    _check(rc, c, 2 if splits > 1 or tc else 1)
     vdim = w_uv.shape[1]
     out = torch.empty((t, h * vdim), dtype=torch.bfloat16, device=dev)
     _head_gemm(lat_out, h * kv_lora, kv_lora, w_uv, out.view(t, h, vdim))
@@ -1878,7 +1878,7 @@ def latent_attention(q, uk_t, uv, ukv, cache, meta: AttnMeta, rot: int, scale: f
         splits = _latent_splits(n, heads, longest, tc, c.sms)
         splits = max(1, min(splits, c.attn_part.numel() // (n * heads * (lat + 1) * 4)))
         rc = lib().pg_latent_attention(_ptr(q_abs), *strides, *pe, *where, _ci(row0), _ci(meta.num_seqs), _ci(n), _ci(heads), _ci(lat), _ci(rot), _ci(ps), _cf(scale), _ci(window), *extra, _ci(splits),
-                                       _ci(int(tc)), _ptr(c.attn_part), _ptr(c.attn_part[n * heads * splits * lat * 4 :]), _ll(cache.shape[0]), _ptr(c.status), _stream())
+                                       _ci(int(tc)), _ptr(c.attn_part), _ptr(c.attn_part[n * heads * splits * lat * 4 :]), _ll(c.attn_part.numel()), _ll(cache.shape[0]), _ptr(c.status), _stream())
         _check(rc, c, 2 if splits > 1 else 1)
     else:
         assert row0 == 0
