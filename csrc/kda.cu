@@ -22,6 +22,8 @@
 //
 // Functional parity with pegainfer-k3/kernels/tilelang_defs.py:67-139 (attnres_scores / attnres_mix) and
 // :304-410 (kda_core) and pegainfer-kernels/csrc/k3/k3_flash_kda.cu (chunked prefill of the same rule).
+#include <atomic>
+
 #include "api.h"
 #include "common.cuh"
 #include "mma_frag.cuh"
@@ -279,299 +281,481 @@ int run_rule(int rule, RecArgs<T> p, int num_seqs, int max_q_len, cudaStream_t s
 }
 
 // ---------------------------------------------------------------------------------
-// The delta rule with bounded channel decays, KB_T tokens at a time (prompts, 128-wide keys).  Inside a block
-//   kd_t = k_t * P_t, qd_t = q_t * P_t      (P_t: product of the block's decays up to and with token t)
-//   kh_t = k_t * (product of the decays behind t),   A_ts = k_t . (k_s * decays of s+1 .. t),   B_ts likewise with q_t
-// do not depend on the state, so a warp forms them once per block for all columns of the CTA, and per state column
-//   d_t = beta_t (v_t - kd_t . S0 - sum_{s<t} A_ts d_s),   o_t = qd_t . S0 + sum_{s<=t} B_ts d_s,
-//   S   = (all decays) * S0 + sum_t kh_t d_t
-// Everything stays f32 (products of decays only, no quotients, so nothing can overflow).  Against the token-by-token walk
-// this takes 3.25 multiply-adds per state element and token instead of 4, and one reduction, one solve per KB_T tokens.
-// A lane holds 16 rows x 4 columns of the state as row pairs for the packed f32x2 instructions; the 8 lanes of a column
-// group read 128 contiguous bytes of a vector at a time, which is what the walk, with 32 elements of one column per thread,
-// was short of: shared-memory reads (three vectors per 32 elements and token there, 13 per 64 elements and 4 tokens here).
-// 3001 tokens in two prompts, 96 heads: 2550 us before, 1145 us now; 16 heads, one prompt of 3000: 1644 and 1099.  Decode rows
-// beside a prompt stay on the walk (64 rows and 300 tokens, 96 heads: 398 us with every row in a block of four, 333 now).  What bounds it: FMA issue and shared-memory reads
-// (both near half of their rate) by warps that wait for their own sums, few of them where a step has few sequences.
-constexpr int KB_T = 4;        // tokens per block
-constexpr int KB_BLOCKS = 4;   // blocks per stage: one per warp to prepare
-constexpr int KB_COLS = 64;    // state columns per CTA, 16 per warp
-constexpr int KB_DK = 128;
+// The delta rule with bounded channel decays, KC_T tokens at a time (prompts, 128-wide keys), on the tensor cores.  With P_t the
+// product of the chunk's decays up to and with token t, and token 7 as the reference,
+//   rk_t = k_t P_t / P_7,   rq_t = q_t P_t / P_7,   c_s = k_s P_7 / P_s,   S' = P_7 S0,
+//   A_ts = rk_t . c_s,   B_ts = rq_t . c_s,   T = (I + diag(beta) A_strict)^-1 diag(beta),
+//   d = T (v - rk S'),   o = rq S' + B d  (s <= t),   S = P_15 / P_7 (S' + sum_s c_s d_s)
+// so everything but T, 16 x 16 and solved by one warp, is a product of matrices.  None is rounded to less than f32: each factor
+// is split into two tf32 numbers, x = hi + lo with 22 bits, and lo hi, hi lo and hi hi are added (mma.sync, f32 sums); sums over more than
+// 32 channels and the state itself are added outside of the tensor core, which cuts sums off.  With lower >= KC_LOWER all
+// factors are numbers of f32: quotients P_t / P_7 reach exp(8 |lower|), and the state goes from one chunk's reference to the next one's by
+// a product of sixteen decays, exp(16 lower) = 3e-37 at least.
+//
+// A warp keeps 16 state columns as S^T (columns x 128 channels) in mma accumulators.  A product over the channels takes them as its
+// left operand where they are: accumulator columns 2 t, 2 t + 1 become the operand's channels t, t + 4, and the right operand is
+// stored in the same order, a pair of channels (or of tokens) with its low parts in 16 bytes.  The same holds for d^T.  Four warps
+// prepare chunks together (a lane has four channels of four tokens) while four others, of 16 columns each, walk the chunk before: a
+// sequence is one chain of chunks, and what a block takes for a chunk is what a prompt takes.  rk and rq exist once: they are free when
+// the walk has multiplied them with S', and the next ones written while it does the rest; c, T and B exist twice.
+// A NaN in a token reaches the other tokens of its chunk, the earlier ones too.
+// Against four tokens at a time on the FMA units (one group of four warps to prepare and to walk; 53 % of FMA issue):  3001 tokens in two
+// prompts, 96 heads 1150 -> 966 us; one prompt of 3000 tokens, 16 heads 1105 -> 795; eight of 125, 32 heads 151 -> 145; 4 x 50 48 -> 42.  State
+// against 64 bits, 2-norm: 8.4e-7 and 8.4e-7 (900 tokens), 1.12e-6 and 1.12e-6 (2000).  What bounds it: the chain of a chunk, some 8000
+// cycles, half of it preparation whose steps wait for each other; the products themselves are 350 a scheduler, eight cycles each.
+constexpr int KC_T = 16;      // tokens per chunk, four per warp to prepare
+constexpr int KC_COLS = 64;   // state columns per CTA, 16 per warp
+constexpr int KC_DK = 128;
+constexpr float KC_LOWER = -5.25f;
+// Registers of the two groups of four warps: what the block is launched with (128 a thread; kc_allow checks it), moved to the walking
+// warps, whose state alone takes 64.  96 / 160: 989 us, 112 / 144: 1015, 128 each: 1087 (two prompts below).
+constexpr int KC_REGS_PREP = 104, KC_REGS_WALK = 152;
 
-struct KdaBlock {
-  float kd[KB_T][KB_DK], qd[KB_T][KB_DK], kh[KB_T][KB_DK], dp[KB_DK];
-  float v[KB_T][KB_COLS];
-  float ab[16];  // A_ts at t (t - 1) / 2 + s, B_ts at 6 + t (t + 1) / 2 + s
-  float beta[KB_T];
-};
-struct KdaBlockSmem {  // 47 KB: no attribute needed
-  KdaBlock blk[KB_BLOCKS];
-  bf16 raw[KB_BLOCKS][3][KB_T][KB_DK];  // q, k, f rows of the stage after this one
-  bf16 raw_v[KB_BLOCKS][KB_T][KB_COLS];
-  float u[4][KB_T][16], o[4][KB_T][16];  // per warp: kd . S0, then d; qd . S0
+struct KcSmem {
+  float4 rk[KC_T][KC_DK / 2], rq[KC_T][KC_DK / 2];  // [token][pair of channels, ^ 4 on odd tokens]: hi, hi, lo, lo
+  float4 c[2][KC_T / 2][KC_DK];                     // [pair of tokens][channel ^ 2 (pair % 4)]: hi, hi, lo, lo
+  bf16 raw[4][3][4][KC_DK];                         // q, k, f rows of the next chunk to prepare, by warp
+  bf16 raw_v[4][KC_T][KC_COLS];
+  float tot[4][KC_DK];  // products of each warp's four decays
+  float fac[KC_DK], tail[KC_DK];  // (P_15 / P_7 of the chunk before) P_7, and this chunk's P_15 / P_7
+  float m[KC_T][KC_T];  // [s][t]: beta_t A_ts, s < t
+  float beta[2][KC_T];
+  float4 tf[2][3][32], bf[2][3][32];  // T and B (s <= t) as right operands: tokens (0 - 7, 0 - 7), (8 - 15, 0 - 7), (8 - 15, 8 - 15)
 };
 
-static_assert(sizeof(KdaBlockSmem) <= 48 * 1024, "more needs the kernel's attribute, on every device");
-__device__ __forceinline__ unsigned long long kb_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
+// hi: x rounded to the eleven bits of a tf32 number (a NaN's hi may be a number, its lo is a NaN); lo: what is left, of which the tensor
+// core reads the first eleven bits
+__device__ __forceinline__ void kc_split(float x, float& hi, float& lo) {
+  hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+  lo = x - hi;
 }
-__device__ __forceinline__ unsigned long long kb_mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
+struct KcA {  // left operand, rows g and g + 8, columns (2 t of both, 2 t + 1 of both)
+  float hi[4], lo[4];
+};
+// from accumulators: (g, 2t), (g, 2t + 1), (g + 8, 2t), (g + 8, 2t + 1)
+__device__ __forceinline__ void kc_left(const float* c, KcA& a) {
+  kc_split(c[0], a.hi[0], a.lo[0]);
+  kc_split(c[2], a.hi[1], a.lo[1]);
+  kc_split(c[1], a.hi[2], a.lo[2]);
+  kc_split(c[3], a.hi[3], a.lo[3]);
 }
-__device__ __forceinline__ unsigned long long kb_pair(float lo, float hi) {
-  unsigned long long d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
+__device__ __forceinline__ void kc_mma1(float* d, const float* a, float b0, float b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
 }
-__device__ __forceinline__ float2 kb_split(unsigned long long a) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(a));
-  return f;
-}
-// Sum over lanes of N values per lane, scattered: every step halves the values a lane still carries.  Bit `top` of the lane
-// picks the upper half first.
+// low[i] and high[i] += left[i] right[i], right = (hi, hi, lo, lo), the two products with a low part, which add up to a small number, apart.
+// The order is that of issue: a product waits some 35 cycles for one in front of it that adds to the same sums, so N of them take turns.
 template <int N>
-__device__ __forceinline__ void kb_reduce_scatter(float* v, int lane, int top) {
+__device__ __forceinline__ void kc_mma(float* const (&low)[N], float* const (&high)[N], const KcA* const (&left)[N], const float4 (&right)[N]) {
 #pragma unroll
-  for (int n = N / 2, bit = top; n > 0 && bit > 0; n >>= 1, bit >>= 1) {
-    const bool up = lane & bit;
+  for (int i = 0; i < N; ++i) kc_mma1(low[i], left[i]->lo, right[i].x, right[i].y);
 #pragma unroll
-    for (int j = 0; j < n; ++j) {
-      const float send = up ? v[j] : v[j + n], keep = up ? v[j + n] : v[j];
-      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
-    }
-  }
+  for (int i = 0; i < N; ++i) kc_mma1(high[i], left[i]->hi, right[i].x, right[i].y);
+#pragma unroll
+  for (int i = 0; i < N; ++i) kc_mma1(low[i], left[i]->hi, right[i].z, right[i].w);
 }
 
-__global__ void __launch_bounds__(128, 3)
-kda_block_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v, long long ld, const bf16* __restrict__ f, long long ldf, const bf16* __restrict__ b, long long ldb,
+// d += a b, b = (hi, hi, lo, lo): the two products with a low part apart, which add up to a small number, as their own chain
+__device__ __forceinline__ void kc_mma_low(float* d, const KcA& a, const float4& b) {
+  kc_mma1(d, a.lo, b.x, b.y);
+  kc_mma1(d, a.hi, b.z, b.w);
+}
+__device__ __forceinline__ void kc_mma_high(float* d, const KcA& a, const float4& b) { kc_mma1(d, a.hi, b.x, b.y); }
+
+// named barriers: among the preparing warps; rk and rq are free; rk, rq and fac are there; T, B and c are there (by parity of the chunk)
+enum { KC_BAR_PREP = 1, KC_BAR_FREE = 2, KC_BAR_ROWS = 3, KC_BAR_T = 4 };
+__device__ __forceinline__ void kc_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void kc_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+__global__ void __launch_bounds__(256, 2)
+kda_chunk_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v, long long ld, const bf16* __restrict__ f, long long ldf, const bf16* __restrict__ b, long long ldb,
                  const float* __restrict__ a_log, const float* __restrict__ dt_bias, float lower, float* __restrict__ state, bf16* __restrict__ out, const int* __restrict__ q_indptr,
                  const int* __restrict__ slots, int heads, int dv, int min_len) {
-  extern __shared__ __align__(16) uint8_t kb_raw[];
-  KdaBlockSmem& sm = *reinterpret_cast<KdaBlockSmem*>(kb_raw);
-  const int groups = dv / KB_COLS;
-  const int h = blockIdx.x / groups, c0 = blockIdx.x % groups * KB_COLS, seq = blockIdx.y;
+  extern __shared__ __align__(16) uint8_t kc_raw[];
+  KcSmem& sm = *reinterpret_cast<KcSmem*>(kc_raw);
+  const int groups = dv / KC_COLS;
+  const int h = blockIdx.x / groups, c0 = blockIdx.x % groups * KC_COLS, seq = blockIdx.y;
   const int slot = slots[seq];
   const int q0 = q_indptr[seq], q1 = q_indptr[seq + 1];
   if (q1 - q0 < min_len || slot < 0) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rg = lane & 7, cg = lane >> 3;
-  const int col = c0 + warp * 16 + cg * 4;  // the lane's first state column
-  float* S = state + ((long long)slot * heads + h) * KB_DK * dv;
+  const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t4 = lane & 3;
+  const int sw = (g & 1) << 2;  // of the rows g and g + 8 of rk and rq
 
-  // raw rows of this warp's block of the stage that starts at token t0; rows past the end are zero
+  if (threadIdx.x < 128) {
+  // ================ preparing warps ================
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(KC_REGS_PREP));
+
+  // raw rows of this warp's four tokens of the chunk that starts at token t0; rows past the end are zero
   float b_next = 0.f;
-  auto fetch = [&](int t0) {
-    const int t = t0 + warp * KB_T;
+  auto fetch = [&](int t0, int chunk) {
+    const int t = t0 + warp * 4;
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
       const int c = lane + 32 * (i & 1), r = c >> 4, ch = (c & 15) * 8;
       const bool ok = t + r < q1;
       const long long row = ok ? t + r : q0;
       const bf16* src = i < 2 ? q + row * ld : i < 4 ? k + row * ld : f + row * ldf;
-      cp_async16(&sm.raw[warp][i >> 1][r][ch], src + (long long)h * KB_DK + ch, ok);
+      cp_async16(&sm.raw[warp][i >> 1][r][ch], src + (long long)h * KC_DK + ch, ok);
     }
     const int r = lane >> 3, ch = (lane & 7) * 8;
     const bool ok = t + r < q1;
-    cp_async16(&sm.raw_v[warp][r][ch], v + (ok ? t + r : q0) * ld + (long long)h * dv + c0 + ch, ok);
+    cp_async16(&sm.raw_v[chunk & 3][warp * 4 + r][ch], v + (ok ? t + r : q0) * ld + (long long)h * dv + c0 + ch, ok);
     cp_async_commit();
-    b_next = lane < KB_T && t + lane < q1 ? to_f32(b[(long long)(t + lane) * ldb + h]) : 0.f;
+    b_next = lane < 4 && t + lane < q1 ? to_f32(b[(long long)(t + lane) * ldb + h]) : 0.f;
   };
-  fetch(q0);
+  fetch(q0, 0);
 
-  unsigned long long s2[4][2][4];  // rows 32 i + 4 rg + {0, 1} and {2, 3}, columns col .. col + 3
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      const float4 lo = *reinterpret_cast<const float4*>(S + (long long)(32 * i + 4 * rg + 2 * p) * dv + col);
-      const float4 hi = *reinterpret_cast<const float4*>(S + (long long)(32 * i + 4 * rg + 2 * p + 1) * dv + col);
-      s2[i][p][0] = kb_pair(lo.x, hi.x);
-      s2[i][p][1] = kb_pair(lo.y, hi.y);
-      s2[i][p][2] = kb_pair(lo.z, hi.z);
-      s2[i][p][3] = kb_pair(lo.w, hi.w);
-    }
-  const float a = __expf(a_log[h]), q_scale = rsqrtf((float)KB_DK);
+  const float a = __expf(a_log[h]), q_scale = rsqrtf((float)KC_DK);
+  // a lane prepares channels 2 lane, 2 lane + 1 and 64 further on
+  const float2 bias0 = *reinterpret_cast<const float2*>(dt_bias + h * KC_DK + 2 * lane), bias1 = *reinterpret_cast<const float2*>(dt_bias + h * KC_DK + 64 + 2 * lane);
+  const float bias[4] = {bias0.x, bias0.y, bias1.x, bias1.y};
+  float tail[4] = {1.f, 1.f, 1.f, 1.f};
 
-  for (int t0 = q0; t0 < q1; t0 += KB_T * KB_BLOCKS) {
-    // ---- each warp prepares one block; a lane has four key channels of its four tokens ----
+  for (int t0 = q0, chunk = 0; t0 < q1; t0 += KC_T, ++chunk) {
+    // ---- unit rows and decays of the warp's four tokens ----
     cp_async_wait_all();
     __syncwarp();
-    {
-      KdaBlock& B = sm.blk[warp];
-      const int first = t0 + warp * KB_T;
-      float kk[KB_T][4], qq[KB_T][4], dec[KB_T][4];
-      const float4 db = *reinterpret_cast<const float4*>(dt_bias + h * KB_DK + lane * 4);
-      const float bias[4] = {db.x, db.y, db.z, db.w};
+    float kk[4][4], qq[4][4], dec[4][4], all[4] = {1.f, 1.f, 1.f, 1.f};
+    const int first = t0 + warp * 4;
+    float sq[8];  // sums of squares of q, k of each token
 #pragma unroll
-      for (int t = 0; t < KB_T; ++t) {
-        float x[3][4], qs = 0.f, ks = 0.f;
+    for (int t = 0; t < 4; ++t) {
+      float x[3][4];
 #pragma unroll
-        for (int w = 0; w < 3; ++w) {
-          const uint2 raw = *reinterpret_cast<const uint2*>(&sm.raw[warp][w][t][lane * 4]);
-          const float2 lo = __bfloat1622float2(*reinterpret_cast<const bf162*>(&raw.x)), hi = __bfloat1622float2(*reinterpret_cast<const bf162*>(&raw.y));
-          x[w][0] = lo.x, x[w][1] = lo.y, x[w][2] = hi.x, x[w][3] = hi.y;
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          qs += x[0][e] * x[0][e];
-          ks += x[1][e] * x[1][e];
-        }
-        qs = warp_sum(qs);
-        ks = warp_sum(ks);
-        const float qn = rsqrtf(qs + 1e-6f) * q_scale, kn = rsqrtf(ks + 1e-6f);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          qq[t][e] = x[0][e] * qn;
-          kk[t][e] = x[1][e] * kn;
-          const float raw = x[2][e] + bias[e];
-          dec[t][e] = first + t < q1 ? __expf(lower / (1.f + __expf(-a * raw))) : 1.f;
-        }
+      for (int w = 0; w < 3; ++w) {
+        const float2 lo = __bfloat1622float2(*reinterpret_cast<const bf162*>(&sm.raw[warp][w][t][2 * lane])), hi = __bfloat1622float2(*reinterpret_cast<const bf162*>(&sm.raw[warp][w][t][64 + 2 * lane]));
+        x[w][0] = lo.x, x[w][1] = lo.y, x[w][2] = hi.x, x[w][3] = hi.y;
       }
-      float ab[16], w[KB_T][4];
+      sq[2 * t] = (x[0][0] * x[0][0] + x[0][1] * x[0][1]) + (x[0][2] * x[0][2] + x[0][3] * x[0][3]);
+      sq[2 * t + 1] = (x[1][0] * x[1][0] + x[1][1] * x[1][1]) + (x[1][2] * x[1][2] + x[1][3] * x[1][3]);
 #pragma unroll
-      for (int s = 0; s < KB_T; ++s) {
+      for (int e = 0; e < 4; ++e) {
+        qq[t][e] = x[0][e];
+        kk[t][e] = x[1][e];
+        dec[t][e] = first + t < q1 ? __expf(lower / (1.f + __expf(-a * (x[2][e] + bias[e])))) : 1.f;
+        all[e] *= dec[t][e];
+      }
+    }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) w[s][e] = kk[s][e];
+    for (int m = 16; m > 0; m >>= 1) {  // (one after the other the eight sums took a third of a chunk's time)
+      float y[8];
 #pragma unroll
-        for (int t = s; t < KB_T; ++t) {  // w[s] = k_s times the decays of s + 1 .. t
-          float x = 0.f, y = 0.f;
+      for (int i = 0; i < 8; ++i) y[i] = __shfl_xor_sync(0xffffffffu, sq[i], m);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sq[i] += y[i];
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float qn = rsqrtf(sq[2 * t] + 1e-6f) * q_scale, kn = rsqrtf(sq[2 * t + 1] + 1e-6f);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        qq[t][e] *= qn;
+        kk[t][e] *= kn;
+      }
+    }
+    *reinterpret_cast<float2*>(&sm.tot[warp][2 * lane]) = make_float2(all[0], all[1]);
+    *reinterpret_cast<float2*>(&sm.tot[warp][64 + 2 * lane]) = make_float2(all[2], all[3]);
+    if (lane < 4) sm.beta[chunk & 1][warp * 4 + lane] = first + lane < q1 ? 1.f / (1.f + __expf(-b_next)) : 0.f;
+    kc_sync(KC_BAR_PREP, 128);
+    if (t0 + KC_T < q1) fetch(t0 + KC_T, chunk + 1);
+    if (chunk > 0) kc_sync(KC_BAR_FREE, 256);
+    const int par = chunk & 1;
+    {
+      float run[4];  // the product between the warp's tokens and token 7
+      const bool behind = warp >= 2;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int ch = (e >> 1) * 64 + 2 * lane + (e & 1);
+        run[e] = warp == 3 ? sm.tot[2][ch] : warp == 0 ? sm.tot[1][ch] : 1.f;
+      }
+      float held[4];  // c of the pair's other token
+      auto put = [&](int t, bool second, const float* r, const float* ci) {  // r = P_t / P_7, ci its inverse
+        const int row = warp * 4 + t, p = row >> 1;
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) {
+          const int pair = ((e >> 1) * 32 + lane) ^ ((t & 1) << 2);
+          float4 o;
+          kc_split(kk[t][e] * r[e], o.x, o.z);
+          kc_split(kk[t][e + 1] * r[e + 1], o.y, o.w);
+          sm.rk[row][pair] = o;
+          kc_split(qq[t][e] * r[e], o.x, o.z);
+          kc_split(qq[t][e + 1] * r[e + 1], o.y, o.w);
+          sm.rq[row][pair] = o;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float x = kk[t][e] * ci[e];
+          if (second) {
+            float4 o;
+            kc_split((t & 1) ? held[e] : x, o.x, o.z);
+            kc_split((t & 1) ? x : held[e], o.y, o.w);
+            sm.c[par][p][((e >> 1) * 64 + 2 * lane + (e & 1)) ^ ((p & 3) << 1)] = o;
+          } else {
+            held[e] = x;
+          }
+        }
+      };
+      if (behind) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          float inv[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            if (t > s) w[s][e] *= dec[t][e];
-            x += kk[t][e] * w[s][e];
-            y += qq[t][e] * w[s][e];
+            run[e] *= dec[t][e];
+            inv[e] = 1.f / run[e];
           }
-          if (t > s) ab[t * (t - 1) / 2 + s] = x;
-          ab[6 + t * (t + 1) / 2 + s] = y;
+          put(t, t & 1, run, inv);
         }
-        *reinterpret_cast<float4*>(&B.kh[s][lane * 4]) = make_float4(w[s][0], w[s][1], w[s][2], w[s][3]);
-      }
-      float cum[4] = {1.f, 1.f, 1.f, 1.f};
+      } else {
 #pragma unroll
-      for (int t = 0; t < KB_T; ++t) {
+        for (int t = 3; t >= 0; --t) {
+          float inv[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) cum[e] *= dec[t][e];
-        *reinterpret_cast<float4*>(&B.kd[t][lane * 4]) = make_float4(kk[t][0] * cum[0], kk[t][1] * cum[1], kk[t][2] * cum[2], kk[t][3] * cum[3]);
-        *reinterpret_cast<float4*>(&B.qd[t][lane * 4]) = make_float4(qq[t][0] * cum[0], qq[t][1] * cum[1], qq[t][2] * cum[2], qq[t][3] * cum[3]);
-        const float2 vv = __bfloat1622float2(*reinterpret_cast<const bf162*>(&sm.raw_v[warp][t][lane * 2]));
-        *reinterpret_cast<float2*>(&B.v[t][lane * 2]) = vv;
+          for (int e = 0; e < 4; ++e) inv[e] = 1.f / run[e];
+          put(t, !(t & 1), inv, run);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) run[e] *= dec[t][e];
+        }
       }
-      *reinterpret_cast<float4*>(&B.dp[lane * 4]) = make_float4(cum[0], cum[1], cum[2], cum[3]);
-      kb_reduce_scatter<16>(ab, lane, 16);
-      ab[0] += __shfl_xor_sync(0xffffffffu, ab[0], 1);
-      if (!(lane & 1)) B.ab[lane >> 1] = ab[0];
-      if (lane < KB_T) B.beta[lane] = first + lane < q1 ? 1.f / (1.f + __expf(-b_next)) : 0.f;
+      if (warp == 0) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int ch = (e >> 1) * 64 + 2 * lane + (e & 1);
+          sm.fac[ch] = tail[e] * (all[e] * sm.tot[1][ch]);
+          tail[e] = sm.tot[2][ch] * sm.tot[3][ch];
+          sm.tail[ch] = tail[e];
+        }
+      }
     }
-    __syncthreads();
-    if (t0 + KB_T * KB_BLOCKS < q1) fetch(t0 + KB_T * KB_BLOCKS);
+    kc_arrive(KC_BAR_ROWS, 256);
+    kc_sync(KC_BAR_PREP, 128);
+    // ---- A (warps 0, 1) and B (warps 2, 3), eight tokens s each ----
+    {
+      const float4* left = &(warp < 2 ? sm.rk : sm.rq)[g][t4];
+      const int sn = warp & 1, tok = sn * 8 + g, p = tok >> 1;
+      const float* right = reinterpret_cast<const float*>(&sm.c[par][p][(2 * t4) ^ ((p & 3) << 1)]) + (tok & 1);
+      float sum[4] = {0.f, 0.f, 0.f, 0.f}, low[2][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) low[0][i] = low[1][i] = 0.f;
+#pragma unroll
+      for (int jg = 0; jg < 4; ++jg) {
+        float high[2][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) high[0][i] = high[1][i] = 0.f;
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+          const int j = jg * 4 + jj, at = 4 * j + (j & 1 ? -sw : sw);
+          const float4 u = left[at], w = left[8 * (KC_DK / 2) + at];
+          KcA l;
+          l.hi[0] = u.x, l.hi[1] = w.x, l.hi[2] = u.y, l.hi[3] = w.y;
+          l.lo[0] = u.z, l.lo[1] = w.z, l.lo[2] = u.w, l.lo[3] = w.w;
+          const float* cp = right + 32 * j;
+          const float4 r = make_float4(cp[0], cp[4], cp[2], cp[6]);
+          kc_mma_low(low[jj & 1], l, r);
+          kc_mma_high(high[jj & 1], l, r);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[i] += high[0][i] + high[1][i];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sum[i] += low[0][i] + low[1][i];
+      const int s0 = sn * 8 + 2 * t4;
+      if (warp < 2) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int t = g + (i >> 1) * 8, ss = s0 + (i & 1);
+          sm.m[ss][t] = ss < t ? sum[i] * sm.beta[par][t] : 0.f;
+        }
+      } else {
+#pragma unroll
+        for (int tb = 0; tb < 2; ++tb) {
+          if (tb < sn) continue;
+          float4 o;
+          kc_split(s0 <= g + 8 * tb ? sum[2 * tb] : 0.f, o.x, o.z);
+          kc_split(s0 + 1 <= g + 8 * tb ? sum[2 * tb + 1] : 0.f, o.y, o.w);
+          sm.bf[par][tb + sn][lane] = o;
+        }
+      }
+    }
+    kc_sync(KC_BAR_PREP, 128);
+    if (warp == (chunk & 3)) {
+      // T, a column to a lane (lanes 16 .. 31 the same ones again)
+      const int c = lane & 15;
+      float x[KC_T];
+#pragma unroll
+      for (int t = 0; t < KC_T; ++t) x[t] = t == c ? 1.f : 0.f;
+#pragma unroll
+      for (int s = 0; s < KC_T - 1; ++s)
+#pragma unroll
+        for (int t = (s + 1) & ~3; t < KC_T; t += 4) {
+          const float4 mm = *reinterpret_cast<const float4*>(&sm.m[s][t]);
+          if (t > s) x[t] -= mm.x * x[s];
+          if (t + 1 > s) x[t + 1] -= mm.y * x[s];
+          if (t + 2 > s) x[t + 2] -= mm.z * x[s];
+          x[t + 3] -= mm.w * x[s];
+        }
+      const float be = sm.beta[par][c];
+#pragma unroll
+      for (int t = 0; t < KC_T; ++t) {
+        const int tb = t >> 3;
+        float hi, lo;
+        kc_split(x[t] * be, hi, lo);
+        if ((c >> 3) <= tb) reinterpret_cast<float*>(&sm.tf[par][tb + (c >> 3)][(t & 7) * 4 + ((c & 7) >> 1)])[(c & 1) + (lane >= 16 ? 2 : 0)] = lane >= 16 ? lo : hi;
+      }
+    }
+    kc_arrive(KC_BAR_T + par, 256);
+  }
+  return;
+  }
 
-    // ---- every warp walks the stage's blocks over its 16 columns ----
-    const int blocks = min(KB_BLOCKS, (q1 - t0 + KB_T - 1) / KB_T);
-#pragma unroll 1
-    for (int n = 0; n < blocks; ++n) {
-      const KdaBlock& B = sm.blk[n];
-      unsigned long long ak[KB_T][4], aq[KB_T][4];
+  // ================ walking warps ================
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(KC_REGS_WALK));
+  float* S = state + ((long long)slot * heads + h) * KC_DK * dv + c0 + warp * 16 + g;
+  float s[16][4];  // S^T: columns (g, g + 8), channels 8 j + 2 t4 + {0, 1}
 #pragma unroll
-      for (int t = 0; t < KB_T; ++t)
+  for (int j = 0; j < 16; ++j) {
+    const float* p = S + (long long)(8 * j + 2 * t4) * dv;
+    s[j][0] = p[0];
+    s[j][1] = p[dv];
+    s[j][2] = p[8];
+    s[j][3] = p[dv + 8];
+  }
+  for (int t0 = q0, chunk = 0; t0 < q1; t0 += KC_T, ++chunk) {
+    const int par = chunk & 1;
+    kc_sync(KC_BAR_ROWS, 256);
+    // ---- rk S' and rq S' for the warp's columns ----
+    float u[2][4], o[2][4], ul[2][4], ol[2][4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) ak[t][c] = aq[t][c] = 0ull;
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 4; ++i) u[n][i] = o[n][i] = ul[n][i] = ol[n][i] = 0.f;
+    const float4 *rk = &sm.rk[g][t4], *rq = &sm.rq[g][t4];
+    const float* fac = &sm.fac[2 * t4];
 #pragma unroll
-        for (int t = 0; t < KB_T; ++t) {
-          const ulonglong2 x = reinterpret_cast<const ulonglong2*>(B.kd[t])[i * 8 + rg], y = reinterpret_cast<const ulonglong2*>(B.qd[t])[i * 8 + rg];
+    for (int jg = 0; jg < 4; ++jg) {
+      float uh[2][4], oh[2][4];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            ak[t][c] = kb_fma2(s2[i][1][c], x.y, kb_fma2(s2[i][0][c], x.x, ak[t][c]));
-            aq[t][c] = kb_fma2(s2[i][1][c], y.y, kb_fma2(s2[i][0][c], y.x, aq[t][c]));
-          }
-        }
-      float sum[32];  // a token's four columns of kd, then of qd
+      for (int n = 0; n < 2; ++n)
 #pragma unroll
-      for (int t = 0; t < KB_T; ++t)
+        for (int i = 0; i < 4; ++i) uh[n][i] = oh[n][i] = 0.f;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float2 x = kb_split(ak[t][c]), y = kb_split(aq[t][c]);
-          sum[t * 8 + c] = x.x + x.y;
-          sum[t * 8 + 4 + c] = y.x + y.y;
-        }
-      // over the eight row groups (lane bits 0 .. 2): four columns of one token's kd or qd are left to each lane
-      kb_reduce_scatter<32>(sum, lane, 4);
-      *reinterpret_cast<float4*>(lane & 1 ? &sm.o[warp][(lane >> 1) & 3][cg * 4] : &sm.u[warp][(lane >> 1) & 3][cg * 4]) = make_float4(sum[0], sum[1], sum[2], sum[3]);
-      __syncwarp();
-      {
-        const int c = lane & 15;  // lanes l and l + 16 solve the same column
-        const float4 be = *reinterpret_cast<const float4*>(B.beta);
-        float ab[16];
+      for (int jj = 0; jj < 4; ++jj) {
+        const int j = jg * 4 + jj, at = 4 * j + (j & 1 ? -sw : sw);
+        const float2 fc = *reinterpret_cast<const float2*>(fac + 8 * j);
+        s[j][0] *= fc.x;
+        s[j][1] *= fc.y;
+        s[j][2] *= fc.x;
+        s[j][3] *= fc.y;
+        KcA l;
+        kc_left(s[j], l);
 #pragma unroll
-        for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(ab + i) = *reinterpret_cast<const float4*>(B.ab + i);
-        const float d0 = be.x * (B.v[0][warp * 16 + c] - sm.u[warp][0][c]);
-        const float d1 = be.y * (B.v[1][warp * 16 + c] - sm.u[warp][1][c] - ab[0] * d0);
-        const float d2 = be.z * (B.v[2][warp * 16 + c] - sm.u[warp][2][c] - ab[1] * d0 - ab[2] * d1);
-        const float d3 = be.w * (B.v[3][warp * 16 + c] - sm.u[warp][3][c] - ab[3] * d0 - ab[4] * d1 - ab[5] * d2);
-        const float o0 = sm.o[warp][0][c] + ab[6] * d0;
-        const float o1 = sm.o[warp][1][c] + ab[7] * d0 + ab[8] * d1;
-        const float o2 = sm.o[warp][2][c] + ab[9] * d0 + ab[10] * d1 + ab[11] * d2;
-        const float o3 = sm.o[warp][3][c] + ab[12] * d0 + ab[13] * d1 + ab[14] * d2 + ab[15] * d3;
-        const int t = t0 + n * KB_T + (lane >> 4) * 2;
-        bf16* dst = out + ((long long)t * heads + h) * dv + c0 + warp * 16 + c;
-        if (t < q1) dst[0] = __float2bfloat16(lane < 16 ? o0 : o2);
-        if (t + 1 < q1) dst[(long long)heads * dv] = __float2bfloat16(lane < 16 ? o1 : o3);
-        __syncwarp();  // both lanes of a column have read u
-        if (lane < 16) {
-          sm.u[warp][0][c] = d0;
-          sm.u[warp][1][c] = d1;
-          sm.u[warp][2][c] = d2;
-          sm.u[warp][3][c] = d3;
+        for (int n = 0; n < 2; ++n) {
+          const float4 x = rk[n * 8 * (KC_DK / 2) + at], y = rq[n * 8 * (KC_DK / 2) + at];
+          kc_mma_low(ul[n], l, x);
+          kc_mma_high(uh[n], l, x);
+          kc_mma_low(ol[n], l, y);
+          kc_mma_high(oh[n], l, y);
         }
       }
-      __syncwarp();
-      unsigned long long d2[KB_T][4];
 #pragma unroll
-      for (int t = 0; t < KB_T; ++t) {
-        const float4 x = *reinterpret_cast<const float4*>(&sm.u[warp][t][cg * 4]);
-        d2[t][0] = kb_pair(x.x, x.x);
-        d2[t][1] = kb_pair(x.y, x.y);
-        d2[t][2] = kb_pair(x.z, x.z);
-        d2[t][3] = kb_pair(x.w, x.w);
-      }
-      __syncwarp();  // d is read; the next block may put its sums there
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          u[n][i] += uh[n][i];
+          o[n][i] += oh[n][i];
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const ulonglong2 x = reinterpret_cast<const ulonglong2*>(B.dp)[i * 8 + rg];
+        u[n][i] += ul[n][i];
+        o[n][i] += ol[n][i];
+      }
+    if (t0 + KC_T < q1) kc_arrive(KC_BAR_FREE, 256);
+    kc_sync(KC_BAR_T + par, 256);
+    // ---- d = T (v - u), o += B d ----
+    KcA d[2];
+    {
+      KcA x[2];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          s2[i][0][c] = kb_mul2(s2[i][0][c], x.x);
-          s2[i][1][c] = kb_mul2(s2[i][1][c], x.y);
+      for (int n = 0; n < 2; ++n) {
+        float y[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[i] = to_f32(sm.raw_v[chunk & 3][8 * n + 2 * t4 + (i & 1)][warp * 16 + g + (i >> 1) * 8]) - u[n][i];
+        kc_left(y, x[n]);
+      }
+      const float4 tf[3] = {sm.tf[par][0][lane], sm.tf[par][1][lane], sm.tf[par][2][lane]}, bf[3] = {sm.bf[par][0][lane], sm.bf[par][1][lane], sm.bf[par][2][lane]};
+      float lo3[3][4], hi3[3][4];
+      auto both = [&](const KcA* l, const float4 (&r)[3], float (&sum)[2][4]) {  // sum[n] = the products of l and r, tokens up to n
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) lo3[k][i] = hi3[k][i] = 0.f;
+        kc_mma<3>({lo3[0], lo3[1], lo3[2]}, {hi3[0], hi3[1], hi3[2]}, {&l[0], &l[0], &l[1]}, r);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          sum[0][i] = hi3[0][i] + lo3[0][i];
+          sum[1][i] = (hi3[1][i] + hi3[2][i]) + (lo3[1][i] + lo3[2][i]);
         }
+      };
+      float dd[2][4];
+      both(x, tf, dd);
+      kc_left(dd[0], d[0]);
+      kc_left(dd[1], d[1]);
+      both(d, bf, dd);
 #pragma unroll
-        for (int t = 0; t < KB_T; ++t) {
-          const ulonglong2 y = reinterpret_cast<const ulonglong2*>(B.kh[t])[i * 8 + rg];
+      for (int n = 0; n < 2; ++n)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            s2[i][0][c] = kb_fma2(y.x, d2[t][c], s2[i][0][c]);
-            s2[i][1][c] = kb_fma2(y.y, d2[t][c], s2[i][1][c]);
-          }
+        for (int i = 0; i < 4; ++i) {
+          const int t = t0 + 8 * n + 2 * t4 + (i & 1);
+          if (t < q1) out[((long long)t * heads + h) * dv + c0 + warp * 16 + g + (i >> 1) * 8] = __float2bfloat16(o[n][i] + dd[n][i]);
         }
+    }
+    // ---- S' + sum c_s d_s ----
+    const float4* cp = &sm.c[par][t4][g ^ (t4 << 1)];
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+      float lo[4][4], hi[4][4];  // by j and half of the tokens
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) lo[k][i] = hi[k][i] = 0.f;
+      const float4 r[4] = {cp[8 * j], cp[4 * KC_DK + 8 * j], cp[8 * j + 8], cp[4 * KC_DK + 8 * j + 8]};
+      kc_mma<4>({lo[0], lo[1], lo[2], lo[3]}, {hi[0], hi[1], hi[2], hi[3]}, {&d[0], &d[1], &d[0], &d[1]}, r);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        s[j][i] += (hi[0][i] + hi[1][i]) + (lo[0][i] + lo[1][i]);
+        s[j + 1][i] += (hi[2][i] + hi[3][i]) + (lo[2][i] + lo[3][i]);
       }
     }
-    __syncthreads();  // the blocks may be written again
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      float2 x[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) x[c] = kb_split(s2[i][p][c]);
-      *reinterpret_cast<float4*>(S + (long long)(32 * i + 4 * rg + 2 * p) * dv + col) = make_float4(x[0].x, x[1].x, x[2].x, x[3].x);
-      *reinterpret_cast<float4*>(S + (long long)(32 * i + 4 * rg + 2 * p + 1) * dv + col) = make_float4(x[0].y, x[1].y, x[2].y, x[3].y);
-    }
+  for (int j = 0; j < 16; ++j) {
+    const float2 e = *reinterpret_cast<const float2*>(&sm.tail[8 * j + 2 * t4]);
+    float* p = S + (long long)(8 * j + 2 * t4) * dv;
+    p[0] = s[j][0] * e.x;
+    p[dv] = s[j][1] * e.y;
+    p[8] = s[j][2] * e.x;
+    p[dv + 8] = s[j][3] * e.y;
+  }
+}
+
+// More shared memory than a kernel gets unasked, on every device; and whether the registers that the walking warps will ask for are
+// in the block's share.
+cudaError_t kc_allow() {
+  static std::atomic<bool> set[64];
+  int dev = 0;
+  if (cudaError_t e = cudaGetDevice(&dev)) return e;
+  if (set[dev & 63].load(std::memory_order_acquire)) return cudaSuccess;
+  cudaFuncAttributes fa;
+  if (cudaError_t e = cudaFuncGetAttributes(&fa, kda_chunk_kernel)) return e;
+  if (2 * fa.numRegs < KC_REGS_PREP + KC_REGS_WALK) return cudaErrorLaunchOutOfResources;
+  if (cudaError_t e = cudaFuncSetAttribute(kda_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KcSmem))) return e;
+  set[dev & 63].store(true, std::memory_order_release);
+  return cudaSuccess;
 }
 
 constexpr int ATTNRES_MAX = 16;  // candidates of one mix (snapshots + the current row)
@@ -631,7 +815,7 @@ __global__ void __launch_bounds__(256) attnres_mix_kernel(const bf16* __restrict
 
 }  // namespace
 
-// Sequences of min_len tokens and more go four tokens at a time where rows and state are runs of 16-byte pieces, shorter ones (of
+// Sequences of min_len tokens and more go in chunks where rows and state are runs of 16-byte pieces, shorter ones (of
 // up to `short_len` tokens; 0: there are none) token by token in a launch of their own, so that a decode row beside a prompt is
 // what it is in a step of decode rows.
 extern "C" int pg_kda_recurrent(const void* q, const void* k, const void* v, long long ld, const void* f, long long ldf, const void* b, long long ldb,
@@ -642,10 +826,10 @@ extern "C" int pg_kda_recurrent(const void* q, const void* k, const void* v, lon
   if (num_seqs == 0) return PG_OK;
   RecArgs<bf16> p = {(const bf16*)q, (const bf16*)k, (const bf16*)v, ld, f, ldf, (const bf16*)b, ldb, (const float*)a_log, (const float*)dt_bias, nullptr, lower,
                      (float*)state, (bf16*)out, (const int*)q_indptr, (const int*)slots, heads, heads, dk, dv, (dv + KDA_COLS - 1) / KDA_COLS, 0};
-  const bool blocks = max_q_len >= min_len && dk == KB_DK && dv % KB_COLS == 0 && ld % 8 == 0 && ldf % 8 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)f | (uintptr_t)dt_bias | (uintptr_t)state) & 15) == 0;
+  const bool blocks = max_q_len >= min_len && dk == KC_DK && dv % KC_COLS == 0 && lower >= KC_LOWER && ld % 8 == 0 && ldf % 8 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)f | (uintptr_t)dt_bias | (uintptr_t)state) & 15) == 0;
   if (blocks) {
-    kda_block_kernel<<<dim3(heads * (dv / KB_COLS), num_seqs), 128, sizeof(KdaBlockSmem), stream>>>(p.q, p.k, p.v, ld, (const bf16*)f, ldf, p.b, ldb, p.a_log, p.dt_bias, lower, p.state, p.out, p.q_indptr, p.slots,
-                                                                                                     heads, dv, min_len);
+    PG_CUDA(kc_allow());
+    kda_chunk_kernel<<<dim3(heads * (dv / KC_COLS), num_seqs), 256, sizeof(KcSmem), stream>>>(p.q, p.k, p.v, ld, (const bf16*)f, ldf, p.b, ldb, p.a_log, p.dt_bias, lower, p.state, p.out, p.q_indptr, p.slots, heads, dv, min_len);
     PG_LAUNCH_CHECK();
     if (short_len <= 0) return PG_OK;
     p.skip_len = min_len;

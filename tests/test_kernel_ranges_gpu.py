@@ -523,3 +523,32 @@ def test_int4_experts_of_ragged_rows(m, k, bn, aligned):
         assert ((got[at : at + n].double() - a @ w.T).abs() <= bound).all()
         at += n
     assert cu().read_status(DEV) == 0
+
+
+@pytest.mark.parametrize("lower", [-5.0, -5.25, -5.5])  # chunks of 16 tokens down to -5.25, token by token below
+@pytest.mark.parametrize("shift", [6.0, -6.0, 0.0])  # decays near exp(lower), near one, both
+def test_kda_chunks_of_strong_and_weak_decays(lower, shift):
+    torch.manual_seed(int(shift) + 20)
+    heads, dk, dv, q_lens = 2, 128, 128, [15, 16, 17, 31, 32, 48, 65]
+    meta, t, n = _state_meta(q_lens, list(range(1, len(q_lens) + 1))), sum(q_lens), len(q_lens)
+    q, k, v = (torch.randn(t, heads, dk, device=DEV).bfloat16() for _ in range(3))
+    f, b = (torch.randn(t, heads * dk, device=DEV) * (8 if shift == 0 else 1) + shift).bfloat16(), torch.randn(t, heads, device=DEV).bfloat16()
+    a_log, dt = torch.zeros(heads, device=DEV), torch.zeros(heads * dk, device=DEV)
+    st1 = torch.randn(n + 1, heads, dk, dv, device=DEV)
+    st2 = st1.double()
+    o1 = cu().kda_recurrent(q, k, v, f, b, a_log, dt, lower, st1, meta)
+    unit = lambda x: x * torch.rsqrt(x.pow(2).sum(-1, keepdim=True) + 1e-6)  # noqa: E731
+    qd, kd = unit(q.double()) * dk ** -0.5, unit(k.double())
+    dec, beta, at = torch.exp(lower * torch.sigmoid(f.double().view(t, heads, dk))), torch.sigmoid(b.double()), 0
+    for s, m in enumerate(q_lens):
+        S = st2[s + 1]
+        for i in range(at, at + m):
+            S = S * dec[i].unsqueeze(-1)
+            d = (v[i].double() - torch.einsum("hkv,hk->hv", S, kd[i])) * beta[i].unsqueeze(-1)
+            S = S + kd[i].unsqueeze(-1) * d.unsqueeze(1)
+            want = torch.einsum("hkv,hk->hv", S, qd[i])
+            # bf16 output; f32 sums of 128 channels and 16 tokens, 2^-23 a step
+            assert (o1[i].double() - want).abs().max() <= 2 ** -8 * want.abs().max() + 1e-5
+        st2[s + 1] = S
+        at += m
+    assert (st1.double() - st2).abs().max() < 2 ** -17 * st2.abs().max()
