@@ -281,6 +281,302 @@ int run_rule(int rule, RecArgs<T> p, int num_seqs, int max_q_len, cudaStream_t s
 }
 
 // ---------------------------------------------------------------------------------
+// The delta rule with bounded channel decays, KB_T tokens at a time (short prompts, 128-wide keys).  Inside a block
+//   kd_t = k_t * P_t, qd_t = q_t * P_t      (P_t: product of the block's decays up to and with token t)
+//   kh_t = k_t * (product of the decays behind t),   A_ts = k_t . (k_s * decays of s+1 .. t),   B_ts likewise with q_t
+// do not depend on the state, so a warp forms them once per block for all columns of the CTA, and per state column
+//   d_t = beta_t (v_t - kd_t . S0 - sum_{s<t} A_ts d_s),   o_t = qd_t . S0 + sum_{s<=t} B_ts d_s,
+//   S   = (all decays) * S0 + sum_t kh_t d_t
+// Everything stays f32 (products of decays only, no quotients, so nothing can overflow).  Against the token-by-token walk
+// this takes 3.25 multiply-adds per state element and token instead of 4, and one reduction, one solve per KB_T tokens.
+// A lane holds 16 rows x 4 columns of the state as row pairs for the packed f32x2 instructions; the 8 lanes of a column
+// group read 128 contiguous bytes of a vector at a time, which is what the walk, with 32 elements of one column per thread,
+// was short of: shared-memory reads (three vectors per 32 elements and token there, 13 per 64 elements and 4 tokens here).
+// 3001 tokens in two prompts, 96 heads: 2550 us before, 1145 us now; 16 heads, one prompt of 3000: 1644 and 1099.  Decode rows
+// beside a prompt stay on the walk (64 rows and 300 tokens, 96 heads: 398 us with every row in a block of four, 333 now).  What bounds it: FMA issue and shared-memory reads
+// (both near half of their rate) by warps that wait for their own sums, few of them where a step has few sequences.
+constexpr int KB_T = 4;        // tokens per block
+constexpr int KB_BLOCKS = 4;   // blocks per stage: one per warp to prepare
+constexpr int KB_COLS = 64;    // state columns per CTA, 16 per warp
+constexpr int KB_DK = 128;
+
+struct KdaBlock {
+  float kd[KB_T][KB_DK], qd[KB_T][KB_DK], kh[KB_T][KB_DK], dp[KB_DK];
+  float v[KB_T][KB_COLS];
+  float ab[16];  // A_ts at t (t - 1) / 2 + s, B_ts at 6 + t (t + 1) / 2 + s
+  float beta[KB_T];
+};
+struct KdaBlockSmem {  // 47 KB: no attribute needed
+  KdaBlock blk[KB_BLOCKS];
+  bf16 raw[KB_BLOCKS][3][KB_T][KB_DK];  // q, k, f rows of the stage after this one
+  bf16 raw_v[KB_BLOCKS][KB_T][KB_COLS];
+  float u[4][KB_T][16], o[4][KB_T][16];  // per warp: kd . S0, then d; qd . S0
+};
+
+static_assert(sizeof(KdaBlockSmem) <= 48 * 1024, "more needs the kernel's attribute, on every device");
+__device__ __forceinline__ unsigned long long kb_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long kb_mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long kb_pair(float lo, float hi) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float2 kb_split(unsigned long long a) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(a));
+  return f;
+}
+// Sum over lanes of N values per lane, scattered: every step halves the values a lane still carries.  Bit `top` of the lane
+// picks the upper half first.
+template <int N>
+__device__ __forceinline__ void kb_reduce_scatter(float* v, int lane, int top) {
+#pragma unroll
+  for (int n = N / 2, bit = top; n > 0 && bit > 0; n >>= 1, bit >>= 1) {
+    const bool up = lane & bit;
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+      const float send = up ? v[j] : v[j + n], keep = up ? v[j + n] : v[j];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(128, 3)
+kda_block_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v, long long ld, const bf16* __restrict__ f, long long ldf, const bf16* __restrict__ b, long long ldb,
+                 const float* __restrict__ a_log, const float* __restrict__ dt_bias, float lower, float* __restrict__ state, bf16* __restrict__ out, const int* __restrict__ q_indptr,
+                 const int* __restrict__ slots, int heads, int dv, int min_len) {
+  extern __shared__ __align__(16) uint8_t kb_raw[];
+  KdaBlockSmem& sm = *reinterpret_cast<KdaBlockSmem*>(kb_raw);
+  const int groups = dv / KB_COLS;
+  const int h = blockIdx.x / groups, c0 = blockIdx.x % groups * KB_COLS, seq = blockIdx.y;
+  const int slot = slots[seq];
+  const int q0 = q_indptr[seq], q1 = q_indptr[seq + 1];
+  if (q1 - q0 < min_len || slot < 0) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rg = lane & 7, cg = lane >> 3;
+  const int col = c0 + warp * 16 + cg * 4;  // the lane's first state column
+  float* S = state + ((long long)slot * heads + h) * KB_DK * dv;
+
+  // raw rows of this warp's block of the stage that starts at token t0; rows past the end are zero
+  float b_next = 0.f;
+  auto fetch = [&](int t0) {
+    const int t = t0 + warp * KB_T;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      const int c = lane + 32 * (i & 1), r = c >> 4, ch = (c & 15) * 8;
+      const bool ok = t + r < q1;
+      const long long row = ok ? t + r : q0;
+      const bf16* src = i < 2 ? q + row * ld : i < 4 ? k + row * ld : f + row * ldf;
+      cp_async16(&sm.raw[warp][i >> 1][r][ch], src + (long long)h * KB_DK + ch, ok);
+    }
+    const int r = lane >> 3, ch = (lane & 7) * 8;
+    const bool ok = t + r < q1;
+    cp_async16(&sm.raw_v[warp][r][ch], v + (ok ? t + r : q0) * ld + (long long)h * dv + c0 + ch, ok);
+    cp_async_commit();
+    b_next = lane < KB_T && t + lane < q1 ? to_f32(b[(long long)(t + lane) * ldb + h]) : 0.f;
+  };
+  fetch(q0);
+
+  unsigned long long s2[4][2][4];  // rows 32 i + 4 rg + {0, 1} and {2, 3}, columns col .. col + 3
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const float4 lo = *reinterpret_cast<const float4*>(S + (long long)(32 * i + 4 * rg + 2 * p) * dv + col);
+      const float4 hi = *reinterpret_cast<const float4*>(S + (long long)(32 * i + 4 * rg + 2 * p + 1) * dv + col);
+      s2[i][p][0] = kb_pair(lo.x, hi.x);
+      s2[i][p][1] = kb_pair(lo.y, hi.y);
+      s2[i][p][2] = kb_pair(lo.z, hi.z);
+      s2[i][p][3] = kb_pair(lo.w, hi.w);
+    }
+  const float a = __expf(a_log[h]), q_scale = rsqrtf((float)KB_DK);
+
+  for (int t0 = q0; t0 < q1; t0 += KB_T * KB_BLOCKS) {
+    // ---- each warp prepares one block; a lane has four key channels of its four tokens ----
+    cp_async_wait_all();
+    __syncwarp();
+    {
+      KdaBlock& B = sm.blk[warp];
+      const int first = t0 + warp * KB_T;
+      float kk[KB_T][4], qq[KB_T][4], dec[KB_T][4];
+      const float4 db = *reinterpret_cast<const float4*>(dt_bias + h * KB_DK + lane * 4);
+      const float bias[4] = {db.x, db.y, db.z, db.w};
+#pragma unroll
+      for (int t = 0; t < KB_T; ++t) {
+        float x[3][4], qs = 0.f, ks = 0.f;
+#pragma unroll
+        for (int w = 0; w < 3; ++w) {
+          const uint2 raw = *reinterpret_cast<const uint2*>(&sm.raw[warp][w][t][lane * 4]);
+          const float2 lo = __bfloat1622float2(*reinterpret_cast<const bf162*>(&raw.x)), hi = __bfloat1622float2(*reinterpret_cast<const bf162*>(&raw.y));
+          x[w][0] = lo.x, x[w][1] = lo.y, x[w][2] = hi.x, x[w][3] = hi.y;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          qs += x[0][e] * x[0][e];
+          ks += x[1][e] * x[1][e];
+        }
+        qs = warp_sum(qs);
+        ks = warp_sum(ks);
+        const float qn = rsqrtf(qs + 1e-6f) * q_scale, kn = rsqrtf(ks + 1e-6f);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          qq[t][e] = x[0][e] * qn;
+          kk[t][e] = x[1][e] * kn;
+          const float raw = x[2][e] + bias[e];
+          dec[t][e] = first + t < q1 ? __expf(lower / (1.f + __expf(-a * raw))) : 1.f;
+        }
+      }
+      float ab[16], w[KB_T][4];
+#pragma unroll
+      for (int s = 0; s < KB_T; ++s) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[s][e] = kk[s][e];
+#pragma unroll
+        for (int t = s; t < KB_T; ++t) {  // w[s] = k_s times the decays of s + 1 .. t
+          float x = 0.f, y = 0.f;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (t > s) w[s][e] *= dec[t][e];
+            x += kk[t][e] * w[s][e];
+            y += qq[t][e] * w[s][e];
+          }
+          if (t > s) ab[t * (t - 1) / 2 + s] = x;
+          ab[6 + t * (t + 1) / 2 + s] = y;
+        }
+        *reinterpret_cast<float4*>(&B.kh[s][lane * 4]) = make_float4(w[s][0], w[s][1], w[s][2], w[s][3]);
+      }
+      float cum[4] = {1.f, 1.f, 1.f, 1.f};
+#pragma unroll
+      for (int t = 0; t < KB_T; ++t) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) cum[e] *= dec[t][e];
+        *reinterpret_cast<float4*>(&B.kd[t][lane * 4]) = make_float4(kk[t][0] * cum[0], kk[t][1] * cum[1], kk[t][2] * cum[2], kk[t][3] * cum[3]);
+        *reinterpret_cast<float4*>(&B.qd[t][lane * 4]) = make_float4(qq[t][0] * cum[0], qq[t][1] * cum[1], qq[t][2] * cum[2], qq[t][3] * cum[3]);
+        const float2 vv = __bfloat1622float2(*reinterpret_cast<const bf162*>(&sm.raw_v[warp][t][lane * 2]));
+        *reinterpret_cast<float2*>(&B.v[t][lane * 2]) = vv;
+      }
+      *reinterpret_cast<float4*>(&B.dp[lane * 4]) = make_float4(cum[0], cum[1], cum[2], cum[3]);
+      kb_reduce_scatter<16>(ab, lane, 16);
+      ab[0] += __shfl_xor_sync(0xffffffffu, ab[0], 1);
+      if (!(lane & 1)) B.ab[lane >> 1] = ab[0];
+      if (lane < KB_T) B.beta[lane] = first + lane < q1 ? 1.f / (1.f + __expf(-b_next)) : 0.f;
+    }
+    __syncthreads();
+    if (t0 + KB_T * KB_BLOCKS < q1) fetch(t0 + KB_T * KB_BLOCKS);
+
+    // ---- every warp walks the stage's blocks over its 16 columns ----
+    const int blocks = min(KB_BLOCKS, (q1 - t0 + KB_T - 1) / KB_T);
+#pragma unroll 1
+    for (int n = 0; n < blocks; ++n) {
+      const KdaBlock& B = sm.blk[n];
+      unsigned long long ak[KB_T][4], aq[KB_T][4];
+#pragma unroll
+      for (int t = 0; t < KB_T; ++t)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) ak[t][c] = aq[t][c] = 0ull;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int t = 0; t < KB_T; ++t) {
+          const ulonglong2 x = reinterpret_cast<const ulonglong2*>(B.kd[t])[i * 8 + rg], y = reinterpret_cast<const ulonglong2*>(B.qd[t])[i * 8 + rg];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            ak[t][c] = kb_fma2(s2[i][1][c], x.y, kb_fma2(s2[i][0][c], x.x, ak[t][c]));
+            aq[t][c] = kb_fma2(s2[i][1][c], y.y, kb_fma2(s2[i][0][c], y.x, aq[t][c]));
+          }
+        }
+      float sum[32];  // a token's four columns of kd, then of qd
+#pragma unroll
+      for (int t = 0; t < KB_T; ++t)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float2 x = kb_split(ak[t][c]), y = kb_split(aq[t][c]);
+          sum[t * 8 + c] = x.x + x.y;
+          sum[t * 8 + 4 + c] = y.x + y.y;
+        }
+      // over the eight row groups (lane bits 0 .. 2): four columns of one token's kd or qd are left to each lane
+      kb_reduce_scatter<32>(sum, lane, 4);
+      *reinterpret_cast<float4*>(lane & 1 ? &sm.o[warp][(lane >> 1) & 3][cg * 4] : &sm.u[warp][(lane >> 1) & 3][cg * 4]) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+      __syncwarp();
+      {
+        const int c = lane & 15;  // lanes l and l + 16 solve the same column
+        const float4 be = *reinterpret_cast<const float4*>(B.beta);
+        float ab[16];
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(ab + i) = *reinterpret_cast<const float4*>(B.ab + i);
+        const float d0 = be.x * (B.v[0][warp * 16 + c] - sm.u[warp][0][c]);
+        const float d1 = be.y * (B.v[1][warp * 16 + c] - sm.u[warp][1][c] - ab[0] * d0);
+        const float d2 = be.z * (B.v[2][warp * 16 + c] - sm.u[warp][2][c] - ab[1] * d0 - ab[2] * d1);
+        const float d3 = be.w * (B.v[3][warp * 16 + c] - sm.u[warp][3][c] - ab[3] * d0 - ab[4] * d1 - ab[5] * d2);
+        const float o0 = sm.o[warp][0][c] + ab[6] * d0;
+        const float o1 = sm.o[warp][1][c] + ab[7] * d0 + ab[8] * d1;
+        const float o2 = sm.o[warp][2][c] + ab[9] * d0 + ab[10] * d1 + ab[11] * d2;
+        const float o3 = sm.o[warp][3][c] + ab[12] * d0 + ab[13] * d1 + ab[14] * d2 + ab[15] * d3;
+        const int t = t0 + n * KB_T + (lane >> 4) * 2;
+        bf16* dst = out + ((long long)t * heads + h) * dv + c0 + warp * 16 + c;
+        if (t < q1) dst[0] = __float2bfloat16(lane < 16 ? o0 : o2);
+        if (t + 1 < q1) dst[(long long)heads * dv] = __float2bfloat16(lane < 16 ? o1 : o3);
+        __syncwarp();  // both lanes of a column have read u
+        if (lane < 16) {
+          sm.u[warp][0][c] = d0;
+          sm.u[warp][1][c] = d1;
+          sm.u[warp][2][c] = d2;
+          sm.u[warp][3][c] = d3;
+        }
+      }
+      __syncwarp();
+      unsigned long long d2[KB_T][4];
+#pragma unroll
+      for (int t = 0; t < KB_T; ++t) {
+        const float4 x = *reinterpret_cast<const float4*>(&sm.u[warp][t][cg * 4]);
+        d2[t][0] = kb_pair(x.x, x.x);
+        d2[t][1] = kb_pair(x.y, x.y);
+        d2[t][2] = kb_pair(x.z, x.z);
+        d2[t][3] = kb_pair(x.w, x.w);
+      }
+      __syncwarp();  // d is read; the next block may put its sums there
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const ulonglong2 x = reinterpret_cast<const ulonglong2*>(B.dp)[i * 8 + rg];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          s2[i][0][c] = kb_mul2(s2[i][0][c], x.x);
+          s2[i][1][c] = kb_mul2(s2[i][1][c], x.y);
+        }
+#pragma unroll
+        for (int t = 0; t < KB_T; ++t) {
+          const ulonglong2 y = reinterpret_cast<const ulonglong2*>(B.kh[t])[i * 8 + rg];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            s2[i][0][c] = kb_fma2(y.x, d2[t][c], s2[i][0][c]);
+            s2[i][1][c] = kb_fma2(y.y, d2[t][c], s2[i][1][c]);
+          }
+        }
+      }
+    }
+    __syncthreads();  // the blocks may be written again
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      float2 x[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) x[c] = kb_split(s2[i][p][c]);
+      *reinterpret_cast<float4*>(S + (long long)(32 * i + 4 * rg + 2 * p) * dv + col) = make_float4(x[0].x, x[1].x, x[2].x, x[3].x);
+      *reinterpret_cast<float4*>(S + (long long)(32 * i + 4 * rg + 2 * p + 1) * dv + col) = make_float4(x[0].y, x[1].y, x[2].y, x[3].y);
+    }
+}
+
+// ---------------------------------------------------------------------------------
 // The delta rule with bounded channel decays, KC_T tokens at a time (prompts, 128-wide keys), on the tensor cores.  With P_t the
 // product of the chunk's decays up to and with token t, and token 7 as the reference,
 //   rk_t = k_t P_t / P_7,   rq_t = q_t P_t / P_7,   c_s = k_s P_7 / P_s,   S' = P_7 S0,
@@ -815,21 +1111,27 @@ __global__ void __launch_bounds__(256) attnres_mix_kernel(const bf16* __restrict
 
 }  // namespace
 
-// Sequences of min_len tokens and more go in chunks where rows and state are runs of 16-byte pieces, shorter ones (of
+// Sequences of min_len tokens and more go in blocks of four tokens, or in chunks of sixteen, where rows and state are runs of 16-byte pieces, shorter ones (of
 // up to `short_len` tokens; 0: there are none) token by token in a launch of their own, so that a decode row beside a prompt is
 // what it is in a step of decode rows.
 extern "C" int pg_kda_recurrent(const void* q, const void* k, const void* v, long long ld, const void* f, long long ldf, const void* b, long long ldb,
                                 const void* a_log, const void* dt_bias, float lower, void* state, void* out, const void* q_indptr, const void* slots,
-                                int num_seqs, int heads, int dk, int dv, int max_q_len, int min_len, int short_len, cudaStream_t stream) {
+                                int num_seqs, int heads, int dk, int dv, int max_q_len, int min_len, int chunks, int short_len, cudaStream_t stream) {
   PG_REQUIRE(dv <= 128 && lower < 0.f, "kda_recurrent: dv=%d must be <= 128 and the decay lower bound %f negative", dv, (double)lower);
   PG_REQUIRE(min_len >= 1, "kda_recurrent: blocks for sequences of %d tokens", min_len);
   if (num_seqs == 0) return PG_OK;
   RecArgs<bf16> p = {(const bf16*)q, (const bf16*)k, (const bf16*)v, ld, f, ldf, (const bf16*)b, ldb, (const float*)a_log, (const float*)dt_bias, nullptr, lower,
                      (float*)state, (bf16*)out, (const int*)q_indptr, (const int*)slots, heads, heads, dk, dv, (dv + KDA_COLS - 1) / KDA_COLS, 0};
-  const bool blocks = max_q_len >= min_len && dk == KC_DK && dv % KC_COLS == 0 && lower >= KC_LOWER && ld % 8 == 0 && ldf % 8 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)f | (uintptr_t)dt_bias | (uintptr_t)state) & 15) == 0;
+  const bool blocks = max_q_len >= min_len && dk == KC_DK && dv % KC_COLS == 0 && ld % 8 == 0 && ldf % 8 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)f | (uintptr_t)dt_bias | (uintptr_t)state) & 15) == 0;
   if (blocks) {
-    PG_CUDA(kc_allow());
-    kda_chunk_kernel<<<dim3(heads * (dv / KC_COLS), num_seqs), 256, sizeof(KcSmem), stream>>>(p.q, p.k, p.v, ld, (const bf16*)f, ldf, p.b, ldb, p.a_log, p.dt_bias, lower, p.state, p.out, p.q_indptr, p.slots, heads, dv, min_len);
+    static_assert(KB_COLS == KC_COLS && KB_DK == KC_DK, "both kernels take the same steps");
+    const dim3 all(heads * (dv / KC_COLS), num_seqs);
+    if (chunks && lower >= KC_LOWER) {
+      PG_CUDA(kc_allow());
+      kda_chunk_kernel<<<all, 256, sizeof(KcSmem), stream>>>(p.q, p.k, p.v, ld, (const bf16*)f, ldf, p.b, ldb, p.a_log, p.dt_bias, lower, p.state, p.out, p.q_indptr, p.slots, heads, dv, min_len);
+    } else {
+      kda_block_kernel<<<all, 128, sizeof(KdaBlockSmem), stream>>>(p.q, p.k, p.v, ld, (const bf16*)f, ldf, p.b, ldb, p.a_log, p.dt_bias, lower, p.state, p.out, p.q_indptr, p.slots, heads, dv, min_len);
+    }
     PG_LAUNCH_CHECK();
     if (short_len <= 0) return PG_OK;
     p.skip_len = min_len;

@@ -525,11 +525,11 @@ def test_int4_experts_of_ragged_rows(m, k, bn, aligned):
     assert cu().read_status(DEV) == 0
 
 
-@pytest.mark.parametrize("lower", [-5.0, -5.25, -5.5])  # chunks of 16 tokens down to -5.25, token by token below
+@pytest.mark.parametrize("lower", [-5.0, -5.25, -5.5])  # chunks of 16 tokens down to -5.25, blocks of four below
 @pytest.mark.parametrize("shift", [6.0, -6.0, 0.0])  # decays near exp(lower), near one, both
 def test_kda_chunks_of_strong_and_weak_decays(lower, shift):
     torch.manual_seed(int(shift) + 20)
-    heads, dk, dv, q_lens = 2, 128, 128, [15, 16, 17, 31, 32, 48, 65]
+    heads, dk, dv, q_lens = 2, 128, 128, [15, 16, 17, 31, 48, 400, 401]
     meta, t, n = _state_meta(q_lens, list(range(1, len(q_lens) + 1))), sum(q_lens), len(q_lens)
     q, k, v = (torch.randn(t, heads, dk, device=DEV).bfloat16() for _ in range(3))
     f, b = (torch.randn(t, heads * dk, device=DEV) * (8 if shift == 0 else 1) + shift).bfloat16(), torch.randn(t, heads, device=DEV).bfloat16()
