@@ -295,7 +295,8 @@ __global__ void __launch_bounds__(ST) sample_kernel(const T* __restrict__ logits
 // descent with counts and masses, which ends after its first level where they are all alike (64 rows of 151936 equal logits: 114 us;
 // 237 with the four radix levels of all tokens).  Bound by the latency of the passes and of the eight cluster barriers between them, with
 // every row of a batch of 64 resident at once (clusters of four).  64 x 151936 bf16, top-k 50, top-p 0.9: 200 us with all tokens
-// taking part in each of four radix levels, one warp match per 32 tokens; 61 us now (1 row: 36 us).
+// taking part in each of four radix levels, one warp match per 32 tokens; 61 us with a key formed for every token in every pass, 47 with those
+// passed over whose piece of eight has its largest logit below what the pass looks for (1 row: 33 and 28 us).
 // ---------------------------------------------------------------------------------
 constexpr int SC_THREADS = 512;
 constexpr int SC_WARPS = SC_THREADS / 32;
@@ -346,9 +347,25 @@ struct ScShared {
 // floor(e * 2^40) of a token by its bits (2^-40 <= e < 2^24), in integer instructions: a conversion to 64 bits takes several
 // times as long as the rest of a token's work
 __device__ __forceinline__ unsigned long long sc_fx(uint32_t key) {
-  const unsigned long long mant = (key & 0x7fffffu) | 0x800000u;
-  const int shift = (int)(key >> 23) - (127 - 40 + 23);
-  return shift >= 0 ? mant << shift : mant >> -shift;
+  const uint32_t mant = (key & 0x7fffffu) | 0x800000u, hi = mant >> 15, lo = mant << 17;
+  const int r = 127 - (int)(key >> 23);  // (hi, lo) = mantissa * 2^17, shifted right by 0 .. 40 (left, where e is 2 and more)
+  if (r < 0) return (unsigned long long)mant << (17 - r);
+  const uint32_t both = __funnelshift_r(lo, hi, r), high = hi >> (r & 31);
+  return r & 32 ? (unsigned long long)high : (unsigned long long)high << 32 | both;
+}
+
+// Largest of the logits in 16 bytes; a NaN only where all are.
+template <typename T>
+__device__ __forceinline__ float sc_max(const uint4& x);
+template <>
+__device__ __forceinline__ float sc_max<bf16>(const uint4& x) {
+  const bf162* p = reinterpret_cast<const bf162*>(&x);
+  const bf162 a = __hmax2(__hmax2(p[0], p[1]), __hmax2(p[2], p[3]));
+  return fmaxf(__low2float(a), __high2float(a));
+}
+template <>
+__device__ __forceinline__ float sc_max<float>(const uint4& x) {
+  return fmaxf(fmaxf(__uint_as_float(x.x), __uint_as_float(x.y)), fmaxf(__uint_as_float(x.z), __uint_as_float(x.w)));
 }
 
 // Totals of the lanes above this one, of three quantities.
@@ -404,25 +421,24 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
   };
 
   // the slice into shared memory (slices start at multiples of eight tokens); local max
-  float m = -FLT_MAX;
+  float raw = -INFINITY;  // (the largest logit is the largest tempered one: a product with one positive factor keeps the order)
   constexpr int VEC = 16 / sizeof(T);
   int done = 0;
   if (((reinterpret_cast<uintptr_t>(r) | (uintptr_t)(i0 * sizeof(T))) & 15) == 0) {
     done = n / VEC * VEC;
+#pragma unroll 4
     for (int i = tid; i < n / VEC; i += SC_THREADS) {
       const uint4 x = reinterpret_cast<const uint4*>(r + i0)[i];
       reinterpret_cast<uint4*>(vals)[i] = x;
-      const T* e = reinterpret_cast<const T*>(&x);
-#pragma unroll
-      for (int j = 0; j < VEC; ++j) m = fmaxf(m, ldf(e, j) * inv_t);
+      raw = fmaxf(raw, sc_max<T>(x));
     }
   }
   for (int i = done + tid; i < n; i += SC_THREADS) {
     const T x = r[i0 + i];
     vals[i] = x;
-    m = fmaxf(m, ldf(&x, 0) * inv_t);
+    raw = fmaxf(raw, ldf(&x, 0));
   }
-  m = block_max_f(m, red);
+  float m = block_max_f(fmaxf(raw * inv_t, -FLT_MAX), red);
   if (tid == 0) {
     sh.x_f32 = m;
     sh.list_n = 0u;
@@ -446,11 +462,13 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
     return e > 0.f ? min(__float_as_uint(e), SC_ONE) : 0u;
   };
   // f(keys) for the slice's tokens `from` + VEC * first .. `to`, 16 bytes of them at a time, every `step` pieces; all lanes of a
-  // warp come together (tokens behind `to` have key 0)
-  auto walk = [&](int from, int to, int first, int step, auto&& f) {
+  // warp come together (tokens behind `to` have key 0) unless there is a cut: lanes whose tokens all lie below it stay away.
+  // (What is looked for is mostly some hundred tokens; a key takes some 15 instructions, the largest of eight logits four.)
+  auto walk = [&](int from, int to, int first, int step, float cut, auto&& f) {
     for (int b = from + (first - lane) * VEC; b < to; b += step * VEC) {
       const int i = b + lane * VEC;
       const uint4 x = i < to ? *reinterpret_cast<const uint4*>(vals + i) : make_uint4(0u, 0u, 0u, 0u);
+      if (sc_max<T>(x) * inv_t - m < cut) continue;
       uint32_t key[VEC];
 #pragma unroll
       for (int j = 0; j < VEC; ++j) key[j] = i + j < to ? key_of(ldf(reinterpret_cast<const T*>(&x), j)) : 0u;
@@ -458,6 +476,8 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
     }
   };
 
+  // tokens with s - m below it have keys below `key`, however the logarithm and the exponential round
+  auto cut_of = [&](uint32_t key) { return __logf(__uint_as_float(key)) - 1e-3f; };
   const uint32_t kk = top_k[row] > 0 ? (uint32_t)min(top_k[row], vocab) : (uint32_t)vocab;
   const float tp = top_p[row];
   const float mp = min_p[row];
@@ -465,7 +485,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
   if (kk < (uint32_t)vocab || tp < 1.f) {  // the same for the whole cluster: every CTA reads the row's controls
     // ---- coarse counts and the normaliser ----
     unsigned long long z = 0ull;
-    walk(0, n, tid, SC_THREADS, [&](const uint32_t (&key)[VEC]) {
+    walk(0, n, tid, SC_THREADS, -INFINITY, [&](const uint32_t (&key)[VEC]) {
       bool same = key[0] >= SC_LOW;  // (equal logits: one atomic for all of a thread's)
 #pragma unroll
       for (int j = 1; j < VEC; ++j) same = same && key[j] == key[0];
@@ -554,7 +574,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
       unsigned long long above = 0ull;
       uint32_t n_above = 0u;
       uint32_t least = SC_ONE, most = 0u;
-      walk(0, n, tid, SC_THREADS, [&](const uint32_t (&key)[VEC]) {
+      walk(0, n, tid, SC_THREADS, cut_of(k_lo), [&](const uint32_t (&key)[VEC]) {
 #pragma unroll
         for (int j = 0; j < VEC; ++j)
           if (key[j] >= k_hi) {
@@ -636,7 +656,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
             add(key, key >= k_lo);
           }
         } else {
-          walk(0, n, tid, SC_THREADS, [&](const uint32_t (&key)[VEC]) {
+          walk(0, n, tid, SC_THREADS, -INFINITY, [&](const uint32_t (&key)[VEC]) {
 #pragma unroll
             for (int j = 0; j < VEC; ++j) add(key[j], key[j] >= k_lo && key[j] < k_hi);
           });
@@ -723,7 +743,8 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
   const int run = ((n + SC_WARPS - 1) / SC_WARPS + 31) & ~31;  // (a multiple of a 16-byte piece)
   const int c0 = min(n, warp * run), c1 = min(n, c0 + run);
   unsigned long long local = 0ull;
-  walk(c0, c1, lane, 32, [&](const uint32_t (&key)[VEC]) {
+  const float cut = cut_of(thr_key);
+  walk(c0, c1, lane, 32, cut, [&](const uint32_t (&key)[VEC]) {
 #pragma unroll
     for (int j = 0; j < VEC; ++j)
       if (key[j] >= thr_key) local += sc_fx(key[j]);
@@ -754,11 +775,19 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
   if (target >= total && total > 0ull) target = total - 1ull;
   before += cta_before;
   if (local > 0ull && before <= target && target < before + local) {
-    for (int b = c0; b < c1; b += 32) {
-      const int i = b + lane;
-      const uint32_t key = i < c1 ? key_of(ldf(vals, i)) : 0u;
-      unsigned long long incl = i < c1 && key >= thr_key ? sc_fx(key) : 0ull;
-      if (!__any_sync(0xffffffffu, incl > 0ull)) continue;
+    for (int b = c0; b < c1; b += 32 * VEC) {  // a lane has the tokens of one piece
+      const int i = b + lane * VEC;
+      const uint4 x = i < c1 ? *reinterpret_cast<const uint4*>(vals + i) : make_uint4(0u, 0u, 0u, 0u);
+      unsigned long long fx[VEC], mine = 0ull;
+      const bool none = i >= c1 || sc_max<T>(x) * inv_t - m < cut;
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) {
+        const uint32_t key = !none && i + j < c1 ? key_of(ldf(reinterpret_cast<const T*>(&x), j)) : 0u;
+        fx[j] = key >= thr_key ? sc_fx(key) : 0ull;
+        mine += fx[j];
+      }
+      if (!__any_sync(0xffffffffu, mine > 0ull)) continue;
+      unsigned long long incl = mine;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
@@ -766,7 +795,17 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
       }
       const uint32_t past = __ballot_sync(0xffffffffu, before + incl > target);
       if (past) {
-        if (lane == 0) out[row] = i0 + b + __ffs(past) - 1;
+        if (lane == __ffs(past) - 1) {
+          unsigned long long at = before + incl - mine;
+          int pick = 0;
+          bool found = false;
+#pragma unroll
+          for (int j = 0; j < VEC; ++j) {
+            at += fx[j];
+            if (!found && at > target) pick = j, found = true;
+          }
+          out[row] = i0 + i + pick;
+        }
         break;
       }
       before += __shfl_sync(0xffffffffu, incl, 31);
