@@ -3,11 +3,12 @@
 //
 // Routes arrive as a flat list of local expert ids (anything outside [0, e_local) means "not for this rank").  Every warp
 // owns one contiguous slice of the list and walks it 32 entries at a time: lanes with the same expert find each other by a
-// ballot per bit of the id (a warp match takes several times as long), the first of them moves the warp's counter of it.  A
-// first walk counts, a scan over (expert, warp) turns the counts into cursors, a second walk hands out positions, so the order
-// inside an expert is the route order (stable: the f32 summation order downstream never depends on scheduling).  Bound by the
-// latency of the walks, n / 512 steps each; with every warp scanning the whole list for its own experts instead, 10266 routes
-// to 64 experts took 140 us and 1024 routes 14 us; 20 us and 4.6 us now.  Up to 256 routes to at most 16 experts, a warp per
+// ballot per bit of the id (a warp match takes several times as long), the first of them moves the warp's counter of it.  In
+// front of that walk another one counts (atomics on the warp's counters, which need no order), a scan over (expert, warp)
+// turns the counts into cursors, and the walk hands out positions, so the order inside an expert is the route order (stable:
+// the f32 summation order downstream never depends on scheduling).  Bound by the latency of the walk, n / 512 steps; with
+// every warp scanning the whole list for its own experts instead, 10266 routes to 64 experts took 140 us and 1024 routes
+// 14 us; 18.8 and 4.9 us with two ordered walks, 12.5 and 3.5 now.  Up to 256 routes to at most 16 experts, a warp per
 // expert does scan the list, which it holds in registers (8 experts, 48 routes: 2.0 us, with slices 3.3).
 //
 // Takes the place of the reference's per-layer host-side routing bookkeeping and of the
@@ -36,8 +37,21 @@ __device__ __forceinline__ void route_sort_sliced(RouteSortSmem& sm, int n, int 
   const int used = AHEAD == 1 ? (n + 31) / 32 : ROUTE_SORT_WARPS;  // warps that are looked at
   int* cursor = sm.cursor[warp];
   const int bits = 32 - __clz(e_local - 1);  // of a local expert id (none for a single expert)
-  // `place`: the second walk
-  auto walk = [&](bool place) {
+  // counts need no order
+  auto count = [&]() {
+    for (int base = i_begin; base < i_end; base += 32 * AHEAD) {
+      int id[AHEAD];
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a) {
+        const int i = base + 32 * a + lane;
+        id[a] = i < i_end ? load(i) : -1;
+      }
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a)
+        if (id[a] >= 0 && id[a] < e_local) atomicAdd(&cursor[id[a]], 1);
+    }
+  };
+  auto place = [&]() {
     for (int base = i_begin; base < i_end; base += 32 * AHEAD) {
       int id[AHEAD];
 #pragma unroll
@@ -60,7 +74,7 @@ __device__ __forceinline__ void route_sort_sliced(RouteSortSmem& sm, int n, int 
         __syncwarp();
         if (mine && lane == __ffs(peers) - 1) cursor[id[a]] = before + __popc(peers);
         __syncwarp();
-        if (place && i < i_end) emit(i, mine ? before + __popc(peers & ((1u << lane) - 1u)) : -1);
+        if (i < i_end) emit(i, mine ? before + __popc(peers & ((1u << lane) - 1u)) : -1);
       }
     }
   };
@@ -68,7 +82,7 @@ __device__ __forceinline__ void route_sort_sliced(RouteSortSmem& sm, int n, int 
   for (int w = 0; w < ROUTE_SORT_WARPS; ++w)
     if (w < used) sm.cursor[w][tid] = 0;
   __syncthreads();
-  walk(false);
+  count();
   __syncthreads();
   int total = 0;  // of expert `tid`
 #pragma unroll
@@ -96,7 +110,7 @@ __device__ __forceinline__ void route_sort_sliced(RouteSortSmem& sm, int n, int 
       at += c;
     }
   __syncthreads();
-  walk(true);
+  place();
 }
 
 // `load(i)` returns the local expert id of flat entry i (0 <= i < n); `emit(i, pos)` is called
