@@ -8,19 +8,20 @@
 // global memory by each thread they were 128 sectors a k-block): 256-deep stages make a row of eight of them the 16 bytes that
 // a TMA row needs.
 //
-// 48 experts of 7168 x 2048, top 8 (routing and both products): 128 tokens 684 us with the A tile in shared memory, 451 now, of
+// 48 experts of 7168 x 2048, top 8 (routing and both products): 128 tokens 684 us with the A tile in shared memory, 445 now, of
 // which 70 by the issue of products from uniform registers (gemm_sm100.cu).  The weights' bytes take 182 us; a product of 128 rows
 // and few columns occupies the tensor core for 45 cycles whatever its columns, 165 us of this.
 //
 // warp 0 TMA producer | warp 1 MMA issuer + TMEM owner | warps 2-5 epilogue | then Q4_GROUPS groups of four dequant warps.
-// Group g expands the k-blocks g, g + Q4_GROUPS, .. of the four of a stage into one of eight TMEM buffers.
+// Group g expands the k-blocks g, g + Q4_GROUPS, .. of the four of a stage into TMEM buffers of two or three stages.
 constexpr int Q4_GROUPS = 4;             // divides 4; two groups: 534 us where four take 474 (128 tokens), 688 and 703 (512)
 constexpr int Q4_BK = 256;               // weights of a row in one stage: 128 bytes
 constexpr int Q4_RAW = BM * Q4_BK / 2;   // packed tile
 constexpr int Q4_SC = BM * (Q4_BK / 32) * 2;
 constexpr int Q4_STAGES = 8;             // at most
-constexpr int Q4_BUFS = 8;               // A buffers of 32 columns in TMEM columns 256..511
-constexpr int Q4_MAX_BN = 128;           // two accumulators in columns 0..255
+constexpr int Q4_TURNS = 3;              // at most: stages whose A is in tensor memory, four buffers of 32 columns each, behind two accumulators (two: 452 us, three: 445)
+constexpr int Q4_BUFS = 4 * Q4_TURNS;
+constexpr int Q4_MAX_BN = 128;
 constexpr int Q4_THREADS = 192 + Q4_GROUPS * 128;
 
 __global__ void __launch_bounds__(Q4_THREADS, 1)
@@ -70,6 +71,8 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
   pdl_launch_dependents();  // (behind the allocation above: a dependent that takes tensor memory must not be first)
   const uint32_t tmem_base = *tmem_slot;
   const int total = s_total;
+  const int turns = min(Q4_TURNS, (512 - 2 * p.bn) / 128);
+  const uint32_t a_col = 512u - 128u * (uint32_t)turns;
   const int depth = (p.K + Q4_BK - 1) / Q4_BK;  // stages of an item; TMA fills what lies past K with zeros on every operand
   uint32_t ep_epoch = 0;
   if (p.scatter_src != nullptr) ep_epoch = *((volatile uint32_t*)(p.peer_flags[p.rank] + p.site * 32 + 16));
@@ -118,15 +121,15 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
       const uint32_t idesc = umma_idesc_bf16_f32(BM, (uint32_t)p.bn);
       const uint64_t x_desc0 = umma_desc_k_sw128(smem_u32(tiles) + Q4_RAW + Q4_SC);
       int stage = 0;
-      uint32_t phase = 0, turn = 0;
-      int acc = 0;
+      uint32_t phase = 0, a_phase = 0;
+      int turn = 0, acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < total && ok; item += gridDim.x) {
         if (!mbar_wait(&tempty[acc], acc_phase ^ 1u, abort_flag)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * p.bn);
-        for (int d = 0; d < depth && ok; ++d, ++turn) {
+        for (int d = 0; d < depth && ok; ++d) {
           if (!mbar_wait(&full[stage], phase, abort_flag)) {
             ok = false;
             break;
@@ -134,8 +137,8 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
           const uint64_t x_desc = x_desc0 + (uint32_t)(stage * (stage_bytes >> 4));
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const int b = (int)(turn & 1u) * 4 + i;
-            if (!mbar_wait(&aready[b], (turn >> 1) & 1u, abort_flag)) {
+            const int b = turn * 4 + i;
+            if (!mbar_wait(&aready[b], a_phase, abort_flag)) {
               ok = false;
               break;
             }
@@ -143,7 +146,7 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             if (leader) {
 #pragma unroll
               for (int k = 0; k < BK / 16; ++k)
-                umma_bf16_ts(d_tmem, tmem_base + 256u + (uint32_t)(b * 32 + k * 8), x_desc + (uint32_t)(i * (x_bytes >> 4) + k * 2), idesc, (d | i | k) ? 1u : 0u);
+                umma_bf16_ts(d_tmem, tmem_base + a_col + (uint32_t)(b * 32 + k * 8), x_desc + (uint32_t)(i * (x_bytes >> 4) + k * 2), idesc, (d | i | k) ? 1u : 0u);
               umma_commit(&afree[b]);
               if (i == 3) umma_commit(&empty[stage]);
             }
@@ -152,6 +155,10 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
           if (++stage == p.stages) {
             stage = 0;
             phase ^= 1u;
+          }
+          if (++turn == turns) {
+            turn = 0;
+            a_phase ^= 1u;
           }
         }
         if (!ok) break;
@@ -184,13 +191,13 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     const int wq = warp & 3;  // TMEM lanes of this warp: 32 wq ..
     const int grp = (warp - 6) >> 2;
     const int r = wq * 32 + lane;
-    const uint32_t a_row = tmem_base + ((uint32_t)(wq * 32) << 16) + 256u;
+    const uint32_t a_row = tmem_base + ((uint32_t)(wq * 32) << 16) + a_col;
     const int groups_per_row = p.K / 32;
     const bf162 bias = __floats2bfloat162_rn(136.f, 136.f);
     uint32_t mask, magic;  // in registers: as two constants of one operation they make it two (474 us where this takes 451)
     asm volatile("mov.b32 %0, 0x000F000F;\n\tmov.b32 %1, 0x43004300;" : "=r"(mask), "=r"(magic));
-    int stage = 0;
-    uint32_t phase = 0, turn = 0;
+    int stage = 0, turn = 0;
+    uint32_t phase = 0, a_phase = 0;
     ItemCursor cur;
     Item it;
     bool ok = true;
@@ -198,12 +205,12 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
       if (!locate(p, s_tiles, item, cur, it)) break;
       const int m = it.m_tile * BM + r;
       const bf16* srow = reinterpret_cast<const bf16*>(p.scales) + ((size_t)it.e * p.M + (m < p.M ? m : 0)) * groups_per_row;
-      for (int d = 0; d < depth; ++d, ++turn) {
+      for (int d = 0; d < depth; ++d) {
         ok = __all_sync(0xffffffffu, mbar_wait(&full[stage], phase, abort_flag));
         if (!ok) break;
         const uint8_t* st = tiles + stage * stage_bytes;
         for (int i = grp; i < 4; i += Q4_GROUPS) {
-          const int b = (int)(turn & 1u) * 4 + i;
+          const int b = turn * 4 + i;
           uint32_t words[8];
           *reinterpret_cast<uint4*>(words) = *reinterpret_cast<const uint4*>(st + r * 128 + (((2 * i) ^ (r & 7)) << 4));
           *reinterpret_cast<uint4*>(words + 4) = *reinterpret_cast<const uint4*>(st + r * 128 + (((2 * i + 1) ^ (r & 7)) << 4));
@@ -215,7 +222,7 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             if (g < groups_per_row) sc.x = srow[g];
             if (g + 1 < groups_per_row) sc.y = srow[g + 1];
           }
-          ok = __all_sync(0xffffffffu, mbar_wait(&afree[b], ((turn >> 1) & 1u) ^ 1u, abort_flag));
+          ok = __all_sync(0xffffffffu, mbar_wait(&afree[b], a_phase ^ 1u, abort_flag));
           if (!ok) break;
           tc_fence_after();
 #pragma unroll
@@ -245,6 +252,10 @@ moe_gemm_int4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
         if (++stage == p.stages) {
           stage = 0;
           phase ^= 1u;
+        }
+        if (++turn == turns) {
+          turn = 0;
+          a_phase ^= 1u;
         }
       }
     }
