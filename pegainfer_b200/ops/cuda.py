@@ -1639,6 +1639,7 @@ def _latent_tc(rows: int, heads: int, lat: int, rot: int, keys: int, max_q_len: 
     return keys > (96 if heads <= 32 or 3 * blocks < 4 * sms else 32)
 
 
+_LATENT_WHOLE = 256  # rows of up to so many keys are not shared between blocks (csrc/mla_decode_tc.cu): steps of nothing else need no scratch, and no join
 _LATENT_FEW = 16  # rows of a sequence in a decode step or in one that checks drafted tokens
 
 
@@ -1774,7 +1775,7 @@ def mla_attention(q: "_MlaQ", w_uk, w_uv, latent_layer, meta: AttnMeta, scale, k
     lat_out = torch.empty((t, h, kv_lora), dtype=torch.bfloat16, device=dev)
     rc = lib().pg_mla_attention(_ptr(q_abs), _ptr(q.pe), _ptr(latent_layer), _ptr(lat_out), _ptr(meta.q_indptr), _ptr(meta.kv_lens), _ptr(meta.block_table),
                                 _ci(meta.block_table.stride(0)), _ptr(unit_seq), _ci(meta.num_seqs), _ci(t), _ci(h), _ci(kv_lora), _ci(rope), _ci(page_size), _cf(scale),
-                                _ci(splits), _ci(int(tc)), _ptr(part_o), _ptr(part_lse), _ll(part_o.numel()), _ll(latent_layer.shape[0]), _ptr(c.status), _stream())
+                                _ci(splits), _ci(int(tc)), _ptr(part_o), _ptr(part_lse), _ll(part_o.numel() if meta.max_kv_len > _LATENT_WHOLE else 0), _ll(latent_layer.shape[0]), _ptr(c.status), _stream())
     _check(rc, c, 2 if splits > 1 or tc else 1)
     vdim = w_uv.shape[1]
     out = torch.empty((t, h * vdim), dtype=torch.bfloat16, device=dev)
@@ -1896,7 +1897,7 @@ def latent_attention(q, uk_t, uv, ukv, cache, meta: AttnMeta, rot: int, scale: f
         splits = _latent_splits(n, heads, longest, tc, c.sms)
         splits = max(1, min(splits, c.attn_part.numel() // (n * heads * (lat + 1) * 4)))
         rc = lib().pg_latent_attention(_ptr(q_abs), *strides, *pe, *where, _ci(row0), _ci(meta.num_seqs), _ci(n), _ci(heads), _ci(lat), _ci(rot), _ci(ps), _cf(scale), _ci(window), *extra, _ci(splits),
-                                       _ci(int(tc)), _ptr(c.attn_part), _ptr(c.attn_part[n * heads * splits * lat * 4 :]), _ll(c.attn_part.numel()), _ll(cache.shape[0]), _ptr(c.status), _stream())
+                                       _ci(int(tc)), _ptr(c.attn_part), _ptr(c.attn_part[n * heads * splits * lat * 4 :]), _ll(c.attn_part.numel() if longest > _LATENT_WHOLE else 0), _ll(cache.shape[0]), _ptr(c.status), _stream())
         _check(rc, c, 2 if splits > 1 else 1)
     else:
         assert row0 == 0
