@@ -1809,7 +1809,11 @@ def _head_gemm(x, x_tok: int, x_head: int, w, y, gate=None):
     y_f32 = _ci(int(y.dtype == torch.float32))
     if w.dtype == torch.bfloat16 and k % 8 == 0 and x_tok % 8 == 0 and x_head % 8 == 0 and x.data_ptr() % 16 == 0 and heads <= 512:
         bn, tiles = _token_tile(heads * rows, heads), heads * ((m + 127) // 128)
-        while bn > 16 and tiles * ((rows + bn - 1) // bn) < c.sms:  # narrower token tiles until every SM has one (a head's weights come from L2 again)
+        # Narrower token tiles until four of five SMs have one; each reads its head's weights again from L2, and a tile of the second
+        # round waits for its loads anew.  Latent decode, whole calls, tiles until every SM has one against this rule against two of
+        # five: 128 rows x 64 heads 82.6, 78.9 and 77.5 us (contexts of 100 keys 39.4, 35.8 and 35.2), 64 rows x 128 heads 41.3,
+        # 37.6 and 37.9, 40 rows x 64 heads 30.7, 29.0 and 28.9, 100 rows x 16 heads 22.7, 21.0 and 22.9.
+        while bn > 16 and 5 * tiles * ((rows + bn - 1) // bn) < 4 * c.sms:
             bn //= 2
         _check(lib().pg_head_gemm(*front, y_f32, *rest, _ci(bn), _ptr(c.status), _stream()), c)
     else:

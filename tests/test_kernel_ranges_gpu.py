@@ -552,3 +552,15 @@ def test_kda_chunks_of_strong_and_weak_decays(lower, shift):
         st2[s + 1] = S
         at += m
     assert (st1.double() - st2).abs().max() < 2 ** -17 * st2.abs().max()
+
+
+@pytest.mark.parametrize("n,m", [(5, 130), (59, 128), (60, 136), (117, 48), (118, 32)])  # around four of five SMs
+@pytest.mark.parametrize("t", [1, 17, 64, 65, 129])
+def test_products_per_head_where_token_tiles_narrow(t, n, m):
+    g = torch.Generator().manual_seed(t * 1000 + m)
+    k = 72
+    x, w = torch.randn(t, n, k, generator=g).bfloat16(), torch.randn(n, m, k, generator=g).bfloat16()
+    y = cu().multi_dense(x.to(DEV), w.to(DEV)).cpu().double()
+    want, size = torch.einsum("tnk,nmk->tnm", x.double(), w.double()), torch.einsum("tnk,nmk->tnm", x.double().abs(), w.double().abs())
+    # one rounding to bf16 of a sum of k products in f32
+    assert ((y - want).abs() <= 2 ** -8 * want.abs() + k * 2 ** -23 * size).all()
