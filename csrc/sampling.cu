@@ -476,8 +476,9 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(const T* 
     }
   };
 
-  // tokens with s - m below it have keys below `key`, however the logarithm and the exponential round
-  auto cut_of = [&](uint32_t key) { return __logf(__uint_as_float(key)) - 1e-3f; };
+  // tokens with s - m below it have keys below `key`, however the logarithm and the exponential round, and the product in s: it may be
+  // part of a fused multiply-add, exact beside a maximum that is rounded (2^-24 of it, far above 1e-3 at temperatures of 1e-3 and less)
+  auto cut_of = [&](uint32_t key) { return __logf(__uint_as_float(key)) - fmaf(fabsf(m), 0x1p-22f, 1e-3f); };
   const uint32_t kk = top_k[row] > 0 ? (uint32_t)min(top_k[row], vocab) : (uint32_t)vocab;
   const float tp = top_p[row];
   const float mp = min_p[row];

@@ -119,6 +119,24 @@ def test_sampler_brackets(vocab, dtype):
             assert (at >= target - slack).all() and (at - mass.gather(-1, got[rows, None]) <= target + slack).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("temp", [1e-5, 7e-5, 3e-4, 1e-3])
+def test_sampler_at_low_temperatures(temp, dtype):
+    """Tempered logits of 10^4 to 10^7, whose products round by more than tokens of mass may differ: only the largest has mass (the next one
+    is a thousand units and more below it), so every row gives the largest, whatever its piece of eight."""
+    g = torch.Generator(device=DEV).manual_seed(1)
+    top = torch.arange(128, 512, device=DEV)
+    top = torch.cat([(1 + (top % 128) / 128) * 2.0 ** (top // 128 + 2), -(1 + (top % 128) / 128) * 2.0 ** (top // 128 + 2)])  # every bf16 number of 8 to 64
+    rows, vocab = top.numel(), 24577
+    lg = (top[:, None] - 1 - torch.rand(rows, vocab, device=DEV, generator=g) * 8).to(dtype)
+    want = torch.randint(0, vocab, (rows,), device=DEV, generator=g)
+    lg[torch.arange(rows, device=DEV), want] = top.to(dtype)
+    one = torch.ones(rows, device=DEV)
+    for k, p, m in ((1, 1.0, 0.0), (50, 1.0, 0.0), (0, 0.9, 0.0), (0, 1.0, 1.0), (0, 1.0, 0.05), (0, 1.0, 0.0), (20, 0.8, 0.1)):
+        got = cu().sample(lg, one * temp, torch.full((rows,), k, dtype=torch.int32, device=DEV), one * p, one * m, torch.rand(rows, device=DEV, generator=g))
+        assert torch.equal(got.long(), want)
+
+
 @pytest.mark.parametrize("heads,page,splits", [(16, 16, 1), (16, 64, 5), (32, 32, 2), (64, 16, 1), (64, 16, 3), (96, 16, 2)])
 def test_latent_decode_tiles(heads, page, splits, monkeypatch):
     """Absorbed attention around tiles of 64 keys, padding rows, splits without keys, and rows behind a sequence's end that
