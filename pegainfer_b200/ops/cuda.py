@@ -622,7 +622,7 @@ def set_batch_invariant(on: bool) -> None:
     """Numeric policy for ``--batch-invariant`` serving: a row's result must not depend on what
     else rides in the batch.  GEMMs run with one k-split (the k order inside a CTA is fixed and
     independent of the token tile), decode attention uses a constant number of KV splits (the
-    split boundaries then depend on the sequence's own length only); the default policy picks
+    split boundaries then depend on the sequence's own length only), latent rows are summed whole on one kernel; the default policy picks
     both from the batch shape.  Reference: pegainfer-kernels/src/ops/linear.rs NumericPolicy,
     pegainfer-qwen3/src/lib.rs:498-548."""
     global _BATCH_INVARIANT
@@ -1629,7 +1629,7 @@ def _latent_tc(rows: int, heads: int, lat: int, rot: int, keys: int, max_q_len: 
     100), 64 heads 0.88 - 1.0 at 40, but 1.02 at 80 with a second wave that is nearly empty (150 rows)."""
     if lat != 512 or rot not in (0, 64):
         return False
-    if max_q_len <= _LATENT_FEW:
+    if max_q_len <= _LATENT_FEW or _BATCH_INVARIANT:
         return True
     blocks = rows * ((heads + 63) // 64)
     if blocks <= sms:
@@ -1643,8 +1643,16 @@ _LATENT_WHOLE = 256  # rows of up to so many keys are not shared between blocks 
 _LATENT_FEW = 16  # rows of a sequence in a decode step or in one that checks drafted tokens
 
 
+def _latent_scratch(part, longest: int) -> int:
+    """Bytes of ``part`` for the rows that blocks of the tcgen05 kernel share; without any no row is cut.  Where a row is cut follows from the
+    lengths of all rows of the step, so none are under the batch-invariant policy."""
+    return part.numel() if longest > _LATENT_WHOLE and not _BATCH_INVARIANT else 0
+
+
 def _latent_splits(rows: int, heads: int, longest: int, tc: bool, sms: int) -> int:
     """Blocks that share one row's keys in the absorbed kernels."""
+    if _BATCH_INVARIANT:
+        return 1
     if tc:  # csrc/mla_decode_tc.cu: a block owns an SM and serves up to 64 heads; blocks share the keys by themselves, this says how few heads one gets
         return max(1, min(16, sms // (rows * ((heads + 63) // 64)), (longest + 255) // 256))
     return max(1, min(16, (4 * sms) // (rows * ((heads + 15) // 16)), (min(longest, 4096) + 127) // 128))
@@ -1775,7 +1783,7 @@ def mla_attention(q: "_MlaQ", w_uk, w_uv, latent_layer, meta: AttnMeta, scale, k
     lat_out = torch.empty((t, h, kv_lora), dtype=torch.bfloat16, device=dev)
     rc = lib().pg_mla_attention(_ptr(q_abs), _ptr(q.pe), _ptr(latent_layer), _ptr(lat_out), _ptr(meta.q_indptr), _ptr(meta.kv_lens), _ptr(meta.block_table),
                                 _ci(meta.block_table.stride(0)), _ptr(unit_seq), _ci(meta.num_seqs), _ci(t), _ci(h), _ci(kv_lora), _ci(rope), _ci(page_size), _cf(scale),
-                                _ci(splits), _ci(int(tc)), _ptr(part_o), _ptr(part_lse), _ll(part_o.numel() if meta.max_kv_len > _LATENT_WHOLE else 0), _ll(latent_layer.shape[0]), _ptr(c.status), _stream())
+                                _ci(splits), _ci(int(tc)), _ptr(part_o), _ptr(part_lse), _ll(_latent_scratch(part_o, meta.max_kv_len)), _ll(latent_layer.shape[0]), _ptr(c.status), _stream())
     _check(rc, c, 2 if splits > 1 or tc else 1)
     vdim = w_uv.shape[1]
     out = torch.empty((t, h * vdim), dtype=torch.bfloat16, device=dev)
@@ -1901,7 +1909,7 @@ def latent_attention(q, uk_t, uv, ukv, cache, meta: AttnMeta, rot: int, scale: f
         splits = _latent_splits(n, heads, longest, tc, c.sms)
         splits = max(1, min(splits, c.attn_part.numel() // (n * heads * (lat + 1) * 4)))
         rc = lib().pg_latent_attention(_ptr(q_abs), *strides, *pe, *where, _ci(row0), _ci(meta.num_seqs), _ci(n), _ci(heads), _ci(lat), _ci(rot), _ci(ps), _cf(scale), _ci(window), *extra, _ci(splits),
-                                       _ci(int(tc)), _ptr(c.attn_part), _ptr(c.attn_part[n * heads * splits * lat * 4 :]), _ll(c.attn_part.numel() if longest > _LATENT_WHOLE else 0), _ll(cache.shape[0]), _ptr(c.status), _stream())
+                                       _ci(int(tc)), _ptr(c.attn_part), _ptr(c.attn_part[n * heads * splits * lat * 4 :]), _ll(_latent_scratch(c.attn_part, longest)), _ll(cache.shape[0]), _ptr(c.status), _stream())
         _check(rc, c, 2 if splits > 1 else 1)
     else:
         assert row0 == 0

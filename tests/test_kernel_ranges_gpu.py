@@ -395,6 +395,53 @@ def test_latent_window_and_empty_splits(heads, rot, window, splits, reps, tc, ex
     assert cu().read_status(DEV) == 0
 
 
+def _latent_rows(kv_lens, heads, seed, q_lens=None, page=16, lat=512, rot=64, dim=128):
+    """A decode step (or rows of up to 16 tokens) over scattered pages: (meta of chosen sequences, q, up-projections, cache, angles)."""
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    q_lens = q_lens or [1] * len(kv_lens)
+    per = [(x + page - 1) // page for x in kv_lens]
+    order = (torch.randperm(sum(per), device=DEV, generator=g) + 1).int().cpu()
+    table, at = torch.zeros(len(kv_lens), max(per), dtype=torch.int32), 0
+    for i, m in enumerate(per):
+        table[i, :m] = order[at : at + m]
+        at += m
+    draw = lambda *shape: torch.randn(*shape, device=DEV, generator=g)  # noqa: E731
+
+    def meta(rows):
+        n, ql, kl = len(rows), [q_lens[i] for i in rows], [kv_lens[i] for i in rows]
+        qi = torch.tensor([0] + ql).cumsum(0)
+        pos = torch.cat([torch.arange(k - m, k).clamp(min=0) for k, m in zip(kl, ql)]).int().to(DEV)
+        return R.AttnMeta(qi.int().to(DEV), torch.tensor(kl, dtype=torch.int32, device=DEV), table[rows].to(DEV), pos, pos, page, n, sum(ql), max(ql), max(kl), max(ql) == 1, qi.tolist(), kl)
+
+    angles = draw(max(kv_lens) + 1, max(rot // 2, 1))
+    return (meta, draw(sum(q_lens), heads * (dim + rot)).bfloat16(), (draw(heads, lat, dim) * 0.05).bfloat16(), (draw(heads, dim, lat) * 0.05).bfloat16(), draw(sum(per) + 1, page * (lat + rot)).bfloat16(),
+            (angles.cos(), angles.sin()))
+
+
+@pytest.mark.parametrize("heads,rot", [(16, 64), (64, 64), (64, 0)])
+def test_latent_rows_whatever_shares_their_step(heads, rot):
+    """Under the batch-invariant policy a latent decode row has the same bytes alone, beside rows of other lengths and behind a prompt."""
+    K = cu()
+    kv_lens = [700, 1500, 300, 40, 2000, 3001, 257, 256, 65]
+    n = len(kv_lens)
+    meta, q, uk_t, uv, cache, cs = _latent_rows(kv_lens + [90], heads, 3, [1] * n + [50], rot=rot)
+    uk, turn = uk_t.transpose(1, 2).contiguous(), R.rope_tables(4096, 64, 1e4, torch.bfloat16, DEV)
+    before = K.batch_invariant()
+    K.set_batch_invariant(True)
+    try:
+        def run(seqs, x):
+            m = meta(seqs)
+            y = K.latent_attention(x, uk_t, uv, None, cache, m, rot, 0.07, 0, *cs)
+            return torch.cat([y, K.mla_attention(K.mla_rope_q(x.view(-1, heads, 192), *turn, m, 128), uk, uv, cache.view(-1, 16, 576), m, 0.07, 512)], 1) if rot else y
+
+        step, beside = run(list(range(n)), q[:n]), run([n] + list(range(n)), torch.cat([q[n:], q[:n]]))[50:]
+        for i in range(n):
+            alone = run([i], q[i : i + 1])[0]
+            assert torch.equal(step[i], alone) and torch.equal(beside[i], alone), kv_lens[i]
+    finally:
+        K.set_batch_invariant(before)
+
+
 @pytest.mark.parametrize("lens,past,heads,tc", [([1] * 8, 7, 16, True), ([1] * 150, 100, 16, True), ([16] * 3, 0, 16, True), ([17] * 3, 0, 16, False), ([80], 0, 16, False), ([90], 0, 16, True),
                                                  ([20] * 10, 80, 16, False), ([20] * 10, 130, 16, True), ([20] * 10, 15, 64, False), ([20] * 10, 30, 64, True), ([300] * 3, 0, 32, True)])
 def test_latent_kernels_where_the_rule_changes(lens, past, heads, tc, monkeypatch):
