@@ -194,7 +194,7 @@ int pg_gdn_recurrent(const void* q, const void* k, long long ld_qk, const void* 
 // gate projections (the decay and beta arithmetic runs in the kernel); state [slots, heads, dk, dv] f32.
 int pg_kda_recurrent(const void* q, const void* k, const void* v, long long ld, const void* f, long long ldf, const void* b, long long ldb,
                      const void* a_log, const void* dt_bias, float lower, void* state, void* out, const void* q_indptr, const void* slots,
-                     int num_seqs, int heads, int dk, int dv, int max_q_len, int min_len, int chunks, int short_len, cudaStream_t stream);
+                     int num_seqs, int heads, int dk, int dv, int max_q_len, int min_len, int short_len, cudaStream_t stream);
 // Further rules of the same kernel, bf16 or f32 rows, key width up to 256.  channel_delta: decay exp(-exp(A_log) *
 // softplus(f + dt_bias)) with f in f32, query / key heads shared by heads / kv_heads value heads.  decay_recurrent: linear
 // attention with a fixed decay per head, SiLU on q, k, v inside.  skip_len > 0 leaves sequences of at least that many rows out.

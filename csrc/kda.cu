@@ -22,8 +22,6 @@
 //
 // Functional parity with pegainfer-k3/kernels/tilelang_defs.py:67-139 (attnres_scores / attnres_mix) and
 // :304-410 (kda_core) and pegainfer-kernels/csrc/k3/k3_flash_kda.cu (chunked prefill of the same rule).
-#include <atomic>
-
 #include "api.h"
 #include "common.cuh"
 #include "mma_frag.cuh"
@@ -281,7 +279,7 @@ int run_rule(int rule, RecArgs<T> p, int num_seqs, int max_q_len, cudaStream_t s
 }
 
 // ---------------------------------------------------------------------------------
-// The delta rule with bounded channel decays, KB_T tokens at a time (short prompts, 128-wide keys).  Inside a block
+// The delta rule with bounded channel decays, KB_T tokens at a time (prompts, 128-wide keys).  Inside a block
 //   kd_t = k_t * P_t, qd_t = q_t * P_t      (P_t: product of the block's decays up to and with token t)
 //   kh_t = k_t * (product of the decays behind t),   A_ts = k_t . (k_s * decays of s+1 .. t),   B_ts likewise with q_t
 // do not depend on the state, so a warp forms them once per block for all columns of the CTA, and per state column
@@ -576,484 +574,6 @@ kda_block_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const b
     }
 }
 
-// ---------------------------------------------------------------------------------
-// The delta rule with bounded channel decays, KC_T tokens at a time (prompts, 128-wide keys), on the tensor cores.  With P_t the
-// product of the chunk's decays up to and with token t, and token 7 as the reference,
-//   rk_t = k_t P_t / P_7,   rq_t = q_t P_t / P_7,   c_s = k_s P_7 / P_s,   S' = P_7 S0,
-//   A_ts = rk_t . c_s,   B_ts = rq_t . c_s,   T = (I + diag(beta) A_strict)^-1 diag(beta),
-//   d = T (v - rk S'),   o = rq S' + B d  (s <= t),   S = P_15 / P_7 (S' + sum_s c_s d_s)
-// so everything but T, 16 x 16 and solved by one warp, is a product of matrices.  None is rounded to less than f32: each factor
-// is split into two tf32 numbers, x = hi + lo with 22 bits, and lo hi, hi lo and hi hi are added (mma.sync, f32 sums); sums over more than
-// 32 channels and the state itself are added outside of the tensor core, which cuts sums off.  With lower >= KC_LOWER all
-// factors are numbers of f32: quotients P_t / P_7 reach exp(8 |lower|), and the state goes from one chunk's reference to the next one's by
-// a product of sixteen decays, exp(16 lower) = 3e-37 at least.
-//
-// A warp keeps 16 state columns as S^T (columns x 128 channels) in mma accumulators.  A product over the channels takes them as its
-// left operand where they are: accumulator columns 2 t, 2 t + 1 become the operand's channels t, t + 4, and the right operand is
-// stored in the same order, a pair of channels (or of tokens) with its low parts in 16 bytes.  The same holds for d^T.  Four warps
-// prepare chunks together (a lane has four channels of four tokens) while four others, of 16 columns each, walk the chunk before: a
-// sequence is one chain of chunks, and what a block takes for a chunk is what a prompt takes.  rk and rq exist once: they are free when
-// the walk has multiplied them with S', and the next ones written while it does the rest; c, T and B exist twice.
-// A NaN in a token reaches the other tokens of its chunk, the earlier ones too.
-// Against four tokens at a time on the FMA units (one group of four warps to prepare and to walk; 53 % of FMA issue):  3001 tokens in two
-// prompts, 96 heads 1150 -> 966 us; one prompt of 3000 tokens, 16 heads 1105 -> 795; eight of 125, 32 heads 151 -> 145; 4 x 50 48 -> 42.  State
-// against 64 bits, 2-norm: 8.4e-7 and 8.4e-7 (900 tokens), 1.12e-6 and 1.12e-6 (2000).  What bounds it: the chain of a chunk, some 8000
-// cycles, half of it preparation whose steps wait for each other; the products themselves are 350 a scheduler, eight cycles each.
-constexpr int KC_T = 16;      // tokens per chunk, four per warp to prepare
-constexpr int KC_COLS = 64;   // state columns per CTA, 16 per warp
-constexpr int KC_DK = 128;
-constexpr float KC_LOWER = -5.25f;
-// Registers of the two groups of four warps: what the block is launched with (128 a thread; kc_allow checks it), moved to the walking
-// warps, whose state alone takes 64.  96 / 160: 989 us, 112 / 144: 1015, 128 each: 1087 (two prompts below).
-constexpr int KC_REGS_PREP = 104, KC_REGS_WALK = 152;
-
-struct KcSmem {
-  float4 rk[KC_T][KC_DK / 2], rq[KC_T][KC_DK / 2];  // [token][pair of channels, ^ 4 on odd tokens]: hi, hi, lo, lo
-  float4 c[2][KC_T / 2][KC_DK];                     // [pair of tokens][channel ^ 2 (pair % 4)]: hi, hi, lo, lo
-  bf16 raw[4][3][4][KC_DK];                         // q, k, f rows of the next chunk to prepare, by warp
-  bf16 raw_v[4][KC_T][KC_COLS];
-  float tot[4][KC_DK];  // products of each warp's four decays
-  float fac[KC_DK], tail[KC_DK];  // (P_15 / P_7 of the chunk before) P_7, and this chunk's P_15 / P_7
-  float m[KC_T][KC_T];  // [s][t]: beta_t A_ts, s < t
-  float beta[2][KC_T];
-  float4 tf[2][3][32], bf[2][3][32];  // T and B (s <= t) as right operands: tokens (0 - 7, 0 - 7), (8 - 15, 0 - 7), (8 - 15, 8 - 15)
-};
-
-// hi: x rounded to the eleven bits of a tf32 number (a NaN's hi may be a number, its lo is a NaN); lo: what is left, of which the tensor
-// core reads the first eleven bits
-__device__ __forceinline__ void kc_split(float x, float& hi, float& lo) {
-  hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
-  lo = x - hi;
-}
-struct KcA {  // left operand, rows g and g + 8, columns (2 t of both, 2 t + 1 of both)
-  float hi[4], lo[4];
-};
-// from accumulators: (g, 2t), (g, 2t + 1), (g + 8, 2t), (g + 8, 2t + 1)
-__device__ __forceinline__ void kc_left(const float* c, KcA& a) {
-  kc_split(c[0], a.hi[0], a.lo[0]);
-  kc_split(c[2], a.hi[1], a.lo[1]);
-  kc_split(c[1], a.hi[2], a.lo[2]);
-  kc_split(c[3], a.hi[3], a.lo[3]);
-}
-__device__ __forceinline__ void kc_mma1(float* d, const float* a, float b0, float b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
-}
-// low[i] and high[i] += left[i] right[i], right = (hi, hi, lo, lo), the two products with a low part, which add up to a small number, apart.
-// The order is that of issue: a product waits some 35 cycles for one in front of it that adds to the same sums, so N of them take turns.
-template <int N>
-__device__ __forceinline__ void kc_mma(float* const (&low)[N], float* const (&high)[N], const KcA* const (&left)[N], const float4 (&right)[N]) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) kc_mma1(low[i], left[i]->lo, right[i].x, right[i].y);
-#pragma unroll
-  for (int i = 0; i < N; ++i) kc_mma1(high[i], left[i]->hi, right[i].x, right[i].y);
-#pragma unroll
-  for (int i = 0; i < N; ++i) kc_mma1(low[i], left[i]->hi, right[i].z, right[i].w);
-}
-
-// d += a b, b = (hi, hi, lo, lo): the two products with a low part apart, which add up to a small number, as their own chain
-__device__ __forceinline__ void kc_mma_low(float* d, const KcA& a, const float4& b) {
-  kc_mma1(d, a.lo, b.x, b.y);
-  kc_mma1(d, a.hi, b.z, b.w);
-}
-__device__ __forceinline__ void kc_mma_high(float* d, const KcA& a, const float4& b) { kc_mma1(d, a.hi, b.x, b.y); }
-
-// named barriers: among the preparing warps; rk and rq are free; rk, rq and fac are there; T, B and c are there (by parity of the chunk)
-enum { KC_BAR_PREP = 1, KC_BAR_FREE = 2, KC_BAR_ROWS = 3, KC_BAR_T = 4 };
-__device__ __forceinline__ void kc_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
-__device__ __forceinline__ void kc_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
-
-__global__ void __launch_bounds__(256, 2)
-kda_chunk_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v, long long ld, const bf16* __restrict__ f, long long ldf, const bf16* __restrict__ b, long long ldb,
-                 const float* __restrict__ a_log, const float* __restrict__ dt_bias, float lower, float* __restrict__ state, bf16* __restrict__ out, const int* __restrict__ q_indptr,
-                 const int* __restrict__ slots, int heads, int dv, int min_len) {
-  extern __shared__ __align__(16) uint8_t kc_raw[];
-  KcSmem& sm = *reinterpret_cast<KcSmem*>(kc_raw);
-  const int groups = dv / KC_COLS;
-  const int h = blockIdx.x / groups, c0 = blockIdx.x % groups * KC_COLS, seq = blockIdx.y;
-  const int slot = slots[seq];
-  const int q0 = q_indptr[seq], q1 = q_indptr[seq + 1];
-  if (q1 - q0 < min_len || slot < 0) return;
-  const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t4 = lane & 3;
-  const int sw = (g & 1) << 2;  // of the rows g and g + 8 of rk and rq
-
-  if (threadIdx.x < 128) {
-  // ================ preparing warps ================
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(KC_REGS_PREP));
-
-  // raw rows of this warp's four tokens of the chunk that starts at token t0; rows past the end are zero
-  float b_next = 0.f;
-  auto fetch = [&](int t0, int chunk) {
-    const int t = t0 + warp * 4;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      const int c = lane + 32 * (i & 1), r = c >> 4, ch = (c & 15) * 8;
-      const bool ok = t + r < q1;
-      const long long row = ok ? t + r : q0;
-      const bf16* src = i < 2 ? q + row * ld : i < 4 ? k + row * ld : f + row * ldf;
-      cp_async16(&sm.raw[warp][i >> 1][r][ch], src + (long long)h * KC_DK + ch, ok);
-    }
-    const int r = lane >> 3, ch = (lane & 7) * 8;
-    const bool ok = t + r < q1;
-    cp_async16(&sm.raw_v[chunk & 3][warp * 4 + r][ch], v + (ok ? t + r : q0) * ld + (long long)h * dv + c0 + ch, ok);
-    cp_async_commit();
-    b_next = lane < 4 && t + lane < q1 ? to_f32(b[(long long)(t + lane) * ldb + h]) : 0.f;
-  };
-  fetch(q0, 0);
-
-  const float a = __expf(a_log[h]), q_scale = rsqrtf((float)KC_DK);
-  // a lane prepares channels 2 lane, 2 lane + 1 and 64 further on
-  const float2 bias0 = *reinterpret_cast<const float2*>(dt_bias + h * KC_DK + 2 * lane), bias1 = *reinterpret_cast<const float2*>(dt_bias + h * KC_DK + 64 + 2 * lane);
-  const float bias[4] = {bias0.x, bias0.y, bias1.x, bias1.y};
-  float tail[4] = {1.f, 1.f, 1.f, 1.f};
-
-  for (int t0 = q0, chunk = 0; t0 < q1; t0 += KC_T, ++chunk) {
-    // ---- unit rows and decays of the warp's four tokens ----
-    cp_async_wait_all();
-    __syncwarp();
-    float kk[4][4], qq[4][4], dec[4][4], all[4] = {1.f, 1.f, 1.f, 1.f};
-    const int first = t0 + warp * 4;
-    float sq[8];  // sums of squares of q, k of each token
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      float x[3][4];
-#pragma unroll
-      for (int w = 0; w < 3; ++w) {
-        const float2 lo = __bfloat1622float2(*reinterpret_cast<const bf162*>(&sm.raw[warp][w][t][2 * lane])), hi = __bfloat1622float2(*reinterpret_cast<const bf162*>(&sm.raw[warp][w][t][64 + 2 * lane]));
-        x[w][0] = lo.x, x[w][1] = lo.y, x[w][2] = hi.x, x[w][3] = hi.y;
-      }
-      sq[2 * t] = (x[0][0] * x[0][0] + x[0][1] * x[0][1]) + (x[0][2] * x[0][2] + x[0][3] * x[0][3]);
-      sq[2 * t + 1] = (x[1][0] * x[1][0] + x[1][1] * x[1][1]) + (x[1][2] * x[1][2] + x[1][3] * x[1][3]);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        qq[t][e] = x[0][e];
-        kk[t][e] = x[1][e];
-        dec[t][e] = first + t < q1 ? __expf(lower / (1.f + __expf(-a * (x[2][e] + bias[e])))) : 1.f;
-        all[e] *= dec[t][e];
-      }
-    }
-#pragma unroll
-    for (int m = 16; m > 0; m >>= 1) {  // (one after the other the eight sums took a third of a chunk's time)
-      float y[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) y[i] = __shfl_xor_sync(0xffffffffu, sq[i], m);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) sq[i] += y[i];
-    }
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const float qn = rsqrtf(sq[2 * t] + 1e-6f) * q_scale, kn = rsqrtf(sq[2 * t + 1] + 1e-6f);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        qq[t][e] *= qn;
-        kk[t][e] *= kn;
-      }
-    }
-    *reinterpret_cast<float2*>(&sm.tot[warp][2 * lane]) = make_float2(all[0], all[1]);
-    *reinterpret_cast<float2*>(&sm.tot[warp][64 + 2 * lane]) = make_float2(all[2], all[3]);
-    if (lane < 4) sm.beta[chunk & 1][warp * 4 + lane] = first + lane < q1 ? 1.f / (1.f + __expf(-b_next)) : 0.f;
-    kc_sync(KC_BAR_PREP, 128);
-    if (t0 + KC_T < q1) fetch(t0 + KC_T, chunk + 1);
-    if (chunk > 0) kc_sync(KC_BAR_FREE, 256);
-    const int par = chunk & 1;
-    {
-      float run[4];  // the product between the warp's tokens and token 7
-      const bool behind = warp >= 2;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int ch = (e >> 1) * 64 + 2 * lane + (e & 1);
-        run[e] = warp == 3 ? sm.tot[2][ch] : warp == 0 ? sm.tot[1][ch] : 1.f;
-      }
-      float held[4];  // c of the pair's other token
-      auto put = [&](int t, bool second, const float* r, const float* ci) {  // r = P_t / P_7, ci its inverse
-        const int row = warp * 4 + t, p = row >> 1;
-#pragma unroll
-        for (int e = 0; e < 4; e += 2) {
-          const int pair = ((e >> 1) * 32 + lane) ^ ((t & 1) << 2);
-          float4 o;
-          kc_split(kk[t][e] * r[e], o.x, o.z);
-          kc_split(kk[t][e + 1] * r[e + 1], o.y, o.w);
-          sm.rk[row][pair] = o;
-          kc_split(qq[t][e] * r[e], o.x, o.z);
-          kc_split(qq[t][e + 1] * r[e + 1], o.y, o.w);
-          sm.rq[row][pair] = o;
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float x = kk[t][e] * ci[e];
-          if (second) {
-            float4 o;
-            kc_split((t & 1) ? held[e] : x, o.x, o.z);
-            kc_split((t & 1) ? x : held[e], o.y, o.w);
-            sm.c[par][p][((e >> 1) * 64 + 2 * lane + (e & 1)) ^ ((p & 3) << 1)] = o;
-          } else {
-            held[e] = x;
-          }
-        }
-      };
-      if (behind) {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          float inv[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            run[e] *= dec[t][e];
-            inv[e] = 1.f / run[e];
-          }
-          put(t, t & 1, run, inv);
-        }
-      } else {
-#pragma unroll
-        for (int t = 3; t >= 0; --t) {
-          float inv[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) inv[e] = 1.f / run[e];
-          put(t, !(t & 1), inv, run);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) run[e] *= dec[t][e];
-        }
-      }
-      if (warp == 0) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int ch = (e >> 1) * 64 + 2 * lane + (e & 1);
-          sm.fac[ch] = tail[e] * (all[e] * sm.tot[1][ch]);
-          tail[e] = sm.tot[2][ch] * sm.tot[3][ch];
-          sm.tail[ch] = tail[e];
-        }
-      }
-    }
-    kc_arrive(KC_BAR_ROWS, 256);
-    kc_sync(KC_BAR_PREP, 128);
-    // ---- A (warps 0, 1) and B (warps 2, 3), eight tokens s each ----
-    {
-      const float4* left = &(warp < 2 ? sm.rk : sm.rq)[g][t4];
-      const int sn = warp & 1, tok = sn * 8 + g, p = tok >> 1;
-      const float* right = reinterpret_cast<const float*>(&sm.c[par][p][(2 * t4) ^ ((p & 3) << 1)]) + (tok & 1);
-      float sum[4] = {0.f, 0.f, 0.f, 0.f}, low[2][4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) low[0][i] = low[1][i] = 0.f;
-#pragma unroll
-      for (int jg = 0; jg < 4; ++jg) {
-        float high[2][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) high[0][i] = high[1][i] = 0.f;
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-          const int j = jg * 4 + jj, at = 4 * j + (j & 1 ? -sw : sw);
-          const float4 u = left[at], w = left[8 * (KC_DK / 2) + at];
-          KcA l;
-          l.hi[0] = u.x, l.hi[1] = w.x, l.hi[2] = u.y, l.hi[3] = w.y;
-          l.lo[0] = u.z, l.lo[1] = w.z, l.lo[2] = u.w, l.lo[3] = w.w;
-          const float* cp = right + 32 * j;
-          const float4 r = make_float4(cp[0], cp[4], cp[2], cp[6]);
-          kc_mma_low(low[jj & 1], l, r);
-          kc_mma_high(high[jj & 1], l, r);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) sum[i] += high[0][i] + high[1][i];
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) sum[i] += low[0][i] + low[1][i];
-      const int s0 = sn * 8 + 2 * t4;
-      if (warp < 2) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int t = g + (i >> 1) * 8, ss = s0 + (i & 1);
-          sm.m[ss][t] = ss < t ? sum[i] * sm.beta[par][t] : 0.f;
-        }
-      } else {
-#pragma unroll
-        for (int tb = 0; tb < 2; ++tb) {
-          if (tb < sn) continue;
-          float4 o;
-          kc_split(s0 <= g + 8 * tb ? sum[2 * tb] : 0.f, o.x, o.z);
-          kc_split(s0 + 1 <= g + 8 * tb ? sum[2 * tb + 1] : 0.f, o.y, o.w);
-          sm.bf[par][tb + sn][lane] = o;
-        }
-      }
-    }
-    kc_sync(KC_BAR_PREP, 128);
-    if (warp == (chunk & 3)) {
-      // T, a column to a lane (lanes 16 .. 31 the same ones again)
-      const int c = lane & 15;
-      float x[KC_T];
-#pragma unroll
-      for (int t = 0; t < KC_T; ++t) x[t] = t == c ? 1.f : 0.f;
-#pragma unroll
-      for (int s = 0; s < KC_T - 1; ++s)
-#pragma unroll
-        for (int t = (s + 1) & ~3; t < KC_T; t += 4) {
-          const float4 mm = *reinterpret_cast<const float4*>(&sm.m[s][t]);
-          if (t > s) x[t] -= mm.x * x[s];
-          if (t + 1 > s) x[t + 1] -= mm.y * x[s];
-          if (t + 2 > s) x[t + 2] -= mm.z * x[s];
-          x[t + 3] -= mm.w * x[s];
-        }
-      const float be = sm.beta[par][c];
-#pragma unroll
-      for (int t = 0; t < KC_T; ++t) {
-        const int tb = t >> 3;
-        float hi, lo;
-        kc_split(x[t] * be, hi, lo);
-        if ((c >> 3) <= tb) reinterpret_cast<float*>(&sm.tf[par][tb + (c >> 3)][(t & 7) * 4 + ((c & 7) >> 1)])[(c & 1) + (lane >= 16 ? 2 : 0)] = lane >= 16 ? lo : hi;
-      }
-    }
-    kc_arrive(KC_BAR_T + par, 256);
-  }
-  return;
-  }
-
-  // ================ walking warps ================
-  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(KC_REGS_WALK));
-  float* S = state + ((long long)slot * heads + h) * KC_DK * dv + c0 + warp * 16 + g;
-  float s[16][4];  // S^T: columns (g, g + 8), channels 8 j + 2 t4 + {0, 1}
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const float* p = S + (long long)(8 * j + 2 * t4) * dv;
-    s[j][0] = p[0];
-    s[j][1] = p[dv];
-    s[j][2] = p[8];
-    s[j][3] = p[dv + 8];
-  }
-  for (int t0 = q0, chunk = 0; t0 < q1; t0 += KC_T, ++chunk) {
-    const int par = chunk & 1;
-    kc_sync(KC_BAR_ROWS, 256);
-    // ---- rk S' and rq S' for the warp's columns ----
-    float u[2][4], o[2][4], ul[2][4], ol[2][4];
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) u[n][i] = o[n][i] = ul[n][i] = ol[n][i] = 0.f;
-    const float4 *rk = &sm.rk[g][t4], *rq = &sm.rq[g][t4];
-    const float* fac = &sm.fac[2 * t4];
-#pragma unroll
-    for (int jg = 0; jg < 4; ++jg) {
-      float uh[2][4], oh[2][4];
-#pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) uh[n][i] = oh[n][i] = 0.f;
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        const int j = jg * 4 + jj, at = 4 * j + (j & 1 ? -sw : sw);
-        const float2 fc = *reinterpret_cast<const float2*>(fac + 8 * j);
-        s[j][0] *= fc.x;
-        s[j][1] *= fc.y;
-        s[j][2] *= fc.x;
-        s[j][3] *= fc.y;
-        KcA l;
-        kc_left(s[j], l);
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-          const float4 x = rk[n * 8 * (KC_DK / 2) + at], y = rq[n * 8 * (KC_DK / 2) + at];
-          kc_mma_low(ul[n], l, x);
-          kc_mma_high(uh[n], l, x);
-          kc_mma_low(ol[n], l, y);
-          kc_mma_high(oh[n], l, y);
-        }
-      }
-#pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          u[n][i] += uh[n][i];
-          o[n][i] += oh[n][i];
-        }
-    }
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        u[n][i] += ul[n][i];
-        o[n][i] += ol[n][i];
-      }
-    if (t0 + KC_T < q1) kc_arrive(KC_BAR_FREE, 256);
-    kc_sync(KC_BAR_T + par, 256);
-    // ---- d = T (v - u), o += B d ----
-    KcA d[2];
-    {
-      KcA x[2];
-#pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        float y[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) y[i] = to_f32(sm.raw_v[chunk & 3][8 * n + 2 * t4 + (i & 1)][warp * 16 + g + (i >> 1) * 8]) - u[n][i];
-        kc_left(y, x[n]);
-      }
-      const float4 tf[3] = {sm.tf[par][0][lane], sm.tf[par][1][lane], sm.tf[par][2][lane]}, bf[3] = {sm.bf[par][0][lane], sm.bf[par][1][lane], sm.bf[par][2][lane]};
-      float lo3[3][4], hi3[3][4];
-      auto both = [&](const KcA* l, const float4 (&r)[3], float (&sum)[2][4]) {  // sum[n] = the products of l and r, tokens up to n
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) lo3[k][i] = hi3[k][i] = 0.f;
-        kc_mma<3>({lo3[0], lo3[1], lo3[2]}, {hi3[0], hi3[1], hi3[2]}, {&l[0], &l[0], &l[1]}, r);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          sum[0][i] = hi3[0][i] + lo3[0][i];
-          sum[1][i] = (hi3[1][i] + hi3[2][i]) + (lo3[1][i] + lo3[2][i]);
-        }
-      };
-      float dd[2][4];
-      both(x, tf, dd);
-      kc_left(dd[0], d[0]);
-      kc_left(dd[1], d[1]);
-      both(d, bf, dd);
-#pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int t = t0 + 8 * n + 2 * t4 + (i & 1);
-          if (t < q1) out[((long long)t * heads + h) * dv + c0 + warp * 16 + g + (i >> 1) * 8] = __float2bfloat16(o[n][i] + dd[n][i]);
-        }
-    }
-    // ---- S' + sum c_s d_s ----
-    const float4* cp = &sm.c[par][t4][g ^ (t4 << 1)];
-#pragma unroll
-    for (int j = 0; j < 16; j += 2) {
-      float lo[4][4], hi[4][4];  // by j and half of the tokens
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) lo[k][i] = hi[k][i] = 0.f;
-      const float4 r[4] = {cp[8 * j], cp[4 * KC_DK + 8 * j], cp[8 * j + 8], cp[4 * KC_DK + 8 * j + 8]};
-      kc_mma<4>({lo[0], lo[1], lo[2], lo[3]}, {hi[0], hi[1], hi[2], hi[3]}, {&d[0], &d[1], &d[0], &d[1]}, r);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        s[j][i] += (hi[0][i] + hi[1][i]) + (lo[0][i] + lo[1][i]);
-        s[j + 1][i] += (hi[2][i] + hi[3][i]) + (lo[2][i] + lo[3][i]);
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const float2 e = *reinterpret_cast<const float2*>(&sm.tail[8 * j + 2 * t4]);
-    float* p = S + (long long)(8 * j + 2 * t4) * dv;
-    p[0] = s[j][0] * e.x;
-    p[dv] = s[j][1] * e.y;
-    p[8] = s[j][2] * e.x;
-    p[dv + 8] = s[j][3] * e.y;
-  }
-}
-
-// More shared memory than a kernel gets unasked, on every device; and whether the registers that the walking warps will ask for are
-// in the block's share.
-cudaError_t kc_allow() {
-  static std::atomic<bool> set[64];
-  int dev = 0;
-  if (cudaError_t e = cudaGetDevice(&dev)) return e;
-  if (set[dev & 63].load(std::memory_order_acquire)) return cudaSuccess;
-  cudaFuncAttributes fa;
-  if (cudaError_t e = cudaFuncGetAttributes(&fa, kda_chunk_kernel)) return e;
-  if (2 * fa.numRegs < KC_REGS_PREP + KC_REGS_WALK) return cudaErrorLaunchOutOfResources;
-  if (cudaError_t e = cudaFuncSetAttribute(kda_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KcSmem))) return e;
-  set[dev & 63].store(true, std::memory_order_release);
-  return cudaSuccess;
-}
-
 constexpr int ATTNRES_MAX = 16;  // candidates of one mix (snapshots + the current row)
 
 // One CTA of 256 threads per token.  Pass 1: sum of squares and dot with score_w for every candidate; pass 2: softmax of
@@ -1111,27 +631,21 @@ __global__ void __launch_bounds__(256) attnres_mix_kernel(const bf16* __restrict
 
 }  // namespace
 
-// Sequences of min_len tokens and more go in blocks of four tokens, or in chunks of sixteen, where rows and state are runs of 16-byte pieces, shorter ones (of
+// Sequences of min_len tokens and more go four tokens at a time where rows and state are runs of 16-byte pieces, shorter ones (of
 // up to `short_len` tokens; 0: there are none) token by token in a launch of their own, so that a decode row beside a prompt is
 // what it is in a step of decode rows.
 extern "C" int pg_kda_recurrent(const void* q, const void* k, const void* v, long long ld, const void* f, long long ldf, const void* b, long long ldb,
                                 const void* a_log, const void* dt_bias, float lower, void* state, void* out, const void* q_indptr, const void* slots,
-                                int num_seqs, int heads, int dk, int dv, int max_q_len, int min_len, int chunks, int short_len, cudaStream_t stream) {
+                                int num_seqs, int heads, int dk, int dv, int max_q_len, int min_len, int short_len, cudaStream_t stream) {
   PG_REQUIRE(dv <= 128 && lower < 0.f, "kda_recurrent: dv=%d must be <= 128 and the decay lower bound %f negative", dv, (double)lower);
   PG_REQUIRE(min_len >= 1, "kda_recurrent: blocks for sequences of %d tokens", min_len);
   if (num_seqs == 0) return PG_OK;
   RecArgs<bf16> p = {(const bf16*)q, (const bf16*)k, (const bf16*)v, ld, f, ldf, (const bf16*)b, ldb, (const float*)a_log, (const float*)dt_bias, nullptr, lower,
                      (float*)state, (bf16*)out, (const int*)q_indptr, (const int*)slots, heads, heads, dk, dv, (dv + KDA_COLS - 1) / KDA_COLS, 0};
-  const bool blocks = max_q_len >= min_len && dk == KC_DK && dv % KC_COLS == 0 && ld % 8 == 0 && ldf % 8 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)f | (uintptr_t)dt_bias | (uintptr_t)state) & 15) == 0;
+  const bool blocks = max_q_len >= min_len && dk == KB_DK && dv % KB_COLS == 0 && ld % 8 == 0 && ldf % 8 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)f | (uintptr_t)dt_bias | (uintptr_t)state) & 15) == 0;
   if (blocks) {
-    static_assert(KB_COLS == KC_COLS && KB_DK == KC_DK, "both kernels take the same steps");
-    const dim3 all(heads * (dv / KC_COLS), num_seqs);
-    if (chunks && lower >= KC_LOWER) {
-      PG_CUDA(kc_allow());
-      kda_chunk_kernel<<<all, 256, sizeof(KcSmem), stream>>>(p.q, p.k, p.v, ld, (const bf16*)f, ldf, p.b, ldb, p.a_log, p.dt_bias, lower, p.state, p.out, p.q_indptr, p.slots, heads, dv, min_len);
-    } else {
-      kda_block_kernel<<<all, 128, sizeof(KdaBlockSmem), stream>>>(p.q, p.k, p.v, ld, (const bf16*)f, ldf, p.b, ldb, p.a_log, p.dt_bias, lower, p.state, p.out, p.q_indptr, p.slots, heads, dv, min_len);
-    }
+    kda_block_kernel<<<dim3(heads * (dv / KB_COLS), num_seqs), 128, sizeof(KdaBlockSmem), stream>>>(p.q, p.k, p.v, ld, (const bf16*)f, ldf, p.b, ldb, p.a_log, p.dt_bias, lower, p.state, p.out, p.q_indptr, p.slots,
+                                                                                                     heads, dv, min_len);
     PG_LAUNCH_CHECK();
     if (short_len <= 0) return PG_OK;
     p.skip_len = min_len;

@@ -876,14 +876,9 @@ def gdn_recurrent(q, k, v, g, beta, state, meta: AttnMeta, chunked: Optional[boo
     return out
 
 
-# Sequences of at least this many tokens go four at a time (csrc/kda.cu).  In blocks / token by token, us: one sequence of 8, 9, 16 tokens
+# Sequences of at least this many tokens go four tokens at a time (csrc/kda.cu).  In blocks / token by token, us: one sequence of 8, 9, 16 tokens
 # and 16 heads 7.4 / 6.7, 8.4 / 8.3, 9.4 / 11.1; 64 of them and 96 heads 373 / 447, 431 / 518, 495 / 780; 64 x 5 370 / 354.
 _KDA_BLOCK_MIN = 9
-# Steps whose sequences have so many tokens on average go sixteen at a time on the tensor cores, where every chunk is paid in full (not where a
-# sequence's sums must not depend on the others).  Chunks / blocks, us, equal lengths: 4 x 96 heads
-# 57 / 47 (17 tokens), 120 / 117 (65), 200 / 209 (129), 361 / 395 (257); 2 x 96 heads 45 / 37 (33), 111 / 108 (129), 199 / 201 (257);
-# 8 x 32 heads 54 / 49 (33), 83 / 82 (65), 137 / 148 (129); 1 x 96 heads 27 / 29 (33), 122 / 150 (257).
-_KDA_CHUNK_MEAN = 128
 
 
 def kda_recurrent(q, k, v, f, b, a_log, dt_bias, lower: float, state, meta: AttnMeta):
@@ -897,15 +892,11 @@ def kda_recurrent(q, k, v, f, b, a_log, dt_bias, lower: float, state, meta: Attn
     assert f.stride(1) == 1 and b.stride(1) == 1 and f.shape[1] == h * dk and b.shape[1] == h
     assert state.is_contiguous() and state.dtype == torch.float32 and a_log.dtype == torch.float32 and dt_bias.dtype == torch.float32
     out = torch.empty((t, h, dv), dtype=q.dtype, device=q.device)
-    short, tokens, seqs = min(int(meta.max_q_len), _KDA_BLOCK_MIN - 1), int(meta.max_q_len), 1  # longest of the sequences that go token by token; the others
+    short = min(int(meta.max_q_len), _KDA_BLOCK_MIN - 1)  # longest of the sequences that go token by token
     if meta.h_q_indptr is not None:
-        lens = [meta.h_q_indptr[i + 1] - meta.h_q_indptr[i] for i in range(meta.num_seqs)]
-        short = max((n for n in lens if n < _KDA_BLOCK_MIN), default=0)
-        lens = [n for n in lens if n >= _KDA_BLOCK_MIN]
-        tokens, seqs = sum(lens), len(lens)
-    chunks = not _BATCH_INVARIANT and seqs > 0 and tokens >= _KDA_CHUNK_MEAN * seqs
+        short = max((n for i in range(meta.num_seqs) if (n := meta.h_q_indptr[i + 1] - meta.h_q_indptr[i]) < _KDA_BLOCK_MIN), default=0)
     rc = lib().pg_kda_recurrent(_ptr(q), _ptr(k), _ptr(v), _ll(q.stride(0)), _ptr(f), _ll(f.stride(0)), _ptr(b), _ll(b.stride(0)), _ptr(a_log), _ptr(dt_bias), _cf(lower),
-                                _ptr(state), _ptr(out), _ptr(meta.q_indptr), _ptr(meta.state_slots), _ci(meta.num_seqs), _ci(h), _ci(dk), _ci(dv), _ci(int(meta.max_q_len)), _ci(_KDA_BLOCK_MIN), _ci(int(chunks)), _ci(short), _stream())
+                                _ptr(state), _ptr(out), _ptr(meta.q_indptr), _ptr(meta.state_slots), _ci(meta.num_seqs), _ci(h), _ci(dk), _ci(dv), _ci(int(meta.max_q_len)), _ci(_KDA_BLOCK_MIN), _ci(short), _stream())
     _check(rc, ctx(q.device), 2 if short and meta.max_q_len >= _KDA_BLOCK_MIN else 1)
     return out
 
