@@ -1640,6 +1640,11 @@ def _latent_scratch(part, longest: int) -> int:
     return part.numel() if longest > _LATENT_WHOLE and not _BATCH_INVARIANT else 0
 
 
+def _latent_launches(tc: bool, rows: int, splits: int, scratch: int) -> int:
+    """Kernels of one absorbed call: the second one joins rows that are, or may be, cut (csrc/mla_decode_tc.cu: in steps of up to 512 rows)."""
+    return 2 if (scratch > 0 and rows <= 512 if tc else splits > 1) else 1
+
+
 def _latent_splits(rows: int, heads: int, longest: int, tc: bool, sms: int) -> int:
     """Blocks that share one row's keys in the absorbed kernels."""
     if _BATCH_INVARIANT:
@@ -1769,13 +1774,13 @@ def mla_attention(q: "_MlaQ", w_uk, w_uv, latent_layer, meta: AttnMeta, scale, k
     need = t * h * splits * (kv_lora + 1) * 4
     if need > c.attn_part.numel():
         splits = 1
-    part_o = c.attn_part
+    part_o, scratch = c.attn_part, _latent_scratch(c.attn_part, meta.max_kv_len)
     part_lse = c.attn_part[t * h * splits * kv_lora * 4 :]
     lat_out = torch.empty((t, h, kv_lora), dtype=torch.bfloat16, device=dev)
     rc = lib().pg_mla_attention(_ptr(q_abs), _ptr(q.pe), _ptr(latent_layer), _ptr(lat_out), _ptr(meta.q_indptr), _ptr(meta.kv_lens), _ptr(meta.block_table),
                                 _ci(meta.block_table.stride(0)), _ptr(unit_seq), _ci(meta.num_seqs), _ci(t), _ci(h), _ci(kv_lora), _ci(rope), _ci(page_size), _cf(scale),
-                                _ci(splits), _ci(int(tc)), _ptr(part_o), _ptr(part_lse), _ll(_latent_scratch(part_o, meta.max_kv_len)), _ll(latent_layer.shape[0]), _ptr(c.status), _stream())
-    _check(rc, c, 2 if splits > 1 or tc else 1)
+                                _ci(splits), _ci(int(tc)), _ptr(part_o), _ptr(part_lse), _ll(scratch), _ll(latent_layer.shape[0]), _ptr(c.status), _stream())
+    _check(rc, c, _latent_launches(tc, t, splits, scratch))
     vdim = w_uv.shape[1]
     out = torch.empty((t, h * vdim), dtype=torch.bfloat16, device=dev)
     _head_gemm(lat_out, h * kv_lora, kv_lora, w_uv, out.view(t, h, vdim))
@@ -1898,10 +1903,10 @@ def latent_attention(q, uk_t, uv, ukv, cache, meta: AttnMeta, rot: int, scale: f
         longest = min(longest, window + 31) if window else longest
         tc = _latent_tc(n, heads, lat, rot, _latent_keys(meta, row0, window), 1 if row0 else meta.max_q_len, c.sms)  # (behind prompts: decode rows)
         splits = _latent_splits(n, heads, longest, tc, c.sms)
-        splits = max(1, min(splits, c.attn_part.numel() // (n * heads * (lat + 1) * 4)))
+        splits, scratch = max(1, min(splits, c.attn_part.numel() // (n * heads * (lat + 1) * 4))), _latent_scratch(c.attn_part, longest)
         rc = lib().pg_latent_attention(_ptr(q_abs), *strides, *pe, *where, _ci(row0), _ci(meta.num_seqs), _ci(n), _ci(heads), _ci(lat), _ci(rot), _ci(ps), _cf(scale), _ci(window), *extra, _ci(splits),
-                                       _ci(int(tc)), _ptr(c.attn_part), _ptr(c.attn_part[n * heads * splits * lat * 4 :]), _ll(_latent_scratch(c.attn_part, longest)), _ll(cache.shape[0]), _ptr(c.status), _stream())
-        _check(rc, c, 2 if splits > 1 else 1)
+                                       _ci(int(tc)), _ptr(c.attn_part), _ptr(c.attn_part[n * heads * splits * lat * 4 :]), _ll(scratch), _ll(cache.shape[0]), _ptr(c.status), _stream())
+        _check(rc, c, _latent_launches(tc, n, splits, scratch))
     else:
         assert row0 == 0
         _check(lib().pg_latent_attention_plain(_ptr(q_abs), *strides, *pe, *where, _ci(n), _ci(heads), _ci(lat), _ci(rot), _ci(ps), _cf(scale), _ci(window), *extra, _ci(f32), _stream()), c)

@@ -442,6 +442,25 @@ def test_latent_rows_whatever_shares_their_step(heads, rot):
         K.set_batch_invariant(before)
 
 
+@pytest.mark.parametrize("kv_lens,heads", [([40, 200], 16), ([40, 700], 16), ([700] * 64, 64), ([300] * 513, 16)])
+def test_latent_launches_are_counted(kv_lens, heads):
+    """``launch_count`` against the profiler: steps of short rows, rows that may be cut (with the kernel that joins them), and too many for that."""
+    K = cu()
+    meta, q, uk_t, uv, cache, cs = _latent_rows(kv_lens, heads, 4)
+    m = meta(list(range(len(kv_lens))))
+    uk = uk_t.transpose(1, 2).contiguous()
+    hq = K.mla_rope_q(q.view(len(kv_lens), heads, 192), *R.rope_tables(1024, 64, 1e4, torch.bfloat16, DEV), m, 128)
+    for call in (lambda: K.latent_attention(q, uk_t, uv, None, cache, m, 64, 0.07, 0, *cs), lambda: K.mla_attention(hq, uk, uv, cache.view(-1, 16, 576), m, 0.07, 512)):
+        call()
+        torch.cuda.synchronize()
+        n0 = K.launch_count(DEV)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            call()
+            torch.cuda.synchronize()
+        seen = sum(e.count for e in prof.key_averages() if "mla_" in e.key or "moe_gemm" in e.key)
+        assert seen > 0 and K.launch_count(DEV) - n0 == seen
+
+
 @pytest.mark.parametrize("lens,past,heads,tc", [([1] * 8, 7, 16, True), ([1] * 150, 100, 16, True), ([16] * 3, 0, 16, True), ([17] * 3, 0, 16, False), ([80], 0, 16, False), ([90], 0, 16, True),
                                                  ([20] * 10, 80, 16, False), ([20] * 10, 130, 16, True), ([20] * 10, 15, 64, False), ([20] * 10, 30, 64, True), ([300] * 3, 0, 32, True)])
 def test_latent_kernels_where_the_rule_changes(lens, past, heads, tc, monkeypatch):
