@@ -139,8 +139,8 @@ def test_sampler_at_low_temperatures(temp, dtype):
 
 @pytest.mark.parametrize("heads,page,splits", [(16, 16, 1), (16, 64, 5), (32, 32, 2), (64, 16, 1), (64, 16, 3), (96, 16, 2)])
 def test_latent_decode_tiles(heads, page, splits, monkeypatch):
-    """Absorbed attention around tiles of 64 keys, padding rows, splits without keys, and rows behind a sequence's end that
-    hold NaN."""
+    """Absorbed attention around tiles of 64 keys, padding rows, blocks of 16 to 64 heads (``splits``: blocks that a row may have, from
+    which their heads follow; where its keys are cut follows from all rows' lengths), and rows behind a sequence's end that hold NaN."""
     torch.manual_seed(heads + page)
     kv_lens = [1, 63, 64, 65, 0, 129, 200, 511, 1000, 77]
     n = len(kv_lens)
@@ -353,14 +353,15 @@ def test_chain_that_gives_up_leaves_nothing_behind(t):
 @pytest.mark.parametrize("extras", [False, True])
 @pytest.mark.parametrize(
     "heads,rot,window,splits,reps,tc",
-    # blocks of 16 heads; of 32 (60 rows of 64 heads) and 64 (120 rows), with one and three splits, and a second group of 32 heads
+    # blocks of 16 heads; of 32 (60 rows of 64 heads) and 64 (120 rows), and a second group of 32 heads
     [(16, 64, 70, 1, 1, True), (64, 64, 70, 3, 1, True), (5, 0, 33, 1, 1, True), (40, 64, 200, 2, 1, True), (64, 0, 64, 16, 1, True), (16, 64, 0, 16, 1, True),
      (64, 64, 70, 1, 5, True), (64, 64, 0, 1, 10, True), (64, 64, 70, 3, 10, True), (96, 64, 130, 2, 10, True), (33, 0, 33, 1, 15, True),
      (16, 64, 70, 1, 1, False), (5, 0, 64, 3, 1, False), (64, 64, 0, 16, 1, False)],
 )
 def test_latent_window_and_empty_splits(heads, rot, window, splits, reps, tc, extras, monkeypatch):
-    """Rows in front of a window and behind the last key hold NaN (pages that others have written since); splits without keys,
-    also with a sink and a gate per head, which belong to the merged row; on both kernels."""
+    """Rows in front of a window and behind the last key hold NaN (pages that others have written since), also with a sink and a gate per
+    head, which belong to the joined row; on both kernels (``splits``: how many blocks share a row on the mma.sync kernel, some without
+    keys; on tcgen05 how few heads a block gets)."""
     torch.manual_seed(heads + window)
     kv_lens, page, lat, dim, vdim = [1, 63, 64, 65, 0, 129, 200, 511, 1000, 77, 96, 270] * reps, 16, 512, 128, 128
     n = len(kv_lens)
@@ -459,6 +460,82 @@ def test_latent_launches_are_counted(kv_lens, heads):
             torch.cuda.synchronize()
         seen = sum(e.count for e in prof.key_averages() if "mla_" in e.key or "moe_gemm" in e.key)
         assert seen > 0 and K.launch_count(DEV) - n0 == seen
+
+
+_SHARED_ROWS = {
+    "long": [20000, 1, 0, 300, 65],  # 78 pieces of a row: more than a warp has lanes
+    "longest first and last": [9000, 0, 64, 0, 12345],
+    "lines": [256, 257, 320, 0, 255, 64, 0, 0, 321, 319] * 3,  # rows of four tiles stay whole, rows of five may be cut
+    "wave": [700] * 150 + [0, 3000],
+    "most": [270] * 511 + [5000],  # the most rows that are shared
+    "more": [270] * 512 + [5000],  # and one more
+}
+
+
+@pytest.mark.parametrize("heads,rot,window,extras", [(16, 64, 0, False), (64, 64, 0, True), (96, 0, 0, False), (40, 64, 3000, True), (16, 0, 130, False)])
+@pytest.mark.parametrize("lens", _SHARED_ROWS)
+def test_latent_rows_that_blocks_share(lens, heads, rot, window, extras, monkeypatch):
+    """Rows cut between blocks, few pieces and many, against the restatement and against whole rows; the same bytes every time."""
+    K, kv_lens = cu(), _SHARED_ROWS[lens]
+    meta, q, uk_t, uv, cache, cs = _latent_rows(kv_lens, heads, heads, rot=rot)
+    n = len(kv_lens)
+    m = meta(list(range(n)))
+    q[n // 2] *= 8  # scores that pass the reference value by far in a later tile
+    g = torch.Generator(device=DEV).manual_seed(1)
+    more = dict(head_gate=torch.randn(n, heads, device=DEV, generator=g).bfloat16(), sink=torch.randn(heads, device=DEV, generator=g)) if extras else {}
+    run = lambda f: f(q, uk_t, uv, None, cache, m, rot, 0.07, window, *cs, **more).float()  # noqa: E731
+    got, want = run(K.latent_attention), run(R.latent_attention)
+    monkeypatch.setattr(K, "_latent_scratch", lambda part, longest: 0)
+    whole = run(K.latent_attention)
+    monkeypatch.undo()
+    # weights and rows of all are rounded to bf16 (2^-8 each), the sums are of some hundred terms that matter: 2^-6 of a row's largest
+    lim = 2 ** -6 * want.abs().amax(-1, keepdim=True)
+    assert ((got - want).abs() <= lim).all() and ((got - whole).abs() <= lim).all() and torch.equal(got, run(K.latent_attention))
+    short = torch.tensor([x <= 256 for x in kv_lens], device=DEV)
+    assert torch.equal(got[short], whole[short]) and not got[[i for i, x in enumerate(kv_lens) if x == 0]].any()
+    assert K.read_status(DEV) == 0
+
+
+@pytest.mark.parametrize("heads", [16, 64])
+def test_latent_rows_behind_prompts_are_shared(heads):
+    """Decode rows, long ones among them, behind a prompt that takes the expanded form."""
+    K, kv_lens, q_lens = cu(), [200, 700, 4000, 100, 9000, 1], [128, 72, 1, 1, 1, 1]
+    meta, q, uk_t, uv, cache, cs = _latent_rows(kv_lens, heads, 7, q_lens)
+    m, calls = meta(list(range(6))), K.PREFILL_TC_CALLS["latent"]
+    ukv = torch.cat([uk_t.transpose(1, 2).reshape(heads * 128, 512), uv.reshape(heads * 128, 512)])
+    got, want = (f(q.clone(), uk_t, uv, ukv, cache, m, 64, 0.07, 0, *cs).float() for f in (K.latent_attention, R.latent_attention))
+    assert K.PREFILL_TC_CALLS["latent"] == calls + 1
+    assert ((got - want).abs() <= 2 ** -6 * want.abs().amax(-1, keepdim=True)).all()  # as above
+
+
+@pytest.mark.parametrize("heads", [16, 64])
+def test_latent_rows_in_a_graph_with_a_bound(heads):
+    """A captured step knows a bound on its rows' keys only: short rows have the bytes of a step whose lengths are known, others those of a
+    step with the bound."""
+    K, kv_lens = cu(), [1, 64, 65, 200, 256, 0, 129, 1000, 3000]
+    meta, q, uk_t, uv, cache, cs = _latent_rows(kv_lens, heads, 9)
+    n = len(kv_lens)
+    run = lambda m: K.latent_attention(q[: m.num_seqs], uk_t, uv, None, cache, m, 64, 0.07, 0, *cs)  # noqa: E731
+    known, bound = meta(list(range(7))), meta(list(range(7)))
+    bound.max_kv_len = 4096
+    bound.h_kv_lens = bound.h_q_indptr = None
+    assert torch.equal(run(known), run(bound))
+    m = meta(list(range(n)))
+    m.max_kv_len = 4096
+    m.h_kv_lens = m.h_q_indptr = None
+    eager, real = run(m), m.kv_lens.clone()
+    m.kv_lens.fill_(1)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        run(m)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = run(m)
+    m.kv_lens.copy_(real)
+    graph.replay()
+    assert torch.equal(out, eager)
 
 
 @pytest.mark.parametrize("lens,past,heads,tc", [([1] * 8, 7, 16, True), ([1] * 150, 100, 16, True), ([16] * 3, 0, 16, True), ([17] * 3, 0, 16, False), ([80], 0, 16, False), ([90], 0, 16, True),
