@@ -1,5 +1,6 @@
 """Kernels at the edges of the ranges that their launch rules draw: tile and segment edges, remainders, odd widths, the
 smallest and largest sizes, against the PyTorch restatements."""
+import ctypes
 import os
 import subprocess
 import sys
@@ -445,8 +446,9 @@ def test_latent_rows_whatever_shares_their_step(heads, rot):
 
 @pytest.mark.parametrize("kv_lens,heads", [([40, 200], 16), ([40, 700], 16), ([700] * 64, 64), ([300] * 513, 16)])
 def test_latent_launches_are_counted(kv_lens, heads):
-    """``launch_count`` against the profiler: steps of short rows, rows that may be cut (with the kernel that joins them), and too many for that."""
-    K = cu()
+    """``launch_count`` against the kernels of a captured graph: steps of short rows, rows that may be cut (with the kernel that joins
+    them), and too many for that."""
+    K, driver = cu(), ctypes.CDLL("libcuda.so.1")
     meta, q, uk_t, uv, cache, cs = _latent_rows(kv_lens, heads, 4)
     m = meta(list(range(len(kv_lens))))
     uk = uk_t.transpose(1, 2).contiguous()
@@ -454,12 +456,12 @@ def test_latent_launches_are_counted(kv_lens, heads):
     for call in (lambda: K.latent_attention(q, uk_t, uv, None, cache, m, 64, 0.07, 0, *cs), lambda: K.mla_attention(hq, uk, uv, cache.view(-1, 16, 576), m, 0.07, 512)):
         call()
         torch.cuda.synchronize()
-        n0 = K.launch_count(DEV)
-        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        graph, n0 = torch.cuda.CUDAGraph(keep_graph=True), K.launch_count(DEV)
+        with torch.cuda.graph(graph):
             call()
-            torch.cuda.synchronize()
-        seen = sum(e.count for e in prof.key_averages() if "mla_" in e.key or "moe_gemm" in e.key)
-        assert seen > 0 and K.launch_count(DEV) - n0 == seen
+        nodes = ctypes.c_size_t()
+        assert driver.cuGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None, ctypes.byref(nodes)) == 0
+        assert nodes.value >= 3 and K.launch_count(DEV) - n0 == nodes.value  # kernels are all that is captured
 
 
 _SHARED_ROWS = {
