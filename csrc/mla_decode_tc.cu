@@ -8,7 +8,9 @@
 // 36 copies of 2 KB a tile, which took 1.25 us to issue), and the operand descriptors step from box to box.  Two tiles of
 // 72 KB, Q (72 KB at 64 heads) and P fill the shared memory, so a CTA owns an SM.  Up to DT_ROWS rows the CTAs, one an SM, share all tiles
 // of the step evenly (dt_shares): a CTA walks pieces of rows one behind the other, copies and queries of the next piece under the
-// last tiles of the one before, and a second kernel joins the rows that were cut.
+// last tiles of the one before, and a second kernel joins the rows that were cut.  So a row of more than DT_WHOLE tiles is cut where the
+// lengths of all rows of the step say, and weights are rounded to bf16 against a reference that starts anew with a piece: its sums
+// are those of the step, not of the row alone.  A caller that wants the latter gives no scratch, and a block walks a row.
 //
 // A product of 64 rows leaves them in the lower half of each warp's tensor-memory lanes: a warp has 16 keys, and a thread
 // reads two of them for a quarter of the heads.  Rows are reduced across threads only when it matters: exponentials refer to
@@ -33,7 +35,9 @@ constexpr int DT_KEYS = 64;
 constexpr int DT_P = DT_KEYS * 128;      // weights: 64 keys x 64 heads
 constexpr int DT_THREADS = 320;          // producer, MMA, four softmax / epilogue warps, four warps that fetch queries
 constexpr int DT_ROWS = 512;             // rows whose keys the blocks share
-constexpr int DT_WHOLE = 4;              // rows of up to so many tiles are not cut (steps without longer ones get no scratch, no shares and no join: 128 rows of 100 keys 40 us the whole operation, 44 with them)
+// Rows of up to so many tiles are not cut.  Steps whose longest row the host knows to be no longer get no scratch, no shares and no join (128 rows of
+// 100 keys 32 us the whole operation, 36 with them); a captured step, which knows a bound only, has them all the same.
+constexpr int DT_WHOLE = 4;
 constexpr float DT_NONE = -1e30f;        // reference of a head that has seen no key; also "no keys" among the partial results
 
 template <int HN>

@@ -168,8 +168,8 @@ __device__ __forceinline__ void store_tile(const MoeGemmParams& p, const Item& i
           }
         }
         const long long at = (p.head_rows ? it.e * p.y_head : 0ll) + (long long)(it.row0 + c) * p.ldy + m;
-        // (a pointer that steps, and no test per row: 1711 tokens through 64 bf16 experts, both products, 351 us with an address
-        // formed for each of the 16 stores, 302 now; 128 tokens through 48 INT4 experts 451 and 405)
+        // (a pointer that steps, and no test per row: 1711 tokens through 64 bf16 experts, both products, 232 us with an address
+        // formed for each of the 16 stores, 226 now, the whole operation 351 and 345; 128 tokens through 48 INT4 experts 390 and 386)
         const bool all = c + 16 <= it.rows;
         if (p.y_f32 != nullptr) {
           float* dst = p.y_f32 + at;

@@ -1594,7 +1594,7 @@ def mla_rope_q(q, cos, sin, meta: AttnMeta, nope):
 
 def _latent_keys(meta: AttnMeta, row0: int = 0, window: int = 0) -> int:
     """Keys of a typical row of a step from row ``row0`` on, for the choice of a kernel: the rows' mean where the lengths are known here, but at
-    least half of the longest, which one block walks."""
+    least half of the longest, whose rows end last."""
     longest = min(meta.max_kv_len, window) if window else meta.max_kv_len
     qi, kvl = meta.h_q_indptr, meta.h_kv_lens
     if qi is None or kvl is None:
@@ -1630,7 +1630,9 @@ def _latent_tc(rows: int, heads: int, lat: int, rot: int, keys: int, max_q_len: 
     return keys > (96 if heads <= 32 or 3 * blocks < 4 * sms else 32)
 
 
-_LATENT_WHOLE = 256  # rows of up to so many keys are not shared between blocks (csrc/mla_decode_tc.cu): steps of nothing else need no scratch, and no join
+# Rows of up to so many keys are not shared between blocks (csrc/mla_decode_tc.cu): steps of nothing else need no scratch, and no join.  That
+# goes by what is known here, in a captured graph a bound on the keys, so a served graph has both; its short rows are whole all the same.
+_LATENT_WHOLE = 256
 _LATENT_FEW = 16  # rows of a sequence in a decode step or in one that checks drafted tokens
 
 
@@ -1646,10 +1648,11 @@ def _latent_launches(tc: bool, rows: int, splits: int, scratch: int) -> int:
 
 
 def _latent_splits(rows: int, heads: int, longest: int, tc: bool, sms: int) -> int:
-    """Blocks that share one row's keys in the absorbed kernels."""
+    """Blocks that are to share one row's keys: the mma.sync kernel splits a row so.  Blocks of the tcgen05 kernel, which own an SM and serve
+    up to 64 heads, share the keys by themselves and take it for how few heads one gets."""
     if _BATCH_INVARIANT:
         return 1
-    if tc:  # csrc/mla_decode_tc.cu: a block owns an SM and serves up to 64 heads; blocks share the keys by themselves, this says how few heads one gets
+    if tc:
         return max(1, min(16, sms // (rows * ((heads + 63) // 64)), (longest + 255) // 256))
     return max(1, min(16, (4 * sms) // (rows * ((heads + 15) // 16)), (min(longest, 4096) + 127) // 128))
 
